@@ -409,6 +409,37 @@ __global__ void __launch_bounds__(kCmThreads) k_amr_corner_moments(
   }
 }
 
+// J alone (a run's current output, without the 243-term M): one thread per
+// (corner, component) in host order instead of k_amr_corner_moments' CTA per
+// corner, of which only 3 of 256 threads have work when M is not asked for.
+// Same entries in the same order with the same pair sums, so the values equal
+// that kernel's J bit for bit.  Bound: the corner's ~8 scattered 12-byte reads
+// of cellJ (one L2 sector each) and, for a page-locked destination that the
+// kernel writes itself, the host link's 12 MB.  500,832 corners: 0.1 ms where
+// the CTA form's 16 launches took 1.36 ms.
+__global__ void __launch_bounds__(256) k_amr_corner_j(long long n3, const int* __restrict__ start,
+                                                      const int* __restrict__ ent,
+                                                      const float* __restrict__ cellJ,
+                                                      const float* __restrict__ ivh,
+                                                      const float* __restrict__ ivl,
+                                                      double* __restrict__ J) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n3) return;
+  const long long cc = t / 3;
+  const int jc = (int)(t - 3 * cc);
+  const int e0 = start[cc], e1 = start[cc + 1];
+  FF sum{0.f, 0.f};
+#pragma unroll 4
+  for (int e = e0; e < e1; e++) {
+    const int en = ent[e];
+    const long long cell = en >> 3;
+    const int q = en & 7, b = (int)(cell / AMPS_CPB);
+    const FF p = ff_mul(cellJ[cellJ_at(cell, (q ^ ((q >> 1) & 1)) * 3 + jc)], 0.f, ivh[b], ivl[b]);
+    ff_acc(sum, p.s, p.q);
+  }
+  J[t] = widen(sum.s) + widen(sum.q);
+}
+
 // the corner-layout moments of an AMR context (k_amr_corner_moments) into
 // host J[nvc][3], M[nvc][243] (mesh corner numbering).  The kernel writes a
 // device buffer in kCmChunks corner ranges; each range's copy to the host
@@ -421,14 +452,17 @@ amps_gpu_status amr_export_corner_moments(amps_gpu_ctx* c, double* J, double* M)
   amps_gpu_status st = corner_csr_setup(c);
   if (st) return st;
   if (!J && !M) return AMPS_GPU_OK;
-  if (!c->d_amrJ) {
-    if (cudaMalloc(reinterpret_cast<void**>(&c->d_amrJ), sizeof(double) * 3 * (size_t)c->nvc) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void**>(&c->d_amrM), sizeof(double) * 243 * (size_t)c->nvc) != cudaSuccess) {
-      cudaGetLastError();
-      cudaFree(c->d_amrJ);
-      c->d_amrJ = nullptr;
-      return set_err(c, AMPS_GPU_CUDA_ERROR, "export_moments: allocation failed");
-    }
+  if (!c->d_amrJ && cudaMalloc(reinterpret_cast<void**>(&c->d_amrJ),
+                               sizeof(double) * 3 * (size_t)c->nvc) != cudaSuccess) {
+    cudaGetLastError();
+    c->d_amrJ = nullptr;
+    return set_err(c, AMPS_GPU_CUDA_ERROR, "export_moments: allocation failed");
+  }
+  if (M && !c->d_amrM && cudaMalloc(reinterpret_cast<void**>(&c->d_amrM),
+                                    sizeof(double) * 243 * (size_t)c->nvc) != cudaSuccess) {
+    cudaGetLastError();
+    c->d_amrM = nullptr;
+    return set_err(c, AMPS_GPU_CUDA_ERROR, "export_moments: allocation failed");
   }
   if (!c->d_bivh) {
     // 1/dx^3 per block as an FP32 pair
@@ -450,6 +484,22 @@ amps_gpu_status amr_export_corner_moments(amps_gpu_ctx* c, double* J, double* M)
     if ((st = cuda_check(c, cudaMemcpy(c->d_bivh, iv.data(), sizeof(float) * iv.size(),
                                        cudaMemcpyHostToDevice), "block volumes")))
       return st;
+  }
+  if (!M) {
+    const long long n3 = 3 * c->nvc;
+    double* direct = host_mapped(J);
+    cudaError_t e;
+    {
+      TimedLaunch t(c, "amr_corner_j");
+      k_amr_corner_j<<<(unsigned)((n3 + 255) / 256), 256, 0, c->stream>>>(
+          n3, c->d_spec_start, c->d_spec_ent, c->d_cellJ, c->d_bivh, c->d_bivh + c->nb,
+          direct ? direct : c->d_amrJ);
+    }
+    e = cudaGetLastError();
+    if (e == cudaSuccess && !direct)
+      e = cudaMemcpyAsync(J, c->d_amrJ, sizeof(double) * (size_t)n3, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    return cuda_check(c, e, "export corner current");
   }
   if (!c->copy_stream) {
     if ((st = cuda_check(c, cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking),

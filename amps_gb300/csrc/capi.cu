@@ -319,7 +319,8 @@ bool alloc_context(amps_gpu_ctx* c) {
   if (!c->amr) ok = ok && !dalloc(&c->d_J, 3 * nc) && !dalloc(&c->d_M, 243 * nc);
   if (c->amr) ok = ok && !dalloc(&c->d_y32, 3 * nv);
   ok = ok && !dalloc(&c->d_rhs, 3 * nv) && !dalloc(&c->d_x, 3 * nv) &&
-       !dalloc(&c->d_V, (size_t)(c->restart + 1) * 3 * nv) && !dalloc(&c->d_w, 3 * nv) &&
+       !dalloc(&c->d_V, (size_t)(c->restart + 1) * ((3 * nv + 3) & ~3LL)) &&
+       !dalloc(&c->d_w, (3 * nv + 3) & ~3LL) &&
        !dalloc(&c->d_dinv, 3 * nv) && !dalloc(&c->d_red, 12288);
   ok = ok && cudaMallocHost(&c->h_red, 128 * sizeof(double)) == cudaSuccess;
   ok = ok && !dalloc(&c->d_stencil_push, (size_t)c->nb * AMPS_SC * AMPS_PUSH_STRIDE) &&

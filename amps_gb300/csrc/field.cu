@@ -12,8 +12,8 @@
 //               srcInterface/LinearSystemCornerNode.h:3067-3205)
 //   GMRES       restarted GMRES(30), x0 = 0, right preconditioner (none,
 //               Jacobi, learned), classical Gram-Schmidt with one
-//               re-orthogonalisation; each Arnoldi step is matvec + three fused
-//               sweep/reduction kernels with FP64 warp-shuffle reductions
+//               re-orthogonalisation; each Arnoldi step is matvec + one
+//               cooperative kernel on FP32-pair vectors (k_arnoldi_tile)
 //               (the external linear_solver_wrapper of LinearSystemCornerNode.h:3282)
 //   k_update_b  UpdateB (:5160-5711), k_c2n InterpolateB_C2N (:5715),
 //   k_update_e  UpdateE with the wave-energy sum (:5909-6001)
@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "precond.cuh"
+#include "ptx.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -36,6 +37,7 @@ constexpr int kMaxV = 32;
 constexpr int kRedBlocks = 304;  // 2 x 152 SMs
 constexpr int kGmOffset = 10240;  // doubles into d_red (12288 doubles)
 constexpr int kArnMaxGrid = 1024;  // CTAs of the cooperative Arnoldi step (at most)
+constexpr uint32_t kWaitLimit = 1u << 24;
 
 struct Taps {
   double K[3][3][27];  // operator taps without the mass matrix
@@ -396,15 +398,16 @@ __device__ void gm_update(GmState* __restrict__ S, int jj, const double* h1, con
                           double n2) {
   if (S->done) return;
   double* H = S->H;
-  for (int i = 0; i <= jj; i++) H[i * kMaxV + jj] = h1[i] + h2[i];
   const double hn = sqrt(n2);
-  H[(jj + 1) * kMaxV + jj] = hn;
+  // the column runs through the rotations in a register
+  double a = h1[0] + h2[0];
+  const double b = hn;
+#pragma unroll 4
   for (int i = 0; i < jj; i++) {
-    const double a = H[i * kMaxV + jj], b = H[(i + 1) * kMaxV + jj];
-    H[i * kMaxV + jj] = S->cs[i] * a + S->sn[i] * b;
-    H[(i + 1) * kMaxV + jj] = -S->sn[i] * a + S->cs[i] * b;
+    const double hb = h1[i + 1] + h2[i + 1], c0 = S->cs[i], s0 = S->sn[i];
+    H[i * kMaxV + jj] = c0 * a + s0 * hb;
+    a = -s0 * a + c0 * hb;
   }
-  const double a = H[jj * kMaxV + jj], b = H[(jj + 1) * kMaxV + jj];
   const double r = sqrt(a * a + b * b);
   const double c = r > 0.0 ? a / r : 1.0, s = r > 0.0 ? b / r : 0.0;
   S->cs[jj] = c;
@@ -429,19 +432,14 @@ __global__ void k_gm_solve(GmState* __restrict__ S) {
   }
 }
 
-// one CGS2 Arnoldi orthogonalisation with a register budget fitted to nv
 // ---- Krylov vectors in FP32 pairs ----------------------------------------------
-// One whole Arnoldi step after the operator runs in one cooperative launch
-// (co-resident CTAs, grid-wide barriers between the phases): CGS2 against
-// V_0..V_nv-1 (h1 = V^T w, w -= V h1, h2 = V^T w, w -= V h2), ||w||,
-// V_nv = w / ||w||, and the Givens update of the least-squares state.  Every
-// CTA reduces the per-CTA partial sums of a phase itself, so the phases need
-// no further launches; each phase writes its own partial buffer.
-constexpr int kArnThreads = 256;
 // The Arnoldi basis and the operator output are stored as FP32 pairs (hi, lo:
 // 48 significant bits, the bytes of a double vector): FP64 arithmetic runs at
 // ~1/70 of the FP32 rate on this part, and CGS2 is 4 nv n multiply-adds per
-// step, so the sweeps run in pair arithmetic and only per-block sums touch FP64.
+// step, so the sweeps run in pair arithmetic and only the sums over the CTAs
+// touch FP64.  One whole Arnoldi step after the operator is one cooperative
+// launch (grid-wide barriers between the sweeps); every CTA adds up the per-CTA
+// partial sums of a sweep itself.
 
 // a += (xh + xl)(yh + yl)
 __device__ __forceinline__ void ff_dot_acc(FF& a, float xh, float xl, float yh, float yl) {
@@ -460,256 +458,416 @@ __device__ __forceinline__ FF ff_warp_sum(FF a) {
   return a;
 }
 
-// Reduce acc[0..nv) over the block into row[2i], row[2i+1] (a pair per entry).
-template <int NVM>
-__device__ __forceinline__ void arn_block_store_ff(const FF (&acc)[NVM], int nv, float* __restrict__ row,
-                                                   float* __restrict__ s_red) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// One Arnoldi step on pair vectors: CGS2 of w against V_0..V_{nv-1} (h1 = V^T w,
+// w' = w - V h1, h2 = V^T w', w'' = w' - V h2), V_nv = w'' / ||w''||, and the
+// Givens update of the least-squares state.  Vectors are pair streams: hi at
+// V + 2 i ld, lo ld behind it, ld = n rounded up to 4 so that every stream
+// starts on 16 bytes.
+//
+// Bound: reading the basis (n = 1.34M, 15 vectors: 161 MB a sweep).  One
+// persistent CTA per SM; a producer warp brings tiles of kArnT elements of
+// every stream into a ring of shared-memory stages by bulk copies (up to 200 KB
+// in flight per SM, which per-thread loads at 2 CTAs per SM did not reach), and
+// 16 consumer warps work on the staged tile:
+//   - update: thread pairs split an element's vectors (even / odd);
+//   - dots: a warp owns whole vectors (or an element range of one when there
+//     are fewer vectors than warps), so the register cost does not grow with
+//     nv and no sums cross warps inside the sweep.
+// The staged tile serves both halves of the second sweep (w' and then h2), the
+// third sweep needs V's hi halves only (h2 is of the order of the pair
+// arithmetic's own rounding, 2^-48 |w|; times a lo half, 2^-24 |V|, it is far
+// below the last bit of w''), and tiles are walked in alternating directions so
+// a sweep starts on what the last one left in L2: 2.5 basis reads per step.
+// ||w''||^2 = ||w'||^2 - ||h2||^2 (V orthonormal) spares a sweep and a grid
+// barrier; where the second projection took more than half of ||w'||^2 (w in
+// the span of V) it is summed instead, from a sweep with the full pairs.
+// A CTA whose tiles all fit its stages reads them once.  Mean step of a
+// 55-iteration solve with 1.34M unknowns (1 to 30 vectors): 150 us, where the
+// form with per-thread streams and accumulators in registers (four basis reads,
+// three barriers) took 304 us; 1.50M unknowns, 1 to 8 vectors: 71 against 81 us.
+constexpr int kArnT = 256;                  // elements per tile and element per thread
+constexpr int kArnCons = 512;               // consumer threads (16 warps)
+constexpr int kArnBlock = kArnCons + 32;    // + the producer warp
+constexpr int kArnWarps = kArnCons / 32;
+constexpr int kArnMaxStages = 16;
+constexpr size_t kArnRing = 200 * 1024;     // ring budget
+constexpr int kArnDots = kMaxV;             // dots per sweep: nv, and ||w'||^2
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// orders this thread's generic writes before later bulk copies of the same addresses
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+__device__ __forceinline__ void bar_consumers() {
+  asm volatile("bar.sync 1, %0;" ::"n"(kArnCons) : "memory");
+}
+__device__ __forceinline__ void bar_all() { asm volatile("bar.sync 2, %0;" ::"n"(kArnBlock) : "memory"); }
+
+template <int M>
+__global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
+    long long n, long long ld, const float* __restrict__ V, float* __restrict__ w, int nv,
+    float* __restrict__ vnext, float2* __restrict__ part, GmState* gs, int jj, float* __restrict__ xf,
+    const float* __restrict__ dh, int stages, unsigned long long* flags) {
+  cg::grid_group grid = cg::this_grid();
+  extern __shared__ __align__(16) float s_ring[];
+  __shared__ __align__(8) uint64_t full[kArnMaxStages], empty[kArnMaxStages];
+  __shared__ float2 s_red[kArnWarps][2];
+  __shared__ double s_h1[kMaxV], s_h2[kMaxV], s_n2, s_inv;
+  __shared__ float2 s_f[kArnDots];               // the coefficients of the running sweep as pairs
+  __shared__ int s_slow;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int nblk = gridDim.x;
+  constexpr int T = kArnT * M;
+  const int tiles = (int)((n + T - 1) / T);
+  const int nt = (tiles - (int)blockIdx.x + nblk - 1) / nblk;  // this CTA's tiles (grid <= tiles)
+  const bool resident = nt <= stages;
+  constexpr int slot = 2 * T;                    // floats per staged vector (hi, lo)
+  const size_t stage_f = (size_t)(nv + 1) * slot;
+  float* s_w = s_ring + stages * stage_f;        // w' of the tile in work: hi, lo
+  float2* s_part = reinterpret_cast<float2*>(s_w + slot);  // odd vectors' share of the update
+  auto tile_of = [&](int k) { return (long long)blockIdx.x + (long long)k * nblk; };
+  auto count_of = [&](int k) { return (int)min((long long)T, n - tile_of(k) * T); };
+  if (tid == 0) {
+    for (int s = 0; s < stages; s++) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], kArnWarps);
+    }
+    fence_mbar_init();
+  }
+  __syncthreads();
+
+  if (wid == kArnWarps) {
+    // ---- producer warp: tile k of the sweep as the ring's use number c
+    // (dlo: D's tile in the place of V_0's lo half, in the sweep that reads hi halves)
+    auto issue = [&](int c, int k, bool lo, const float* dlo) {
+      const int s = c % stages;
+      if (c >= stages && !mbar_wait_bounded(&empty[s], ((c / stages) - 1) & 1, kWaitLimit) && lane == 0)
+        atomicAdd(flags + 2, 1ull);
+      const long long e0 = tile_of(k) * T;
+      const uint32_t bytes = (uint32_t)((count_of(k) + 3) & ~3) * 4u;
+      float* dst = s_ring + (size_t)s * stage_f;
+      if (lane == 0)
+        mbar_arrive_expect_tx(&full[s], bytes * (uint32_t)(lo ? 2 * nv + 2 : nv + 2 + (dlo ? 1 : 0)));
+      __syncwarp();
+      for (int q = lane; q < 2 * nv + 2; q += 32) {
+        const int i = q >> 1, half = q & 1;
+        const float* src = (i < nv ? V + 2 * (size_t)i * ld : w) + (half ? ld : 0);
+        if (half && !lo && i < nv) {
+          if (i > 0 || !dlo) continue;
+          src = dlo;
+        }
+        bulk_copy_g2s(dst + (size_t)i * slot + half * T, src + e0, bytes, &full[s]);
+      }
+    };
+    for (int k = 0; k < nt; k++) issue(k, k, true, nullptr);
+    const int pre = min(nt, stages);  // the second sweep's first tiles load across the barrier
+    if (!resident)
+      for (int k = 0; k < pre; k++) issue(nt + k, nt - 1 - k, true, nullptr);
+    grid.sync();
+    if (!resident)
+      for (int k = pre; k < nt; k++) issue(nt + k, nt - 1 - k, true, nullptr);
+    grid.sync();
+    bar_all();  // s_slow
+    const bool slow = s_slow != 0;
+    if (!resident)
+      for (int k = 0; k < nt; k++) issue(2 * nt + k, k, slow, slow || !xf ? nullptr : dh);
+    if (slow) {
+      grid.sync();
+      bar_all();  // s_n2
+    }
+    if (blockIdx.x == 0 && lane == 0) gm_update(gs, jj, s_h1, s_h2, s_n2);
+    return;
+  }
+
+  // ---- consumers
+  auto acquire = [&](int c) -> float* {
+    const int s = c % stages;
+    if (!mbar_wait_bounded(&full[s], (c / stages) & 1, kWaitLimit) && lane == 0) atomicAdd(flags + 2, 1ull);
+    return s_ring + (size_t)s * stage_f;
+  };
+  auto release = [&](int c) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[c % stages]);
+  };
+  // dots of the staged w with nd vectors (number nv: w itself): warp -> vector
+  // and, with fewer vectors than warps, element range
+  FF acc[2];
+  int dots_n = 0, dots_p = 1, dots_g = 1;
+  auto dots_begin = [&](int nd) {
+    dots_n = nd;
+    dots_p = 1;
+    while (dots_p < nd && dots_p < kArnWarps) dots_p *= 2;
+    dots_g = kArnWarps / dots_p;  // element ranges per vector
+    acc[0] = acc[1] = FF{0.f, 0.f};
+  };
+  auto dots = [&](const float* st, const float* wt, int count) {
+    const int g = wid / dots_p;
 #pragma unroll
-  for (int i = 0; i < NVM; i++) {
-    if (i < nv) {
-      const FF v = ff_warp_sum(acc[i]);
+    for (int r = 0; r < 2; r++) {
+      const int i = wid % dots_p + kArnWarps * r;
+      if (i >= dots_n) continue;
+      const float* v = i < nv ? st + (size_t)i * slot : wt;
+#pragma unroll 4
+      for (int e = g * 32 + lane; e < count; e += 32 * dots_g)
+        ff_dot_acc(acc[r], v[e], v[T + e], wt[e], wt[T + e]);
+    }
+  };
+  // block sums to part[i * nblk + blk]; all blocks' sums after the barrier
+  auto dots_end = [&](float2* __restrict__ out) {
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const FF t = ff_norm(ff_warp_sum(acc[r]));
+      if (lane == 0) s_red[wid][r] = make_float2(t.s, t.q);
+    }
+    bar_consumers();
+    if (tid < dots_n) {
+      const int r = tid / kArnWarps, wi = tid % kArnWarps;
+      FF t{0.f, 0.f};
+      for (int g = 0; g < dots_g; g++) {
+        const float2 q = s_red[wi % dots_p + g * dots_p][r];
+        ff_acc(t, q.x, q.y);
+      }
+      t = ff_norm(t);
+      out[(size_t)tid * nblk + blockIdx.x] = make_float2(t.s, t.q);
+    }
+  };
+  auto grid_sums = [&](const float2* __restrict__ in, int nd, double* __restrict__ h) {
+    for (int i = wid; i < nd; i += kArnWarps) {
+      FF t{0.f, 0.f};
+      for (int b = lane; b < nblk; b += 32) {
+        const float2 q = __ldcg(in + (size_t)i * nblk + b);
+        ff_acc(t, q.x, q.y);
+      }
+      t = ff_norm(ff_warp_sum(t));
       if (lane == 0) {
-        s_red[2 * (wid * kMaxV + i)] = v.s;
-        s_red[2 * (wid * kMaxV + i) + 1] = v.q;
+        s_f[i] = make_float2(t.s, t.q);
+        if (i < nv) h[i] = (double)t.s + (double)t.q;
+        else s_n2 = (double)t.s + (double)t.q;
       }
     }
-  }
-  __syncthreads();
-  if (threadIdx.x < nv) {
-    FF t{0.f, 0.f};
-    for (int w = 0; w < kArnThreads / 32; w++)
-      ff_acc(t, s_red[2 * (w * kMaxV + threadIdx.x)], s_red[2 * (w * kMaxV + threadIdx.x) + 1]);
-    t = ff_norm(t);
-    row[2 * threadIdx.x] = t.s;
-    row[2 * threadIdx.x + 1] = t.q;
-  }
-  __syncthreads();
-}
+    bar_consumers();
+  };
+  // sum_i V_i f_i of the staged tile at this thread's M elements, its share of
+  // the vectors (half 0 even, half 1 odd)
+  const int e0 = tid & (kArnT - 1), half = tid / kArnT;
+  auto share = [&](const float* st, bool lo, FF (&p)[M]) {
+#pragma unroll
+    for (int m = 0; m < M; m++) p[m] = FF{0.f, 0.f};
+#pragma unroll(M >= 4 ? 2 : 4)
+    for (int i = half; i < nv; i += 2) {
+      const float* v = st + (size_t)i * slot + e0;
+      const float2 f = s_f[i];
+#pragma unroll
+      for (int m = 0; m < M; m++) {
+        const FF u = ff_mul(v[kArnT * m], lo ? v[T + kArnT * m] : 0.f, f.x, f.y);
+        ff_acc(p[m], u.s, u.q);
+      }
+    }
+    if (half) {
+#pragma unroll
+      for (int m = 0; m < M; m++) s_part[e0 + kArnT * m] = make_float2(p[m].s, p[m].q);
+    }
+    bar_consumers();
+  };
+  // w - V f at element e (half 0; p: its own share)
+  auto minus = [&](const float* wt, int e, const FF& p) {
+    FF t{wt[e], wt[T + e]};
+    ff_acc(t, -p.s, -p.q);
+    const float2 o = s_part[e];
+    ff_acc(t, -o.x, -o.y);
+    return ff_norm(t);
+  };
 
-// Sum of the blocks' pairs: s_out[i] (FP64) and s_outf[i] (the pair, renormalised)
-__device__ __forceinline__ void arn_grid_reduce_ff(const float* __restrict__ part, int nblk, int nv,
-                                                   double* __restrict__ s_out, float (*s_outf)[2]) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int i = wid; i < nv; i += kArnThreads / 32) {
+  // sweep 1: h1 = V^T w
+  dots_begin(nv);
+  for (int k = 0; k < nt; k++) {
+    const float* st = acquire(k);
+    dots(st, st + (size_t)nv * slot, count_of(k));
+    if (!resident) release(k);
+  }
+  dots_end(part);
+  grid.sync();
+  grid_sums(part, nv, s_h1);
+  // sweep 2: w' = w - V h1; h2 = V^T w', ||w'||^2.  w' stays out of the ring's
+  // w slot (the copies of later tiles write there) unless the tiles stay.
+  float2* part2 = part + (size_t)kArnDots * nblk;
+  dots_begin(nv + 1);
+  for (int q = 0; q < nt; q++) {
+    const int k = nt - 1 - q, c = resident ? k : nt + q;
+    float* st = resident ? s_ring + (size_t)(k % stages) * stage_f : acquire(c);
+    float* wt = st + (size_t)nv * slot;
+    float* wn = resident ? wt : s_w;
+    const int count = count_of(k);
+    FF p[M];
+    share(st, true, p);
+    if (!half) {
+#pragma unroll
+      for (int m = 0; m < M; m++) {
+        const int e = e0 + kArnT * m;
+        const FF t = minus(wt, e, p[m]);
+        wn[e] = t.s;
+        wn[T + e] = t.q;
+        if (!resident && e < count) {
+          const long long g = tile_of(k) * T + e;
+          w[g] = t.s;
+          w[ld + g] = t.q;
+        }
+      }
+    }
+    bar_consumers();
+    dots(st, wn, count);
+    if (!resident) release(c);
+  }
+  if (!resident) fence_proxy_async();  // the third sweep's copies read the w' written here
+  dots_end(part2);
+  grid.sync();
+  grid_sums(part2, nv + 1, s_h2);
+  if (wid == 0) {
+    double t = lane < nv ? s_h2[lane] * s_h2[lane] : 0.0;
+    t = warp_sum(t);
+    if (lane == 0) {
+      const double w2 = s_n2, n2 = w2 - t;
+      s_slow = !(n2 >= 0.5 * w2) || !(n2 > 0.0);
+      s_n2 = n2;
+      s_inv = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
+    }
+  }
+  bar_all();
+  const bool slow = s_slow != 0;
+  // V_nv = (w' - V h2) / ||w''||, and the next operator's FP32 input fp32(D V_nv)
+  auto put = [&](long long g, const FF& t, float ih, float il, float d) {
+    const FF u = ff_norm(ff_mul(t.s, t.q, ih, il));
+    vnext[g] = u.s;
+    vnext[ld + g] = u.q;
+    if (xf) xf[g] = u.s * d;
+  };
+  const bool scaled = xf && dh;
+  const float ih = (float)s_inv, il = (float)(s_inv - (double)ih);
+  FF nacc{0.f, 0.f};
+  for (int k = 0; k < nt; k++) {
+    const int c = 2 * nt + k, count = count_of(k);
+    const float* st = resident ? s_ring + (size_t)(k % stages) * stage_f : acquire(c);
+    float dv[M];
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+      const int e = e0 + kArnT * m;
+      dv[m] = 1.f;
+      if (!half && scaled && !slow && e < count) dv[m] = resident ? dh[tile_of(k) * T + e] : st[T + e];
+    }
+    FF p[M];
+    share(st, slow, p);
+    if (!half) {
+#pragma unroll
+      for (int m = 0; m < M; m++) {
+        const int e = e0 + kArnT * m;
+        const FF t = minus(st + (size_t)nv * slot, e, p[m]);
+        if (e < count) {
+          const long long g = tile_of(k) * T + e;
+          if (slow) {
+            w[g] = t.s;
+            w[ld + g] = t.q;
+            ff_dot_acc(nacc, t.s, t.q, t.s, t.q);
+          } else {
+            put(g, t, ih, il, dv[m]);
+          }
+        }
+      }
+    }
+    if (!resident) release(c);
+    bar_consumers();  // s_part is rewritten
+  }
+  if (!slow) return;
+  // w was (nearly) in the span of V: its remainder's norm from the sum itself
+  float2* part3 = part2 + (size_t)kArnDots * nblk;
+  dots_n = 1;
+  dots_p = 1;
+  dots_g = kArnWarps;
+  acc[0] = nacc;
+  acc[1] = FF{0.f, 0.f};
+  dots_end(part3);
+  grid.sync();
+  if (wid == 0) {
     FF t{0.f, 0.f};
-    for (int b = lane; b < nblk; b += 32)
-      ff_acc(t, __ldcg(part + 2 * ((size_t)b * kMaxV + i)), __ldcg(part + 2 * ((size_t)b * kMaxV + i) + 1));
+    for (int b = lane; b < nblk; b += 32) {
+      const float2 q = __ldcg(part3 + b);
+      ff_acc(t, q.x, q.y);
+    }
     t = ff_norm(ff_warp_sum(t));
     if (lane == 0) {
-      s_out[i] = (double)t.s + (double)t.q;
-      s_outf[i][0] = t.s;
-      s_outf[i][1] = t.q;
+      s_n2 = (double)t.s + (double)t.q;
+      s_inv = s_n2 > 0.0 ? 1.0 / sqrt(s_n2) : 0.0;
     }
   }
-  __syncthreads();
+  bar_all();
+  if (half) return;
+  const float jh = (float)s_inv, jl = (float)(s_inv - (double)jh);
+  for (int k = 0; k < nt; k++)
+    for (int m = 0; m < M; m++) {
+      const int e = e0 + kArnT * m;
+      const long long g = tile_of(k) * T + e;
+      if (e < count_of(k)) put(g, FF{w[g], w[ld + g]}, jh, jl, scaled ? dh[g] : 1.f);
+    }
 }
 
-// One Arnoldi step on pair vectors: CGS2 of w against V_0..V_{nv-1},
-// V_nv = w / ||w||, and the Givens update of the least-squares state.  The
-// sweeps are latency-bound at the occupancy the accumulators allow, so each
-// thread moves L consecutive elements per load (L = 4: 16-byte loads of every
-// hi and lo stream, when n is a multiple of 4; else L = 1).
-template <int L>
-__device__ __forceinline__ void ldv(const float* __restrict__ p, long long t, float (&o)[L]) {
-  if constexpr (L == 4) {
-    const float4 q = reinterpret_cast<const float4*>(p)[t];
-    o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
-  } else if constexpr (L == 2) {
-    const float2 q = reinterpret_cast<const float2*>(p)[t];
-    o[0] = q.x; o[1] = q.y;
-  } else {
-    o[0] = p[t];
+// pair stream length of an n-element Krylov vector
+__host__ __device__ __forceinline__ long long ff_ld(long long n) { return (n + 3) & ~3LL; }
+
+template <int M>
+cudaError_t launch_arnoldi_m(cudaStream_t s, int sms, long long n, const float* V, float* w, int nv,
+                             float* vnext, double* d_arn, GmState* gs, int jj, float* xf, const float* dh,
+                             unsigned long long* flags) {
+  constexpr int T = kArnT * M;
+  constexpr size_t extra = sizeof(float) * 4 * T;  // w' and the odd shares
+  static unsigned long long ready = 0;             // per device
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!((ready >> dev) & 1ull)) {
+    int per = 0;
+    cudaError_t e = cudaFuncSetAttribute(k_arnoldi_tile<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(kArnRing + extra));
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_arnoldi_tile<M>, kArnBlock, kArnRing + extra);
+    if (e != cudaSuccess) return e;
+    if (per < 1) return cudaErrorLaunchOutOfResources;
+    ready |= 1ull << dev;
   }
-}
-template <int L>
-__device__ __forceinline__ void stv(float* __restrict__ p, long long t, const float (&o)[L]) {
-  if constexpr (L == 4) {
-    reinterpret_cast<float4*>(p)[t] = make_float4(o[0], o[1], o[2], o[3]);
-  } else if constexpr (L == 2) {
-    reinterpret_cast<float2*>(p)[t] = make_float2(o[0], o[1]);
-  } else {
-    p[t] = o[0];
-  }
+  const long long tiles = (n + T - 1) / T;
+  const unsigned g = (unsigned)std::max<long long>(1, std::min<long long>(sms, tiles));
+  const size_t stage = sizeof(float) * 2 * T * (size_t)(nv + 1);
+  const long long most = (tiles + g - 1) / g;  // tiles of a CTA
+  int stages = (int)std::min<long long>({(long long)kArnMaxStages, (long long)(kArnRing / stage), most});
+  long long ld = ff_ld(n);
+  float2* part = reinterpret_cast<float2*>(d_arn);
+  void* args[] = {&n, &ld, &V, &w, &nv, &vnext, &part, &gs, &jj, &xf, &dh, &stages, &flags};
+  return cudaLaunchCooperativeKernel((const void*)k_arnoldi_tile<M>, dim3(g), dim3(kArnBlock), args,
+                                     stage * stages + extra, s);
 }
 
-template <int NVM, int L>
-__global__ void __launch_bounds__(kArnThreads) k_arnoldi_ff(long long n, const float* __restrict__ V,
-                                                             float* __restrict__ w, int nv,
-                                                             float* __restrict__ vnext,
-                                                             float* __restrict__ part, GmState* gs,
-                                                             int jj, float* __restrict__ xf,
-                                                             const float* __restrict__ dh) {
-  cg::grid_group grid = cg::this_grid();
-  __shared__ float s_red[2 * (kArnThreads / 32) * kMaxV];
-  __shared__ double s_h1[kMaxV], s_h2[kMaxV], s_n2[1];
-  __shared__ float s_f1[kMaxV][2], s_f2[kMaxV][2], s_fn[1][2];
-  const int nblk = gridDim.x;
-  float* pA = part;
-  float* pB = part + 2 * (size_t)nblk * kMaxV;
-  float* pC = pB + 2 * (size_t)nblk * kMaxV;
-  const long long nl = n / L;
-  const long long stride = (long long)nblk * kArnThreads;
-  const long long t0 = (long long)blockIdx.x * kArnThreads + threadIdx.x;
-  float* wl = w + n;
-  auto vh = [&](int i) { return V + 2 * (size_t)i * n; };
-  FF acc[NVM];
-  // pass 1: h1 = V^T w
-#pragma unroll
-  for (int i = 0; i < NVM; i++) acc[i] = FF{0.f, 0.f};
-  for (long long t = t0; t < nl; t += stride) {
-    float a[L], b[L];
-    ldv<L>(w, t, a);
-    ldv<L>(wl, t, b);
-#pragma unroll
-    for (int i = 0; i < NVM; i++)
-      if (i < nv) {
-        float x[L], y[L];
-        ldv<L>(vh(i), t, x);
-        ldv<L>(vh(i) + n, t, y);
-#pragma unroll
-        for (int k = 0; k < L; k++) ff_dot_acc(acc[i], x[k], y[k], a[k], b[k]);
-      }
-  }
-  arn_block_store_ff<NVM>(acc, nv, pA + 2 * (size_t)blockIdx.x * kMaxV, s_red);
-  grid.sync();
-  arn_grid_reduce_ff(pA, nblk, nv, s_h1, s_f1);
-  // pass 2: w -= V h1; h2 = V^T w
-#pragma unroll
-  for (int i = 0; i < NVM; i++) acc[i] = FF{0.f, 0.f};
-  for (long long t = t0; t < nl; t += stride) {
-    float a[L], b[L];
-    ldv<L>(w, t, a);
-    ldv<L>(wl, t, b);
-    FF wt[L];
-#pragma unroll
-    for (int k = 0; k < L; k++) wt[k] = FF{a[k], b[k]};
-#pragma unroll
-    for (int i = 0; i < NVM; i++)
-      if (i < nv) {
-        float x[L], y[L];
-        ldv<L>(vh(i), t, x);
-        ldv<L>(vh(i) + n, t, y);
-#pragma unroll
-        for (int k = 0; k < L; k++) {
-          const FF u = ff_mul(x[k], y[k], s_f1[i][0], s_f1[i][1]);
-          ff_acc(wt[k], -u.s, -u.q);
-        }
-      }
-#pragma unroll
-    for (int k = 0; k < L; k++) {
-      wt[k] = ff_norm(wt[k]);
-      a[k] = wt[k].s;
-      b[k] = wt[k].q;
-    }
-    stv<L>(w, t, a);
-    stv<L>(wl, t, b);
-    // the V loads again (cache hits) rather than 2 L more registers per vector
-#pragma unroll
-    for (int i = 0; i < NVM; i++)
-      if (i < nv) {
-        float x[L], y[L];
-        ldv<L>(vh(i), t, x);
-        ldv<L>(vh(i) + n, t, y);
-#pragma unroll
-        for (int k = 0; k < L; k++) ff_dot_acc(acc[i], x[k], y[k], a[k], b[k]);
-      }
-  }
-  arn_block_store_ff<NVM>(acc, nv, pB + 2 * (size_t)blockIdx.x * kMaxV, s_red);
-  grid.sync();
-  arn_grid_reduce_ff(pB, nblk, nv, s_h2, s_f2);
-  // pass 3: w -= V h2; ||w||^2
-  FF nacc[1] = {FF{0.f, 0.f}};
-  for (long long t = t0; t < nl; t += stride) {
-    float a[L], b[L];
-    ldv<L>(w, t, a);
-    ldv<L>(wl, t, b);
-    FF wt[L];
-#pragma unroll
-    for (int k = 0; k < L; k++) wt[k] = FF{a[k], b[k]};
-#pragma unroll
-    for (int i = 0; i < NVM; i++)
-      if (i < nv) {
-        float x[L], y[L];
-        ldv<L>(vh(i), t, x);
-        ldv<L>(vh(i) + n, t, y);
-#pragma unroll
-        for (int k = 0; k < L; k++) {
-          const FF u = ff_mul(x[k], y[k], s_f2[i][0], s_f2[i][1]);
-          ff_acc(wt[k], -u.s, -u.q);
-        }
-      }
-#pragma unroll
-    for (int k = 0; k < L; k++) {
-      wt[k] = ff_norm(wt[k]);
-      a[k] = wt[k].s;
-      b[k] = wt[k].q;
-      ff_dot_acc(nacc[0], a[k], b[k], a[k], b[k]);
-    }
-    stv<L>(w, t, a);
-    stv<L>(wl, t, b);
-  }
-  arn_block_store_ff<1>(nacc, 1, pC + 2 * (size_t)blockIdx.x * kMaxV, s_red);
-  grid.sync();
-  arn_grid_reduce_ff(pC, nblk, 1, s_n2, s_fn);
-  // V_nv = w / ||w|| (the elements this thread wrote in pass 3)
-  const double inv = s_n2[0] > 0.0 ? 1.0 / sqrt(s_n2[0]) : 0.0;
-  const float ih = (float)inv, il = (float)(inv - (double)ih);
-  for (long long t = t0; t < nl; t += stride) {
-    float a[L], b[L];
-    ldv<L>(w, t, a);
-    ldv<L>(wl, t, b);
-#pragma unroll
-    for (int k = 0; k < L; k++) {
-      const FF u = ff_norm(ff_mul(a[k], b[k], ih, il));
-      a[k] = u.s;
-      b[k] = u.q;
-    }
-    stv<L>(vnext, t, a);
-    stv<L>(vnext + n, t, b);
-    if (xf) {
-      // the next operator's FP32 input fp32(D V_nv), written while it is in registers
-      if (dh) {
-        float dd[L];
-        ldv<L>(dh, t, dd);
-#pragma unroll
-        for (int k = 0; k < L; k++) a[k] *= dd[k];
-      }
-      stv<L>(xf, t, a);
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) gm_update(gs, jj, s_h1, s_h2, s_n2[0]);
-}
-
-template <int NVM, int L>
-cudaError_t launch_arnoldi_ff_l(cudaStream_t s, long long n, const float* V, float* w, int nv,
-                                float* vnext, float* part, GmState* gs, int jj, float* xf, const float* dh) {
-  static int grid[64] = {0};  // per device: co-resident CTAs
+// Tile length: the longest of 1024, 512, 256 elements at which a stage is at
+// most a third of the ring (three loads in flight) and every CTA still gets 8
+// tiles (a tile costs two or three CTA barriers and the warps' latency: short
+// bases need long tiles, short vectors need tiles for every SM).
+cudaError_t launch_arnoldi(cudaStream_t s, long long n, const float* V, float* w, int nv, float* vnext,
+                           double* d_arn, GmState* gs, int jj, float* xf, const float* dh,
+                           unsigned long long* flags) {
+  static int sms[64] = {0};  // per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (grid[dev] == 0) {
-    int sms = 0, per = 0;
-    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_arnoldi_ff<NVM, L>, kArnThreads, 0);
+  if (sms[dev] == 0) {
+    int v = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    if (per < 1) return cudaErrorLaunchOutOfResources;
-    grid[dev] = std::min(sms * per, kArnMaxGrid);
+    sms[dev] = std::min(v, kArnMaxGrid);
   }
-  const long long want = (n / L + kArnThreads - 1) / kArnThreads;
-  const unsigned g = (unsigned)std::max<long long>(1, std::min<long long>(grid[dev], want));
-  void* args[] = {&n, &V, &w, &nv, &vnext, &part, &gs, &jj, &xf, &dh};
-  return cudaLaunchCooperativeKernel((const void*)k_arnoldi_ff<NVM, L>, dim3(g), dim3(kArnThreads), args, 0, s);
-}
-
-// the widest streams at which every pair vector's hi and lo start aligned
-template <int NVM>
-cudaError_t launch_arnoldi_ff(cudaStream_t s, long long n, const float* V, float* w, int nv,
-                              float* vnext, float* part, GmState* gs, int jj, float* xf, const float* dh) {
-  if (n % 4 == 0) return launch_arnoldi_ff_l<NVM, 4>(s, n, V, w, nv, vnext, part, gs, jj, xf, dh);
-  if (n % 2 == 0) return launch_arnoldi_ff_l<NVM, 2>(s, n, V, w, nv, vnext, part, gs, jj, xf, dh);
-  return launch_arnoldi_ff_l<NVM, 1>(s, n, V, w, nv, vnext, part, gs, jj, xf, dh);
+  if (nv + 1 > kArnDots) return cudaErrorInvalidValue;
+  const size_t unit = sizeof(float) * 2 * kArnT * (size_t)(nv + 1);
+  const long long units = n / kArnT / (8LL * sms[dev]);
+  if (3 * 4 * unit <= kArnRing && units >= 4)
+    return launch_arnoldi_m<4>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  if (3 * 2 * unit <= kArnRing && units >= 2)
+    return launch_arnoldi_m<2>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  return launch_arnoldi_m<1>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
 }
 
 // V0 = r / ||r|| as a pair vector (nrm2: ||r||^2)
@@ -722,7 +880,7 @@ __global__ void __launch_bounds__(256) k_start_ff(long long n, const double* __r
     const double x = r[t] * sc;
     const float h = (float)x;
     v[t] = h;
-    v[n + t] = (float)(x - (double)h);
+    v[ff_ld(n) + t] = (float)(x - (double)h);
     if (xf) xf[t] = dh ? h * dh[t] : h;  // the first operator's FP32 input
   }
 }
@@ -734,13 +892,13 @@ __global__ void __launch_bounds__(256) k_to_ff(long long n, const double* __rest
     const double a = x[t];
     const float h = (float)a;
     v[t] = h;
-    v[n + t] = (float)(a - (double)h);
+    v[ff_ld(n) + t] = (float)(a - (double)h);
   }
 }
 __global__ void __launch_bounds__(256) k_from_ff(long long n, const float* __restrict__ v, double* __restrict__ x) {
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x)
-    x[t] = (double)v[t] + (double)v[n + t];
+    x[t] = (double)v[t] + (double)v[ff_ld(n) + t];
 }
 
 // x += D sum_i y_i V_i, V pair vectors, D as pairs (or none); nv from *d_nv
@@ -752,6 +910,7 @@ __global__ void __launch_bounds__(256) k_combine_ff(long long n, const float* __
                                                     const float* __restrict__ dff,
                                                     double* __restrict__ x) {
   __shared__ float s_y[kMaxV][2];
+  const long long ld = ff_ld(n);
   const int nv = min(*d_nv, NVM);
   if (threadIdx.x < kMaxV) {
     const double v = threadIdx.x < nv ? y[threadIdx.x] : 0.0;
@@ -765,8 +924,8 @@ __global__ void __launch_bounds__(256) k_combine_ff(long long n, const float* __
 #pragma unroll
     for (int i = 0; i < NVM; i++)
       if (i < nv) {
-        vh[i] = V[2 * (size_t)i * n + t];
-        vl[i] = V[2 * (size_t)i * n + n + t];
+        vh[i] = V[2 * (size_t)i * ld + t];
+        vl[i] = V[2 * (size_t)i * ld + ld + t];
       }
     FF a{0.f, 0.f};
 #pragma unroll
@@ -950,7 +1109,7 @@ unsigned gridr(long long n, int cap = kRedBlocks, int ept = 4) {
 
 // ============================================================================
 // FP32 pair split of an operator input into the context's scratch (hi_only:
-// the FP32 rounding alone).  d_xs is also where k_start_ff / k_arnoldi_ff
+// the FP32 rounding alone).  d_xs is also where k_start_ff / k_arnoldi_tile
 // leave the FP32 input of the next Krylov vector's operator application: this
 // split, k_rhs and the AMR operators overwrite it, so none of them may run
 // between an Arnoldi step and the operator application that follows it.
@@ -1069,7 +1228,7 @@ cudaError_t launch_update_e(amps_gpu_ctx* c) {
 // ends when the FP64 residual satisfies ||b - A x|| <= tol ||b||.  The
 // preconditioner is none (precond 0), Jacobi (1, z = D v) or the learned block
 // network (2, z = D v + N(D v); flexible form: the directions z_j are kept).
-// Each Arnoldi step is the operator plus one cooperative kernel (k_arnoldi:
+// Each Arnoldi step is the operator plus one cooperative kernel (k_arnoldi_tile:
 // CGS2, normalisation and the Givens update).  The host does not wait for each
 // step: it queues as many Arnoldi steps as the last cycle took before it first
 // reads the device's convergence flag, then one step per read; steps queued
@@ -1103,7 +1262,8 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
   // bytes of d_V / d_w); the Jacobi scaling is used as pairs
   float* Vf = reinterpret_cast<float*>(c->d_V);
   float* wf = reinterpret_cast<float*>(c->d_w);
-  auto vf = [&](int j) { return Vf + 2 * (size_t)j * n; };
+  const long long ld = ff_ld(n);
+  auto vf = [&](int j) { return Vf + 2 * (size_t)j * ld; };
   const float* dh = nullptr;
   const float* dl = nullptr;
   if (dinv) {
@@ -1116,7 +1276,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     CK(cudaMalloc(reinterpret_cast<void**>(&c->d_tmpv), sizeof(double) * 2 * n));
   // w = A (D v_j), or A z_j for the flexible directions, as pairs
   // the FP32 operator input of the next Krylov vector is written by the step
-  // that makes the vector (k_start_ff, k_arnoldi_ff) when the operator takes V
+  // that makes the vector (k_start_ff, k_arnoldi_tile) when the operator takes V
   // directly (no learned directions, FP32 inner operator)
   // (nothing that writes d_xs -- split_input, k_rhs, the AMR operators -- runs
   // between a step that writes it and the inner_matvec that reads it)
@@ -1130,12 +1290,12 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
         in.vd = zj;
       } else {
         in.vh = vf(jj);
-        in.vl = vf(jj) + n;
+        in.vl = vf(jj) + ld;
         in.dh = dh;
         in.dl = dl;
         in.xf_ready = pre_xf;
       }
-      return launch_matvec32_ff(c, in, wf, wf + n);
+      return launch_matvec32_ff(c, in, wf, wf + ld);
     }
     // FP64 inner operator, through FP64 copies
     const double* x = zj;
@@ -1192,12 +1352,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
       }
     }
     TimedLaunch t(c, "gmres_orth");
-    float* part = reinterpret_cast<float*>(c->d_arn);
-    float* vnext = vf(nv);
-    if (nv <= 4) return launch_arnoldi_ff<4>(s, n, Vf, wf, nv, vnext, part, gs, jj, xf_next, dh);
-    if (nv <= 8) return launch_arnoldi_ff<8>(s, n, Vf, wf, nv, vnext, part, gs, jj, xf_next, dh);
-    if (nv <= 16) return launch_arnoldi_ff<16>(s, n, Vf, wf, nv, vnext, part, gs, jj, xf_next, dh);
-    return launch_arnoldi_ff<32>(s, n, Vf, wf, nv, vnext, part, gs, jj, xf_next, dh);
+    return launch_arnoldi(s, n, Vf, wf, nv, vf(nv), c->d_arn, gs, jj, xf_next, dh, c->d_flags);
   };
   // end of a cycle of at most nv_max steps: least squares, x += (D) V y, the
   // true FP64 residual into w and its squared norm into d_n2

@@ -26,6 +26,7 @@
 
 #include <mutex>
 
+#include "assemble_core.cuh"
 #include "common.cuh"
 #include "deposit_core.cuh"
 
@@ -48,26 +49,6 @@ static __device__ unsigned long long g_na_flags[4];
 constexpr int kMaxDevices = 64;
 unsigned char* g_scratch_addr[kMaxDevices] = {nullptr};
 std::mutex g_setup_mu;
-
-// (slot, cell, weight monomial) entries of the corner assembly grouped by slot,
-// and the table index of the corner inside each of its 8 cells (the same tables
-// the context path builds at run time).
-struct NaEntry {
-  unsigned char slot, cell, mono, pad;
-};
-__constant__ NaEntry c_na_asm[64] = {
-    {0, 0, 0, 0}, {0, 1, 2, 0}, {0, 2, 6, 0}, {0, 3, 8, 0}, {0, 4, 18, 0}, {0, 5, 20, 0},
-    {0, 6, 24, 0}, {0, 7, 26, 0}, {1, 1, 1, 0}, {1, 3, 7, 0}, {1, 5, 19, 0}, {1, 7, 25, 0},
-    {2, 0, 1, 0}, {2, 2, 7, 0}, {2, 4, 19, 0}, {2, 6, 25, 0}, {3, 2, 3, 0}, {3, 3, 5, 0},
-    {3, 6, 21, 0}, {3, 7, 23, 0}, {4, 3, 4, 0}, {4, 7, 22, 0}, {5, 2, 4, 0}, {5, 6, 22, 0},
-    {6, 0, 3, 0}, {6, 1, 5, 0}, {6, 4, 21, 0}, {6, 5, 23, 0}, {7, 1, 4, 0}, {7, 5, 22, 0},
-    {8, 0, 4, 0}, {8, 4, 22, 0}, {9, 4, 9, 0}, {9, 5, 11, 0}, {9, 6, 15, 0}, {9, 7, 17, 0},
-    {10, 5, 10, 0}, {10, 7, 16, 0}, {11, 4, 10, 0}, {11, 6, 16, 0}, {12, 6, 12, 0}, {12, 7, 14, 0},
-    {13, 7, 13, 0}, {14, 6, 13, 0}, {15, 4, 12, 0}, {15, 5, 14, 0}, {16, 5, 13, 0}, {17, 4, 13, 0},
-    {18, 0, 9, 0}, {18, 1, 11, 0}, {18, 2, 15, 0}, {18, 3, 17, 0}, {19, 1, 10, 0}, {19, 3, 16, 0},
-    {20, 0, 10, 0}, {20, 2, 16, 0}, {21, 2, 12, 0}, {21, 3, 14, 0}, {22, 3, 13, 0}, {23, 2, 13, 0},
-    {24, 0, 12, 0}, {24, 1, 14, 0}, {25, 1, 13, 0}, {26, 0, 13, 0}};
-__constant__ unsigned char c_na_corner[8] = {0, 1, 3, 2, 4, 5, 7, 6};
 
 struct NaMesh {
   int nbx, nby, nbz;
@@ -171,50 +152,38 @@ __global__ void __launch_bounds__(256) k_na_deposit(NaArgs a) {
   reduce_energy(ff_value(en), s_en, a.energy);
 }
 
-__global__ void __launch_bounds__(256) k_na_assemble(NaMesh m, long long ncor,
-                                                     const float* __restrict__ cellM,
-                                                     const float* __restrict__ cellJ,
-                                                     double inv_vol, double* __restrict__ M,
-                                                     double* __restrict__ J) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncor) return;
-  const int b = (int)(c / AMPS_CPB), l = (int)(c % AMPS_CPB);
-  const int i = l & 7, j = (l >> 3) & 7, k = l >> 6;
-  const long long g = m.global(b, i, j, k);
-  long long cell[8];
+// Corner assembly (assemble_core.cuh) into the global corner layout, FP64: the
+// tile's 32 x 243 sums go through shared memory so that a warp writes
+// consecutive doubles of a corner.  6144 corners: 32 us (a thread per corner:
+// 74 us, writes of 8 bytes at a stride of 1944 included).
+constexpr size_t kNaAsmSmem = kAsmSmem + sizeof(float) * kAsmCorners * AMPS_CELLM;
+
+__global__ void __launch_bounds__(kAsmThreads) k_na_assemble(NaMesh m, const float* __restrict__ cellM,
+                                                             const float* __restrict__ cellJ,
+                                                             double inv_vol, double* __restrict__ M,
+                                                             double* __restrict__ J) {
+  extern __shared__ __align__(16) float4 s_dyn[];
+  float* s_c = reinterpret_cast<float*>(s_dyn);
+  float* s_o = s_c + kAsmSmem / sizeof(float);
+  const int b = blockIdx.x / kAsmPerBlock, tile = blockIdx.x % kAsmPerBlock;
+  const int j0 = 4 * (tile & 1), k = tile >> 1;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  auto cell_id = [&](int ci, int cj, int ck) { return m.owned(b, ci, cj, ck); };
+  asm_stage(s_c, cellM, j0, k, cell_id);
+  asm_slots(s_c, wid, lane, [&](int slot, const float* acc) {
 #pragma unroll
-  for (int co = 0; co < 8; co++)
-    cell[co] = m.owned(b, i - (co & 1), j - ((co >> 1) & 1), k - ((co >> 2) & 1));
-  float acc[9];
-  int cur = c_na_asm[0].slot;
-#pragma unroll
-  for (int e = 0; e < 9; e++) acc[e] = 0.f;
-  for (int t = 0; t < 64; t++) {
-    const NaEntry en = c_na_asm[t];
-    if (en.slot != cur) {
-#pragma unroll
-      for (int e = 0; e < 9; e++) {
-        M[243 * g + cur * 9 + e] = widen(acc[e]);
-        acc[e] = 0.f;
-      }
-      cur = en.slot;
-    }
-    const float* src = cellM + cellM_at(cell[en.cell], en.mono * 9);
-#pragma unroll
-    for (int e = 0; e < 9; e++) acc[e] += src[e];
+    for (int e = 0; e < 9; e++) s_o[lane * AMPS_CELLM + slot * 9 + e] = acc[e];
+  });
+  __syncthreads();
+  // the tile's corners lie in four runs of 8 consecutive global indices
+  for (int t = threadIdx.x; t < kAsmCorners * AMPS_CELLM; t += kAsmThreads) {
+    const int r = t / (8 * AMPS_CELLM);
+    M[243 * m.global(b, 0, j0 + r, k) + (t - r * 8 * AMPS_CELLM)] = widen(s_o[t]);
   }
-#pragma unroll
-  for (int e = 0; e < 9; e++) M[243 * g + cur * 9 + e] = widen(acc[e]);
-  float jj[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-  for (int co = 0; co < 8; co++) {
-    const float* src = cellJ + cellJ_at(cell[co], c_na_corner[co] * 3);
-    jj[0] += src[0];
-    jj[1] += src[1];
-    jj[2] += src[2];
+  if (wid < 3) {
+    const int i = lane & 7, j = j0 + (lane >> 3);
+    J[3 * m.global(b, i, j, k) + wid] = widen(asm_current(cellJ, i, j, k, wid, cell_id)) * inv_vol;
   }
-#pragma unroll
-  for (int d = 0; d < 3; d++) J[3 * g + d] = widen(jj[d]) * inv_vol;
 }
 
 // Resolves the scratch address on `dev` (current) once; 0 on success.
@@ -226,6 +195,8 @@ cudaError_t setup_device(int dev, unsigned char** out) {
     if (e != cudaSuccess) return e;
     const int smem = (int)(AMPS_SC * sizeof(float4) + kNaWarps * kFields * kFS * sizeof(float));
     e = cudaFuncSetAttribute(k_na_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_na_assemble, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNaAsmSmem);
     if (e != cudaSuccess) return e;
     g_scratch_addr[dev] = static_cast<unsigned char*>(p);
   }
@@ -265,7 +236,6 @@ amps_gpu_status deposit_noalloc(const amps_gpu_config* cfg, long long n, const i
   float* cellJ = reinterpret_cast<float*>(base + kStencilBytes + kCellMBytes);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const NaMesh m{cfg->nbx, cfg->nby, cfg->nbz};
-  const long long ncor = nb * AMPS_CPB;
   if (cudaMemsetAsync(d_energy, 0, sizeof(double), s) != cudaSuccess) return AMPS_GPU_CUDA_ERROR;
   k_na_pack<<<(unsigned)nb, 256, 0, s>>>(m, d_B_corner, stencil);
   NaArgs a;
@@ -289,8 +259,8 @@ amps_gpu_status deposit_noalloc(const amps_gpu_config* cfg, long long n, const i
   const size_t smem = AMPS_SC * sizeof(float4) + kNaWarps * kFields * kFS * sizeof(float);
   k_na_deposit<<<dim3((unsigned)nb, AMPS_NC), kNaWarps * 32, smem, s>>>(a);
   const double inv_vol = 1.0 / (cfg->dx[0] * cfg->dx[1] * cfg->dx[2]);
-  k_na_assemble<<<(unsigned)((ncor + 255) / 256), 256, 0, s>>>(m, ncor, cellM, cellJ, inv_vol,
-                                                               d_M, d_J);
+  k_na_assemble<<<(unsigned)(nb * kAsmPerBlock), kAsmThreads, kNaAsmSmem, s>>>(m, cellM, cellJ, inv_vol,
+                                                                               d_M, d_J);
   return cudaGetLastError() == cudaSuccess ? AMPS_GPU_OK : AMPS_GPU_CUDA_ERROR;
 }
 

@@ -47,6 +47,7 @@
 #include <cmath>
 #include <cstdio>
 
+#include "assemble_core.cuh"
 #include "common.cuh"
 #include "deposit_core.cuh"
 
@@ -970,60 +971,27 @@ __global__ void __launch_bounds__(256) k_deposit(StepArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Corner assembly.  For corner c and each of its 8 cells, the pair (c, c2) of
-// that cell lands in slot(c2 - c) of M_c; its block is the cell's partial of
-// the pair's weight monomial.  The 64 (slot, cell, monomial) entries are
-// grouped by slot so each output slot is written once.
-struct AsmEntry {
-  unsigned char slot, cell, mono, pad;
-};
-__constant__ AsmEntry c_asm[64];
-__constant__ unsigned char c_asm_corner[8];
-
-__global__ void __launch_bounds__(256) k_assemble(long long ncor, const int* __restrict__ nbr,
-                                                  const float* __restrict__ cellM,
-                                                  const float* __restrict__ cellJ, double inv_vol,
-                                                  float* __restrict__ M, double* __restrict__ J) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncor) return;
-  const int b = (int)(c / AMPS_CPB), l = (int)(c % AMPS_CPB);
-  const int i = l & 7, j = (l >> 3) & 7, k = l >> 6;
-  int cell[8];
+// Corner assembly (assemble_core.cuh): M in 243 FP32 planes, J in FP64.
+// 32,768 corners: 26 us; 512 corners: 8 us (a thread per corner reading the
+// partials from global memory: 39 and 35 us).
+__global__ void __launch_bounds__(kAsmThreads, 2) k_assemble(long long ncor, const int* __restrict__ nbr,
+                                                          const float* __restrict__ cellM,
+                                                          const float* __restrict__ cellJ, double inv_vol,
+                                                          float* __restrict__ M, double* __restrict__ J) {
+  extern __shared__ __align__(16) float4 s_dyn[];
+  float* s_c = reinterpret_cast<float*>(s_dyn);
+  const int b = blockIdx.x / kAsmPerBlock, tile = blockIdx.x % kAsmPerBlock;
+  const int j0 = 4 * (tile & 1), k = tile >> 1;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  auto cell_id = [&](int ci, int cj, int ck) { return (long long)local_id(nbr, b, ci, cj, ck); };
+  asm_stage(s_c, cellM, j0, k, cell_id);
+  const long long c = (long long)b * AMPS_CPB + 64 * k + 8 * j0 + lane;
+  asm_slots(s_c, wid, lane, [&](int slot, const float* acc) {
 #pragma unroll
-  for (int co = 0; co < 8; co++)
-    cell[co] = local_id(nbr, b, i - (co & 1), j - ((co >> 1) & 1), k - ((co >> 2) & 1));
-  // sums of at most 8 FP32 partials per element (stored FP32)
-  float acc[9];
-  int cur = c_asm[0].slot;
-#pragma unroll
-  for (int e = 0; e < 9; e++) acc[e] = 0.f;
-  for (int t = 0; t < 64; t++) {
-    const AsmEntry en = c_asm[t];
-    if (en.slot != cur) {
-#pragma unroll
-      for (int e = 0; e < 9; e++) {
-        M[(size_t)(cur * 9 + e) * ncor + c] = acc[e];
-        acc[e] = 0.f;
-      }
-      cur = en.slot;
-    }
-    const float* src = cellM + cellM_at(cell[en.cell], en.mono * 9);
-#pragma unroll
-    for (int e = 0; e < 9; e++) acc[e] += src[e];
-  }
-#pragma unroll
-  for (int e = 0; e < 9; e++) M[(size_t)(cur * 9 + e) * ncor + c] = acc[e];
-  float jj[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-  for (int co = 0; co < 8; co++) {
-    const float* src = cellJ + cellJ_at(cell[co], c_asm_corner[co] * 3);
-    jj[0] += src[0];
-    jj[1] += src[1];
-    jj[2] += src[2];
-  }
-  J[c] = widen(jj[0]) * inv_vol;
-  J[ncor + c] = widen(jj[1]) * inv_vol;
-  J[2 * ncor + c] = widen(jj[2]) * inv_vol;
+    for (int e = 0; e < 9; e++) M[(size_t)(slot * 9 + e) * ncor + c] = acc[e];
+  });
+  if (wid < 3)
+    J[wid * ncor + c] = widen(asm_current(cellJ, lane & 7, j0 + (lane >> 3), k, wid, cell_id)) * inv_vol;
 }
 
 // ---------------------------------------------------------------------------
@@ -1723,42 +1691,6 @@ int grid_for(long long n, int threads) {
   return (int)g;
 }
 
-bool g_asm_ready = false;
-
-void init_asm_table() {
-  if (g_asm_ready) return;
-  static const int off[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
-                                {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
-  auto tidx = [&](int x, int y, int z) {
-    for (int t = 0; t < 8; t++)
-      if (off[t][0] == x && off[t][1] == y && off[t][2] == z) return t;
-    return -1;
-  };
-  AsmEntry e[64];
-  unsigned char corner_of[8];
-  int n = 0;
-  for (int slot = 0; slot < 27; slot++)
-    for (int co = 0; co < 8; co++) {
-      // cell = corner - (co&1, (co>>1)&1, (co>>2)&1): the corner sits at local
-      // offset (co&1, (co>>1)&1, (co>>2)&1) of that cell
-      const int lx = co & 1, ly = (co >> 1) & 1, lz = (co >> 2) & 1;
-      const int c1 = tidx(lx, ly, lz);
-      corner_of[co] = (unsigned char)c1;
-      for (int c2 = 0; c2 < 8; c2++) {
-        const int ddx = off[c2][0] - lx, ddy = off[c2][1] - ly, ddz = off[c2][2] - lz;
-        if (mm_slot(ddx, ddy, ddz) != slot) continue;
-        e[n].slot = (unsigned char)slot;
-        e[n].cell = (unsigned char)co;
-        e[n].mono = (unsigned char)pair_monomial(c1, c2);
-        e[n].pad = 0;
-        n++;
-      }
-    }
-  cudaMemcpyToSymbol(c_asm, e, sizeof(e));
-  cudaMemcpyToSymbol(c_asm_corner, corner_of, sizeof(corner_of));
-  g_asm_ready = true;
-}
-
 StepArgs step_args(amps_gpu_ctx* c) {
   StepArgs a;
   a.nbr = c->d_nbr;
@@ -1819,6 +1751,7 @@ void set_smem_attrs() {
   cudaFuncSetAttribute(k_arrivals<false, 16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_arr(16));
   cudaFuncSetAttribute(k_arrivals<true, 32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_arr(32));
   cudaFuncSetAttribute(k_arrivals<false, 32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_arr(32));
+  cudaFuncSetAttribute(k_assemble, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAsmSmem);
   done = true;
 }
 
@@ -1883,12 +1816,9 @@ cudaError_t place_ranked(amps_gpu_ctx* c, long long n) {
 // ===========================================================================
 // launchers
 
-// one-time host-side setup of the particle kernels (kernel attributes, the
-// constant assembly table); must precede any stream capture
-void particles_prepare() {
-  set_smem_attrs();
-  init_asm_table();
-}
+// one-time host-side setup of the particle kernels (kernel attributes); must
+// precede any stream capture
+void particles_prepare() { set_smem_attrs(); }
 
 cudaError_t launch_pack_stencils(amps_gpu_ctx* c, const double* Eh, const double* Bprev,
                                  const double* Bcur) {
@@ -1908,10 +1838,9 @@ cudaError_t launch_pack_stencils(amps_gpu_ctx* c, const double* Eh, const double
 // On AMR meshes the field operator reads the per-cell partials directly.
 static cudaError_t launch_assemble(amps_gpu_ctx* c) {
   if (c->amr) return cudaSuccess;
-  init_asm_table();
   TimedLaunch t(c, "assemble");
   const double inv_vol = 1.0 / (c->cfg.dx[0] * c->cfg.dx[1] * c->cfg.dx[2]);
-  k_assemble<<<(unsigned)((c->ncor + 255) / 256), 256, 0, c->stream>>>(
+  k_assemble<<<(unsigned)(c->nb * kAsmPerBlock), kAsmThreads, kAsmSmem, c->stream>>>(
       c->ncor, c->d_nbr, c->d_cellM, c->d_cellJ, inv_vol, c->d_M, c->d_J);
   return cudaGetLastError();
 }

@@ -24,6 +24,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace {
 
@@ -33,17 +34,6 @@ constexpr int kAsmRows = 10;                 // rows of 8 cells: 5 in y, 2 in z
 constexpr int kAsmRowF = 8 * AMPS_CELLM;     // floats of a row
 constexpr int kAsmThreads = 256;
 constexpr size_t kAsmSmem = sizeof(float) * (kAsmRows * kAsmRowF + kAsmRows * AMPS_CELLM);
-
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
 
 // slots by the number of entries: warp w of 8 takes s_asm_slot[first[w] .. first[w+1])
 __constant__ unsigned char c_asm_slot[27] = {0,  1,  2,  3,  6,  9,  18, 4,  5,  7,  8,  10, 11, 19,

@@ -13,8 +13,8 @@
 // Layouts: activations [sample][voxel of R, (k*10 + j)*10 + i][channel];
 // weights [tap (dx+1)+3(dy+1)+9(dz+1)][in channel][out channel].
 //
-// Kernels here (FP32 CUDA cores): k_conv (forward; with flipped, transposed
-// weights also the input gradient), k_wgrad (weight gradient), k_loss, k_adam,
+// Kernels (FP32 CUDA cores): the convolutions and weight gradients of
+// precond_conv.cuh; here k_loss, k_adam,
 // k_harvest (pairs from a solve), k_gather_region / k_scatter_z (inference on
 // the mesh).  The BF16 tensor-core inference kernel is in precond_tc.cu.
 #include <cuda_runtime.h>
@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "precond.cuh"
+#include "precond_conv.cuh"
 
 namespace {
 
@@ -35,126 +36,8 @@ constexpr int kR = 10;            // region edge
 constexpr int kRV = kR * kR * kR;  // region voxels
 constexpr int kOwn = 512;
 
-__host__ __device__ __forceinline__ int tap_dx(int t) { return t % 3 - 1; }
-__host__ __device__ __forceinline__ int tap_dy(int t) { return (t / 3) % 3 - 1; }
-__host__ __device__ __forceinline__ int tap_dz(int t) { return t / 9 - 1; }
 __device__ __forceinline__ bool owned_voxel(int i, int j, int k) {
   return i >= 1 && i <= 8 && j >= 1 && j <= 8 && k >= 1 && k <= 8;
-}
-
-// out[s][v][o] = sum_t sum_c W[t][c][o] in[s][v + off_t][c]   (zero outside R)
-// grid (10 planes, S), 256 threads; one plane of R per CTA.
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(256) k_conv(const float* __restrict__ in,
-                                              const float* __restrict__ W,
-                                              float* __restrict__ out, int owned_only) {
-  constexpr int CP = CIN + 1;  // padded smem row (bank spread)
-  extern __shared__ float smem[];
-  float* sW = smem;                         // 27*CIN*COUT
-  float* sIn = smem + 27 * CIN * COUT;      // 3 planes x 100 voxels x CP
-  const int kz = blockIdx.x, s = blockIdx.y;
-  for (int t = threadIdx.x; t < 27 * CIN * COUT; t += blockDim.x) sW[t] = W[t];
-  const float* ins = in + (size_t)s * kRV * CIN;
-  for (int t = threadIdx.x; t < 300 * CIN; t += blockDim.x) {
-    const int c = t % CIN, pv = t / CIN, pl = pv / 100, v = pv % 100;
-    const int z = kz + pl - 1;
-    sIn[pv * CP + c] = (z >= 0 && z < kR) ? ins[(size_t)(z * 100 + v) * CIN + c] : 0.f;
-  }
-  __syncthreads();
-  constexpr int OG = COUT >= 8 ? 8 : COUT;  // output channels per thread
-  constexpr int NG = COUT / OG;
-  float* outs = out + (size_t)s * kRV * COUT;
-  for (int item = threadIdx.x; item < 100 * NG; item += blockDim.x) {
-    const int v = item % 100, og = item / 100;
-    const int i = v % 10, j = v / 10;
-    float acc[OG];
-#pragma unroll
-    for (int o = 0; o < OG; o++) acc[o] = 0.f;
-    const bool active = !owned_only || owned_voxel(i, j, kz);
-    if (active) {
-      for (int t = 0; t < 27; t++) {
-        const int ii = i + tap_dx(t), jj = j + tap_dy(t), pl = 1 + tap_dz(t);
-        if (ii < 0 || ii >= kR || jj < 0 || jj >= kR) continue;
-        const float* src = sIn + (pl * 100 + jj * 10 + ii) * CP;
-        const float* w = sW + t * CIN * COUT + og * OG;
-#pragma unroll 4
-        for (int c = 0; c < CIN; c++) {
-          const float a = src[c];
-#pragma unroll
-          for (int o = 0; o < OG; o++) acc[o] = fmaf(a, w[c * COUT + o], acc[o]);
-        }
-      }
-    }
-#pragma unroll
-    for (int o = 0; o < OG; o++) outs[(size_t)(kz * 100 + v) * COUT + og * OG + o] = acc[o];
-  }
-}
-
-// Wt[t][o][c] = W[26 - t][c][o]: the input gradient is a convolution of the
-// output gradient with flipped taps and transposed channels
-__global__ void k_flip(const float* __restrict__ W, float* __restrict__ Wt, int cin, int cout) {
-  const int n = 27 * cin * cout;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-    const int t = q / (cin * cout), r = q % (cin * cout), c = r / cout, o = r % cout;
-    Wt[((size_t)(26 - t) * cout + o) * cin + c] = W[q];
-  }
-}
-
-// dW[t][c][o] += sum_{s,v} dout[s][v][o] in[s][v + off_t][c]
-// grid (27 taps, sample chunks), 256 threads; voxel tiles of 64 in shared memory.
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(256) k_wgrad(int S, int chunk, const float* __restrict__ dout,
-                                               const float* __restrict__ in,
-                                               float* __restrict__ dW) {
-  constexpr int TV = 64;
-  constexpr int NP = CIN * COUT;
-  constexpr int PT = (NP + 255) / 256;  // (c,o) pairs per thread
-  __shared__ float sD[TV][COUT + 1];
-  __shared__ float sI[TV][CIN + 1];
-  const int t = blockIdx.x;
-  const int dx = tap_dx(t), dy = tap_dy(t), dz = tap_dz(t);
-  const int s0 = blockIdx.y * chunk, s1 = min(S, s0 + chunk);
-  float acc[PT];
-#pragma unroll
-  for (int q = 0; q < PT; q++) acc[q] = 0.f;
-  for (int s = s0; s < s1; s++) {
-    const float* ds = dout + (size_t)s * kRV * COUT;
-    const float* is = in + (size_t)s * kRV * CIN;
-    for (int v0 = 0; v0 < kRV; v0 += TV) {
-      __syncthreads();
-      for (int q = threadIdx.x; q < TV * COUT; q += blockDim.x) {
-        const int vv = q / COUT, o = q % COUT, v = v0 + vv;
-        sD[vv][o] = v < kRV ? ds[(size_t)v * COUT + o] : 0.f;
-      }
-      for (int q = threadIdx.x; q < TV * CIN; q += blockDim.x) {
-        const int vv = q / CIN, c = q % CIN, v = v0 + vv;
-        float a = 0.f;
-        if (v < kRV) {
-          const int i = v % 10 + dx, j = (v / 10) % 10 + dy, k = v / 100 + dz;
-          if (i >= 0 && i < kR && j >= 0 && j < kR && k >= 0 && k < kR)
-            a = is[(size_t)((k * 10 + j) * 10 + i) * CIN + c];
-        }
-        sI[vv][c] = a;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < PT; q++) {
-        const int pidx = threadIdx.x + q * 256;
-        if (pidx < NP) {
-          const int c = pidx / COUT, o = pidx % COUT;
-          float a = acc[q];
-#pragma unroll 8
-          for (int vv = 0; vv < TV; vv++) a = fmaf(sD[vv][o], sI[vv][c], a);
-          acc[q] = a;
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < PT; q++) {
-    const int pidx = threadIdx.x + q * 256;
-    if (pidx < NP) atomicAdd(dW + (size_t)t * NP + pidx, acc[q]);
-  }
 }
 
 // loss = mean over owned voxels, channels of (x + y - e)^2; dy = dloss/dy
@@ -338,31 +221,14 @@ __global__ void k_owned_out(int S, const float* __restrict__ y, float* __restric
   }
 }
 
-template <int CIN, int COUT>
-size_t conv_smem() {
-  return sizeof(float) * (27 * CIN * COUT + 300 * (CIN + 1));
-}
-
-template <int CIN, int COUT>
-cudaError_t conv(PrecondState* P, cudaStream_t st, int S, const float* in, const float* W,
-                 float* out, int owned_only) {
-  const size_t sm = conv_smem<CIN, COUT>();
-  static unsigned long long attr_set = 0;  // per device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!((attr_set >> dev) & 1ull)) {
-    cudaFuncSetAttribute(k_conv<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    attr_set |= 1ull << dev;
-  }
-  k_conv<CIN, COUT><<<dim3(kR, S), 256, sm, st>>>(in, W, out, owned_only);
-  return cudaGetLastError();
-}
-
-template <int CIN, int COUT>
-cudaError_t wgrad(cudaStream_t st, int S, const float* dout, const float* in, float* dW) {
-  const int chunk = 4;
-  k_wgrad<CIN, COUT><<<dim3(27, (S + chunk - 1) / chunk), 256, 0, st>>>(S, chunk, dout, in, dW);
-  return cudaGetLastError();
+cudaError_t device_sms(int* dev, int* sms) {
+  cudaError_t e = cudaGetDevice(dev);
+  if (e == cudaSuccess && (*dev < 0 || *dev >= 64)) e = cudaErrorInvalidDevice;
+  static int n[64] = {0};
+  if (e == cudaSuccess && n[*dev] == 0)
+    e = cudaDeviceGetAttribute(&n[*dev], cudaDevAttrMultiProcessorCount, *dev);
+  if (e == cudaSuccess) *sms = n[*dev];
+  return e;
 }
 
 }  // namespace
@@ -371,11 +237,12 @@ cudaError_t wgrad(cudaStream_t st, int S, const float* dout, const float* in, fl
 const int kWSize[3] = {27 * 3 * 32, 27 * 32 * 32, 27 * 32 * 3};
 
 static void free_work(PrecondState* P) {
-  float* ws[] = {P->wx, P->we, P->h1, P->h2, P->y, P->dy, P->dh1, P->dh2, P->wt};
+  float* ws[] = {P->wx, P->we, P->h1, P->h2, P->y, P->dy, P->dh1, P->dh2, P->part};
   for (float* p : ws) cudaFree(p);
   cudaFree(P->perm);
-  P->wx = P->we = P->h1 = P->h2 = P->y = P->dy = P->dh1 = P->dh2 = P->wt = nullptr;
+  P->wx = P->we = P->h1 = P->h2 = P->y = P->dy = P->dh1 = P->dh2 = P->part = nullptr;
   P->perm = nullptr;
+  P->perm_n = 0;
   P->work_S = 0;
 }
 
@@ -394,7 +261,7 @@ cudaError_t precond_work(PrecondState* P, int S) {
   al(&P->dy, (size_t)S * kRV * 3);
   al(&P->dh1, (size_t)S * kRV * 32);
   al(&P->dh2, (size_t)S * kRV * 32);
-  al(&P->wt, (size_t)27 * 32 * 32);
+  al(&P->part, (size_t)27 * 32 * 32 * std::min(2 * S, kMaxParts));
   if (e == cudaSuccess) P->work_S = S;
   return e;
 }
@@ -427,10 +294,12 @@ void precond_free(PrecondState* P) {
 
 // forward of the FP32 training path: wx -> h1 -> h2 -> y (owned voxels)
 cudaError_t precond_forward32(PrecondState* P, cudaStream_t st, int S) {
-  cudaError_t e;
-  if ((e = conv<3, 32>(P, st, S, P->wx, P->w[0], P->h1, 0)) != cudaSuccess) return e;
-  if ((e = conv<32, 32>(P, st, S, P->h1, P->w[1], P->h2, 0)) != cudaSuccess) return e;
-  return conv<32, 3>(P, st, S, P->h2, P->w[2], P->y, 1);
+  int dev = 0, sms = 0;
+  cudaError_t e = device_sms(&dev, &sms);
+  if (e != cudaSuccess) return e;
+  if ((e = conv32<3, false>(st, S, sms, dev, P->wx, P->w[0], P->h1)) != cudaSuccess) return e;
+  if ((e = conv32<32, false>(st, S, sms, dev, P->h1, P->w[1], P->h2)) != cudaSuccess) return e;
+  return conv_out(st, S, sms, dev, P->h2, P->w[2], P->y);
 }
 
 // loss (added into *d_loss) and weight gradients (added into g) of the batch in wx/we
@@ -438,13 +307,13 @@ cudaError_t precond_backward32(PrecondState* P, cudaStream_t st, int S, double* 
   cudaError_t e;
   if ((e = precond_forward32(P, st, S)) != cudaSuccess) return e;
   k_loss<<<std::min(S * 4, 1024), 256, 0, st>>>(S, P->wx, P->y, P->we, P->dy, d_loss);
-  if ((e = wgrad<32, 3>(st, S, P->dy, P->h2, P->g[2])) != cudaSuccess) return e;
-  k_flip<<<64, 256, 0, st>>>(P->w[2], P->wt, 32, 3);
-  if ((e = conv<3, 32>(P, st, S, P->dy, P->wt, P->dh2, 0)) != cudaSuccess) return e;
-  if ((e = wgrad<32, 32>(st, S, P->dh2, P->h1, P->g[1])) != cudaSuccess) return e;
-  k_flip<<<64, 256, 0, st>>>(P->w[1], P->wt, 32, 32);
-  if ((e = conv<32, 32>(P, st, S, P->dh2, P->wt, P->dh1, 0)) != cudaSuccess) return e;
-  return wgrad<3, 32>(st, S, P->dh1, P->wx, P->g[0]);
+  int dev = 0, sms = 0;
+  if ((e = device_sms(&dev, &sms)) != cudaSuccess) return e;
+  if ((e = wgrad(st, S, sms, dev, 2, P->dy, P->h2, P->part, P->g[2])) != cudaSuccess) return e;
+  if ((e = conv32<3, true>(st, S, sms, dev, P->dy, P->w[2], P->dh2)) != cudaSuccess) return e;
+  if ((e = wgrad(st, S, sms, dev, 0, P->dh2, P->h1, P->part, P->g[1])) != cudaSuccess) return e;
+  if ((e = conv32<32, true>(st, S, sms, dev, P->dh2, P->w[1], P->dh1)) != cudaSuccess) return e;
+  return wgrad(st, S, sms, dev, 1, P->dh1, P->wx, P->part, P->g[0]);
 }
 
 cudaError_t precond_zero_grads(PrecondState* P, cudaStream_t st) {

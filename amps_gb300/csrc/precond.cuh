@@ -42,7 +42,8 @@ struct PrecondState {
   // work buffers for S samples
   int work_S = 0;
   float *wx = nullptr, *we = nullptr, *h1 = nullptr, *h2 = nullptr, *y = nullptr;
-  float *dy = nullptr, *dh1 = nullptr, *dh2 = nullptr, *wt = nullptr;
+  float *dy = nullptr, *dh1 = nullptr, *dh2 = nullptr;
+  float* part = nullptr;  // the CTAs' partial weight gradients (precond_conv.cuh)
   int* perm = nullptr;
   long long perm_n = 0;
   double* dloss = nullptr;  // device loss accumulator

@@ -25,6 +25,11 @@ constexpr double kPi = 3.14159265358979323846264338327950288;
 __constant__ int c_off[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
                                 {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
 
+// offset bit d of corner c in the table order above
+__host__ __device__ constexpr int off_bit(int c, int d) {
+  return d == 0 ? (((c + 1) >> 1) & 1) : (d == 1 ? ((c >> 1) & 1) : (c >> 2));
+}
+
 struct Hang {
   const int* hs;
   const int* hp;
@@ -53,18 +58,6 @@ __device__ __forceinline__ double cval(const double* __restrict__ F, const doubl
     const int p = h.hp[t];
     v += h.hw[t] * (dinv ? dinv[d * nvc + p] * F[d * nvc + p] : F[d * nvc + p]);
   }
-  return v;
-}
-
-// FP32 value of corner c, component d (xf already scaled), P applied
-__device__ __forceinline__ float cval_f(const float* __restrict__ xf, long long nvc, int c, int d,
-                                        const Hang& h) {
-  // the value is loaded alongside the hanging test (one dependent load fewer)
-  const float v0 = xf[d * nvc + c];
-  const int s = h.hs[c], e = h.hs[c + 1];
-  if (s == e) return v0;
-  float v = 0.f;
-  for (int t = s; t < e; t++) v = fmaf(h.hwh[t], xf[d * nvc + h.hp[t]], v);
   return v;
 }
 
@@ -168,9 +161,9 @@ __device__ __forceinline__ void scatter_row(T* __restrict__ y, long long nvc, co
 }
 
 // per cell size (index log2 of the block's cell size in finest cells): the
-// operator's scale factors, FP32 for the inner operator and as FP32 pairs
+// operator's scale factors as FP32 pairs (the FP32 inner operator takes the hi
+// halves)
 struct LevelK {
-  float dx, V;                       // FP32 inner operator
   float curl[2], cc[2], id[2], m[2], bb[2];  // 0.25/dx, th2dt2 V 0.25/dx, V/8, f V, thdt V 0.25/dx
 };
 constexpr int kMaxScale = 8;
@@ -178,6 +171,7 @@ constexpr int kMaxScale = 8;
 struct ApplyArgs {
   long long ncell, nvc;
   const int* ctab;
+  const int* ctabh;     // ctab with hanging corners as ~id
   Hang h;
   const int* bscale;
   LevelK lk[kMaxScale];
@@ -196,44 +190,174 @@ struct ApplyArgs {
 };
 
 // ---------------------------------------------------------------------------
-// The operator per cell (weak form, see above), y += its contributions.  A CTA
-// serves 32 cells with 3 threads each (one per output component p; warp p
-// takes the 32 cells): the cells' run of partials (31,104 contiguous bytes) is
-// brought into shared memory by one bulk copy while the threads gather the
-// corner values (each value once, shared through shared memory), and each
-// thread reads the rows 3p..3p+2 of its cell's 27 monomial blocks from there
-// (stride 243 words between a warp's cells: conflict-free).
-//   ACC 0: FP32 inner operator (curl-curl + mass; identity added in FP64 by
-//          k_amr_finish32), FP32 atomics;
-//   ACC 1: the full operator to FP64 accuracy (outer residuals);
-//   ACC 2: the RHS to FP64 accuracy.
-// ACC 1/2 run in FP32 pairs (FF, common.cuh): FP64 arithmetic is a small
-// fraction of the FP32 rate on this part; the pairs carry FP64 accuracy.
+// The operator per cell (weak form, see above), y += its contributions, on
+// tiles of 32 cells (an 8 x 4 x 1 slab of a block: 9 x 5 x 2 corners, 31,104
+// contiguous bytes of partials) with 3 threads per cell: warp p takes the 32
+// cells' output component p and reads the rows 3p..3p+2 of each cell's 27
+// monomial blocks from shared memory (stride 243 words between the lanes'
+// cells: conflict-free).
 constexpr int kTileCells = 32;
 constexpr int kTileThreads = 3 * kTileCells;
 constexpr uint32_t kTileBytes = kTileCells * AMPS_CELLM * 4;  // 31,104
+constexpr int kTC = 90;  // tile corners, (i, j, k) at i + 9 (j + 5 k)
 
+// The FP32 inner operator (curl-curl + mass; identity added in pairs by
+// k_amr_finish_ff).  Bound: reading the partials (478 MB at 491,520 cells).
+// Persistent CTAs, three per SM with two tile buffers each: the next tile's
+// bulk copy, its corner values and the corner ids of the one after are in
+// flight while a tile is computed (one tile per CTA, six CTAs per SM, held its
+// buffer through the whole chain of dependent loads: 3.8 TB/s).  Each corner
+// value is gathered once per tile; the corner table carries hanging corners as
+// ~id, so the common corner needs no look at the constraint rows.  The cells'
+// contributions to a corner are added by shuffles along x and y, and go out as
+// one global reduction per tile corner and component (P^T for hanging ones).
+// 491,520 cells: XX us, before 132.
+__global__ void __launch_bounds__(kTileThreads) k_amr_tile32(ApplyArgs a, int tiles, float* __restrict__ y32) {
+  extern __shared__ __align__(16) float s_m[];  // two tiles of partials
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ float s_x[3][kTC];
+  __shared__ int s_id[kTC];
+  const int tid = threadIdx.x, p = tid / 32, lane = tid & 31;
+  const int step = gridDim.x;
+  if (tid == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  auto copy = [&](int tile, int buf) {
+    mbar_arrive_expect_tx(&bar[buf], kTileBytes);
+    bulk_copy_g2s(s_m + (size_t)buf * (kTileBytes / 4), a.cellM + (size_t)tile * kTileCells * AMPS_CELLM,
+                  kTileBytes, &bar[buf]);
+  };
+  // thread t < 90 owns tile corner t
+  const int ti = tid % 9, tj = (tid / 9) % 5, tk = tid / 45;
+  auto corner_id = [&](int tile) {
+    if (tile >= tiles || tid >= kTC) return 0;
+    const int b = tile >> 4, l = (tile & 15) * kTileCells;  // 16 tiles per block
+    return __ldg(a.ctabh + b * 729 + ti + 9 * (((l >> 3) & 7) + tj + 9 * ((l >> 6) + tk)));
+  };
+  auto corner_values = [&](int id, float (&x)[3]) {
+    if (id >= 0) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) x[d] = a.xf[d * a.nvc + id];
+    } else {
+      const int h = ~id, s = a.h.hs[h], e = a.h.hs[h + 1];
+#pragma unroll
+      for (int d = 0; d < 3; d++) x[d] = 0.f;
+      for (int t = s; t < e; t++) {
+        const float w = a.h.hwh[t];
+        const int q = a.h.hp[t];
+#pragma unroll
+        for (int d = 0; d < 3; d++) x[d] = fmaf(w, a.xf[d * a.nvc + q], x[d]);
+      }
+    }
+  };
+  int tile = blockIdx.x;  // grid <= tiles
+  if (tid == 0) copy(tile, 0);
+  int id = corner_id(tile), id1 = corner_id(tile + step);
+  float x[3] = {0.f, 0.f, 0.f};
+  if (tid < kTC) corner_values(id, x);
+  int n = 0;  // tiles done
+  for (; tile < tiles; tile += step, n++) {
+    const int buf = n & 1;
+    const bool more = tile + step < tiles;
+    if (tid == 0 && more) copy(tile + step, buf ^ 1);
+    if (tid < kTC) {
+      s_id[tid] = id;
+#pragma unroll
+      for (int d = 0; d < 3; d++) s_x[d][tid] = x[d];
+    }
+    // in flight over this tile's arithmetic
+    const int id2 = corner_id(tile + 2 * step);
+    if (tid < kTC && more) corner_values(id1, x);
+    id = id1;
+    id1 = id2;
+    // CTA-uniform: every thread leaves together on a timeout
+    const bool ok = __syncthreads_and(mbar_wait_bounded(&bar[buf], (n >> 1) & 1, kWaitLimit)) != 0;
+    if (!ok) {
+      if (tid == 0) atomicAdd(a.flags + 2, 1ull);
+      // let the copies land before exiting
+      mbar_wait_bounded(&bar[buf], (n >> 1) & 1, kWaitLimit);
+      if (more) mbar_wait_bounded(&bar[buf ^ 1], ((n + 1) >> 1) & 1, kWaitLimit);
+      return;
+    }
+    const LevelK& K = a.lk[min(__ffs(__ldg(a.bscale + (tile >> 4))) - 1, kMaxScale - 1)];
+    const int i = lane & 7, j = lane >> 3;
+    float e[8][3], out[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      out[c] = 0.f;
+      const int tc = (i + off_bit(c, 0)) + 9 * ((j + off_bit(c, 1)) + 5 * off_bit(c, 2));
+#pragma unroll
+      for (int d = 0; d < 3; d++) e[c][d] = s_x[d][tc];
+    }
+    // mass term, monomial by monomial: the ordered corner pairs that share it
+    const float* mm = s_m + (size_t)buf * (kTileBytes / 4) + lane * AMPS_CELLM + 3 * p;
+#pragma unroll
+    for (int mono = 0; mono < 27; mono++) {
+      const float m0 = mm[9 * mono], m1 = mm[9 * mono + 1], m2 = mm[9 * mono + 2];
+#pragma unroll
+      for (int c1 = 0; c1 < 8; c1++)
+#pragma unroll
+        for (int c2 = 0; c2 < 8; c2++)
+          if (pair_monomial(c1, c2) == mono) out[c1] = fmaf(m0, e[c2][0], fmaf(m1, e[c2][1], fmaf(m2, e[c2][2], out[c1])));
+    }
+    float cu[3];
+    cell_curl<float>(e, K.curl[0], cu);
+    const float fv = K.m[0];
+#pragma unroll
+    for (int c = 0; c < 8; c++) out[c] *= fv;
+    if (p == 0) cell_curl_t_row<float>(cu, K.cc[0], 0, out);
+    else if (p == 1) cell_curl_t_row<float>(cu, K.cc[0], 1, out);
+    else cell_curl_t_row<float>(cu, K.cc[0], 2, out);
+    // out[c] in the table order (0,0) (1,0) (1,1) (0,1), z: add along x and y
+    auto put = [&](int tc, float v) {
+      const int q = s_id[tc];
+      if (q >= 0) {
+        atomicAdd(y32 + p * a.nvc + q, v);
+      } else {
+        const int h = ~q;
+        for (int t = a.h.hs[h]; t < a.h.hs[h + 1]; t++) atomicAdd(y32 + p * a.nvc + a.h.hp[t], a.h.hwh[t] * v);
+      }
+    };
+#pragma unroll
+    for (int z = 0; z < 2; z++) {
+      const float r0 = __shfl_up_sync(0xffffffffu, out[4 * z + 1], 1);
+      const float r1 = __shfl_up_sync(0xffffffffu, out[4 * z + 2], 1);
+      const float c0 = out[4 * z] + (i > 0 ? r0 : 0.f);      // corner (i, j)
+      const float c1 = out[4 * z + 3] + (i > 0 ? r1 : 0.f);  // corner (i, j + 1)
+      const float e0 = out[4 * z + 1], e1 = out[4 * z + 2];  // lanes i = 7: corners (8, j), (8, j + 1)
+      const float d0 = __shfl_up_sync(0xffffffffu, c1, 8), d1 = __shfl_up_sync(0xffffffffu, e1, 8);
+      put(i + 9 * (j + 5 * z), c0 + (j > 0 ? d0 : 0.f));
+      if (i == 7) put(8 + 9 * (j + 5 * z), e0 + (j > 0 ? d1 : 0.f));
+      if (j == 3) put(i + 9 * (4 + 5 * z), c1);
+      if (i == 7 && j == 3) put(8 + 9 * (4 + 5 * z), e1);
+    }
+    __syncthreads();  // s_x, s_id and this buffer are rewritten
+  }
+}
+
+// The operator (ACC 1) and the RHS (ACC 2) to FP64 accuracy, one tile per CTA,
+// in FP32 pairs (FF, common.cuh): FP64 arithmetic is a small fraction of the
+// FP32 rate on this part; the pairs carry FP64 accuracy.  The tile's partials
+// come by one bulk copy while the threads gather the corner values (each value
+// once, shared through shared memory).
 template <int ACC>
-__global__ void __launch_bounds__(kTileThreads) k_amr_cell_tile(ApplyArgs a, float* __restrict__ y32,
-                                                               double* __restrict__ y64) {
+__global__ void __launch_bounds__(kTileThreads) k_amr_cell_tile(ApplyArgs a, double* __restrict__ y64) {
   extern __shared__ __align__(16) float s_m[];
   __shared__ __align__(8) uint64_t bar;
-  // corner values (8 corners x 3): FP32 for ACC 0, FP32 pairs for ACC 1/2
+  // corner values (8 corners x 3) as pairs
   __shared__ float s_eh[kTileCells][24];
-  __shared__ float s_el[ACC == 0 ? 1 : kTileCells][24];
+  __shared__ float s_el[kTileCells][24];
   // the cell's curl (and for the RHS its centre B) as pairs, one component per thread
-  __shared__ float s_cu[ACC == 0 ? 1 : kTileCells][3][2];
+  __shared__ float s_cu[kTileCells][3][2];
   __shared__ float s_b[ACC == 2 ? kTileCells : 1][3][2];
-  // ACC 0: the tile's 32 cells (an 8 x 4 x 1 slab of a block) share 9 x 5 x 2
-  // corners; their contributions are summed in shared memory first, so each
-  // corner gets one global atomic per component instead of up to 8
-  constexpr int kTC = 90;
-  __shared__ float s_acc[ACC == 0 ? 3 * kTC : 1];
+  // the tile corners' sums as pairs, accumulated without atomics: warp p owns
+  // component p, and in round c the 32 cells' corner c are 32 distinct tile
+  // corners
   __shared__ int s_tcid[kTC];
-  // ACC 1/2: the same per-corner sums as pairs, accumulated without atomics:
-  // warp p owns component p, and in round c the 32 cells' corner c are 32
-  // distinct tile corners
-  __shared__ float s_ffacc[ACC == 0 ? 1 : 3][ACC == 0 ? 1 : kTC][2];
+  __shared__ float s_ffacc[3][kTC][2];
   const int tid = threadIdx.x, p = tid / kTileCells, lc = tid % kTileCells;
   const long long cell0 = (long long)blockIdx.x * kTileCells;
   if (tid == 0) {
@@ -262,13 +386,9 @@ __global__ void __launch_bounds__(kTileThreads) k_amr_cell_tile(ApplyArgs a, flo
     cid[c] = a.ctab[b * 729 + (i + c_off[c][0]) + 9 * ((j + c_off[c][1]) + 9 * (k + c_off[c][2]))];
     if (c % 3 == p) s_tcid[tcorner(c)] = cid[c];  // the same id from every cell sharing it
   }
-  if (ACC == 0) {
-    for (int q = tid; q < 3 * kTC; q += kTileThreads) s_acc[q] = 0.f;
-  } else {
-    for (int q = tid; q < 3 * kTC; q += kTileThreads) {
-      s_ffacc[q / kTC][q % kTC][0] = 0.f;
-      s_ffacc[q / kTC][q % kTC][1] = 0.f;
-    }
+  for (int q = tid; q < 3 * kTC; q += kTileThreads) {
+    s_ffacc[q / kTC][q % kTC][0] = 0.f;
+    s_ffacc[q / kTC][q % kTC][1] = 0.f;
   }
   if (ACC == 2) {
     // centre B, component p, split into a pair (the only FP64 arithmetic besides the scatter)
@@ -279,13 +399,9 @@ __global__ void __launch_bounds__(kTileThreads) k_amr_cell_tile(ApplyArgs a, flo
   }
 #pragma unroll
   for (int c = 0; c < 8; c++) {
-    if (ACC == 0) {
-      s_eh[lc][3 * c + p] = cval_f(a.xf, a.nvc, cid[c], p, a.h);
-    } else {
-      const FF v = cval_ff(a.xh, a.xl, a.nvc, cid[c], p, a.h);
-      s_eh[lc][3 * c + p] = v.s;
-      s_el[lc][3 * c + p] = v.q;
-    }
+    const FF v = cval_ff(a.xh, a.xl, a.nvc, cid[c], p, a.h);
+    s_eh[lc][3 * c + p] = v.s;
+    s_el[lc][3 * c + p] = v.q;
   }
   // CTA-uniform: every thread leaves together on a timeout (later barriers)
   const bool ok = __syncthreads_and(mbar_wait_bounded(&bar, 0, kWaitLimit)) != 0;
@@ -295,153 +411,115 @@ __global__ void __launch_bounds__(kTileThreads) k_amr_cell_tile(ApplyArgs a, flo
     return;
   }
   const float* mm = s_m + lc * AMPS_CELLM + 3 * p;  // row p of every monomial block
-  if (ACC == 0) {
-    const float dx = K.dx, V = K.V;
-    float ef[8][3], out[8];
+  const float sg = ACC == 2 ? -1.f : 1.f;
+  FF out[8];
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      out[c] = 0.f;
+  for (int c = 0; c < 8; c++)
+    out[c] = ACC == 1 ? ff_mul(s_eh[lc][3 * c + p], s_el[lc][3 * c + p], K.id[0], K.id[1]) : FF{0.f, 0.f};
+  // the curl's component p: cu_p = 0.25/dx (sum +-E_qa - sum +-E_qb)
+  const int qa = p == 0 ? 2 : (p == 1 ? 0 : 1), qb = p == 0 ? 1 : (p == 1 ? 2 : 0);
+  {
+    FF d{0.f, 0.f};
 #pragma unroll
-      for (int d = 0; d < 3; d++) ef[c][d] = s_eh[lc][3 * c + d];
+    for (int k2 = 0; k2 < 8; k2++) {
+      const bool px = k2 == 1 || k2 == 2 || k2 == 5 || k2 == 6;
+      const bool py = k2 == 2 || k2 == 3 || k2 == 6 || k2 == 7;
+      const bool pz = k2 >= 4;
+      // cu0 = (dEz/dy - dEy/dz), cu1 = (dEx/dz - dEz/dx), cu2 = (dEy/dx - dEx/dy)
+      const bool sga = p == 0 ? py : (p == 1 ? pz : px);
+      const bool sgb = p == 0 ? pz : (p == 1 ? px : py);
+      const float ha = s_eh[lc][3 * k2 + qa], la = s_el[lc][3 * k2 + qa];
+      const float hb = s_eh[lc][3 * k2 + qb], lb = s_el[lc][3 * k2 + qb];
+      ff_acc(d, sga ? ha : -ha, sga ? la : -la);
+      ff_acc(d, sgb ? -hb : hb, sgb ? -lb : lb);
     }
-    float cu[3];
-    cell_curl<float>(ef, 0.25f / dx, cu);
-    cell_curl_t_row<float>(cu, (float)a.th2dt2 * V * 0.25f / dx, p, out);
-    const float fv = (float)a.f * V;
+    d = ff_norm(d);
+    const FF cu = ff_norm(ff_mul(d.s, d.q, K.curl[0], K.curl[1]));
+    s_cu[lc][p][0] = cu.s;
+    s_cu[lc][p][1] = cu.q;
+  }
+  __syncthreads();
+  // out[k] += s (sig1 y[q1] - sig2 y[q2]) for y = the curl (s = sg th2dt2 V 0.25/dx)
+  // and, for the RHS, y = centre B (s = thdt V 0.25/dx): C^T y, component p
+  const int q1 = p == 0 ? 1 : (p == 1 ? 2 : 0), q2 = p == 0 ? 2 : (p == 1 ? 0 : 1);
+  auto curl_t = [&](float (*y)[2], float sh, float sl) {
+    FF tpp{y[q1][0], y[q1][1]}, tpm{y[q1][0], y[q1][1]};
+    ff_acc(tpp, -y[q2][0], -y[q2][1]);  // y1 - y2
+    ff_acc(tpm, y[q2][0], y[q2][1]);    // y1 + y2
+    tpp = ff_norm(tpp);
+    tpm = ff_norm(tpm);
+    const FF upp = ff_mul(tpp.s, tpp.q, sh, sl), upm = ff_mul(tpm.s, tpm.q, sh, sl);
 #pragma unroll
-    for (int c1 = 0; c1 < 8; c1++)
-#pragma unroll
-      for (int c2 = 0; c2 <= c1; c2++) {
-        const float* m3 = mm + pair_monomial(c1, c2) * 9;
-        const float m0 = fv * m3[0], m1 = fv * m3[1], m2 = fv * m3[2];
-        out[c1] += m0 * ef[c2][0] + m1 * ef[c2][1] + m2 * ef[c2][2];
-        if (c1 != c2) out[c2] += m0 * ef[c1][0] + m1 * ef[c1][1] + m2 * ef[c1][2];
-      }
-#pragma unroll
-    for (int c = 0; c < 8; c++) atomicAdd(&s_acc[3 * tcorner(c) + p], out[c]);
-    __syncthreads();
-    // one global atomic per tile corner and component (P^T for hanging corners)
-    for (int q = tid; q < 3 * kTC; q += kTileThreads) {
-      const int tc = q / 3, pp = q % 3, cc = s_tcid[tc];
-      const float v = s_acc[q];
-      const int hs0 = a.h.hs[cc], hs1 = a.h.hs[cc + 1];
-      if (hs0 == hs1) {
-        atomicAdd(y32 + pp * a.nvc + cc, v);
-      } else {
-        for (int t = hs0; t < hs1; t++) atomicAdd(y32 + pp * a.nvc + a.h.hp[t], a.h.hwh[t] * v);
-      }
+    for (int k2 = 0; k2 < 8; k2++) {
+      const bool px = k2 == 1 || k2 == 2 || k2 == 5 || k2 == 6;
+      const bool py = k2 == 2 || k2 == 3 || k2 == 6 || k2 == 7;
+      const bool pz = k2 >= 4;
+      const bool s1 = p == 0 ? pz : (p == 1 ? px : py);
+      const bool s2 = p == 0 ? py : (p == 1 ? pz : px);
+      // s1 y1 - s2 y2: (+,+) y1 - y2, (+,-) y1 + y2, (-,+) -(y1 + y2), (-,-) -(y1 - y2)
+      const FF& u = (s1 == s2) ? upp : upm;
+      const float sgn = s1 ? 1.f : -1.f;
+      ff_acc(out[k2], sgn * u.s, sgn * u.q);
     }
-  } else {
-    const float sg = ACC == 2 ? -1.f : 1.f;
-    FF out[8];
+  };
+  curl_t(s_cu[lc], sg * K.cc[0], sg * K.cc[1]);
+  // mass term: sum over pairs of m (FP32 partial) x e, in FP32 pairs
+  float eh[8][3], el[8][3];
+  FF acc[8];
 #pragma unroll
-    for (int c = 0; c < 8; c++)
-      out[c] = ACC == 1 ? ff_mul(s_eh[lc][3 * c + p], s_el[lc][3 * c + p], K.id[0], K.id[1]) : FF{0.f, 0.f};
-    // the curl's component p: cu_p = 0.25/dx (sum +-E_qa - sum +-E_qb)
-    const int qa = p == 0 ? 2 : (p == 1 ? 0 : 1), qb = p == 0 ? 1 : (p == 1 ? 2 : 0);
-    {
-      FF d{0.f, 0.f};
+  for (int c = 0; c < 8; c++) {
+    acc[c] = FF{0.f, 0.f};
 #pragma unroll
-      for (int k2 = 0; k2 < 8; k2++) {
-        const bool px = k2 == 1 || k2 == 2 || k2 == 5 || k2 == 6;
-        const bool py = k2 == 2 || k2 == 3 || k2 == 6 || k2 == 7;
-        const bool pz = k2 >= 4;
-        // cu0 = (dEz/dy - dEy/dz), cu1 = (dEx/dz - dEz/dx), cu2 = (dEy/dx - dEx/dy)
-        const bool sga = p == 0 ? py : (p == 1 ? pz : px);
-        const bool sgb = p == 0 ? pz : (p == 1 ? px : py);
-        const float ha = s_eh[lc][3 * k2 + qa], la = s_el[lc][3 * k2 + qa];
-        const float hb = s_eh[lc][3 * k2 + qb], lb = s_el[lc][3 * k2 + qb];
-        ff_acc(d, sga ? ha : -ha, sga ? la : -la);
-        ff_acc(d, sgb ? -hb : hb, sgb ? -lb : lb);
-      }
-      d = ff_norm(d);
-      const FF cu = ff_norm(ff_mul(d.s, d.q, K.curl[0], K.curl[1]));
-      s_cu[lc][p][0] = cu.s;
-      s_cu[lc][p][1] = cu.q;
+    for (int d = 0; d < 3; d++) {
+      eh[c][d] = s_eh[lc][3 * c + d];
+      el[c][d] = s_el[lc][3 * c + d];
     }
-    __syncthreads();
-    // out[k] += s (sig1 y[q1] - sig2 y[q2]) for y = the curl (s = sg th2dt2 V 0.25/dx)
-    // and, for the RHS, y = centre B (s = thdt V 0.25/dx): C^T y, component p
-    const int q1 = p == 0 ? 1 : (p == 1 ? 2 : 0), q2 = p == 0 ? 2 : (p == 1 ? 0 : 1);
-    auto curl_t = [&](float (*y)[2], float sh, float sl) {
-      FF tpp{y[q1][0], y[q1][1]}, tpm{y[q1][0], y[q1][1]};
-      ff_acc(tpp, -y[q2][0], -y[q2][1]);  // y1 - y2
-      ff_acc(tpm, y[q2][0], y[q2][1]);    // y1 + y2
-      tpp = ff_norm(tpp);
-      tpm = ff_norm(tpm);
-      const FF upp = ff_mul(tpp.s, tpp.q, sh, sl), upm = ff_mul(tpm.s, tpm.q, sh, sl);
+  }
 #pragma unroll
-      for (int k2 = 0; k2 < 8; k2++) {
-        const bool px = k2 == 1 || k2 == 2 || k2 == 5 || k2 == 6;
-        const bool py = k2 == 2 || k2 == 3 || k2 == 6 || k2 == 7;
-        const bool pz = k2 >= 4;
-        const bool s1 = p == 0 ? pz : (p == 1 ? px : py);
-        const bool s2 = p == 0 ? py : (p == 1 ? pz : px);
-        // s1 y1 - s2 y2: (+,+) y1 - y2, (+,-) y1 + y2, (-,+) -(y1 + y2), (-,-) -(y1 - y2)
-        const FF& u = (s1 == s2) ? upp : upm;
-        const float sgn = s1 ? 1.f : -1.f;
-        ff_acc(out[k2], sgn * u.s, sgn * u.q);
-      }
-    };
-    curl_t(s_cu[lc], sg * K.cc[0], sg * K.cc[1]);
-    // mass term: sum over pairs of m (FP32 partial) x e, in FP32 pairs
-    float eh[8][3], el[8][3];
-    FF acc[8];
+  for (int c1 = 0; c1 < 8; c1++)
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      acc[c] = FF{0.f, 0.f};
+    for (int c2 = 0; c2 <= c1; c2++) {
+      const float* m3 = mm + pair_monomial(c1, c2) * 9;
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        eh[c][d] = s_eh[lc][3 * c + d];
-        el[c][d] = s_el[lc][3 * c + d];
+      for (int q = 0; q < 3; q++) {
+        const float m = m3[q];
+        ff_add(acc[c1], m, eh[c2][q], el[c2][q]);
+        if (c1 != c2) ff_add(acc[c2], m, eh[c1][q], el[c1][q]);
       }
     }
 #pragma unroll
-    for (int c1 = 0; c1 < 8; c1++)
+  for (int c = 0; c < 8; c++) {
+    const FF t = ff_norm(acc[c]);
+    const FF u = ff_mul(t.s, t.q, sg * K.m[0], sg * K.m[1]);
+    ff_acc(out[c], u.s, u.q);
+  }
+  if (ACC == 2) {
+    curl_t(s_b[lc], K.bb[0], K.bb[1]);
+    const float* jj = a.cellJ + cell * 24;
 #pragma unroll
-      for (int c2 = 0; c2 <= c1; c2++) {
-        const float* m3 = mm + pair_monomial(c1, c2) * 9;
+    for (int c = 0; c < 8; c++) ff_add2(out[c], -a.fj[0], -a.fj[1], jj[3 * c + p], 0.f);
+  }
+  // sum over the tile's cells per corner, in pairs (round c: corner c of every cell)
 #pragma unroll
-        for (int q = 0; q < 3; q++) {
-          const float m = m3[q];
-          ff_add(acc[c1], m, eh[c2][q], el[c2][q]);
-          if (c1 != c2) ff_add(acc[c2], m, eh[c1][q], el[c1][q]);
-        }
-      }
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const FF t = ff_norm(acc[c]);
-      const FF u = ff_mul(t.s, t.q, sg * K.m[0], sg * K.m[1]);
-      ff_acc(out[c], u.s, u.q);
-    }
-    if (ACC == 2) {
-      curl_t(s_b[lc], K.bb[0], K.bb[1]);
-      const float* jj = a.cellJ + cell * 24;
-#pragma unroll
-      for (int c = 0; c < 8; c++) ff_add2(out[c], -a.fj[0], -a.fj[1], jj[3 * c + p], 0.f);
-    }
-    // sum over the tile's cells per corner, in pairs (round c: corner c of every cell)
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      float* slot = s_ffacc[p][tcorner(c)];
-      FF v{slot[0], slot[1]};
-      ff_acc(v, out[c].s, out[c].q);
-      slot[0] = v.s;
-      slot[1] = v.q;
-      __syncwarp();
-    }
-    __syncthreads();
-    // scatter with P^T: one FP64 atomic per tile corner and component
-    for (int q = tid; q < 3 * kTC; q += kTileThreads) {
-      const int pp = q / kTC, tc = q % kTC, cc = s_tcid[tc];
-      const FF o = ff_norm(FF{s_ffacc[pp][tc][0], s_ffacc[pp][tc][1]});
-      const int hs0 = a.h.hs[cc], hs1 = a.h.hs[cc + 1];
-      if (hs0 == hs1) {
-        atomicAdd(y64 + pp * a.nvc + cc, ff_value(o));
-      } else {
-        for (int t = hs0; t < hs1; t++)
-          atomicAdd(y64 + pp * a.nvc + a.h.hp[t], ff_value(ff_mul(o.s, o.q, a.h.hwh[t], a.h.hwl[t])));
-      }
+  for (int c = 0; c < 8; c++) {
+    float* slot = s_ffacc[p][tcorner(c)];
+    FF v{slot[0], slot[1]};
+    ff_acc(v, out[c].s, out[c].q);
+    slot[0] = v.s;
+    slot[1] = v.q;
+    __syncwarp();
+  }
+  __syncthreads();
+  // scatter with P^T: one FP64 atomic per tile corner and component
+  for (int q = tid; q < 3 * kTC; q += kTileThreads) {
+    const int pp = q / kTC, tc = q % kTC, cc = s_tcid[tc];
+    const FF o = ff_norm(FF{s_ffacc[pp][tc][0], s_ffacc[pp][tc][1]});
+    const int hs0 = a.h.hs[cc], hs1 = a.h.hs[cc + 1];
+    if (hs0 == hs1) {
+      atomicAdd(y64 + pp * a.nvc + cc, ff_value(o));
+    } else {
+      for (int t = hs0; t < hs1; t++)
+        atomicAdd(y64 + pp * a.nvc + a.h.hp[t], ff_value(ff_mul(o.s, o.q, a.h.hwh[t], a.h.hwl[t])));
     }
   }
 }
@@ -468,17 +546,37 @@ __global__ void __launch_bounds__(256) k_amr_to_f32(long long n, const double* _
     xf[t] = (float)(dinv ? dinv[t] * x[t] : x[t]);
 }
 
-// The same with the input and output as FP32 pairs (Krylov vectors): free
-// rows S (D v) + y32 in pairs, hanging rows (D v)_h - (P D v)_h.
+// w = A (D v) from y32 as FP32 pairs (Krylov vectors): free rows S (D v) + y32
+// in pairs, hanging rows (D v)_h - (P D v)_h; y32 cleared for the next
+// application.  Almost every row of S is its diagonal alone: diag holds it as a
+// pair (0: any other row), so the common row's loads depend on nothing (500,832
+// corners: XX us; through the CSR rows 20 us, plus 4 for clearing y32 before the
+// operator).
 __global__ void __launch_bounds__(256) k_amr_finish_ff(long long nvc, Hang h,
                                                        const int* __restrict__ ss,
                                                        const int* __restrict__ sc,
                                                        const float* __restrict__ svh,
                                                        const float* __restrict__ svl,
-                                                       const float* __restrict__ y32, OpIn in,
+                                                       const float2* __restrict__ diag,
+                                                       float* __restrict__ y32, OpIn in,
                                                        float* __restrict__ wh, float* __restrict__ wl) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nvc) return;
+  const float2 dg = diag[c];
+  if (dg.x != 0.f) {
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const long long t = d * nvc + c;
+      FF acc{y32[t], 0.f};
+      const FF v = opin_value(in, t);
+      ff_add2(acc, dg.x, dg.y, v.s, v.q);
+      acc = ff_norm(acc);
+      wh[t] = acc.s;
+      wl[t] = acc.q;
+      y32[t] = 0.f;
+    }
+    return;
+  }
   int s = h.hs[c], e = h.hs[c + 1];
   const int* col = h.hp;
   const float* cwh = h.hwh;
@@ -511,6 +609,7 @@ __global__ void __launch_bounds__(256) k_amr_finish_ff(long long nvc, Hang h,
     acc = ff_norm(acc);
     wh[d * nvc + c] = acc.s;
     wl[d * nvc + c] = acc.q;
+    y32[d * nvc + c] = 0.f;
   }
 }
 
@@ -521,7 +620,7 @@ __global__ void __launch_bounds__(256) k_amr_finish32(long long nvc, Hang h,
                                                       const int* __restrict__ ss,
                                                       const int* __restrict__ sc,
                                                       const double* __restrict__ sv,
-                                                      const float* __restrict__ y32,
+                                                      float* __restrict__ y32,
                                                       const double* __restrict__ x,
                                                       const double* __restrict__ dinv,
                                                       double* __restrict__ y) {
@@ -555,6 +654,7 @@ __global__ void __launch_bounds__(256) k_amr_finish32(long long nvc, Hang h,
       }
       y[d * nvc + c] = (dinv ? dinv[d * nvc + c] : 1.0) * x[d * nvc + c] - pv;
     }
+    y32[d * nvc + c] = 0.f;
   }
 }
 
@@ -834,6 +934,7 @@ static ApplyArgs apply_args(amps_gpu_ctx* c) {
   a.ncell = c->ncor;
   a.nvc = c->nvc;
   a.ctab = c->d_ctab;
+  a.ctabh = c->d_ctabh;
   a.h = hang_of(c);
   a.bdx = c->d_bdx;
   a.cellM = c->d_cellM;
@@ -851,8 +952,6 @@ static ApplyArgs apply_args(amps_gpu_ctx* c) {
   for (int sc = 0; sc < kMaxScale; sc++) {
     const double dx = c->dxf * (double)(1 << sc), V = dx * dx * dx;
     LevelK& K = a.lk[sc];
-    K.dx = (float)dx;
-    K.V = (float)V;
     split(0.25 / dx, K.curl);
     split(a.th2dt2 * V * 0.25 / dx, K.cc);
     split(0.125 * V, K.id);
@@ -878,7 +977,7 @@ static cudaError_t split_input(amps_gpu_ctx* c, const double* x, const double* d
 }
 
 template <int ACC>
-static cudaError_t launch_tile(amps_gpu_ctx* c, const ApplyArgs& a, float* y32, double* y64) {
+static cudaError_t launch_tile(amps_gpu_ctx* c, const ApplyArgs& a, double* y64) {
   static unsigned long long attr_set = 0;  // per device
   int dev = 0;
   cudaGetDevice(&dev);
@@ -889,8 +988,28 @@ static cudaError_t launch_tile(amps_gpu_ctx* c, const ApplyArgs& a, float* y32, 
     attr_set |= 1ull << dev;
   }
   // AMR meshes hold whole 512-cell blocks: ncell is a multiple of the tile
-  k_amr_cell_tile<ACC><<<(unsigned)(c->ncor / kTileCells), kTileThreads, kTileBytes, c->stream>>>(a, y32,
-                                                                                                 y64);
+  k_amr_cell_tile<ACC><<<(unsigned)(c->ncor / kTileCells), kTileThreads, kTileBytes, c->stream>>>(a, y64);
+  return cudaGetLastError();
+}
+
+// y32 += the FP32 operator on a.xf
+static cudaError_t launch_tile32(amps_gpu_ctx* c, const ApplyArgs& a, float* y32) {
+  static int grid[64] = {0};  // per device: resident CTAs
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (grid[dev] == 0) {
+    int sms = 0, per = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_amr_tile32, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)kTileBytes);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_amr_tile32, kTileThreads, 2 * kTileBytes);
+    if (e != cudaSuccess) return e;
+    grid[dev] = sms * std::max(per, 1);
+  }
+  const int tiles = (int)(c->ncor / kTileCells);
+  k_amr_tile32<<<std::min(grid[dev], tiles), kTileThreads, 2 * kTileBytes, c->stream>>>(a, tiles, y32);
   return cudaGetLastError();
 }
 
@@ -902,15 +1021,15 @@ cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* di
   a.dinv = dinv;
   TimedLaunch t(c, "matvec", 3);
   if ((e = split_input(c, x, dinv, a)) != cudaSuccess) return e;
-  if ((e = launch_tile<1>(c, a, nullptr, y)) != cudaSuccess) return e;
+  if ((e = launch_tile<1>(c, a, y)) != cudaSuccess) return e;
   k_amr_constraint<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, x, dinv, y, 0);
   return cudaGetLastError();
 }
 
+// (d_y32 is zero between applications: the finish kernels clear what they read)
 cudaError_t launch_amr_matvec32(amps_gpu_ctx* c, const double* x, const double* dinv,
                                 double* y) {
-  cudaError_t e = cudaMemsetAsync(c->d_y32, 0, sizeof(float) * 3 * c->nvc, c->stream);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   ApplyArgs a = apply_args(c);
   a.x = x;
   a.dinv = dinv;
@@ -922,15 +1041,14 @@ cudaError_t launch_amr_matvec32(amps_gpu_ctx* c, const double* x, const double* 
   TimedLaunch t(c, "matvec32", 3);
   k_amr_to_f32<<<(unsigned)std::min<long long>((n + 255) / 256, 152LL * 16), 256, 0, c->stream>>>(n, x, dinv,
                                                                                                  c->d_xs);
-  if ((e = launch_tile<0>(c, a, c->d_y32, nullptr)) != cudaSuccess) return e;
+  if ((e = launch_tile32(c, a, c->d_y32)) != cudaSuccess) return e;
   k_amr_finish32<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, c->d_ss, c->d_sc, c->d_sv,
                                                      c->d_y32, x, dinv, y);
   return cudaGetLastError();
 }
 
 cudaError_t launch_amr_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, float* wl) {
-  cudaError_t e = cudaMemsetAsync(c->d_y32, 0, sizeof(float) * 3 * c->nvc, c->stream);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   ApplyArgs a = apply_args(c);
   const long long n = 3 * c->nvc;
   if (!c->d_xs && (e = cudaMalloc(reinterpret_cast<void**>(&c->d_xs), sizeof(float) * 2 * n)) != cudaSuccess)
@@ -938,9 +1056,9 @@ cudaError_t launch_amr_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, f
   a.xf = c->d_xs;
   TimedLaunch t(c, "matvec32", in.xf_ready ? 2 : 3);
   if (!in.xf_ready && (e = launch_in_f32(c, in, c->d_xs)) != cudaSuccess) return e;
-  if ((e = launch_tile<0>(c, a, c->d_y32, nullptr)) != cudaSuccess) return e;
+  if ((e = launch_tile32(c, a, c->d_y32)) != cudaSuccess) return e;
   k_amr_finish_ff<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, c->d_ss, c->d_sc, c->d_svh, c->d_svl,
-                                                      c->d_y32, in, wh, wl);
+                                                      c->d_sdiag, c->d_y32, in, wh, wl);
   return cudaGetLastError();
 }
 
@@ -953,7 +1071,7 @@ cudaError_t launch_amr_rhs(amps_gpu_ctx* c) {
   a.Bcen = c->d_Bc;
   TimedLaunch t(c, "rhs", 3);
   if ((e = split_input(c, c->d_En, nullptr, a)) != cudaSuccess) return e;
-  if ((e = launch_tile<2>(c, a, nullptr, c->d_rhs)) != cudaSuccess) return e;
+  if ((e = launch_tile<2>(c, a, c->d_rhs)) != cudaSuccess) return e;
   k_amr_constraint<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, nullptr, nullptr, c->d_rhs, 1);
   return cudaGetLastError();
 }

@@ -317,7 +317,9 @@ bool alloc_context(amps_gpu_ctx* c) {
        !dalloc(&c->d_Bc2, 3 * nc) && !dalloc(&c->d_Bcor_prev, 3 * nv) &&
        !dalloc(&c->d_Bcor_cur, 3 * nv);
   if (!c->amr) ok = ok && !dalloc(&c->d_J, 3 * nc) && !dalloc(&c->d_M, 243 * nc);
-  if (c->amr) ok = ok && !dalloc(&c->d_y32, 3 * nv);
+  if (c->amr)
+    ok = ok && !dalloc(&c->d_y32, 3 * nv) &&
+         cudaMemsetAsync(c->d_y32, 0, sizeof(float) * 3 * nv, c->stream) == cudaSuccess;
   ok = ok && !dalloc(&c->d_rhs, 3 * nv) && !dalloc(&c->d_x, 3 * nv) &&
        !dalloc(&c->d_V, (size_t)(c->restart + 1) * ((3 * nv + 3) & ~3LL)) &&
        !dalloc(&c->d_w, (3 * nv + 3) & ~3LL) &&
@@ -648,8 +650,19 @@ amps_gpu_status amps_gpu_create_amr(const amps_gpu_config* cfg, const amps_amr_m
       svh[q] = (float)sv[q];
       svl[q] = (float)(sv[q] - (double)svh[q]);
     }
+    // rows that are their diagonal alone; boundary rows are constraints too
+    std::vector<float2> sdiag((size_t)nv, make_float2(0.f, 0.f));
+    for (long long r = 0; r < nv; r++) {
+      const int q = ss[(size_t)r];
+      if (ss[(size_t)r + 1] - q == 1 && sc[(size_t)q] == (int)r && (m->bnd_flag.empty() || !m->bnd_flag[(size_t)r]))
+        sdiag[(size_t)r] = make_float2(svh[(size_t)q], svl[(size_t)q]);
+    }
+    std::vector<int> ctabh(m->corner_tab.begin(), m->corner_tab.end());
+    for (int& q : ctabh)
+      if (hs[(size_t)q + 1] > hs[(size_t)q]) q = ~q;
     ok = ok && upload(&c->d_ss, ss) && upload(&c->d_sc, sc) && upload(&c->d_sv, sv) &&
-         upload(&c->d_svh, svh) && upload(&c->d_svl, svl);
+         upload(&c->d_svh, svh) && upload(&c->d_svl, svl) && upload(&c->d_sdiag, sdiag) &&
+         upload(&c->d_ctabh, ctabh);
   }
   if (!ok) {
     cudaGetLastError();
@@ -720,7 +733,7 @@ amps_gpu_status amps_gpu_destroy(amps_gpu_ctx* c) {
                   c->d_cellM, c->d_cellJ, c->d_energy, c->d_ctab, c->d_hs, c->d_hp, c->d_hw, c->d_hwh, c->d_hwl,
                   c->d_bflag, c->d_bs, c->d_bc, c->d_bw, c->d_bwh, c->d_bwl,
                   c->d_fine_map, c->d_borg, c->d_bscale, c->d_bdx, c->d_bdtdx, c->d_binvvol,
-                  c->d_ss, c->d_sc, c->d_sv, c->d_svh, c->d_svl, c->d_dff, c->d_tmpv, c->d_pc_in, c->d_pc_out_v[0], c->d_pc_out_v[1],
+                  c->d_ss, c->d_sc, c->d_sv, c->d_svh, c->d_svl, c->d_sdiag, c->d_ctabh, c->d_dff, c->d_tmpv, c->d_pc_in, c->d_pc_out_v[0], c->d_pc_out_v[1],
                   c->d_pc_set, c->d_pc_jac_v[0], c->d_pc_jac_v[1]};
   for (void* p : ptrs) cudaFree(p);
   for (int b = 0; b < 2; b++) {

@@ -69,6 +69,7 @@ struct amps_gpu_ctx {
   int lmax = 0;
   double dxf = 0.0;         // finest cell size (AMR)
   int* d_ctab = nullptr;    // [nb*729] block-local corner -> unique corner (AMR)
+  int* d_ctabh = nullptr;   // the same with hanging corners as ~id (field operator)
   int* d_hs = nullptr;      // [nvc+1] hanging CSR start (AMR)
   int* d_hp = nullptr;      // hanging parents
   double* d_hw = nullptr;   // hanging weights
@@ -94,6 +95,7 @@ struct amps_gpu_ctx {
   double* d_sv = nullptr;     //   values
   float* d_svh = nullptr;     //   values as FP32 pairs
   float* d_svl = nullptr;
+  float2* d_sdiag = nullptr;  //   the diagonal of rows that are nothing else, as pairs (0: others)
 
   // fields (FP64, component-major)
   double* d_En = nullptr;
@@ -116,7 +118,8 @@ struct amps_gpu_ctx {
   float* d_dff = nullptr;       // 2n: the Jacobi scaling as FP32 pairs (hi n, lo n)
   double* d_tmpv = nullptr;     // 2n doubles: FP64 copies of Krylov vectors for the
                                 // learned network, its sample harvest and the FP64 inner operator
-  float* d_y32 = nullptr;       // 3*nvc FP32 accumulation of the inner AMR operator
+  float* d_y32 = nullptr;       // 3*nvc FP32 accumulation of the inner AMR operator (zero between
+                                // applications)
   bool inner_fp32 = true;       // GMRES inner operator in FP32 (iterative refinement)
   PrecondState* pn = nullptr;   // learned preconditioner (precond.cu)
   // the network's view of the mesh: per block the 10^3 corner region (block

@@ -211,7 +211,7 @@ constexpr int kTC = 90;  // tile corners, (i, j, k) at i + 9 (j + 5 k)
 // ~id, so the common corner needs no look at the constraint rows.  The cells'
 // contributions to a corner are added by shuffles along x and y, and go out as
 // one global reduction per tile corner and component (P^T for hanging ones).
-// 491,520 cells: XX us, before 132.
+// 491,520 cells: 94 us (5.1 TB/s), before 132.
 __global__ void __launch_bounds__(kTileThreads) k_amr_tile32(ApplyArgs a, int tiles, float* __restrict__ y32) {
   extern __shared__ __align__(16) float s_m[];  // two tiles of partials
   __shared__ __align__(8) uint64_t bar[2];
@@ -548,11 +548,17 @@ __global__ void __launch_bounds__(256) k_amr_to_f32(long long n, const double* _
 
 // w = A (D v) from y32 as FP32 pairs (Krylov vectors): free rows S (D v) + y32
 // in pairs, hanging rows (D v)_h - (P D v)_h; y32 cleared for the next
-// application.  Almost every row of S is its diagonal alone: diag holds it as a
-// pair (0: any other row), so the common row's loads depend on nothing (500,832
-// corners: XX us; through the CSR rows 20 us, plus 4 for clearing y32 before the
-// operator).
-__global__ void __launch_bounds__(256) k_amr_finish_ff(long long nvc, Hang h,
+// application.  Almost every row of S is its diagonal alone (diag, a pair; 0: any
+// other row): a thread takes two corners, whose loads depend on nothing (a CTA's
+// life is one memory latency: more loads per thread, fewer CTAs).
+// The other rows are listed; the CTAs past the first `plain` take them, 8 lanes
+// per row over its entries: one thread walking a row of up to 27 entries, two
+// dependent loads each, set the time of the whole kernel
+// (500,832 corners: 14 us, before 21; clearing y32 before the operator took 4 more).
+constexpr int kRowLanes = 8;
+constexpr int kFinPer = 2;
+__global__ void __launch_bounds__(256) k_amr_finish_ff(long long nvc, Hang h, unsigned plain,
+                                                       int nrows, const int* __restrict__ rows,
                                                        const int* __restrict__ ss,
                                                        const int* __restrict__ sc,
                                                        const float* __restrict__ svh,
@@ -560,56 +566,95 @@ __global__ void __launch_bounds__(256) k_amr_finish_ff(long long nvc, Hang h,
                                                        const float2* __restrict__ diag,
                                                        float* __restrict__ y32, OpIn in,
                                                        float* __restrict__ wh, float* __restrict__ wl) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nvc) return;
-  const float2 dg = diag[c];
-  if (dg.x != 0.f) {
+  if (blockIdx.x < plain) {
+    // kFinPer corners per thread, all their loads in flight together
+    const long long c0 = (long long)blockIdx.x * (256 * kFinPer) + threadIdx.x;
+    float2 dg[kFinPer];
+    float y[kFinPer][3];
+    FF v[kFinPer][3];
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-      const long long t = d * nvc + c;
-      FF acc{y32[t], 0.f};
-      const FF v = opin_value(in, t);
-      ff_add2(acc, dg.x, dg.y, v.s, v.q);
-      acc = ff_norm(acc);
-      wh[t] = acc.s;
-      wl[t] = acc.q;
-      y32[t] = 0.f;
+    for (int k = 0; k < kFinPer; k++) {
+      const long long c = min(c0 + 256 * k, nvc - 1);
+      dg[k] = diag[c];
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        y[k][d] = y32[d * nvc + c];
+        v[k][d] = opin_value(in, d * nvc + c);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kFinPer; k++) {
+      const long long c = c0 + 256 * k;
+      if (c >= nvc || dg[k].x == 0.f) continue;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        FF acc{y[k][d], 0.f};
+        ff_add2(acc, dg[k].x, dg[k].y, v[k][d].s, v[k][d].q);
+        acc = ff_norm(acc);
+        wh[d * nvc + c] = acc.s;
+        wl[d * nvc + c] = acc.q;
+        y32[d * nvc + c] = 0.f;
+      }
     }
     return;
   }
-  int s = h.hs[c], e = h.hs[c + 1];
+  const int r = (int)(blockIdx.x - plain) * (int)(blockDim.x / kRowLanes) + (int)(threadIdx.x / kRowLanes);
+  const int lane = threadIdx.x % kRowLanes;
+  const bool act = r < nrows;
+  const int c = act ? rows[r] : 0;
+  int s = 0, e = 0;
   const int* col = h.hp;
   const float* cwh = h.hwh;
   const float* cwl = h.hwl;
-  const bool bnd = s == e && is_bnd(h, c);
-  if (bnd) {
-    s = h.bs[c];
-    e = h.bs[c + 1];
-    col = h.bc;
-    cwh = h.bwh;
-    cwl = h.bwl;
+  float sign = -1.f;
+  bool con = true;
+  if (act) {
+    s = h.hs[c];
+    e = h.hs[c + 1];
+    if (s == e && is_bnd(h, c)) {  // boundary rows (donors)
+      s = h.bs[c];
+      e = h.bs[c + 1];
+      col = h.bc;
+      cwh = h.bwh;
+      cwl = h.bwl;
+    } else if (s == e) {  // free rows with other entries of S
+      con = false;
+      s = ss[c];
+      e = ss[c + 1];
+      col = sc;
+      cwh = svh;
+      cwl = svl;
+      sign = 1.f;
+    }
+  }
+  FF acc[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+  for (int t = s + lane; t < e; t += kRowLanes) {
+    const int q = col[t];
+    const float mh = sign * cwh[t], ml = sign * cwl[t];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const FF u = opin_value(in, d * nvc + q);
+      ff_add2(acc[d], mh, ml, u.s, u.q);
+    }
   }
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    FF acc;
-    if (s == e && !bnd) {
-      acc = FF{y32[d * nvc + c], 0.f};
-      for (int q = ss[c]; q < ss[c + 1]; q++) {
-        const FF v = opin_value(in, d * nvc + sc[q]);
-        ff_add2(acc, svh[q], svl[q], v.s, v.q);
-      }
-    } else {
-      // constraint rows: hanging (parents) or boundary (donors)
-      acc = opin_value(in, d * nvc + c);
-      for (int t = s; t < e; t++) {
-        const FF v = opin_value(in, d * nvc + col[t]);
-        ff_add2(acc, -cwh[t], -cwl[t], v.s, v.q);
-      }
+  for (int k = kRowLanes / 2; k > 0; k >>= 1)
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const float bs = __shfl_xor_sync(0xffffffffu, acc[d].s, k), bq = __shfl_xor_sync(0xffffffffu, acc[d].q, k);
+      ff_acc(acc[d], bs, bq);
     }
-    acc = ff_norm(acc);
-    wh[d * nvc + c] = acc.s;
-    wl[d * nvc + c] = acc.q;
-    y32[d * nvc + c] = 0.f;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    if (!act || lane != d) continue;
+    const long long o = d * nvc + c;
+    const FF v = opin_value(in, o);
+    FF w = acc[d];
+    ff_acc(w, con ? v.s : y32[o], con ? v.q : 0.f);
+    w = ff_norm(w);
+    wh[o] = w.s;
+    wl[o] = w.q;
+    y32[o] = 0.f;
   }
 }
 
@@ -1057,8 +1102,11 @@ cudaError_t launch_amr_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, f
   TimedLaunch t(c, "matvec32", in.xf_ready ? 2 : 3);
   if (!in.xf_ready && (e = launch_in_f32(c, in, c->d_xs)) != cudaSuccess) return e;
   if ((e = launch_tile32(c, a, c->d_y32)) != cudaSuccess) return e;
-  k_amr_finish_ff<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, c->d_ss, c->d_sc, c->d_svh, c->d_svl,
-                                                      c->d_sdiag, c->d_y32, in, wh, wl);
+  const unsigned plain = (unsigned)((c->nvc + 256 * kFinPer - 1) / (256 * kFinPer));
+  const int per = 256 / kRowLanes;
+  k_amr_finish_ff<<<plain + (unsigned)((c->nsrows + per - 1) / per), 256, 0, c->stream>>>(
+      c->nvc, a.h, plain, c->nsrows, c->d_srows, c->d_ss, c->d_sc, c->d_svh, c->d_svl, c->d_sdiag,
+      c->d_y32, in, wh, wl);
   return cudaGetLastError();
 }
 

@@ -96,6 +96,8 @@ struct amps_gpu_ctx {
   float* d_svh = nullptr;     //   values as FP32 pairs
   float* d_svl = nullptr;
   float2* d_sdiag = nullptr;  //   the diagonal of rows that are nothing else, as pairs (0: others)
+  int* d_srows = nullptr;     //   those other rows (constraints, or more than the diagonal)
+  int nsrows = 0;
 
   // fields (FP64, component-major)
   double* d_En = nullptr;

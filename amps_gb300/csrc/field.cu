@@ -18,7 +18,9 @@
 //   k_update_b  UpdateB (:5160-5711), k_c2n InterpolateB_C2N (:5715),
 //   k_update_e  UpdateE with the wave-energy sum (:5909-6001)
 #include <cooperative_groups.h>
+#include <cuda.h>
 #include <cuda_runtime.h>
+#include <cudaTypedefs.h>
 
 #include <algorithm>
 #include <cmath>
@@ -464,34 +466,43 @@ __device__ __forceinline__ FF ff_warp_sum(FF a) {
 // V + 2 i ld, lo ld behind it, ld = n rounded up to 4 so that every stream
 // starts on 16 bytes.
 //
-// Bound: reading the basis (n = 1.34M, 15 vectors: 161 MB a sweep).  One
-// persistent CTA per SM; a producer warp brings tiles of kArnT elements of
-// every stream into a ring of shared-memory stages by bulk copies (up to 200 KB
-// in flight per SM, which per-thread loads at 2 CTAs per SM did not reach), and
-// 16 consumer warps work on the staged tile:
-//   - update: thread pairs split an element's vectors (even / odd);
+// Bound: reading the basis (n = 1.34M, 15 vectors: 161 MB a sweep).  Two
+// persistent CTAs per SM (one computes while the other waits at a barrier); a
+// producer warp brings tiles of T elements of every stream into a ring of
+// shared-memory stages by tensor copies (all rows of a tile in one: a bulk copy
+// per row, 62 of 512 bytes at 30 vectors, kept the copy engine busy longer than
+// the bytes; up to 200 KB in flight per SM, which per-thread loads at 2 CTAs per
+// SM did not reach), and 8 consumer warps work on the staged tile:
+//   - update: a thread owns T / 256 elements (T = 128: two threads split an
+//     element's vectors, even and odd);
 //   - dots: a warp owns whole vectors (or an element range of one when there
 //     are fewer vectors than warps), so the register cost does not grow with
 //     nv and no sums cross warps inside the sweep.
 // The staged tile serves both halves of the second sweep (w' and then h2), the
-// third sweep needs V's hi halves only (h2 is of the order of the pair
-// arithmetic's own rounding, 2^-48 |w|; times a lo half, 2^-24 |V|, it is far
-// below the last bit of w''), and tiles are walked in alternating directions so
+// third sweep needs V's hi halves only and sums V h2 in FP32 (h2 is of the order
+// of the pair arithmetic's own rounding, 2^-48 |w|; relative errors of 2^-24 in
+// V h2 are far below the last bit of w''), and tiles are walked in alternating directions so
 // a sweep starts on what the last one left in L2: 2.5 basis reads per step.
 // ||w''||^2 = ||w'||^2 - ||h2||^2 (V orthonormal) spares a sweep and a grid
 // barrier; where the second projection took more than half of ||w'||^2 (w in
 // the span of V) it is summed instead, from a sweep with the full pairs.
-// A CTA whose tiles all fit its stages reads them once.  Mean step of a
-// 55-iteration solve with 1.34M unknowns (1 to 30 vectors): 150 us, where the
-// form with per-thread streams and accumulators in registers (four basis reads,
-// three barriers) took 304 us; 1.50M unknowns, 1 to 8 vectors: 71 against 81 us.
-constexpr int kArnT = 256;                  // elements per tile and element per thread
-constexpr int kArnCons = 512;               // consumer threads (16 warps)
+// A CTA whose tiles all fit its stages reads them once.  1.34M unknowns, mean
+// step of a 55-iteration solve (1 to 30 vectors): 103 us, 4 us per vector (the
+// rate of HBM) on ~45 us of barriers and start-up.  Before: 304 us with
+// per-thread streams, four basis reads and three barriers; 150 us with one CTA
+// per SM and a bulk copy per row.  1.50M unknowns, 1 to 8 vectors: 59 us, before
+// 81.
+constexpr int kArnCons = 256;               // consumer threads (8 warps)
 constexpr int kArnBlock = kArnCons + 32;    // + the producer warp
 constexpr int kArnWarps = kArnCons / 32;
 constexpr int kArnMaxStages = 16;
-constexpr size_t kArnRing = 200 * 1024;     // ring budget
+// shared memory of a CTA (two per SM): two tiles of w' and, where two threads
+// split an element's vectors, of the odd shares; the rest is the ring
+constexpr size_t kArnSmem = 108 * 1024;
+constexpr size_t arn_extra(int T) { return sizeof(float) * (T < kArnCons ? 8 : 4) * T; }
+constexpr size_t arn_ring(int T) { return kArnSmem - arn_extra(T); }
 constexpr int kArnDots = kMaxV;             // dots per sweep: nv, and ||w'||^2
+constexpr int kArnRounds = kArnDots / kArnWarps;  // vectors per warp at most
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -503,28 +514,40 @@ __device__ __forceinline__ void bar_consumers() {
 }
 __device__ __forceinline__ void bar_all() { asm volatile("bar.sync 2, %0;" ::"n"(kArnBlock) : "memory"); }
 
-template <int M>
-__global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
-    long long n, long long ld, const float* __restrict__ V, float* __restrict__ w, int nv,
+// Descriptors of the streams as 2D arrays of ld columns: the 2 nv rows of the
+// basis pairs, the nv rows of its hi halves, the 2 rows of w
+struct ArnMaps {
+  CUtensorMap v, h, w;
+};
+
+template <int T>
+__global__ void __launch_bounds__(kArnBlock, 2) k_arnoldi_tile(
+    const __grid_constant__ ArnMaps maps, long long n, long long ld, float* __restrict__ w, int nv,
     float* __restrict__ vnext, float2* __restrict__ part, GmState* gs, int jj, float* __restrict__ xf,
     const float* __restrict__ dh, int stages, unsigned long long* flags) {
   cg::grid_group grid = cg::this_grid();
-  extern __shared__ __align__(16) float s_ring[];
+  extern __shared__ __align__(128) float s_ring[];
   __shared__ __align__(8) uint64_t full[kArnMaxStages], empty[kArnMaxStages];
-  __shared__ float2 s_red[kArnWarps][2];
+  __shared__ float2 s_red[kArnWarps][kArnRounds];
   __shared__ double s_h1[kMaxV], s_h2[kMaxV], s_n2, s_inv;
   __shared__ float2 s_f[kArnDots];               // the coefficients of the running sweep as pairs
   __shared__ int s_slow;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int nblk = gridDim.x;
-  constexpr int T = kArnT * M;
+  constexpr int M = T >= kArnCons ? T / kArnCons : 1;  // chunks of a tile = elements per thread
+  constexpr int C = T / M;                             // elements per chunk (a copy's width)
+  constexpr int G = kArnCons / C;                      // threads per element
   const int tiles = (int)((n + T - 1) / T);
   const int nt = (tiles - (int)blockIdx.x + nblk - 1) / nblk;  // this CTA's tiles (grid <= tiles)
   const bool resident = nt <= stages;
-  constexpr int slot = 2 * T;                    // floats per staged vector (hi, lo)
-  const size_t stage_f = (size_t)(nv + 1) * slot;
-  float* s_w = s_ring + stages * stage_f;        // w' of the tile in work: hi, lo
-  float2* s_part = reinterpret_cast<float2*>(s_w + slot);  // odd vectors' share of the update
+  // a stage: M chunks of 2 nv + 2 rows of C floats (V_0 hi, lo, V_1 hi, .., w hi,
+  // lo; the third sweep: V_0 hi, V_1 hi, .., D in the first nv + 1 rows)
+  const int chunk_f = (2 * nv + 2) * C;
+  const size_t stage_f = (size_t)M * chunk_f;
+  // w' of two tiles (hi, lo): the next tile's is written while slow warps still
+  // read this one's; G = 2: the odd vectors' share of the update, likewise
+  float* s_w = s_ring + stages * stage_f;
+  float2* s_part = reinterpret_cast<float2*>(s_w + 4 * T);
   auto tile_of = [&](int k) { return (long long)blockIdx.x + (long long)k * nblk; };
   auto count_of = [&](int k) { return (int)min((long long)T, n - tile_of(k) * T); };
   if (tid == 0) {
@@ -537,27 +560,26 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
   __syncthreads();
 
   if (wid == kArnWarps) {
-    // ---- producer warp: tile k of the sweep as the ring's use number c
-    // (dlo: D's tile in the place of V_0's lo half, in the sweep that reads hi halves)
-    auto issue = [&](int c, int k, bool lo, const float* dlo) {
+    // ---- producer warp: tile k of the sweep as the ring's use number c; pairs of
+    // V, or its hi halves (and D)
+    auto issue = [&](int c, int k, bool pairs, const float* D) {
       const int s = c % stages;
       if (c >= stages && !mbar_wait_bounded(&empty[s], ((c / stages) - 1) & 1, kWaitLimit) && lane == 0)
         atomicAdd(flags + 2, 1ull);
-      const long long e0 = tile_of(k) * T;
-      const uint32_t bytes = (uint32_t)((count_of(k) + 3) & ~3) * 4u;
-      float* dst = s_ring + (size_t)s * stage_f;
-      if (lane == 0)
-        mbar_arrive_expect_tx(&full[s], bytes * (uint32_t)(lo ? 2 * nv + 2 : nv + 2 + (dlo ? 1 : 0)));
-      __syncwarp();
-      for (int q = lane; q < 2 * nv + 2; q += 32) {
-        const int i = q >> 1, half = q & 1;
-        const float* src = (i < nv ? V + 2 * (size_t)i * ld : w) + (half ? ld : 0);
-        if (half && !lo && i < nv) {
-          if (i > 0 || !dlo) continue;
-          src = dlo;
+      if (lane == 0) {
+        const long long e0 = tile_of(k) * T;
+        const int count = count_of(k);
+        const uint32_t dbytes = D ? (uint32_t)((count + 3) & ~3) * 4u : 0u;
+        mbar_arrive_expect_tx(&full[s], (uint32_t)(T * 4 * (pairs ? 2 * nv + 2 : nv + 2)) + dbytes);
+        for (int m = 0; m < M; m++) {
+          float* dst = s_ring + (size_t)s * stage_f + m * chunk_f;
+          tensor_copy_2d(dst, pairs ? &maps.v : &maps.h, (int)(e0 + m * C), 0, &full[s]);
+          tensor_copy_2d(dst + 2 * nv * C, &maps.w, (int)(e0 + m * C), 0, &full[s]);
+          const int dc = min(C, count - m * C);
+          if (D && dc > 0) bulk_copy_g2s(dst + nv * C, D + e0 + m * C, (uint32_t)((dc + 3) & ~3) * 4u, &full[s]);
         }
-        bulk_copy_g2s(dst + (size_t)i * slot + half * T, src + e0, bytes, &full[s]);
       }
+      __syncwarp();
     };
     for (int k = 0; k < nt; k++) issue(k, k, true, nullptr);
     const int pre = min(nt, stages);  // the second sweep's first tiles load across the barrier
@@ -591,31 +613,36 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
   };
   // dots of the staged w with nd vectors (number nv: w itself): warp -> vector
   // and, with fewer vectors than warps, element range
-  FF acc[2];
+  FF acc[kArnRounds];
   int dots_n = 0, dots_p = 1, dots_g = 1;
   auto dots_begin = [&](int nd) {
     dots_n = nd;
     dots_p = 1;
     while (dots_p < nd && dots_p < kArnWarps) dots_p *= 2;
     dots_g = kArnWarps / dots_p;  // element ranges per vector
-    acc[0] = acc[1] = FF{0.f, 0.f};
+#pragma unroll
+    for (int r = 0; r < kArnRounds; r++) acc[r] = FF{0.f, 0.f};
   };
-  auto dots = [&](const float* st, const float* wt, int count) {
+  // (w at wt, its chunks wstride apart)
+  auto dots = [&](const float* st, const float* wt, int wstride, int count) {
     const int g = wid / dots_p;
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
+    for (int r = 0; r < kArnRounds; r++) {
       const int i = wid % dots_p + kArnWarps * r;
       if (i >= dots_n) continue;
-      const float* v = i < nv ? st + (size_t)i * slot : wt;
-#pragma unroll 4
-      for (int e = g * 32 + lane; e < count; e += 32 * dots_g)
-        ff_dot_acc(acc[r], v[e], v[T + e], wt[e], wt[T + e]);
+      for (int m = 0; m < M; m++) {
+        const float* wm = wt + m * wstride;
+        const float* v = i < nv ? st + m * chunk_f + 2 * i * C : wm;
+        const int cm = min(C, count - m * C);
+#pragma unroll 2
+        for (int e = g * 32 + lane; e < cm; e += 32 * dots_g) ff_dot_acc(acc[r], v[e], v[C + e], wm[e], wm[C + e]);
+      }
     }
   };
   // block sums to part[i * nblk + blk]; all blocks' sums after the barrier
   auto dots_end = [&](float2* __restrict__ out) {
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
+    for (int r = 0; r < kArnRounds; r++) {
       const FF t = ff_norm(ff_warp_sum(acc[r]));
       if (lane == 0) s_red[wid][r] = make_float2(t.s, t.q);
     }
@@ -647,34 +674,46 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
     }
     bar_consumers();
   };
-  // sum_i V_i f_i of the staged tile at this thread's M elements, its share of
-  // the vectors (half 0 even, half 1 odd)
-  const int e0 = tid & (kArnT - 1), half = tid / kArnT;
-  auto share = [&](const float* st, bool lo, FF (&p)[M]) {
+  // sum_i V_i f_i of the staged tile at this thread's M elements (G = 2: its
+  // share of the vectors; half 1 leaves its own in s_part); pass: the tile's
+  // number in the sweep
+  const int e0 = tid & (C - 1), half = tid / C;
+  auto share = [&](const float* st, bool pairs, int pass, FF (&p)[M]) {
 #pragma unroll
     for (int m = 0; m < M; m++) p[m] = FF{0.f, 0.f};
-#pragma unroll(M >= 4 ? 2 : 4)
-    for (int i = half; i < nv; i += 2) {
-      const float* v = st + (size_t)i * slot + e0;
-      const float2 f = s_f[i];
+    if (pairs) {
+#pragma unroll 2
+      for (int i = half; i < nv; i += G) {
+        const float* v = st + 2 * i * C + e0;
+        const float2 f = s_f[i];
 #pragma unroll
-      for (int m = 0; m < M; m++) {
-        const FF u = ff_mul(v[kArnT * m], lo ? v[T + kArnT * m] : 0.f, f.x, f.y);
-        ff_acc(p[m], u.s, u.q);
+        for (int m = 0; m < M; m++) {
+          const FF u = ff_mul(v[m * chunk_f], v[m * chunk_f + C], f.x, f.y);
+          ff_acc(p[m], u.s, u.q);
+        }
+      }
+    } else {
+#pragma unroll 4
+      for (int i = half; i < nv; i += G) {
+        const float* v = st + i * C + e0;
+        const float f = s_f[i].x;
+#pragma unroll
+        for (int m = 0; m < M; m++) p[m].s = fmaf(v[m * chunk_f], f, p[m].s);
       }
     }
-    if (half) {
-#pragma unroll
-      for (int m = 0; m < M; m++) s_part[e0 + kArnT * m] = make_float2(p[m].s, p[m].q);
+    if (G == 2) {
+      if (half) s_part[(pass & 1) * T + e0] = make_float2(p[0].s, p[0].q);
+      bar_consumers();
     }
-    bar_consumers();
   };
-  // w - V f at element e (half 0; p: its own share)
-  auto minus = [&](const float* wt, int e, const FF& p) {
-    FF t{wt[e], wt[T + e]};
+  // w - V f at this thread's element of a chunk (half 0; p: its own share)
+  auto minus = [&](const float* wm, int pass, const FF& p) {
+    FF t{wm[e0], wm[C + e0]};
     ff_acc(t, -p.s, -p.q);
-    const float2 o = s_part[e];
-    ff_acc(t, -o.x, -o.y);
+    if (G == 2) {
+      const float2 o = s_part[(pass & 1) * T + e0];
+      ff_acc(t, -o.x, -o.y);
+    }
     return ff_norm(t);
   };
 
@@ -682,31 +721,32 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
   dots_begin(nv);
   for (int k = 0; k < nt; k++) {
     const float* st = acquire(k);
-    dots(st, st + (size_t)nv * slot, count_of(k));
+    dots(st, st + 2 * nv * C, chunk_f, count_of(k));
     if (!resident) release(k);
   }
   dots_end(part);
   grid.sync();
   grid_sums(part, nv, s_h1);
   // sweep 2: w' = w - V h1; h2 = V^T w', ||w'||^2.  w' stays out of the ring's
-  // w slot (the copies of later tiles write there) unless the tiles stay.
+  // w rows (the copies of later tiles write there) unless the tiles stay.
   float2* part2 = part + (size_t)kArnDots * nblk;
   dots_begin(nv + 1);
   for (int q = 0; q < nt; q++) {
     const int k = nt - 1 - q, c = resident ? k : nt + q;
     float* st = resident ? s_ring + (size_t)(k % stages) * stage_f : acquire(c);
-    float* wt = st + (size_t)nv * slot;
-    float* wn = resident ? wt : s_w;
+    float* wt = st + 2 * nv * C;
+    float* wn = resident ? wt : s_w + (q & 1) * 2 * T;
+    const int wstride = resident ? chunk_f : 2 * C;
     const int count = count_of(k);
     FF p[M];
-    share(st, true, p);
+    share(st, true, q, p);
     if (!half) {
 #pragma unroll
       for (int m = 0; m < M; m++) {
-        const int e = e0 + kArnT * m;
-        const FF t = minus(wt, e, p[m]);
-        wn[e] = t.s;
-        wn[T + e] = t.q;
+        const int e = e0 + C * m;
+        const FF t = minus(wt + m * chunk_f, q, p[m]);
+        wn[m * wstride + e0] = t.s;
+        wn[m * wstride + C + e0] = t.q;
         if (!resident && e < count) {
           const long long g = tile_of(k) * T + e;
           w[g] = t.s;
@@ -715,7 +755,7 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
       }
     }
     bar_consumers();
-    dots(st, wn, count);
+    dots(st, wn, wstride, count);
     if (!resident) release(c);
   }
   if (!resident) fence_proxy_async();  // the third sweep's copies read the w' written here
@@ -742,6 +782,8 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
     if (xf) xf[g] = u.s * d;
   };
   const bool scaled = xf && dh;
+  // resident tiles still hold V's pairs
+  const bool pairs3 = slow || resident;
   const float ih = (float)s_inv, il = (float)(s_inv - (double)ih);
   FF nacc{0.f, 0.f};
   for (int k = 0; k < nt; k++) {
@@ -750,17 +792,18 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
     float dv[M];
 #pragma unroll
     for (int m = 0; m < M; m++) {
-      const int e = e0 + kArnT * m;
+      const int e = e0 + C * m;
       dv[m] = 1.f;
-      if (!half && scaled && !slow && e < count) dv[m] = resident ? dh[tile_of(k) * T + e] : st[T + e];
+      if (!half && scaled && !slow && e < count)
+        dv[m] = resident ? dh[tile_of(k) * T + e] : st[m * chunk_f + nv * C + e0];
     }
     FF p[M];
-    share(st, slow, p);
+    share(st, pairs3, k, p);
     if (!half) {
 #pragma unroll
       for (int m = 0; m < M; m++) {
-        const int e = e0 + kArnT * m;
-        const FF t = minus(st + (size_t)nv * slot, e, p[m]);
+        const int e = e0 + C * m;
+        const FF t = minus(st + 2 * nv * C + m * chunk_f, k, p[m]);
         if (e < count) {
           const long long g = tile_of(k) * T + e;
           if (slow) {
@@ -774,7 +817,6 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
       }
     }
     if (!resident) release(c);
-    bar_consumers();  // s_part is rewritten
   }
   if (!slow) return;
   // w was (nearly) in the span of V: its remainder's norm from the sum itself
@@ -782,8 +824,8 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
   dots_n = 1;
   dots_p = 1;
   dots_g = kArnWarps;
-  acc[0] = nacc;
-  acc[1] = FF{0.f, 0.f};
+#pragma unroll
+  for (int r = 0; r < kArnRounds; r++) acc[r] = r == 0 ? nacc : FF{0.f, 0.f};
   dots_end(part3);
   grid.sync();
   if (wid == 0) {
@@ -803,7 +845,7 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
   const float jh = (float)s_inv, jl = (float)(s_inv - (double)jh);
   for (int k = 0; k < nt; k++)
     for (int m = 0; m < M; m++) {
-      const int e = e0 + kArnT * m;
+      const int e = e0 + C * m;
       const long long g = tile_of(k) * T + e;
       if (e < count_of(k)) put(g, FF{w[g], w[ld + g]}, jh, jl, scaled ? dh[g] : 1.f);
     }
@@ -812,41 +854,64 @@ __global__ void __launch_bounds__(kArnBlock, 1) k_arnoldi_tile(
 // pair stream length of an n-element Krylov vector
 __host__ __device__ __forceinline__ long long ff_ld(long long n) { return (n + 3) & ~3LL; }
 
-template <int M>
-cudaError_t launch_arnoldi_m(cudaStream_t s, int sms, long long n, const float* V, float* w, int nv,
+// rows x cols FP32 array with `pitch` floats between rows, copied in boxes of
+// all rows x `width` columns
+bool arn_map(CUtensorMap* m, const float* base, long long cols, long long pitch, int rows, int width) {
+  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+  if (!encode) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      return false;
+    encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
+  }
+  const cuuint64_t dim[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, stride[1] = {(cuuint64_t)pitch * sizeof(float)};
+  const cuuint32_t box[2] = {(cuuint32_t)width, (cuuint32_t)rows}, one[2] = {1, 1};
+  return encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dim, stride, box, one,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int T>
+cudaError_t launch_arnoldi_t(cudaStream_t s, int sms, long long n, const float* V, float* w, int nv,
                              float* vnext, double* d_arn, GmState* gs, int jj, float* xf, const float* dh,
                              unsigned long long* flags) {
-  constexpr int T = kArnT * M;
-  constexpr size_t extra = sizeof(float) * 4 * T;  // w' and the odd shares
   static unsigned long long ready = 0;             // per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (!((ready >> dev) & 1ull)) {
     int per = 0;
-    cudaError_t e = cudaFuncSetAttribute(k_arnoldi_tile<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kArnRing + extra));
+    cudaError_t e = cudaFuncSetAttribute(k_arnoldi_tile<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kArnSmem);
     if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_arnoldi_tile<M>, kArnBlock, kArnRing + extra);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_arnoldi_tile<T>, kArnBlock, kArnSmem);
     if (e != cudaSuccess) return e;
-    if (per < 1) return cudaErrorLaunchOutOfResources;
+    if (per < 2) return cudaErrorLaunchOutOfResources;
     ready |= 1ull << dev;
   }
   const long long tiles = (n + T - 1) / T;
-  const unsigned g = (unsigned)std::max<long long>(1, std::min<long long>(sms, tiles));
+  const unsigned g = (unsigned)std::max<long long>(1, std::min<long long>(2 * sms, tiles));
   const size_t stage = sizeof(float) * 2 * T * (size_t)(nv + 1);
   const long long most = (tiles + g - 1) / g;  // tiles of a CTA
-  int stages = (int)std::min<long long>({(long long)kArnMaxStages, (long long)(kArnRing / stage), most});
+  int stages = (int)std::min<long long>({(long long)kArnMaxStages, (long long)(arn_ring(T) / stage), most});
   long long ld = ff_ld(n);
   float2* part = reinterpret_cast<float2*>(d_arn);
-  void* args[] = {&n, &ld, &V, &w, &nv, &vnext, &part, &gs, &jj, &xf, &dh, &stages, &flags};
-  return cudaLaunchCooperativeKernel((const void*)k_arnoldi_tile<M>, dim3(g), dim3(kArnBlock), args,
-                                     stage * stages + extra, s);
+  ArnMaps maps;
+  const int width = std::min(T, kArnCons);
+  if (!arn_map(&maps.v, V, ld, ld, 2 * nv, width) || !arn_map(&maps.h, V, ld, 2 * ld, nv, width) ||
+      !arn_map(&maps.w, w, ld, ld, 2, width))
+    return cudaErrorInvalidValue;
+  void* args[] = {&maps, &n, &ld, &w, &nv, &vnext, &part, &gs, &jj, &xf, &dh, &stages, &flags};
+  return cudaLaunchCooperativeKernel((const void*)k_arnoldi_tile<T>, dim3(g), dim3(kArnBlock), args,
+                                     stage * stages + arn_extra(T), s);
 }
 
-// Tile length: the longest of 1024, 512, 256 elements at which a stage is at
-// most a third of the ring (three loads in flight) and every CTA still gets 8
-// tiles (a tile costs two or three CTA barriers and the warps' latency: short
-// bases need long tiles, short vectors need tiles for every SM).
+// Tile length: the longest of 1024, 512, 256, 128 elements at which a CTA's ring
+// holds kArnMinStages tiles and, above 128, every CTA gets 4 (a tile costs a
+// barrier or two and the warps' latency: short bases need long tiles, short
+// vectors need tiles for every SM).
+constexpr int kArnMinStages = 2;
 cudaError_t launch_arnoldi(cudaStream_t s, long long n, const float* V, float* w, int nv, float* vnext,
                            double* d_arn, GmState* gs, int jj, float* xf, const float* dh,
                            unsigned long long* flags) {
@@ -858,16 +923,16 @@ cudaError_t launch_arnoldi(cudaStream_t s, long long n, const float* V, float* w
     int v = 0;
     cudaError_t e = cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    sms[dev] = std::min(v, kArnMaxGrid);
+    sms[dev] = std::min(v, kArnMaxGrid / 2);
   }
   if (nv + 1 > kArnDots) return cudaErrorInvalidValue;
-  const size_t unit = sizeof(float) * 2 * kArnT * (size_t)(nv + 1);
-  const long long units = n / kArnT / (8LL * sms[dev]);
-  if (3 * 4 * unit <= kArnRing && units >= 4)
-    return launch_arnoldi_m<4>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
-  if (3 * 2 * unit <= kArnRing && units >= 2)
-    return launch_arnoldi_m<2>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
-  return launch_arnoldi_m<1>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  auto fits = [&](int T) {
+    return kArnMinStages * sizeof(float) * 2 * T * (size_t)(nv + 1) <= arn_ring(T) && n >= 8LL * sms[dev] * T;
+  };
+  if (fits(1024)) return launch_arnoldi_t<1024>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  if (fits(512)) return launch_arnoldi_t<512>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  if (fits(256)) return launch_arnoldi_t<256>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  return launch_arnoldi_t<128>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
 }
 
 // V0 = r / ||r|| as a pair vector (nrm2: ||r||^2)

@@ -537,15 +537,6 @@ __global__ void __launch_bounds__(256) k_amr_split(long long n, const double* __
   }
 }
 
-// xf = fp32(dinv .* x), the FP32 inner operator's input
-__global__ void __launch_bounds__(256) k_amr_to_f32(long long n, const double* __restrict__ x,
-                                                    const double* __restrict__ dinv,
-                                                    float* __restrict__ xf) {
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x)
-    xf[t] = (float)(dinv ? dinv[t] * x[t] : x[t]);
-}
-
 // w = A (D v) from y32 as FP32 pairs (Krylov vectors): free rows S (D v) + y32
 // in pairs, hanging rows (D v)_h - (P D v)_h; y32 cleared for the next
 // application.  Almost every row of S is its diagonal alone (diag, a pair; 0: any
@@ -655,51 +646,6 @@ __global__ void __launch_bounds__(256) k_amr_finish_ff(long long nvc, Hang h, un
     wh[o] = w.s;
     wl[o] = w.q;
     y32[o] = 0.f;
-  }
-}
-
-// Free rows: the identity part S (D x) in FP64 (S = P^T diag(sum of V/8) P,
-// mostly diagonal, CSR) plus the FP32 accumulation of the other terms.
-// Hanging rows: the constraint x_h - (P x)_h in FP64.
-__global__ void __launch_bounds__(256) k_amr_finish32(long long nvc, Hang h,
-                                                      const int* __restrict__ ss,
-                                                      const int* __restrict__ sc,
-                                                      const double* __restrict__ sv,
-                                                      float* __restrict__ y32,
-                                                      const double* __restrict__ x,
-                                                      const double* __restrict__ dinv,
-                                                      double* __restrict__ y) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nvc) return;
-  int s = h.hs[c], e = h.hs[c + 1];
-  const int* col = h.hp;
-  const double* w = h.hw;
-  const bool bnd = s == e && is_bnd(h, c);
-  if (bnd) {
-    s = h.bs[c];
-    e = h.bs[c + 1];
-    col = h.bc;
-    w = h.bw;
-  }
-#pragma unroll
-  for (int d = 0; d < 3; d++) {
-    if (s == e && !bnd) {
-      double acc = (double)y32[d * nvc + c];
-      for (int q = ss[c]; q < ss[c + 1]; q++) {
-        const int cl = sc[q];
-        acc += sv[q] * (dinv ? dinv[d * nvc + cl] : 1.0) * x[d * nvc + cl];
-      }
-      y[d * nvc + c] = acc;
-    } else {
-      // constraint rows: hanging (parents) or boundary (donors)
-      double pv = 0.0;
-      for (int t = s; t < e; t++) {
-        const int p = col[t];
-        pv += w[t] * (dinv ? dinv[d * nvc + p] : 1.0) * x[d * nvc + p];
-      }
-      y[d * nvc + c] = (dinv ? dinv[d * nvc + c] : 1.0) * x[d * nvc + c] - pv;
-    }
-    y32[d * nvc + c] = 0.f;
   }
 }
 
@@ -1071,27 +1017,7 @@ cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* di
   return cudaGetLastError();
 }
 
-// (d_y32 is zero between applications: the finish kernels clear what they read)
-cudaError_t launch_amr_matvec32(amps_gpu_ctx* c, const double* x, const double* dinv,
-                                double* y) {
-  cudaError_t e = cudaSuccess;
-  ApplyArgs a = apply_args(c);
-  a.x = x;
-  a.dinv = dinv;
-  // the identity part is applied in FP64 by k_amr_finish32
-  const long long n = 3 * c->nvc;
-  if (!c->d_xs && (e = cudaMalloc(reinterpret_cast<void**>(&c->d_xs), sizeof(float) * 2 * n)) != cudaSuccess)
-    return e;
-  a.xf = c->d_xs;
-  TimedLaunch t(c, "matvec32", 3);
-  k_amr_to_f32<<<(unsigned)std::min<long long>((n + 255) / 256, 152LL * 16), 256, 0, c->stream>>>(n, x, dinv,
-                                                                                                 c->d_xs);
-  if ((e = launch_tile32(c, a, c->d_y32)) != cudaSuccess) return e;
-  k_amr_finish32<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, c->d_ss, c->d_sc, c->d_sv,
-                                                     c->d_y32, x, dinv, y);
-  return cudaGetLastError();
-}
-
+// (d_y32 is zero between applications: the finish kernel clears what it reads)
 cudaError_t launch_amr_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, float* wl) {
   cudaError_t e = cudaSuccess;
   ApplyArgs a = apply_args(c);

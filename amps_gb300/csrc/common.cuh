@@ -319,8 +319,6 @@ cudaError_t launch_export(amps_gpu_ctx* c, double* d_x, double* d_v, uint8_t* d_
 // ---- field launchers (field.cu) ----
 cudaError_t launch_rhs(amps_gpu_ctx* c);
 cudaError_t launch_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y);
-// the same operator evaluated in FP32 arithmetic (inner GMRES iterations)
-cudaError_t launch_matvec32(amps_gpu_ctx* c, const double* x, const double* dinv, double* y);
 // Input of the inner operator on a Krylov vector: v as FP32 pairs (vh, vl) or,
 // for the flexible directions, as doubles (vd); the scaling D as FP32 pairs
 // (dh, dl) or none.  The operator computes w = A (D v) and writes it as FP32
@@ -353,7 +351,6 @@ amps_gpu_status field_autotune(amps_gpu_ctx* c, double* ms);
 cudaError_t launch_amr_pack(amps_gpu_ctx* c, const double* Eh, const double* Bprev,
                             const double* Bcur);
 cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y);
-cudaError_t launch_amr_matvec32(amps_gpu_ctx* c, const double* x, const double* dinv, double* y);
 cudaError_t launch_amr_rhs(amps_gpu_ctx* c);
 cudaError_t launch_amr_jacobi(amps_gpu_ctx* c);
 cudaError_t launch_amr_update_b(amps_gpu_ctx* c);

@@ -120,8 +120,7 @@ TapsFF taps_ff(const Taps& T) {
   return t;
 }
 
-// xh + xl = dinv .* x (dinv may be null), split into FP32 pairs (xl null: the
-// FP32 rounding only, the input of the FP32 inner operator)
+// xh + xl = dinv .* x (dinv may be null), split into FP32 pairs
 __global__ void __launch_bounds__(256) k_split(long long n, const double* __restrict__ x,
                                                const double* __restrict__ dinv,
                                                float* __restrict__ xh, float* __restrict__ xl) {
@@ -130,49 +129,8 @@ __global__ void __launch_bounds__(256) k_split(long long n, const double* __rest
     const double v = dinv ? dinv[t] * x[t] : x[t];
     const float h = (float)v;
     xh[t] = h;
-    if (xl) xl[t] = (float)(v - (double)h);
+    xl[t] = (float)(v - (double)h);
   }
-}
-
-// Row (p, corner c) of (K + f M) x to FP64 accuracy: the 27-point taps and
-// the corner's 243 FP32 mass-matrix coefficients against the split input.
-__device__ __forceinline__ double row_ff(long long ncor, const int* __restrict__ nbr,
-                                         const float* __restrict__ M, const float* __restrict__ xh,
-                                         const float* __restrict__ xl, const TapsFF& T, int p,
-                                         long long c, int b, int i, int j, int k) {
-  FF sk{0.f, 0.f}, sm{0.f, 0.f};
-#pragma unroll 3
-  for (int s = 0; s < 27; s++) {
-    const int dig[3] = {s % 3, (s / 3) % 3, s / 9};
-    const int di = dig[0] == 0 ? 0 : (dig[0] == 1 ? -1 : 1);
-    const int dj = dig[1] == 0 ? 0 : (dig[1] == 1 ? -1 : 1);
-    const int dk = dig[2] == 0 ? 0 : (dig[2] == 1 ? -1 : 1);
-    const int nb = local_id(nbr, b, i + di, j + dj, k + dk);
-    const float* Ms = M + (size_t)(9 * s + 3 * p) * ncor + c;
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-      const float h = xh[q * ncor + nb], lo = xl[q * ncor + nb];
-      ff_add2(sk, T.Kh[p][q][s], T.Kl[p][q][s], h, lo);
-      ff_add(sm, Ms[(size_t)q * ncor], h, lo);
-    }
-  }
-  return ff_value(sk) + T.f * ff_value(sm);
-}
-
-// y = A (dinv .* x) to FP64 accuracy from the split input (outer residuals);
-// one thread per (component p, corner)
-__global__ void __launch_bounds__(256) k_matvec(long long ncor, const int* __restrict__ nbr,
-                                                const float* __restrict__ M,
-                                                const float* __restrict__ xh,
-                                                const float* __restrict__ xl,
-                                                double* __restrict__ y, TapsFF T) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * ncor) return;
-  const int p = (int)(t / ncor);
-  const long long c = t - (long long)p * ncor;
-  int b, i, j, k;
-  corner_ijk(c, b, i, j, k);
-  y[t] = row_ff(ncor, nbr, M, xh, xl, T, p, c, b, i, j, k);
 }
 
 struct TapsF {
@@ -189,77 +147,137 @@ TapsF taps_f32(const Taps& T) {
   return t;
 }
 
-// y = A (dinv .* x) with the identity part in FP64 and the rest (curl-curl
-// and mass-matrix terms, a small fraction of A on ECSIM time steps) in FP32
-// arithmetic: the inner operator of the refined GMRES, which never decides
-// convergence.  One thread per (component p, corner).
-__global__ void __launch_bounds__(256) k_matvec32(long long ncor, const int* __restrict__ nbr,
-                                                  const float* __restrict__ M,
-                                                  const float* __restrict__ xf,
-                                                  const double* __restrict__ x,
-                                                  const double* __restrict__ dinv,
-                                                  double* __restrict__ y, TapsF T) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * ncor) return;
-  const int p = (int)(t / ncor);
-  const long long c = t - (long long)p * ncor;
+// ---- the 27-point operator ---------------------------------------------------
+// A CTA takes 32 consecutive corners (ncor is a multiple of 512) and splits the
+// 27 slots over its W = blockDim / 32 warps (slot s: warp s mod W); lane = corner,
+// so the 243 coefficient planes of M are read in whole lines, and a slot's
+// neighbour values serve the three components.  The warps' partial sums meet in
+// shared memory and are added in warp order.  Bound: latency on small meshes --
+// one thread per (component, corner) walked all 27 slots, nine rounds of
+// dependent loads -- and reading M (HBM) on large ones.  us per application,
+// before and now, at 512 and at 32,768 corners: FP32 operator 15.6 -> 8.5, 18.5 ->
+// 15.9; residual operator with its input split 23.2 -> 16.1, 30.5 -> 27.2; RHS
+// likewise 27 -> 16.8, 42 -> 37.
+constexpr int kOpMaxWarps = 8;
+
+__device__ __forceinline__ void slot_offset(int s, int& di, int& dj, int& dk) {
+  const int d0 = s % 3, d1 = (s / 3) % 3, d2 = s / 9;
+  di = d0 == 0 ? 0 : (d0 == 1 ? -1 : 1);
+  dj = d1 == 0 ? 0 : (d1 == 1 ? -1 : 1);
+  dk = d2 == 0 ? 0 : (d2 == 1 ? -1 : 1);
+}
+
+// This warp's slots of (K + f M) x at corner c, all three rows, to FP64 accuracy:
+// sk the taps, sm the mass matrix's FP32 coefficients, against the split input.
+struct RowFF {
+  FF sk[3], sm[3];
+};
+__device__ __forceinline__ RowFF rows_ff(long long ncor, const int* __restrict__ nbr, const float* __restrict__ M,
+                                         const float* __restrict__ xh, const float* __restrict__ xl,
+                                         const TapsFF& T, long long c, int b, int i, int j, int k, int wid,
+                                         int warps) {
+  RowFF r;
+#pragma unroll
+  for (int p = 0; p < 3; p++) r.sk[p] = r.sm[p] = FF{0.f, 0.f};
+#pragma unroll 2
+  for (int s = wid; s < 27; s += warps) {
+    int di, dj, dk;
+    slot_offset(s, di, dj, dk);
+    const int nb = local_id(nbr, b, i + di, j + dj, k + dk);
+    float h[3], lo[3], m[9];
+#pragma unroll
+    for (int q = 0; q < 3; q++) { h[q] = xh[q * ncor + nb]; lo[q] = xl[q * ncor + nb]; }
+#pragma unroll
+    for (int e = 0; e < 9; e++) m[e] = M[(size_t)(9 * s + e) * ncor + c];
+#pragma unroll
+    for (int p = 0; p < 3; p++)
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        ff_add2(r.sk[p], T.Kh[p][q][s], T.Kl[p][q][s], h[q], lo[q]);
+        ff_add(r.sm[p], m[3 * p + q], h[q], lo[q]);
+      }
+  }
+  return r;
+}
+// The warps' rows into s_row[6][warps][32], and component p of the sum at lane
+// (after the barrier)
+__device__ __forceinline__ void rows_store(const RowFF& r, float2 (*s_row)[kOpMaxWarps][32], int wid, int lane) {
+#pragma unroll
+  for (int p = 0; p < 3; p++) {
+    s_row[p][wid][lane] = make_float2(r.sk[p].s, r.sk[p].q);
+    s_row[3 + p][wid][lane] = make_float2(r.sm[p].s, r.sm[p].q);
+  }
+}
+__device__ __forceinline__ double rows_sum(float2 (*s_row)[kOpMaxWarps][32], int warps, int p, int lane, double f) {
+  FF a{0.f, 0.f}, m{0.f, 0.f};
+  for (int w = 0; w < warps; w++) {
+    ff_acc(a, s_row[p][w][lane].x, s_row[p][w][lane].y);
+    ff_acc(m, s_row[3 + p][w][lane].x, s_row[3 + p][w][lane].y);
+  }
+  return ff_value(a) + f * ff_value(m);
+}
+
+// y = A (dinv .* x) to FP64 accuracy from the split input (outer residuals)
+__global__ void __launch_bounds__(32 * kOpMaxWarps) k_matvec(long long ncor, const int* __restrict__ nbr,
+                                                             const float* __restrict__ M,
+                                                             const float* __restrict__ xh,
+                                                             const float* __restrict__ xl,
+                                                             double* __restrict__ y,
+                                                             const __grid_constant__ TapsFF T) {
+  __shared__ float2 s_row[6][kOpMaxWarps][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const long long c = (long long)blockIdx.x * 32 + lane;
   int b, i, j, k;
   corner_ijk(c, b, i, j, k);
-  float acc = 0.f;
-#pragma unroll 3
-  for (int s = 0; s < 27; s++) {
-    const int dig[3] = {s % 3, (s / 3) % 3, s / 9};
-    const int di = dig[0] == 0 ? 0 : (dig[0] == 1 ? -1 : 1);
-    const int dj = dig[1] == 0 ? 0 : (dig[1] == 1 ? -1 : 1);
-    const int dk = dig[2] == 0 ? 0 : (dig[2] == 1 ? -1 : 1);
-    const int nb = local_id(nbr, b, i + di, j + dj, k + dk);
-    const float* Ms = M + (size_t)(9 * s + 3 * p) * ncor + c;
-#pragma unroll
-    for (int q = 0; q < 3; q++)
-      acc = fmaf(fmaf(T.f, Ms[(size_t)q * ncor], T.K[p][q][s]), xf[q * ncor + nb], acc);
-  }
-  const double xi = dinv ? dinv[t] * x[t] : x[t];
-  y[t] = xi + (double)acc;
+  rows_store(rows_ff(ncor, nbr, M, xh, xl, T, c, b, i, j, k, wid, warps), s_row, wid, lane);
+  __syncthreads();
+  for (int p = wid; p < 3; p += warps) y[p * ncor + c] = rows_sum(s_row, warps, p, lane, T.f);
 }
 
 // RHS: theta c dt curl B^n - f J - (curl-curl + f M) E^n, the last term to
 // FP64 accuracy from the split E^n (taps without the identity)
-__global__ void __launch_bounds__(256) k_rhs(long long ncor, const int* __restrict__ nbr,
-                                             const float* __restrict__ M,
-                                             const float* __restrict__ Eh,
-                                             const float* __restrict__ El,
-                                             const double* __restrict__ Bc,
-                                             const double* __restrict__ J,
-                                             double* __restrict__ rhs, TapsFF T, double c4x,
-                                             double c4y, double c4z) {
-  // one thread per (component p, corner)
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * ncor) return;
-  const int p = (int)(t / ncor);
-  const long long c = t - (long long)p * ncor;
+__global__ void __launch_bounds__(32 * kOpMaxWarps) k_rhs(long long ncor, const int* __restrict__ nbr,
+                                                          const float* __restrict__ M,
+                                                          const float* __restrict__ Eh,
+                                                          const float* __restrict__ El,
+                                                          const double* __restrict__ Bc,
+                                                          const double* __restrict__ J,
+                                                          double* __restrict__ rhs,
+                                                          const __grid_constant__ TapsFF T, double c4x,
+                                                          double c4y, double c4z) {
+  __shared__ float2 s_row[6][kOpMaxWarps][32];
+  __shared__ double s_cb[3][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const long long c = (long long)blockIdx.x * 32 + lane;
   int b, i, j, k;
   corner_ijk(c, b, i, j, k);
-  double r = -row_ff(ncor, nbr, M, Eh, El, T, p, c, b, i, j, k);
-  r -= T.f * J[t];
-  // curl B^n from the 2x2 face averages of the 8 cells around the corner
+  // curl B^n from the 2x2 face averages of the 8 cells around the corner,
+  // components from the last warp down (the first have one slot more)
   auto Bv = [&](int ii, int jj, int kk, int comp) {
     return Bc[comp * ncor + local_id(nbr, b, ii, jj, kk)];
   };
-  double cb = 0.0;
-  for (int a = -1; a <= 0; a++)
-    for (int q = -1; q <= 0; q++) {
-      if (p == 0) {
-        cb += c4y * (Bv(i + a, j, k + q, 2) - Bv(i + a, j - 1, k + q, 2));
-        cb += -c4z * (Bv(i + a, j + q, k, 1) - Bv(i + a, j + q, k - 1, 1));
-      } else if (p == 1) {
-        cb += c4z * (Bv(i + a, j + q, k, 0) - Bv(i + a, j + q, k - 1, 0));
-        cb += -c4x * (Bv(i, j + q, k + a, 2) - Bv(i - 1, j + q, k + a, 2));
-      } else {
-        cb += c4x * (Bv(i, j + q, k + a, 1) - Bv(i - 1, j + q, k + a, 1));
-        cb += -c4y * (Bv(i + q, j, k + a, 0) - Bv(i + q, j - 1, k + a, 0));
+  for (int p = warps - 1 - wid; p < 3; p += warps) {
+    double cb = 0.0;
+#pragma unroll
+    for (int a = -1; a <= 0; a++)
+#pragma unroll
+      for (int q = -1; q <= 0; q++) {
+        if (p == 0) {
+          cb += c4y * (Bv(i + a, j, k + q, 2) - Bv(i + a, j - 1, k + q, 2));
+          cb += -c4z * (Bv(i + a, j + q, k, 1) - Bv(i + a, j + q, k - 1, 1));
+        } else if (p == 1) {
+          cb += c4z * (Bv(i + a, j + q, k, 0) - Bv(i + a, j + q, k - 1, 0));
+          cb += -c4x * (Bv(i, j + q, k + a, 2) - Bv(i - 1, j + q, k + a, 2));
+        } else {
+          cb += c4x * (Bv(i, j + q, k + a, 1) - Bv(i - 1, j + q, k + a, 1));
+          cb += -c4y * (Bv(i + q, j, k + a, 0) - Bv(i + q, j - 1, k + a, 0));
+        }
       }
-    }
-  rhs[t] = r + cb;
+    s_cb[p][lane] = cb - T.f * J[p * ncor + c];
+  }
+  rows_store(rows_ff(ncor, nbr, M, Eh, El, T, c, b, i, j, k, wid, warps), s_row, wid, lane);
+  __syncthreads();
+  for (int p = wid; p < 3; p += warps) rhs[p * ncor + c] = s_cb[p][lane] - rows_sum(s_row, warps, p, lane, T.f);
 }
 
 __global__ void __launch_bounds__(256) k_jacobi(long long ncor, const float* __restrict__ M,
@@ -1034,37 +1052,49 @@ __global__ void __launch_bounds__(256) k_in_f32(long long n, OpIn in, float* __r
     xf[t] = in.vd ? (float)in.vd[t] : (in.dh ? in.vh[t] * in.dh[t] : in.vh[t]);
 }
 
-// w = A (D v) with the identity part in pairs and the rest in FP32 (the FP32
-// inner operator of k_matvec32 with pair input and output)
-__global__ void __launch_bounds__(256) k_matvec32_ff(long long ncor, const int* __restrict__ nbr,
-                                                     const float* __restrict__ M,
-                                                     const float* __restrict__ xf, OpIn in,
-                                                     float* __restrict__ wh, float* __restrict__ wl,
-                                                     TapsF T) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * ncor) return;
-  const int p = (int)(t / ncor);
-  const long long c = t - (long long)p * ncor;
+// w = A (D v) with the identity part in pairs and the rest (curl-curl and
+// mass-matrix terms, a small fraction of A on ECSIM time steps) in FP32
+// arithmetic: the inner operator of the refined GMRES, which never decides
+// convergence.  xf = fp32(D v).
+__global__ void __launch_bounds__(32 * kOpMaxWarps) k_matvec32_ff(long long ncor, const int* __restrict__ nbr,
+                                                                  const float* __restrict__ M,
+                                                                  const float* __restrict__ xf, OpIn in,
+                                                                  float* __restrict__ wh, float* __restrict__ wl,
+                                                                  const __grid_constant__ TapsF T) {
+  __shared__ float s_row[3][kOpMaxWarps][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const long long c = (long long)blockIdx.x * 32 + lane;
   int b, i, j, k;
   corner_ijk(c, b, i, j, k);
-  float acc = 0.f;
-#pragma unroll 3
-  for (int s = 0; s < 27; s++) {
-    const int dig[3] = {s % 3, (s / 3) % 3, s / 9};
-    const int di = dig[0] == 0 ? 0 : (dig[0] == 1 ? -1 : 1);
-    const int dj = dig[1] == 0 ? 0 : (dig[1] == 1 ? -1 : 1);
-    const int dk = dig[2] == 0 ? 0 : (dig[2] == 1 ? -1 : 1);
+  float acc[3] = {0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int s = wid; s < 27; s += warps) {
+    int di, dj, dk;
+    slot_offset(s, di, dj, dk);
     const int nb = local_id(nbr, b, i + di, j + dj, k + dk);
-    const float* Ms = M + (size_t)(9 * s + 3 * p) * ncor + c;
+    float x[3], m[9];
 #pragma unroll
-    for (int q = 0; q < 3; q++)
-      acc = fmaf(fmaf(T.f, Ms[(size_t)q * ncor], T.K[p][q][s]), xf[q * ncor + nb], acc);
+    for (int q = 0; q < 3; q++) x[q] = xf[q * ncor + nb];
+#pragma unroll
+    for (int e = 0; e < 9; e++) m[e] = M[(size_t)(9 * s + e) * ncor + c];
+#pragma unroll
+    for (int p = 0; p < 3; p++)
+#pragma unroll
+      for (int q = 0; q < 3; q++) acc[p] = fmaf(fmaf(T.f, m[3 * p + q], T.K[p][q][s]), x[q], acc[p]);
   }
-  FF y = opin_value(in, t);
-  ff_acc(y, acc, 0.f);
-  y = ff_norm(y);
-  wh[t] = y.s;
-  wl[t] = y.q;
+#pragma unroll
+  for (int p = 0; p < 3; p++) s_row[p][wid][lane] = acc[p];
+  __syncthreads();
+  for (int p = wid; p < 3; p += warps) {
+    float a = 0.f;
+    for (int w = 0; w < warps; w++) a += s_row[p][w][lane];
+    const long long t = p * ncor + c;
+    FF y = opin_value(in, t);
+    ff_acc(y, a, 0.f);
+    y = ff_norm(y);
+    wh[t] = y.s;
+    wl[t] = y.q;
+  }
 }
 
 // ---- field updates -----------------------------------------------------------
@@ -1162,7 +1192,6 @@ __global__ void __launch_bounds__(256) k_add(long long n, const double* __restri
 }
 
 unsigned grid1(long long n) { return (unsigned)((n + 255) / 256); }
-unsigned gridt(long long n, int tb) { return (unsigned)((n + tb - 1) / tb); }
 // sweep/reduction grid: at least ept elements per thread, at most cap CTAs
 unsigned gridr(long long n, int cap = kRedBlocks, int ept = 4) {
   long long g = (n + 256LL * ept - 1) / (256LL * ept);
@@ -1173,19 +1202,17 @@ unsigned gridr(long long n, int cap = kRedBlocks, int ept = 4) {
 }  // namespace
 
 // ============================================================================
-// FP32 pair split of an operator input into the context's scratch (hi_only:
-// the FP32 rounding alone).  d_xs is also where k_start_ff / k_arnoldi_tile
+// FP32 pair split of an operator input into the context's scratch.  d_xs is also where k_start_ff / k_arnoldi_tile
 // leave the FP32 input of the next Krylov vector's operator application: this
 // split, k_rhs and the AMR operators overwrite it, so none of them may run
 // between an Arnoldi step and the operator application that follows it.
-static cudaError_t split_input(amps_gpu_ctx* c, const double* x, const double* dinv,
-                               bool hi_only = false) {
+static cudaError_t split_input(amps_gpu_ctx* c, const double* x, const double* dinv) {
   const long long n = 3 * c->nvc;
   if (!c->d_xs) {
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&c->d_xs), sizeof(float) * 2 * n);
     if (e != cudaSuccess) return e;
   }
-  k_split<<<gridr(n), 256, 0, c->stream>>>(n, x, dinv, c->d_xs, hi_only ? nullptr : c->d_xs + n);
+  k_split<<<gridr(n), 256, 0, c->stream>>>(n, x, dinv, c->d_xs, c->d_xs + n);
   return cudaGetLastError();
 }
 
@@ -1196,19 +1223,8 @@ cudaError_t launch_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, 
   cudaError_t e = split_input(c, x, dinv);
   if (e != cudaSuccess) return e;
   const long long n = 3 * c->ncor;
-  k_matvec<<<gridt(n, c->tune_tb), c->tune_tb, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_M,
-                                                               c->d_xs, c->d_xs + n, y, T);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_matvec32(amps_gpu_ctx* c, const double* x, const double* dinv, double* y) {
-  if (c->amr) return launch_amr_matvec32(c, x, dinv, y);
-  const TapsF T = taps_f32(make_taps(c->cfg, false));
-  TimedLaunch t(c, "matvec32", 2);
-  cudaError_t e = split_input(c, x, dinv, true);
-  if (e != cudaSuccess) return e;
-  k_matvec32<<<gridt(3 * c->ncor, c->tune_tb), c->tune_tb, 0, c->stream>>>(c->ncor, c->d_nbr,
-                                                                            c->d_M, c->d_xs, x, dinv, y, T);
+  k_matvec<<<(unsigned)(c->ncor / 32), c->tune_tb, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_M, c->d_xs,
+                                                                   c->d_xs + n, y, T);
   return cudaGetLastError();
 }
 
@@ -1229,8 +1245,8 @@ cudaError_t launch_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, float
   TimedLaunch t(c, "matvec32", in.xf_ready ? 1 : 2);
   cudaError_t e = in.xf_ready ? cudaSuccess : launch_in_f32(c, in, c->d_xs);
   if (e != cudaSuccess) return e;
-  k_matvec32_ff<<<gridt(n, c->tune_tb), c->tune_tb, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_M, c->d_xs, in,
-                                                                     wh, wl, T);
+  k_matvec32_ff<<<(unsigned)(c->ncor / 32), c->tune_tb, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_M, c->d_xs,
+                                                                        in, wh, wl, T);
   return cudaGetLastError();
 }
 
@@ -1243,8 +1259,9 @@ cudaError_t launch_rhs(amps_gpu_ctx* c) {
   cudaError_t e = split_input(c, c->d_En, nullptr);
   if (e != cudaSuccess) return e;
   const long long n = 3 * c->ncor;
-  k_rhs<<<grid1(n), 256, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_M, c->d_xs, c->d_xs + n, c->d_Bc,
-                                         c->d_J, c->d_rhs, T, c4[0], c4[1], c4[2]);
+  k_rhs<<<(unsigned)(c->ncor / 32), c->tune_tb, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_M, c->d_xs,
+                                                                c->d_xs + n, c->d_Bc, c->d_J, c->d_rhs, T,
+                                                                c4[0], c4[1], c4[2]);
   return cudaGetLastError();
 }
 
@@ -1575,7 +1592,9 @@ amps_gpu_status field_autotune(amps_gpu_ctx* c, double* ms) {
     return st;
   };
   double* x = c->d_x;
-  double* y = c->d_w;
+  float* yf = reinterpret_cast<float*>(c->d_w);
+  OpIn in{};
+  in.vd = x;
   if ((e = cudaMemsetAsync(x, 0, sizeof(double) * n, s)) != cudaSuccess) fail(e, "autotune");
   if ((e = cudaMemsetAsync(c->d_V, 0, sizeof(double) * n * 10, s)) != cudaSuccess) fail(e, "autotune");
   const int tbs[3] = {64, 128, 256};
@@ -1584,10 +1603,10 @@ amps_gpu_status field_autotune(amps_gpu_ctx* c, double* ms) {
   for (int q = 0; q < 3 && !st; q++) {
     c->tune_tb = tbs[q];
     for (int w = 0; w < 2 && !st; w++)
-      if ((e = launch_matvec32(c, x, nullptr, y)) != cudaSuccess) fail(e, "autotune matvec");
+      if ((e = launch_matvec32_ff(c, in, yf, yf + ff_ld(n))) != cudaSuccess) fail(e, "autotune matvec");
     cudaEventRecord(a, s);
     for (int r = 0; r < 5 && !st; r++)
-      if ((e = launch_matvec32(c, x, nullptr, y)) != cudaSuccess) fail(e, "autotune matvec");
+      if ((e = launch_matvec32_ff(c, in, yf, yf + ff_ld(n))) != cudaSuccess) fail(e, "autotune matvec");
     cudaEventRecord(b, s);
     cudaEventSynchronize(b);
     float t = 0.f;

@@ -103,10 +103,6 @@ amps_gpu_status upload_vec3(amps_gpu_ctx* c, const double* host, double* dev, lo
   return layout_upload(c, host, dev, n, 3, false);
 }
 
-amps_gpu_status download_vec3(amps_gpu_ctx* c, const double* dev, double* host, long long n) {
-  return layout_download(c, dev, host, n, 3, false);
-}
-
 // staging buffers for particle import/export (allocated on first use)
 struct Staging {
   double* x = nullptr;   // 3n doubles (also 3n floats for the local import)
@@ -876,14 +872,13 @@ amps_gpu_status amps_gpu_import_fields(amps_gpu_ctx* c, const double* E_n, const
                                        const double* B_corner_cur) {
   if (!c) return AMPS_GPU_INVALID_ARG;
   cudaSetDevice(c->cfg.device);
-  cudaStreamSynchronize(c->stream);
-  amps_gpu_status s;
   const long long nv = c->nvc, nc = c->ncor;
-  if ((s = upload_vec3(c, E_n, c->d_En, nv)) || (s = upload_vec3(c, E_half, c->d_Eh, nv)) ||
-      (s = upload_vec3(c, B_center, c->d_Bc, nc)) ||
-      (s = upload_vec3(c, B_corner_prev, c->d_Bcor_prev, nv)) ||
-      (s = upload_vec3(c, B_corner_cur, c->d_Bcor_cur, nv)))
-    return s;
+  double* host[5] = {const_cast<double*>(E_n), const_cast<double*>(E_half), const_cast<double*>(B_center),
+                     const_cast<double*>(B_corner_prev), const_cast<double*>(B_corner_cur)};
+  double* dev[5] = {c->d_En, c->d_Eh, c->d_Bc, c->d_Bcor_prev, c->d_Bcor_cur};
+  const long long n[5] = {nv, nv, nc, nv, nv};
+  amps_gpu_status s = layout_vec3_many(c, false, 5, host, dev, n);
+  if (s) return s;
   // the centre B^n a centre-B push reads before the first field solve
   return cuda_check(c, cudaMemcpyAsync(c->d_Bc2, c->d_Bc, sizeof(double) * 3 * nc,
                                        cudaMemcpyDeviceToDevice, c->stream), "B centre copy");
@@ -894,15 +889,11 @@ amps_gpu_status amps_gpu_export_fields(amps_gpu_ctx* c, double* E_n, double* E_h
                                        double* B_corner_cur) {
   if (!c) return AMPS_GPU_INVALID_ARG;
   cudaSetDevice(c->cfg.device);
-  amps_gpu_status s = cuda_check(c, cudaStreamSynchronize(c->stream), "sync");
-  if (s) return s;
   const long long nv = c->nvc, nc = c->ncor;
-  if ((s = download_vec3(c, c->d_En, E_n, nv)) || (s = download_vec3(c, c->d_Eh, E_half, nv)) ||
-      (s = download_vec3(c, c->d_Bc, B_center, nc)) ||
-      (s = download_vec3(c, c->d_Bcor_prev, B_corner_prev, nv)) ||
-      (s = download_vec3(c, c->d_Bcor_cur, B_corner_cur, nv)))
-    return s;
-  return AMPS_GPU_OK;
+  double* host[5] = {E_n, E_half, B_center, B_corner_prev, B_corner_cur};
+  double* dev[5] = {c->d_En, c->d_Eh, c->d_Bc, c->d_Bcor_prev, c->d_Bcor_cur};
+  const long long n[5] = {nv, nv, nc, nv, nv};
+  return layout_vec3_many(c, true, 5, host, dev, n);
 }
 
 amps_gpu_status amps_gpu_import_moments(amps_gpu_ctx* c, const double* J, const double* M) {
@@ -922,10 +913,8 @@ amps_gpu_status amps_gpu_import_moments(amps_gpu_ctx* c, const double* J, const 
 amps_gpu_status amps_gpu_export_moments(amps_gpu_ctx* c, double* J, double* M) {
   if (!c) return AMPS_GPU_INVALID_ARG;
   cudaSetDevice(c->cfg.device);
-  amps_gpu_status s = cuda_check(c, cudaStreamSynchronize(c->stream), "sync");
-  if (s) return s;
   if (c->amr) return amr_export_corner_moments(c, J, M);
-  s = download_vec3(c, c->d_J, J, c->ncor);
+  amps_gpu_status s = layout_vec3_many(c, true, 1, &J, &c->d_J, &c->ncor);
   if (s) return s;
   if ((s = layout_download(c, c->d_M, M, c->ncor, 243, true))) return s;
   return AMPS_GPU_OK;

@@ -287,6 +287,8 @@ amps_gpu_status layout_upload(amps_gpu_ctx* c, const double* host, void* dev, lo
                               int ncomp, bool dev_f32);
 amps_gpu_status layout_download(amps_gpu_ctx* c, const void* dev, double* host, long long n,
                                 int ncomp, bool dev_f32);
+amps_gpu_status layout_vec3_many(amps_gpu_ctx* c, bool to_host, int count, double* const* host,
+                                 double* const* dev, const long long* n);
 amps_gpu_status layout_cell_moments(amps_gpu_ctx* c, double* hJ, double* hM);
 // device address of a page-locked host array (kernels write it across the host
 // link directly), or null for pageable memory

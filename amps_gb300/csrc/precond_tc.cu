@@ -1,26 +1,40 @@
 // BF16 tensor-core inference of the learned preconditioner on sm_103a:
-// tcgen05.mma with FP32 accumulators in tensor memory, one CTA per mesh block.
+// tcgen05.mma with FP32 accumulators in tensor memory, two CTAs per mesh block.
 //
-// Each 3x3x3 convolution is an implicit GEMM: D[m][n] = sum over taps t and
-// input channels k of A[m + off_t][k] * B_t[k][n], m = voxel of the padded
-// 12^3 region (linear index p = x + 12 y + 144 z, a zero ring around the 10^3
-// region R), off_t = dx + 12 dy + 144 dz.  Activations live in shared memory
-// as BF16 planes of 8 channels, 16 bytes per voxel, so the A operand of tap t
-// is the same buffer read from row m0 + off_t: a K-major, non-swizzled operand
-// whose 8x16-byte core matrices are 8 consecutive voxels (stride-dimension
-// offset 128 B) and whose next 8 channels are the next plane (leading-dimension
-// offset = plane size).  Rows 157 .. 1692 (12 tiles of 128) cover every voxel
-// of R; rows outside R are computed and dropped.
+// Each 3x3x3 convolution over the region R of 10^3 voxels is an implicit GEMM.
+// An x-plane of R is one tile of 128 accumulator rows: voxel (i, j, k) is row
+// j + 11 k of plane i, so a tap (dy, dz) is a shift of dy + 11 dz rows (the zero
+// rows j = 10 and 110 .. 127 are the ring; a plane's lower ring is the end of the
+// plane before it).  Activations live in shared memory as BF16 planes of 8
+// channels, 16 bytes per row, so the A operand of a tap is the same buffer read
+// from a shifted row: a K-major, non-swizzled operand whose 8x16-byte core matrices
+// are 8 consecutive rows (stride-dimension offset 128 B) and whose next 8 channels
+// are the next channel plane (leading-dimension offset = its size).  A tap's dx
+// moves the output by whole tiles: the three dx of one (dy, dz) are side by side in
+// the B operand, [dx = +1 | 0 | -1], and one MMA adds input plane x to the
+// accumulators of planes x-1, x and x+1, which are neighbours in tensor memory.
+// The first (dy, dz) and K chunk goes by single planes, the centre one first and
+// without accumulation, as it starts the sums.
 //
-// A cluster of two CTAs serves one mesh block; each keeps the whole activation
-// buffer and computes 6 of the 12 tiles.  Per layer one thread of each CTA
-// issues 6 tiles x 27 taps x (K/16) MMAs of 128 x N x 16 into tensor memory
-// (N = 32, or 16 for the 3-channel output layer), commits them to an mbarrier,
-// and the four warps read their 32 accumulator lanes back (tcgen05.ld),
-// convert to BF16 and write the rows into both CTAs' activation planes
-// (distributed shared memory; zero on the ring), or write the owned voxels'
-// FP32 output.  A cluster barrier separates the layers.
-// Shared memory per CTA: 4 activation planes (110,592 B) + the three layers'
+// A cluster of two CTAs serves one mesh block; each computes 5 output planes from
+// 6 input planes, counted from the block's outside: u = 0 .. 4 its own, 5 the
+// peer's nearest.  One thread issues the MMAs of 128 x N x 16 (N = 32 a plane, 16
+// in the 3-channel output layer), those of u < 4 first; each half is committed to
+// its own mbarrier.  Warps 0-3 read planes 0-2 back (tcgen05.ld, 32 lanes a warp)
+// and write the next layer's rows while the second half runs, warps 4-7 planes 3-4.
+// Once the peer's MMAs have read their plane 5 (a split cluster barrier), plane 4
+// is written there too (distributed shared memory); the first half of the next
+// layer doesn't need it and is issued before.  The last layer writes the owned
+// voxels' FP32 output.
+//
+// What bounds it: an MMA of M = 128 and K = 16 takes 40 cycles at N = 16 and 32
+// alike (its A rows come from shared memory) and 64 at N = 96, so three dx per MMA
+// count (294 MMAs per CTA instead of 810), and an issue loop in uniform control flow
+// (one elected thread, descriptors in uniform registers; a loop under tid == 0 issues
+// one MMA in 74 cycles); these are 15,000 of the kernel's 25,000 cycles, the chain
+// gather - read-back - exchange the rest.  64 blocks of a mesh: 28 us per
+// application; with an MMA per tap, 4 warps and one commit a layer 60.
+// Shared memory per CTA: 4 channel planes (82,944 B) + the three layers'
 // BF16 weight images (110,592 B, one bulk copy); tensor memory: 256 columns.
 // Every mbarrier wait is bounded; a timeout is counted in flags[2] and the CTA
 // still takes part in every cluster barrier, so its peer never waits on it.
@@ -33,19 +47,20 @@
 
 namespace {
 
-constexpr int kPadV = 1728;                 // 12^3 padded voxels
-constexpr int kPlane = kPadV * 16;          // bytes per 8-channel BF16 plane
-constexpr int kActBytes = 4 * kPlane;       // 110,592
-constexpr int kMBegin = 157;                // padded voxel (1,1,1)
-constexpr int kTiles = 12;                  // rows kMBegin .. kMBegin + 1535
+constexpr int kLead = 16;                   // zero rows before plane 0 (a tap reaches 12 back)
+constexpr int kRows = kLead + 10 * 128;     // ten x-planes of 128 rows
+constexpr int kPlane = kRows * 16;          // bytes per 8-channel BF16 plane
+constexpr int kActBytes = 4 * kPlane;       // 82,944
 constexpr int kSplit = 2;                   // CTAs (cluster) per mesh block
-constexpr int kMyTiles = kTiles / kSplit;
+constexpr int kMine = 5;                    // output planes per CTA
+constexpr int kFirst = 3;                   // of these read back by warps 0-3
 constexpr int kW1 = 27 * 2 * 4 * 128;       // K 16 (3 used), N 32
 constexpr int kW2 = 27 * 4 * 4 * 128;       // K 32, N 32
 constexpr int kW3 = 27 * 4 * 2 * 128;       // K 32, N 16 (3 used)
 constexpr int kWBytes = kW1 + kW2 + kW3;    // 110,592
 constexpr int kSmem = kActBytes + kWBytes + 64;
-constexpr int kTmemCols = 256;             // kMyTiles x 32 columns
+constexpr int kThreads = 256;
+constexpr int kTmemCols = 256;              // kMine x 32 columns, a power of two
 constexpr uint32_t kWait = 1u << 24;
 
 // shared-memory matrix descriptor: no swizzle, K-major
@@ -88,6 +103,10 @@ __device__ __forceinline__ void fence_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+__device__ __forceinline__ void fence_async_cluster() {
+  asm volatile("fence.proxy.async;" ::: "memory");
+}
+
 // 16 consecutive accumulator columns of this warp's 32 lanes; the registers are
 // valid only after tmem_wait() and reg_fence16()
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t r[16]) {
@@ -109,11 +128,6 @@ __device__ __forceinline__ void reg_fence16(uint32_t r[16]) {
                  "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]));
 }
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
 // shared::cluster address of the same offset in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t peer_addr(uint32_t saddr, uint32_t rank) {
   uint32_t r;
@@ -125,9 +139,15 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint4 v) {
                "r"(v.z), "r"(v.w)
                : "memory");
 }
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::
-                   : "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
@@ -135,12 +155,65 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-__device__ __forceinline__ bool interior(int p, int& i, int& j, int& k) {
-  const int pz = p / 144, py = (p / 12) % 12, px = p % 12;
-  i = px - 1;
-  j = py - 1;
-  k = pz - 1;
-  return px >= 1 && px <= 10 && py >= 1 && py <= 10 && pz >= 1 && pz <= 10;
+__device__ __forceinline__ int act_row(int i, int j, int k) { return kLead + 128 * i + 11 * k + j; }
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.b32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
+}
+
+// The MMAs of one half of layer L (0: input planes u < 4, and the first of every
+// sum; 1: u = 4, 5).  Called by a converged warp.
+template <int L>
+__device__ __forceinline__ void issue_half(int half, int rank, uint32_t act_s, uint32_t w_s, uint32_t tmem,
+                                           uint64_t* bar) {
+  constexpr int N1 = L < 2 ? 32 : 16;   // accumulator columns per plane
+  constexpr int G1 = N1 / 8;
+  constexpr int KS = L == 0 ? 1 : 2;    // K steps of 16 channels
+  const bool el = elect_one();
+  const int p0 = rank * kMine;
+  // 18 bits of the shared address: in a cluster the rest holds the CTA's rank
+  const uint32_t act = act_s & 0x3FFFFu;
+  const uint32_t wb = (w_s & 0x3FFFFu) + (L == 0 ? 0 : (L == 1 ? kW1 : kW1 + kW2));
+  const uint64_t adesc0 = sdesc(0, kPlane, 128), bdesc0 = sdesc(0, 3 * G1 * 128, 128);
+  // input plane x of (dy, dz) t and K step ks into the cnt output planes from lo on
+  auto mma = [&](int t, int ks, int x, int lo, int cnt, bool acc) {
+    const int off = t % 3 - 1 + 11 * (t / 3 - 1);
+    const uint32_t a = act + (uint32_t)(2 * ks * kPlane + (kLead + 128 * x + off) * 16);
+    const uint32_t b = wb + (uint32_t)(((t * 2 * KS + 2 * ks) * 3 + lo - (x - 1)) * G1 * 128);
+    if (el)
+      mma_bf16(tmem + (uint32_t)((lo - p0) * N1), adesc0 | (uint64_t)(a >> 4), bdesc0 | (uint64_t)(b >> 4),
+               idesc_bf16(cnt * N1), acc);
+  };
+  const int u0 = half ? 4 : 0, u1 = half ? 6 : 4;
+  if (!half) {
+#pragma unroll
+    for (int u = 0; u < kMine; u++) {
+      const int x = rank ? 9 - u : u;
+      mma(0, 0, x, x, 1, false);
+    }
+  }
+#pragma unroll
+  for (int u = u0; u < u1; u++) {
+    const int x = rank ? 9 - u : u;
+    if (x - 1 >= p0 && x - 1 < p0 + kMine) mma(0, 0, x, x - 1, 1, true);
+    if (x + 1 >= p0 && x + 1 < p0 + kMine) mma(0, 0, x, x + 1, 1, true);
+  }
+#pragma unroll 3
+  for (int t = 0; t < 9; t++)
+#pragma unroll
+    for (int ks = 0; ks < KS; ks++) {
+      if (t == 0 && ks == 0) continue;
+#pragma unroll
+      for (int u = u0; u < u1; u++) {
+        const int x = rank ? 9 - u : u;
+        const int lo = max(x - 1, p0);
+        const int cnt = u == 0 || u == 4 ? 2 : (u == 5 ? 1 : 3);
+        mma(t, ks, x, lo, cnt, true);
+      }
+    }
+  if (el) mma_commit(bar);
 }
 
 // Inputs/outputs: samples mode (x[S][1000][3] -> y[S][1000][3], owned voxels)
@@ -160,28 +233,57 @@ struct MeshIO {
   double* z;
 };
 
-__global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(128, 1)
+__global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kThreads, 1)
     k_precond_tc(const float* __restrict__ x, float* __restrict__ y,
                  const uint16_t* __restrict__ wimg, unsigned long long* __restrict__ flags,
                  MeshIO mesh) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* act = smem;
   uint8_t* wsm = smem + kActBytes;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kActBytes + kWBytes);  // [0] mma, [1] weights
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kActBytes + kWBytes);  // [0], [1] MMA halves, [2] weights
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 3);
   const int s = blockIdx.x / kSplit;
-  const uint32_t rank = cluster_rank(), peer = rank ^ 1u;
-  const int tile0 = (int)rank * kMyTiles;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = (int)(blockIdx.x % kSplit);  // the rank in the cluster
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform, as the issue loop wants it
 
   if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
+    for (int q = 0; q < 3; q++) mbar_init(&bar[q], 1);
     fence_mbar_init();
+    const int wset = (mesh.v && mesh.set) ? mesh.set[s] : 0;
+    mbar_arrive_expect_tx(&bar[2], kWBytes);
+    bulk_copy_g2s(wsm, wimg + (size_t)wset * (kWBytes / 2), kWBytes, &bar[2]);
   }
-  // zero the activation planes (the ring and the unused input channels stay zero)
-  for (int q = tid; q < kActBytes / 16; q += blockDim.x)
+  // layer-1 input, channels 0..2 of channel plane 0: on its way while the planes are
+  // zeroed
+  constexpr int kPer = (1000 + kThreads - 1) / kThreads;
+  const float* xs = x + (size_t)s * 1000 * 3;
+  float xv[kPer][3];
+#pragma unroll
+  for (int q = 0; q < kPer; q++) {
+    const int v = tid + q * kThreads;
+#pragma unroll
+    for (int ch = 0; ch < 3; ch++) xv[q][ch] = 0.f;
+    if (v < 1000) {
+      if (mesh.v) {
+        const int id = mesh.in_map[(size_t)s * 1000 + v];
+#pragma unroll
+        for (int ch = 0; ch < 3; ch++)
+          xv[q][ch] = (float)pc_input(id, ch, mesh.nvc, mesh.v, mesh.dinv, mesh.hs, mesh.hp, mesh.hw);
+      } else {
+#pragma unroll
+        for (int ch = 0; ch < 3; ch++) xv[q][ch] = __ldg(xs + 3 * v + ch);
+      }
+    }
+  }
+  // zero the channel planes of the first layer, and of the others the rows before
+  // planes 0 and 4, the lowest of the two CTAs (the lower ring); the rest is written
+  // before it is read for a voxel of R
+  for (int q = tid; q < 2 * kRows; q += kThreads)
     reinterpret_cast<uint4*>(act)[q] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid < 4 * kLead)
+    reinterpret_cast<uint4*>(act)[(2 + tid / kLead % 2) * kRows + tid / (2 * kLead) * 4 * 128 + tid % kLead] =
+        make_uint4(0u, 0u, 0u, 0u);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tslot)),
@@ -190,136 +292,94 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(128, 1)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   __syncthreads();
-  if (tid == 0) {
-    const int wset = (mesh.v && mesh.set) ? mesh.set[s] : 0;
-    mbar_arrive_expect_tx(&bar[1], kWBytes);
-    bulk_copy_g2s(wsm, wimg + (size_t)wset * (kWBytes / 2), kWBytes, &bar[1]);
+#pragma unroll
+  for (int q = 0; q < kPer; q++) {
+    const int v = tid + q * kThreads;
+    if (v < 1000)
+      *reinterpret_cast<uint4*>(act + (size_t)act_row(v % 10, (v / 10) % 10, v / 100) * 16) =
+          make_uint4(pack_bf16(xv[q][0], xv[q][1]), pack_bf16(xv[q][2], 0.f), 0u, 0u);
   }
-  // layer-1 input: channels 0..2 of plane 0
-  const float* xs = x + (size_t)s * 1000 * 3;
-  {
-    constexpr int kPer = (1000 + 127) / 128;
-    float xv[kPer][3];
-#pragma unroll
-    for (int q = 0; q < kPer; q++) {
-      const int v = tid + q * 128;
-#pragma unroll
-      for (int ch = 0; ch < 3; ch++) xv[q][ch] = 0.f;
-      if (v < 1000) {
-        if (mesh.v) {
-          const int id = mesh.in_map[(size_t)s * 1000 + v];
-#pragma unroll
-          for (int ch = 0; ch < 3; ch++)
-            xv[q][ch] = (float)pc_input(id, ch, mesh.nvc, mesh.v, mesh.dinv, mesh.hs, mesh.hp, mesh.hw);
-        } else {
-#pragma unroll
-          for (int ch = 0; ch < 3; ch++) xv[q][ch] = __ldg(xs + 3 * v + ch);
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < kPer; q++) {
-      const int v = tid + q * 128;
-      if (v < 1000) {
-        const int i = v % 10, j = (v / 10) % 10, k = v / 100;
-        const int p = (k + 1) * 144 + (j + 1) * 12 + (i + 1);
-        uint4 w4;
-        w4.x = pack_bf16(xv[q][0], xv[q][1]);
-        w4.y = pack_bf16(xv[q][2], 0.f);
-        w4.z = 0u;
-        w4.w = 0u;
-        *reinterpret_cast<uint4*>(act + (size_t)p * 16) = w4;
-      }
-    }
-  }
-  // both CTAs' buffers are initialised before either writes into the other's
-  cluster_sync();
   fence_async_smem();
-  __syncthreads();
-  // CTA-uniform status: the warp-collective tcgen05.ld below needs it
-  bool ok = __syncthreads_and(mbar_wait_bounded(&bar[1], 0, kWait)) != 0;
-  tc_fence_after();
+  // CTA-uniform status: the warp-collective tcgen05 calls below need it
+  bool ok = __syncthreads_and(mbar_wait_bounded(&bar[2], 0, kWait)) != 0;
   const uint32_t tmem = *tslot;
   const uint32_t act_s = smem_u32(act), w_s = smem_u32(wsm);
-  const uint32_t act_peer = peer_addr(act_s, peer);
-  uint32_t mma_phase = 0;
-  bool mma_pending = false;
+  const uint32_t act_peer = peer_addr(act_s, (uint32_t)rank ^ 1u);
+  // rows of this thread: row o of the planes u = u0 .. u0 + nu - 1
+  const int half = warp >> 2, u0 = half ? kFirst : 0, nu = half ? kMine - kFirst : kFirst;
+  const int o = (warp & 3) * 32 + lane, k = o / 11, j = o % 11;
+  const bool in = o < 110 && j < 10;
+  uint4 keep[4];
+  int issued = -1;  // the last layer with MMAs on their way
 
   for (int L = 0; L < 3; L++) {
-    const int N = L < 2 ? 32 : 16;
-    const int NQ = L == 0 ? 2 : 4;  // 8-channel K chunks
-    const int NG = N / 8;
-    const uint32_t wbase = w_s + (L == 0 ? 0 : (L == 1 ? kW1 : kW1 + kW2));
-    if (ok && tid == 0) {
-      // taps outer, tiles inner: consecutive MMAs write different accumulators
-      const uint32_t id = idesc_bf16(N);
-      const uint64_t adesc0 = sdesc(0, kPlane, 128);
-      const uint64_t bdesc0 = sdesc(0, (uint32_t)NG * 128u, 128);
-      int off = -157;  // tap (-1,-1,-1)
-      for (int t = 0; t < 27; t++) {
-        for (int ks = 0; ks < NQ / 2; ks++) {
-          const uint64_t bd = bdesc0 | (uint64_t)(((wbase + (uint32_t)((t * NQ + 2 * ks) * NG) * 128u) >> 4) & 0x3FFFu);
-          uint32_t a_addr =
-              act_s + (uint32_t)(2 * ks) * kPlane + (uint32_t)(kMBegin + tile0 * 128 + off) * 16u;
-          const uint32_t acc = (t | ks) != 0 ? 1u : 0u;
-#pragma unroll 3
-          for (int tile = 0; tile < kMyTiles; tile++) {
-            const uint64_t ad = adesc0 | (uint64_t)((a_addr >> 4) & 0x3FFFu);
-            mma_bf16(tmem + (uint32_t)(tile * N), ad, bd, id, acc);
-            a_addr += 128u * 16u;
-          }
-        }
-        // next tap: x fastest, then y, then z
-        off += 1;
-        if (t % 3 == 2) off += 12 - 3;
-        if (t % 9 == 8) off += 144 - 36;
-      }
-      mma_commit(&bar[0]);
-    }
-    mma_pending = ok;
-    __syncwarp();
-    if (mma_pending) {
-      ok = __syncthreads_and(mbar_wait_bounded(&bar[0], mma_phase, kWait)) != 0;
-      if (ok) {
-        mma_phase ^= 1u;
-        mma_pending = false;
-      }
-    }
     tc_fence_after();
-    // epilogue: groups of tiles whose accumulator loads share one wait
-    constexpr int kGroup = 3;
-    for (int t0 = 0; t0 < kMyTiles && ok; t0 += kGroup) {
-      uint32_t r[kGroup][2][16];
+    if (warp == 0 && ok) {
+      if (L == 0) issue_half<0>(0, rank, act_s, w_s, tmem, &bar[0]);
+      if (L == 1) issue_half<1>(0, rank, act_s, w_s, tmem, &bar[0]);
+      if (L == 2) issue_half<2>(0, rank, act_s, w_s, tmem, &bar[0]);
+    }
+    uint32_t r[kFirst][2][16];
+    if (L > 0) {
+      // the peer's MMAs of the layer before have read its plane u = 5: this CTA's
+      // plane u = 4 goes there
+      cluster_wait();
+      if (half && ok) {
+        const uint32_t dst = act_peer + (uint32_t)act_row(rank ? 5 : 4, 0, 0) * 16u + (uint32_t)o * 16u;
 #pragma unroll
-      for (int g = 0; g < kGroup; g++) {
-        const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((t0 + g) * N);
+        for (int q = 0; q < 4; q++)
+          st_cluster_v4(dst + (uint32_t)q * kPlane, keep[q]);
+      }
+      fence_async_cluster();
+      cluster_sync();
+    }
+    if (warp == 0 && ok) {
+      fence_async_smem();
+      if (L == 0) issue_half<0>(1, rank, act_s, w_s, tmem, &bar[1]);
+      if (L == 1) issue_half<1>(1, rank, act_s, w_s, tmem, &bar[1]);
+      if (L == 2) issue_half<2>(1, rank, act_s, w_s, tmem, &bar[1]);
+    }
+    __syncwarp();
+    if (ok) issued = L;
+    // the accumulators (warp-uniform: tcgen05.ld is a warp's)
+    bool mine = false;
+    if (ok) mine = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[half], L & 1, kWait)) != 0;
+    tc_fence_after();
+    if (mine) {
+#pragma unroll
+      for (int g = 0; g < kFirst; g++) {
+        if (g >= nu) break;
+        const int N1 = L < 2 ? 32 : 16;
+        const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) +
+                            (uint32_t)((rank ? kMine - 1 - (u0 + g) : u0 + g) * N1);
         tmem_ld16(ta, r[g][0]);
         if (L < 2) tmem_ld16(ta + 16, r[g][1]);
       }
       tmem_wait();
 #pragma unroll
-      for (int g = 0; g < kGroup; g++) {
+      for (int g = 0; g < kFirst; g++) {
         reg_fence16(r[g][0]);
-        if (L < 2) reg_fence16(r[g][1]);
-        const int m = kMBegin + (tile0 + t0 + g) * 128 + warp * 32 + lane;
-        int i, j, k;
-        const bool in = m < kPadV && interior(m, i, j, k);
-        if (L < 2) {
-          if (m < kPadV) {
+        reg_fence16(r[g][1]);
+      }
+      tc_fence_before();
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-              const uint32_t* src = r[g][q >> 1] + 8 * (q & 1);
-              uint4 w4 = make_uint4(0u, 0u, 0u, 0u);
-              if (in) {
-                w4.x = pack_bf16(__uint_as_float(src[0]), __uint_as_float(src[1]));
-                w4.y = pack_bf16(__uint_as_float(src[2]), __uint_as_float(src[3]));
-                w4.z = pack_bf16(__uint_as_float(src[4]), __uint_as_float(src[5]));
-                w4.w = pack_bf16(__uint_as_float(src[6]), __uint_as_float(src[7]));
-              }
-              const uint32_t off_b = (uint32_t)q * kPlane + (uint32_t)m * 16u;
-              *reinterpret_cast<uint4*>(act + off_b) = w4;
-              st_cluster_v4(act_peer + off_b, w4);
+      for (int g = 0; g < kFirst; g++) {
+        if (g >= nu) break;
+        const int i = rank ? 9 - (u0 + g) : u0 + g;
+        if (L < 2) {
+          // the second half reads no row of planes u < 3 that this changes
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const uint32_t* src = r[g][q >> 1] + 8 * (q & 1);
+            uint4 w4 = make_uint4(0u, 0u, 0u, 0u);
+            if (in) {
+              w4.x = pack_bf16(__uint_as_float(src[0]), __uint_as_float(src[1]));
+              w4.y = pack_bf16(__uint_as_float(src[2]), __uint_as_float(src[3]));
+              w4.z = pack_bf16(__uint_as_float(src[4]), __uint_as_float(src[5]));
+              w4.w = pack_bf16(__uint_as_float(src[6]), __uint_as_float(src[7]));
             }
+            if (g == kMine - 1 - kFirst) keep[q] = w4;  // plane u = 4 of warps 4-7
+            *reinterpret_cast<uint4*>(act + (uint32_t)q * kPlane + (uint32_t)(act_row(i, 0, 0) + o) * 16u) = w4;
           }
         } else if (in && i >= 1 && i <= 8 && j >= 1 && j <= 8 && k >= 1 && k <= 8) {
           if (mesh.v) {
@@ -340,18 +400,22 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(128, 1)
         }
       }
     }
-    tc_fence_before();
-    // the peer's rows of this layer have landed in this CTA's buffer
-    cluster_sync();
+    if (L == 2) {
+      if (!mine) ok = false;
+      break;
+    }
+    // the rows of the next layer are written, this layer's MMAs have read theirs
     fence_async_smem();
-    __syncthreads();
-    tc_fence_after();
+    if (ok) ok = __syncthreads_and(mine) != 0;
+    cluster_arrive();
   }
+  ok = __syncthreads_and(ok) != 0;
   if (!ok) {
     if (tid == 0) atomicAdd(flags + 2, 1ull);
     // let outstanding MMAs and the weight copy finish before releasing memory
-    if (mma_pending) mbar_wait_bounded(&bar[0], mma_phase, kWait);
-    mbar_wait_bounded(&bar[1], 0, kWait);
+    if (issued >= 0)
+      for (int g = 0; g < 2; g++) mbar_wait_bounded(&bar[g], issued & 1, kWait);
+    mbar_wait_bounded(&bar[2], 0, kWait);
   }
   tc_fence_before();
   __syncthreads();
@@ -362,25 +426,26 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(128, 1)
   }
 }
 
-// BF16 operand images of the FP32 weights: layer L, tap t, K chunk q, N group g:
-// core matrix of 8 rows (n = 8g + r) x 8 K elements (k = 8q + e), 128 bytes.
+// BF16 operand images of the FP32 weights: layer, (dy, dz), K chunk q, dx (+1, 0,
+// -1), N group g: core matrix of 8 rows (n = 8g + r) x 8 K elements (k = 8q + e),
+// 128 bytes.
 __global__ void k_pack_wtc(const float* __restrict__ w1, const float* __restrict__ w2,
                            const float* __restrict__ w3, uint16_t* __restrict__ img) {
   const int total = kWBytes / 2;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
-    int byte = q * 2, L, cin, cout, NQ, NG;
+    int byte = q * 2, cin, cout, NQ, NG;
     const float* W;
     if (byte < kW1) {
-      L = 0; W = w1; cin = 3; cout = 32; NQ = 2; NG = 4;
+      W = w1; cin = 3; cout = 32; NQ = 2; NG = 4;
     } else if (byte < kW1 + kW2) {
-      L = 1; W = w2; cin = 32; cout = 32; NQ = 4; NG = 4; byte -= kW1;
+      W = w2; cin = 32; cout = 32; NQ = 4; NG = 4; byte -= kW1;
     } else {
-      L = 2; W = w3; cin = 32; cout = 3; NQ = 4; NG = 2; byte -= kW1 + kW2;
+      W = w3; cin = 32; cout = 3; NQ = 4; NG = 2; byte -= kW1 + kW2;
     }
-    (void)L;
     const int core = byte / 128, within = byte % 128;
     const int r = within / 16, e = (within % 16) / 2;
-    const int g = core % NG, tq = core / NG, qq = tq % NQ, t = tq / NQ;
+    const int g = core % NG, sl = core / NG % 3, tq = core / (3 * NG), qq = tq % NQ;
+    const int t = tq / NQ * 3 + 2 - sl;  // taps count dx fastest
     const int n = 8 * g + r, k = 8 * qq + e;
     const float v = (k < cin && n < cout) ? W[((size_t)t * cin + k) * cout + n] : 0.f;
     const __nv_bfloat16 h = __float2bfloat16_rn(v);
@@ -420,8 +485,8 @@ cudaError_t precond_forward_tc(PrecondState* P, cudaStream_t st, int S, const fl
   cudaError_t e = set_tc_attr();
   if (e != cudaSuccess) return e;
   MeshIO none{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr};
-  k_precond_tc<<<S * kSplit, 128, kSmem, st>>>(x, y, P->wtc + (size_t)P->active * (kWBytes / 2),
-                                               P->flags, none);
+  k_precond_tc<<<S * kSplit, kThreads, kSmem, st>>>(x, y, P->wtc + (size_t)P->active * (kWBytes / 2),
+                                                    P->flags, none);
   return cudaGetLastError();
 }
 
@@ -433,6 +498,6 @@ cudaError_t precond_apply_tc_mesh(PrecondState* P, cudaStream_t st, int nb, cons
   cudaError_t e = set_tc_attr();
   if (e != cudaSuccess) return e;
   MeshIO io{v, dinv, in_map, hs, hp, hw, out_map, set, nvc, z};
-  k_precond_tc<<<nb * kSplit, 128, kSmem, st>>>(nullptr, nullptr, P->wtc, P->flags, io);
+  k_precond_tc<<<nb * kSplit, kThreads, kSmem, st>>>(nullptr, nullptr, P->wtc, P->flags, io);
   return cudaGetLastError();
 }

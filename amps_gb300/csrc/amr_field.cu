@@ -10,8 +10,8 @@
 // edge off its corner lattice are hanging: they take the interpolation of the
 // coarse corners (P), contributions to them are scattered to the parents (P^T),
 // and their rows read x_h - (P x)_h = 0.  On a uniform mesh this is the
-// reference operator times V.  One thread per cell, FP64 atomics for the
-// scatter to the (up to 8) cells sharing a corner.
+// reference operator times V.  Tiles of cells, atomics for the scatter to the (up
+// to 8) cells sharing a corner.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -61,40 +61,6 @@ __device__ __forceinline__ double cval(const double* __restrict__ F, const doubl
   return v;
 }
 
-// corner c, component d of a field given as FP32 pairs (xh + xl), P applied in pairs
-__device__ __forceinline__ FF cval_ff(const float* __restrict__ xh, const float* __restrict__ xl,
-                                     long long nvc, int c, int d, const Hang& h) {
-  const FF v0{xh[d * nvc + c], xl[d * nvc + c]};
-  const int s = h.hs[c], e = h.hs[c + 1];
-  if (s == e) return v0;
-  FF v{0.f, 0.f};
-  for (int t = s; t < e; t++) {
-    const long long q = d * nvc + h.hp[t];
-    ff_add2(v, h.hwh[t], h.hwl[t], xh[q], xl[q]);
-  }
-  return ff_norm(v);
-}
-
-// scatter out[8][3] to the cell's corners with P^T
-template <typename T>
-__device__ __forceinline__ void scatter(T* __restrict__ y, long long nvc, const int cid[8],
-                                        const T out[8][3], const Hang& h) {
-#pragma unroll
-  for (int c = 0; c < 8; c++) {
-    const int cc = cid[c], s = h.hs[cc], e = h.hs[cc + 1];
-    if (s == e) {
-#pragma unroll
-      for (int d = 0; d < 3; d++) atomicAdd(y + d * nvc + cc, out[c][d]);
-    } else {
-      for (int t = s; t < e; t++) {
-        const T w = (T)h.hw[t];
-#pragma unroll
-        for (int d = 0; d < 3; d++) atomicAdd(y + d * nvc + h.hp[t], w * out[c][d]);
-      }
-    }
-  }
-}
-
 template <typename T>
 __device__ __forceinline__ void cell_curl(const T e[8][3], T q, T cu[3]) {
   T a = 0, b = 0, c = 0, d = 0, f = 0, g = 0;
@@ -115,21 +81,6 @@ __device__ __forceinline__ void cell_curl(const T e[8][3], T q, T cu[3]) {
   cu[2] = q * (f - g);
 }
 
-// out += s C^T y  (C with the 1/(4 dx) factor folded into s)
-template <typename T>
-__device__ __forceinline__ void cell_curl_t(const T y[3], T s, T out[8][3]) {
-  const T a0 = s * y[0], a1 = s * y[1], a2 = s * y[2];
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const bool px = k == 1 || k == 2 || k == 5 || k == 6;
-    const bool py = k == 2 || k == 3 || k == 6 || k == 7;
-    const bool pz = k >= 4;
-    out[k][0] += (pz ? a1 : -a1) - (py ? a2 : -a2);
-    out[k][1] += (px ? a2 : -a2) - (pz ? a0 : -a0);
-    out[k][2] += (py ? a0 : -a0) - (px ? a1 : -a1);
-  }
-}
-
 // out[k] += component p of s C^T y on the 8 corners
 template <typename T>
 __device__ __forceinline__ void cell_curl_t_row(const T y[3], T s, int p, T out[8]) {
@@ -142,21 +93,6 @@ __device__ __forceinline__ void cell_curl_t_row(const T y[3], T s, int p, T out[
     if (p == 0) out[k] += (pz ? a1 : -a1) - (py ? a2 : -a2);
     else if (p == 1) out[k] += (px ? a2 : -a2) - (pz ? a0 : -a0);
     else out[k] += (py ? a0 : -a0) - (px ? a1 : -a1);
-  }
-}
-
-// scatter component p of out[8] to the cell's corners with P^T
-template <typename T>
-__device__ __forceinline__ void scatter_row(T* __restrict__ y, long long nvc, const int cid[8], int p,
-                                            const T out[8], const Hang& h) {
-#pragma unroll
-  for (int c = 0; c < 8; c++) {
-    const int cc = cid[c], s = h.hs[cc], e = h.hs[cc + 1];
-    if (s == e) {
-      atomicAdd(y + p * nvc + cc, out[c]);
-    } else {
-      for (int t = s; t < e; t++) atomicAdd(y + p * nvc + h.hp[t], (T)h.hw[t] * out[c]);
-    }
   }
 }
 
@@ -187,6 +123,7 @@ struct ApplyArgs {
   const double* Bcen;  // RHS: centre B (component-major over cells)
   double th2dt2, f, thdt;
   unsigned long long* flags;  // [2]: bounded-wait timeouts
+  int* next;                  // tiles handed out beyond the first two per CTA
 };
 
 // ---------------------------------------------------------------------------
@@ -338,189 +275,294 @@ __global__ void __launch_bounds__(kTileThreads) k_amr_tile32(ApplyArgs a, int ti
   }
 }
 
-// The operator (ACC 1) and the RHS (ACC 2) to FP64 accuracy, one tile per CTA,
-// in FP32 pairs (FF, common.cuh): FP64 arithmetic is a small fraction of the
-// FP32 rate on this part; the pairs carry FP64 accuracy.  The tile's partials
-// come by one bulk copy while the threads gather the corner values (each value
-// once, shared through shared memory).
+// Two FP32 pairs side by side (FF in each half of the registers): packed
+// instructions halve the issue slots of the error-free sums.
+struct FF2 {
+  unsigned long long s, q;
+};
+__device__ __forceinline__ unsigned long long pk(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 upk(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
+                                                   unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// a += m (xh + xl) in both halves, m exact in FP32, nm = -m: the steps of ff_add
+__device__ __forceinline__ void ff2_add(FF2& a, unsigned long long m, unsigned long long nm,
+                                        unsigned long long xh, unsigned long long xl) {
+  const unsigned long long ph = mul2(m, xh);
+  const unsigned long long npl = fma2(nm, xl, fma2(nm, xh, ph));
+  const unsigned long long t = add2(a.s, ph);
+  const unsigned long long bp = sub2(t, a.s);
+  const unsigned long long err = add2(sub2(a.s, sub2(t, bp)), sub2(ph, bp));
+  a.s = t;
+  a.q = add2(a.q, sub2(err, npl));
+}
+
+// The operator (ACC 1) and the RHS (ACC 2) to FP64 accuracy in FP32 pairs (FF,
+// common.cuh): FP64 arithmetic is a small fraction of the FP32 rate on this part;
+// the pairs carry FP64 accuracy.  Bound: issue and the FP32 pipe (192 error-free
+// products of 11 operations per cell and component).  Persistent CTAs as in
+// k_amr_tile32 (the next tile's partials, for the RHS also its currents, and its
+// corner values are in flight while one is computed), on tiles of 16 cells (8 x 2
+// x 1, 9 x 3 x 2 corners): six small CTAs per SM hide each other's barriers, which
+// cost three of twice the size half their time.  Tiles are claimed one by one: those
+// with hanging corners take longer, and a fixed share per CTA left a fifth of the
+// warps idle towards the end (216 us; k_amr_tile32, which waits for memory anyway,
+// gains nothing by it); the kernel launched after this one clears the counter.  A
+// warp takes one component, a lane one cell's corners of y = 0 or of y = 1; two
+// z-neighbours of a corner column share packed instructions: with M_a the monomial
+// block of z-sum a, both sums take e(z=0) times (M_0, M_1) and e(z=1) times (M_1,
+// M_2).  The cells' sums for a corner are added in pairs by shuffles, and one FP64
+// reduction per tile corner and component goes out (from shared memory: in full
+// warps, as the conversion is FP64 too).  491,520 cells: 191 us (32-cell tiles 230;
+// one tile per CTA, scalar pairs and values gathered per cell: 345).
+constexpr int kFFCells = 16;
+constexpr int kFFCorners = 54;                            // (i, j, k) at i + 9 (j + 3 k)
+constexpr uint32_t kFFBytes = kFFCells * AMPS_CELLM * 4;  // 15,552
+constexpr uint32_t kFFJBytes = kFFCells * 24 * 4;
 template <int ACC>
-__global__ void __launch_bounds__(kTileThreads) k_amr_cell_tile(ApplyArgs a, double* __restrict__ y64) {
-  extern __shared__ __align__(16) float s_m[];
-  __shared__ __align__(8) uint64_t bar;
-  // corner values (8 corners x 3) as pairs
-  __shared__ float s_eh[kTileCells][24];
-  __shared__ float s_el[kTileCells][24];
-  // the cell's curl (and for the RHS its centre B) as pairs, one component per thread
-  __shared__ float s_cu[kTileCells][3][2];
-  __shared__ float s_b[ACC == 2 ? kTileCells : 1][3][2];
-  // the tile corners' sums as pairs, accumulated without atomics: warp p owns
-  // component p, and in round c the 32 cells' corner c are 32 distinct tile
-  // corners
-  __shared__ int s_tcid[kTC];
-  __shared__ float s_ffacc[3][kTC][2];
-  const int tid = threadIdx.x, p = tid / kTileCells, lc = tid % kTileCells;
-  const long long cell0 = (long long)blockIdx.x * kTileCells;
+constexpr uint32_t tile_ff_bytes() { return kFFBytes + (ACC == 2 ? kFFJBytes : 0); }
+template <int ACC>
+__global__ void __launch_bounds__(kTileThreads, ACC == 2 ? 5 : 6) k_amr_tile_ff(ApplyArgs a, int tiles, double* __restrict__ y64) {
+  extern __shared__ __align__(16) float s_m[];  // two tiles of partials (and currents)
+  constexpr uint32_t kBytes = tile_ff_bytes<ACC>();
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ float4 s_x[3][kFFCorners];  // corner values as pairs (h, h, l, l)
+  __shared__ float2 s_cu[3][kFFCells];   // the cell's curl and centre B, a component per warp
+  __shared__ float2 s_b[ACC == 2 ? 3 : 1][kFFCells];
+  __shared__ float2 s_out[3][kFFCorners];
+  const int tid = threadIdx.x, p = tid / 32, lane = tid & 31;
+  const int set = lane / kFFCells, lc = lane % kFFCells;
+  // tiles of this CTA: the first two fixed, then as they are asked for
+  __shared__ int s_next;
+  auto claim = [&] { return 2 * (int)gridDim.x + atomicAdd(a.next, 1); };
   if (tid == 0) {
-    mbar_init(&bar, 1);
+    s_next = claim();
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
     fence_mbar_init();
   }
   __syncthreads();
-  if (tid == 0) {
-    mbar_arrive_expect_tx(&bar, kTileBytes);
-    bulk_copy_g2s(s_m, a.cellM + cell0 * AMPS_CELLM, kTileBytes, &bar);
-  }
-  const long long cell = cell0 + lc;
-  const int b = (int)(cell >> 9), l = (int)(cell & 511);
-  const int i = l & 7, j = (l >> 3) & 7, k = l >> 6;
-  const LevelK& K = a.lk[min(__ffs(a.bscale[b]) - 1, kMaxScale - 1)];
-  // the cell's corners and their values, each gathered once by one of its 3
-  // threads (thread p: corner ids c = p, p+3, p+6; values of component p)
-  // tile-local corner of (cell lc, corner c): the slab's cells are i = 0..7,
-  // 4 rows j, one k
-  auto tcorner = [&](int c) { return (lc % 8 + c_off[c][0]) + 9 * ((lc / 8 + c_off[c][1]) + 5 * c_off[c][2]); };
-  // every thread loads its cell's 8 corner ids (cached table), so the value
-  // gathers below wait on one load, not on a barrier
-  int cid[8];
+  auto copy = [&](int tile, int buf) {
+    mbar_arrive_expect_tx(&bar[buf], kBytes);
+    float* dst = s_m + (size_t)buf * (kBytes / 4);
+    bulk_copy_g2s(dst, a.cellM + (size_t)tile * kFFCells * AMPS_CELLM, kFFBytes, &bar[buf]);
+    if (ACC == 2) bulk_copy_g2s(dst + kFFBytes / 4, a.cellJ + (size_t)tile * kFFCells * 24, kFFJBytes, &bar[buf]);
+  };
+  // thread t < 54 owns tile corner t
+  const int ti = tid % 9, tj = (tid / 9) % 3, tk = tid / 27;
+  auto corner_id = [&](int tile) {
+    if (tile >= tiles || tid >= kFFCorners) return 0;
+    const int b = tile >> 5, l = (tile & 31) * kFFCells;  // 32 tiles per block
+    return __ldg(a.ctabh + b * 729 + ti + 9 * (((l >> 3) & 7) + tj + 9 * ((l >> 6) + tk)));
+  };
+  auto corner_values = [&](int id, FF (&x)[3]) {
+    if (id >= 0) {
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    cid[c] = a.ctab[b * 729 + (i + c_off[c][0]) + 9 * ((j + c_off[c][1]) + 9 * (k + c_off[c][2]))];
-    if (c % 3 == p) s_tcid[tcorner(c)] = cid[c];  // the same id from every cell sharing it
-  }
-  for (int q = tid; q < 3 * kTC; q += kTileThreads) {
-    s_ffacc[q / kTC][q % kTC][0] = 0.f;
-    s_ffacc[q / kTC][q % kTC][1] = 0.f;
-  }
-  if (ACC == 2) {
-    // centre B, component p, split into a pair (the only FP64 arithmetic besides the scatter)
-    const double Bv = a.Bcen[p * a.ncell + cell];
-    const float bh = (float)Bv;
-    s_b[lc][p][0] = bh;
-    s_b[lc][p][1] = (float)(Bv - (double)bh);
-  }
+      for (int d = 0; d < 3; d++) x[d] = FF{a.xh[d * a.nvc + id], a.xl[d * a.nvc + id]};
+    } else {
+      const int h = ~id, s = a.h.hs[h], e = a.h.hs[h + 1];
+      FF v[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+      for (int t = s; t < e; t++) {
+        const float wh = a.h.hwh[t], wl = a.h.hwl[t];
+        const int q = a.h.hp[t];
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    const FF v = cval_ff(a.xh, a.xl, a.nvc, cid[c], p, a.h);
-    s_eh[lc][3 * c + p] = v.s;
-    s_el[lc][3 * c + p] = v.q;
-  }
-  // CTA-uniform: every thread leaves together on a timeout (later barriers)
-  const bool ok = __syncthreads_and(mbar_wait_bounded(&bar, 0, kWaitLimit)) != 0;
-  if (!ok) {
-    if (tid == 0) atomicAdd(a.flags + 2, 1ull);
-    mbar_wait_bounded(&bar, 0, kWaitLimit);  // let the copy land before exiting
-    return;
-  }
-  const float* mm = s_m + lc * AMPS_CELLM + 3 * p;  // row p of every monomial block
-  const float sg = ACC == 2 ? -1.f : 1.f;
-  FF out[8];
+        for (int d = 0; d < 3; d++) ff_add2(v[d], wh, wl, a.xh[d * a.nvc + q], a.xl[d * a.nvc + q]);
+      }
 #pragma unroll
-  for (int c = 0; c < 8; c++)
-    out[c] = ACC == 1 ? ff_mul(s_eh[lc][3 * c + p], s_el[lc][3 * c + p], K.id[0], K.id[1]) : FF{0.f, 0.f};
-  // the curl's component p: cu_p = 0.25/dx (sum +-E_qa - sum +-E_qb)
-  const int qa = p == 0 ? 2 : (p == 1 ? 0 : 1), qb = p == 0 ? 1 : (p == 1 ? 2 : 0);
-  {
-    FF d{0.f, 0.f};
-#pragma unroll
-    for (int k2 = 0; k2 < 8; k2++) {
-      const bool px = k2 == 1 || k2 == 2 || k2 == 5 || k2 == 6;
-      const bool py = k2 == 2 || k2 == 3 || k2 == 6 || k2 == 7;
-      const bool pz = k2 >= 4;
-      // cu0 = (dEz/dy - dEy/dz), cu1 = (dEx/dz - dEz/dx), cu2 = (dEy/dx - dEx/dy)
-      const bool sga = p == 0 ? py : (p == 1 ? pz : px);
-      const bool sgb = p == 0 ? pz : (p == 1 ? px : py);
-      const float ha = s_eh[lc][3 * k2 + qa], la = s_el[lc][3 * k2 + qa];
-      const float hb = s_eh[lc][3 * k2 + qb], lb = s_el[lc][3 * k2 + qb];
-      ff_acc(d, sga ? ha : -ha, sga ? la : -la);
-      ff_acc(d, sgb ? -hb : hb, sgb ? -lb : lb);
-    }
-    d = ff_norm(d);
-    const FF cu = ff_norm(ff_mul(d.s, d.q, K.curl[0], K.curl[1]));
-    s_cu[lc][p][0] = cu.s;
-    s_cu[lc][p][1] = cu.q;
-  }
-  __syncthreads();
-  // out[k] += s (sig1 y[q1] - sig2 y[q2]) for y = the curl (s = sg th2dt2 V 0.25/dx)
-  // and, for the RHS, y = centre B (s = thdt V 0.25/dx): C^T y, component p
-  const int q1 = p == 0 ? 1 : (p == 1 ? 2 : 0), q2 = p == 0 ? 2 : (p == 1 ? 0 : 1);
-  auto curl_t = [&](float (*y)[2], float sh, float sl) {
-    FF tpp{y[q1][0], y[q1][1]}, tpm{y[q1][0], y[q1][1]};
-    ff_acc(tpp, -y[q2][0], -y[q2][1]);  // y1 - y2
-    ff_acc(tpm, y[q2][0], y[q2][1]);    // y1 + y2
-    tpp = ff_norm(tpp);
-    tpm = ff_norm(tpm);
-    const FF upp = ff_mul(tpp.s, tpp.q, sh, sl), upm = ff_mul(tpm.s, tpm.q, sh, sl);
-#pragma unroll
-    for (int k2 = 0; k2 < 8; k2++) {
-      const bool px = k2 == 1 || k2 == 2 || k2 == 5 || k2 == 6;
-      const bool py = k2 == 2 || k2 == 3 || k2 == 6 || k2 == 7;
-      const bool pz = k2 >= 4;
-      const bool s1 = p == 0 ? pz : (p == 1 ? px : py);
-      const bool s2 = p == 0 ? py : (p == 1 ? pz : px);
-      // s1 y1 - s2 y2: (+,+) y1 - y2, (+,-) y1 + y2, (-,+) -(y1 + y2), (-,-) -(y1 - y2)
-      const FF& u = (s1 == s2) ? upp : upm;
-      const float sgn = s1 ? 1.f : -1.f;
-      ff_acc(out[k2], sgn * u.s, sgn * u.q);
+      for (int d = 0; d < 3; d++) x[d] = ff_norm(v[d]);
     }
   };
-  curl_t(s_cu[lc], sg * K.cc[0], sg * K.cc[1]);
-  // mass term: sum over pairs of m (FP32 partial) x e, in FP32 pairs
-  float eh[8][3], el[8][3];
-  FF acc[8];
+  auto centre = [&](int tile) { return a.Bcen[p * a.ncell + (long long)tile * kFFCells + lc]; };
+  const float sg = ACC == 2 ? -1.f : 1.f;
+  int tile = blockIdx.x, t1 = tile + gridDim.x, t2 = s_next;  // grid <= tiles
+  if (tid == 0) copy(tile, 0);
+  int id = corner_id(tile), id1 = corner_id(t1);
+  FF x[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+  if (tid < kFFCorners) corner_values(id, x);
+  double bc = ACC == 2 && set == 0 ? centre(tile) : 0.0;
+  int n = 0;  // tiles done
+  while (tile < tiles) {
+    const int buf = n & 1;
+    const bool more = t1 < tiles;
+    if (tid == 0 && more) copy(t1, buf ^ 1);
+    const int t3 = tid == 0 && more ? claim() : tiles;
+    if (tid < kFFCorners) {
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    acc[c] = FF{0.f, 0.f};
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      eh[c][d] = s_eh[lc][3 * c + d];
-      el[c][d] = s_el[lc][3 * c + d];
+      for (int d = 0; d < 3; d++) s_x[d][tid] = make_float4(x[d].s, x[d].s, x[d].q, x[d].q);
     }
-  }
+    if (ACC == 2 && set == 0) {
+      const float bh = (float)bc;
+      s_b[p][lc] = make_float2(bh, (float)(bc - (double)bh));
+      if (more) bc = centre(t1);
+    }
+    // in flight over this tile's arithmetic
+    const int id2 = corner_id(t2);
+    if (tid < kFFCorners && more) corner_values(id1, x);
+    const int idc = id;  // this tile's
+    id = id1;
+    id1 = id2;
+    // CTA-uniform: every thread leaves together on a timeout
+    const bool ok = __syncthreads_and(mbar_wait_bounded(&bar[buf], (n >> 1) & 1, kWaitLimit)) != 0;
+    if (!ok) {
+      if (tid == 0) atomicAdd(a.flags + 2, 1ull);
+      // let the copies land before exiting
+      mbar_wait_bounded(&bar[buf], (n >> 1) & 1, kWaitLimit);
+      if (more) mbar_wait_bounded(&bar[buf ^ 1], ((n + 1) >> 1) & 1, kWaitLimit);
+      return;
+    }
+    const LevelK& K = a.lk[min(__ffs(__ldg(a.bscale + (tile >> 5))) - 1, kMaxScale - 1)];
+    const int i = lc & 7, j = lc >> 3;
+    auto tc = [&](int xx, int yy, int zz) { return i + xx + 9 * (j + yy + 3 * zz); };
+    // the curl's component p: cu_p = 0.25/dx (sum +-E_qa - sum +-E_qb), a sum per set:
+    // cu0 = (dEz/dy - dEy/dz), cu1 = (dEx/dz - dEz/dx), cu2 = (dEy/dx - dEx/dy)
+    {
+      const int q = (p + 2 - set) % 3;   // qa = p + 2, qb = p + 1
+      const int ax = (p + 1 + set) % 3;  // the axis of the difference
+      FF d{0.f, 0.f};
 #pragma unroll
-  for (int c1 = 0; c1 < 8; c1++)
+      for (int c = 0; c < 8; c++) {
+        const float4 v = s_x[q][tc(c & 1, (c >> 1) & 1, c >> 2)];
+        const bool plus = (((c >> ax) & 1) != 0) == (set == 0);
+        ff_acc(d, plus ? v.x : -v.x, plus ? v.z : -v.z);
+      }
+      const float ds = __shfl_xor_sync(0xffffffffu, d.s, kFFCells), dq = __shfl_xor_sync(0xffffffffu, d.q, kFFCells);
+      ff_acc(d, ds, dq);
+      d = ff_norm(d);
+      const FF cu = ff_norm(ff_mul(d.s, d.q, K.curl[0], K.curl[1]));
+      if (set == 0) s_cu[p][lc] = make_float2(cu.s, cu.q);
+    }
+    // mass term: sum over pairs of m (FP32 partial) x e, in FP32 pairs; acc[x] holds
+    // the corners x, y = set of the cell's lower (z = 0) and upper face.  Row p of the
+    // monomial blocks, from y-sum `set` on.
+    const float* tm = s_m + (size_t)buf * (kBytes / 4);
+    const float* mm = tm + lc * AMPS_CELLM + 27 * set + 3 * p;
+    FF2 acc[2] = {{0ull, 0ull}, {0ull, 0ull}};
+#pragma unroll 1
+    for (int q = 0; q < 3; q++) {
 #pragma unroll
-    for (int c2 = 0; c2 <= c1; c2++) {
-      const float* m3 = mm + pair_monomial(c1, c2) * 9;
+      for (int y2 = 0; y2 < 2; y2++) {
+        ulonglong2 e[2][2];  // [x][z], (h, h) and (l, l)
 #pragma unroll
-      for (int q = 0; q < 3; q++) {
-        const float m = m3[q];
-        ff_add(acc[c1], m, eh[c2][q], el[c2][q]);
-        if (c1 != c2) ff_add(acc[c2], m, eh[c1][q], el[c1][q]);
+        for (int x2 = 0; x2 < 2; x2++)
+#pragma unroll
+          for (int z2 = 0; z2 < 2; z2++) e[x2][z2] = *reinterpret_cast<const ulonglong2*>(&s_x[q][tc(x2, y2, z2)]);
+#pragma unroll
+        for (int ax = 0; ax < 3; ax++) {
+          const float* m = mm + 9 * (ax + 3 * y2) + q;
+          const float m0 = m[0], m1 = m[81], m2 = m[162];
+          const unsigned long long mA = pk(m0, m1), mB = pk(m1, m2), nA = pk(-m0, -m1), nB = pk(-m1, -m2);
+#pragma unroll
+          for (int x1 = 0; x1 < 2; x1++) {
+            const int x2 = ax - x1;
+            if (x2 < 0 || x2 > 1) continue;
+            ff2_add(acc[x1], mA, nA, e[x2][0].x, e[x2][0].y);
+            ff2_add(acc[x1], mB, nB, e[x2][1].x, e[x2][1].y);
+          }
+        }
       }
     }
+    FF out[2][2];  // [z][x]
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    const FF t = ff_norm(acc[c]);
-    const FF u = ff_mul(t.s, t.q, sg * K.m[0], sg * K.m[1]);
-    ff_acc(out[c], u.s, u.q);
-  }
-  if (ACC == 2) {
-    curl_t(s_b[lc], K.bb[0], K.bb[1]);
-    const float* jj = a.cellJ + cell * 24;
+    for (int z = 0; z < 2; z++)
 #pragma unroll
-    for (int c = 0; c < 8; c++) ff_add2(out[c], -a.fj[0], -a.fj[1], jj[3 * c + p], 0.f);
-  }
-  // sum over the tile's cells per corner, in pairs (round c: corner c of every cell)
+      for (int xx = 0; xx < 2; xx++) {
+        const float2 as = upk(acc[xx].s), aq = upk(acc[xx].q);
+        const FF t = ff_norm(FF{z ? as.y : as.x, z ? aq.y : aq.x});
+        out[z][xx] = ff_mul(t.s, t.q, sg * K.m[0], sg * K.m[1]);
+        if (ACC == 1) {
+          const float4 v = s_x[p][tc(xx, set, z)];
+          ff_add2(out[z][xx], K.id[0], K.id[1], v.x, v.z);
+        } else {
+          // corner (x, y) in the table order (0,0) (1,0) (1,1) (0,1)
+          const int c = 4 * z + (set ? 3 - xx : xx);
+          ff_add2(out[z][xx], -a.fj[0], -a.fj[1], tm[kFFBytes / 4 + lc * 24 + 3 * c + p], 0.f);
+        }
+      }
+    __syncthreads();  // s_cu complete; s_x is not read again
+    // out += s (sig1 y[q1] - sig2 y[q2]) for y = the curl (s = sg th2dt2 V 0.25/dx)
+    // and, for the RHS, y = centre B (s = thdt V 0.25/dx): C^T y, component p
+    const int q1 = (p + 1) % 3, q2 = (p + 2) % 3;
+    auto curl_t = [&](const float2 (*y)[kFFCells], float sh, float sl) {
+      const float2 y1 = y[q1][lc], y2 = y[q2][lc];
+      FF tpp{y1.x, y1.y}, tpm{y1.x, y1.y};
+      ff_acc(tpp, -y2.x, -y2.y);  // y1 - y2
+      ff_acc(tpm, y2.x, y2.y);    // y1 + y2
+      tpp = ff_norm(tpp);
+      tpm = ff_norm(tpm);
+      const FF upp = ff_mul(tpp.s, tpp.q, sh, sl), upm = ff_mul(tpm.s, tpm.q, sh, sl);
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    float* slot = s_ffacc[p][tcorner(c)];
-    FF v{slot[0], slot[1]};
-    ff_acc(v, out[c].s, out[c].q);
-    slot[0] = v.s;
-    slot[1] = v.q;
-    __syncwarp();
-  }
-  __syncthreads();
-  // scatter with P^T: one FP64 atomic per tile corner and component
-  for (int q = tid; q < 3 * kTC; q += kTileThreads) {
-    const int pp = q / kTC, tc = q % kTC, cc = s_tcid[tc];
-    const FF o = ff_norm(FF{s_ffacc[pp][tc][0], s_ffacc[pp][tc][1]});
-    const int hs0 = a.h.hs[cc], hs1 = a.h.hs[cc + 1];
-    if (hs0 == hs1) {
-      atomicAdd(y64 + pp * a.nvc + cc, ff_value(o));
-    } else {
-      for (int t = hs0; t < hs1; t++)
-        atomicAdd(y64 + pp * a.nvc + a.h.hp[t], ff_value(ff_mul(o.s, o.q, a.h.hwh[t], a.h.hwl[t])));
+      for (int z = 0; z < 2; z++)
+#pragma unroll
+        for (int xx = 0; xx < 2; xx++) {
+          const bool s1 = p == 0 ? z : (p == 1 ? xx : set);
+          const bool s2 = p == 0 ? set : (p == 1 ? z : xx);
+          // s1 y1 - s2 y2: (+,+) y1 - y2, (+,-) y1 + y2, (-,+) -(y1 + y2), (-,-) -(y1 - y2)
+          const float us = s1 == s2 ? upp.s : upm.s, uq = s1 == s2 ? upp.q : upm.q;
+          ff_acc(out[z][xx], s1 ? us : -us, s1 ? uq : -uq);
+        }
+    };
+    curl_t(s_cu, sg * K.cc[0], sg * K.cc[1]);
+    if (ACC == 2) curl_t(s_b, K.bb[0], K.bb[1]);
+    // row j + set: the cell's corner and its left neighbour's; row 1 is of both sets
+    auto row = [&](int xx, int z, FF v) {
+      const float rs = __shfl_down_sync(0xffffffffu, v.s, 8), rq = __shfl_down_sync(0xffffffffu, v.q, 8);
+      const bool both = set == 0 && j == 1;  // lanes 8 .. 15; lanes 16 .. 23 hold the rest
+      ff_acc(v, both ? rs : 0.f, both ? rq : 0.f);
+      const FF o = ff_norm(v);
+      if ((xx == 0 || i == 7) && (set == 0 || j == 1)) s_out[p][tc(xx, set, z)] = make_float2(o.s, o.q);
+    };
+#pragma unroll
+    for (int z = 0; z < 2; z++) {
+      const float rs = __shfl_up_sync(0xffffffffu, out[z][1].s, 1), rq = __shfl_up_sync(0xffffffffu, out[z][1].q, 1);
+      ff_acc(out[z][0], i > 0 ? rs : 0.f, i > 0 ? rq : 0.f);
+      row(0, z, out[z][0]);
+      row(1, z, out[z][1]);
     }
+    if (tid == 0) s_next = t3;
+    __syncthreads();  // s_out, s_next complete; this buffer is not read again
+    // scatter with P^T: one FP64 reduction per tile corner and component
+    if (tid < kFFCorners) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        const FF o{s_out[d][tid].x, s_out[d][tid].y};
+        if (idc >= 0) {
+          atomicAdd(y64 + d * a.nvc + idc, ff_value(o));
+        } else {
+          for (int t = a.h.hs[~idc]; t < a.h.hs[~idc + 1]; t++)
+            atomicAdd(y64 + d * a.nvc + a.h.hp[t], ff_value(ff_mul(o.s, o.q, a.h.hwh[t], a.h.hwl[t])));
+        }
+      }
+    }
+    tile = t1;
+    t1 = t2;
+    t2 = s_next;
+    n++;
   }
 }
 
@@ -653,7 +695,9 @@ __global__ void __launch_bounds__(256) k_amr_finish_ff(long long nvc, Hang h, un
 __global__ void __launch_bounds__(256) k_amr_constraint(long long nvc, Hang h,
                                                         const double* __restrict__ x,
                                                         const double* __restrict__ dinv,
-                                                        double* __restrict__ y, int rhs_mode) {
+                                                        double* __restrict__ y, int rhs_mode,
+                                                        int* __restrict__ next) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0;  // for the next tile kernel
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nvc) return;
   int s = h.hs[c], e = h.hs[c + 1];
@@ -935,6 +979,7 @@ static ApplyArgs apply_args(amps_gpu_ctx* c) {
   a.f = 4.0 * kPi * dt * th;
   a.thdt = th * dt;
   a.flags = c->d_flags;
+  a.next = c->d_next;
   a.bscale = c->d_bscale;
   auto split = [](double v, float* o) {
     o[0] = (float)v;
@@ -967,25 +1012,10 @@ static cudaError_t split_input(amps_gpu_ctx* c, const double* x, const double* d
   return cudaGetLastError();
 }
 
-template <int ACC>
-static cudaError_t launch_tile(amps_gpu_ctx* c, const ApplyArgs& a, double* y64) {
-  static unsigned long long attr_set = 0;  // per device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!((attr_set >> dev) & 1ull)) {
-    cudaError_t e = cudaFuncSetAttribute(k_amr_cell_tile<ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTileBytes);
-    if (e != cudaSuccess) return e;
-    attr_set |= 1ull << dev;
-  }
-  // AMR meshes hold whole 512-cell blocks: ncell is a multiple of the tile
-  k_amr_cell_tile<ACC><<<(unsigned)(c->ncor / kTileCells), kTileThreads, kTileBytes, c->stream>>>(a, y64);
-  return cudaGetLastError();
-}
-
-// y32 += the FP32 operator on a.xf
-static cudaError_t launch_tile32(amps_gpu_ctx* c, const ApplyArgs& a, float* y32) {
-  static int grid[64] = {0};  // per device: resident CTAs
+// CTAs of a persistent tile kernel that the device holds at a time (asked once per
+// device and kernel)
+template <typename Kernel>
+static cudaError_t tile_grid(Kernel kernel, uint32_t smem, int (&grid)[64], int& n) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
@@ -993,14 +1023,36 @@ static cudaError_t launch_tile32(amps_gpu_ctx* c, const ApplyArgs& a, float* y32
     int sms = 0, per = 0;
     cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_amr_tile32, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)kTileBytes);
-    if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_amr_tile32, kTileThreads, 2 * kTileBytes);
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kTileThreads, smem);
     if (e != cudaSuccess) return e;
     grid[dev] = sms * std::max(per, 1);
   }
+  n = grid[dev];
+  return cudaSuccess;
+}
+
+// y64 += the operator (ACC 1) or the RHS (ACC 2) in FP32 pairs
+template <int ACC>
+static cudaError_t launch_tile(amps_gpu_ctx* c, const ApplyArgs& a, double* y64) {
+  static int grid[64] = {0};
+  int n = 0;
+  cudaError_t e = tile_grid(k_amr_tile_ff<ACC>, 2 * tile_ff_bytes<ACC>(), grid, n);
+  if (e != cudaSuccess) return e;
+  // AMR meshes hold whole 512-cell blocks: ncell is a multiple of the tile
+  const int tiles = (int)(c->ncor / kFFCells);
+  k_amr_tile_ff<ACC><<<std::min(n, tiles), kTileThreads, 2 * tile_ff_bytes<ACC>(), c->stream>>>(a, tiles, y64);
+  return cudaGetLastError();
+}
+
+// y32 += the FP32 operator on a.xf
+static cudaError_t launch_tile32(amps_gpu_ctx* c, const ApplyArgs& a, float* y32) {
+  static int grid[64] = {0};
+  int n = 0;
+  cudaError_t e = tile_grid(k_amr_tile32, 2 * kTileBytes, grid, n);
+  if (e != cudaSuccess) return e;
   const int tiles = (int)(c->ncor / kTileCells);
-  k_amr_tile32<<<std::min(grid[dev], tiles), kTileThreads, 2 * kTileBytes, c->stream>>>(a, tiles, y32);
+  k_amr_tile32<<<std::min(n, tiles), kTileThreads, 2 * kTileBytes, c->stream>>>(a, tiles, y32);
   return cudaGetLastError();
 }
 
@@ -1013,7 +1065,7 @@ cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* di
   TimedLaunch t(c, "matvec", 3);
   if ((e = split_input(c, x, dinv, a)) != cudaSuccess) return e;
   if ((e = launch_tile<1>(c, a, y)) != cudaSuccess) return e;
-  k_amr_constraint<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, x, dinv, y, 0);
+  k_amr_constraint<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, x, dinv, y, 0, c->d_next);
   return cudaGetLastError();
 }
 
@@ -1046,7 +1098,7 @@ cudaError_t launch_amr_rhs(amps_gpu_ctx* c) {
   TimedLaunch t(c, "rhs", 3);
   if ((e = split_input(c, c->d_En, nullptr, a)) != cudaSuccess) return e;
   if ((e = launch_tile<2>(c, a, c->d_rhs)) != cudaSuccess) return e;
-  k_amr_constraint<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, nullptr, nullptr, c->d_rhs, 1);
+  k_amr_constraint<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, nullptr, nullptr, c->d_rhs, 1, c->d_next);
   return cudaGetLastError();
 }
 

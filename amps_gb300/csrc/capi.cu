@@ -314,7 +314,8 @@ bool alloc_context(amps_gpu_ctx* c) {
        !dalloc(&c->d_Bcor_cur, 3 * nv);
   if (!c->amr) ok = ok && !dalloc(&c->d_J, 3 * nc) && !dalloc(&c->d_M, 243 * nc);
   if (c->amr)
-    ok = ok && !dalloc(&c->d_y32, 3 * nv) &&
+    ok = ok && !dalloc(&c->d_y32, 3 * nv) && !dalloc(&c->d_next, 1) &&
+         cudaMemsetAsync(c->d_next, 0, sizeof(int), c->stream) == cudaSuccess &&
          cudaMemsetAsync(c->d_y32, 0, sizeof(float) * 3 * nv, c->stream) == cudaSuccess;
   ok = ok && !dalloc(&c->d_rhs, 3 * nv) && !dalloc(&c->d_x, 3 * nv) &&
        !dalloc(&c->d_V, (size_t)(c->restart + 1) * ((3 * nv + 3) & ~3LL)) &&
@@ -727,7 +728,7 @@ amps_gpu_status amps_gpu_destroy(amps_gpu_ctx* c) {
   c->d_hstage = nullptr;
   void* ptrs[] = {c->d_nbr, c->d_En, c->d_Eh, c->d_Bc, c->d_Bc2, c->d_Bcor_prev, c->d_Bcor_cur,
                   c->d_J, c->d_M, c->d_rhs, c->d_x, c->d_V, c->d_w, c->d_dinv, c->d_red, c->d_arn, c->d_xs, c->d_step,
-                  c->d_Z, c->d_y32,
+                  c->d_Z, c->d_y32, c->d_next,
                   c->d_stencil_push, c->d_stencil_dep, c->d_stencil_cprev, c->d_stencil_ccur, c->d_key, c->d_rank, c->d_base, c->d_cnt,
                   c->d_arr, c->d_stay, c->d_tmp, c->d_count, c->d_scan_part, c->d_flags,
                   c->d_cellM, c->d_cellJ, c->d_energy, c->d_ctab, c->d_hs, c->d_hp, c->d_hw, c->d_hwh, c->d_hwl,

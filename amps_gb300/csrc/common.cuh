@@ -120,6 +120,7 @@ struct amps_gpu_ctx {
   float* d_dff = nullptr;       // 2n: the Jacobi scaling as FP32 pairs (hi n, lo n)
   double* d_tmpv = nullptr;     // 2n doubles: FP64 copies of Krylov vectors for the
                                 // learned network, its sample harvest and the FP64 inner operator
+  int* d_next = nullptr;        // next tile of the persistent AMR operator in pairs (zero between launches)
   float* d_y32 = nullptr;       // 3*nvc FP32 accumulation of the inner AMR operator (zero between
                                 // applications)
   bool inner_fp32 = true;       // GMRES inner operator in FP32 (iterative refinement)

@@ -101,6 +101,7 @@ __device__ __forceinline__ void cell_curl_t_row(const T y[3], T s, int p, T out[
 // halves)
 struct LevelK {
   float curl[2], cc[2], id[2], m[2], bb[2];  // 0.25/dx, th2dt2 V 0.25/dx, V/8, f V, thdt V 0.25/dx
+  float dg;                                  // V (1/8 + th2dt2 / (8 dx^2)), of the Jacobi diagonal
 };
 constexpr int kMaxScale = 8;
 
@@ -123,6 +124,7 @@ struct ApplyArgs {
   const double* Bcen;  // RHS: centre B (component-major over cells)
   double th2dt2, f, thdt;
   unsigned long long* flags;  // [2]: bounded-wait timeouts
+  double* diag;               // RHS: += the Jacobi diagonal of free corners (null: not wanted)
   int* next;                  // tiles handed out beyond the first two per CTA
 };
 
@@ -339,7 +341,9 @@ __device__ __forceinline__ void ff2_add(FF2& a, unsigned long long m, unsigned l
 // block of z-sum a, both sums take e(z=0) times (M_0, M_1) and e(z=1) times (M_1,
 // M_2).  The cells' sums for a corner are added in pairs by shuffles, and one FP64
 // reduction per tile corner and component goes out (from shared memory: in full
-// warps, as the conversion is FP64 too).  491,520 cells: 191 us (32-cell tiles 230;
+// warps, as the conversion is FP64 too).  The RHS also sums the Jacobi diagonal,
+// whose entries lie in the staged partials (24 us more; a kernel of its own read half
+// of the partials again: 84).  491,520 cells: 191 us (32-cell tiles 230;
 // one tile per CTA, scalar pairs and values gathered per cell: 345).
 constexpr int kFFCells = 16;
 constexpr int kFFCorners = 54;                            // (i, j, k) at i + 9 (j + 3 k)
@@ -356,6 +360,7 @@ __global__ void __launch_bounds__(kTileThreads, ACC == 2 ? 5 : 6) k_amr_tile_ff(
   __shared__ float2 s_cu[3][kFFCells];   // the cell's curl and centre B, a component per warp
   __shared__ float2 s_b[ACC == 2 ? 3 : 1][kFFCells];
   __shared__ float2 s_out[3][kFFCorners];
+  __shared__ float2 s_dg[ACC == 2 ? 3 : 1][kFFCorners];
   const int tid = threadIdx.x, p = tid / 32, lane = tid & 31;
   const int set = lane / kFFCells, lc = lane % kFFCells;
   // tiles of this CTA: the first two fixed, then as they are asked for
@@ -530,24 +535,43 @@ __global__ void __launch_bounds__(kTileThreads, ACC == 2 ? 5 : 6) k_amr_tile_ff(
     curl_t(s_cu, sg * K.cc[0], sg * K.cc[1]);
     if (ACC == 2) curl_t(s_b, K.bb[0], K.bb[1]);
     // row j + set: the cell's corner and its left neighbour's; row 1 is of both sets
-    auto row = [&](int xx, int z, FF v) {
+    auto row = [&](float2 (*dst)[kFFCorners], int xx, int z, FF v) {
       const float rs = __shfl_down_sync(0xffffffffu, v.s, 8), rq = __shfl_down_sync(0xffffffffu, v.q, 8);
       const bool both = set == 0 && j == 1;  // lanes 8 .. 15; lanes 16 .. 23 hold the rest
       ff_acc(v, both ? rs : 0.f, both ? rq : 0.f);
       const FF o = ff_norm(v);
-      if ((xx == 0 || i == 7) && (set == 0 || j == 1)) s_out[p][tc(xx, set, z)] = make_float2(o.s, o.q);
+      if ((xx == 0 || i == 7) && (set == 0 || j == 1)) dst[p][tc(xx, set, z)] = make_float2(o.s, o.q);
     };
+    auto corners = [&](float2 (*dst)[kFFCorners], FF (&v)[2][2]) {
 #pragma unroll
-    for (int z = 0; z < 2; z++) {
-      const float rs = __shfl_up_sync(0xffffffffu, out[z][1].s, 1), rq = __shfl_up_sync(0xffffffffu, out[z][1].q, 1);
-      ff_acc(out[z][0], i > 0 ? rs : 0.f, i > 0 ? rq : 0.f);
-      row(0, z, out[z][0]);
-      row(1, z, out[z][1]);
+      for (int z = 0; z < 2; z++) {
+        const float rs = __shfl_up_sync(0xffffffffu, v[z][1].s, 1), rq = __shfl_up_sync(0xffffffffu, v[z][1].q, 1);
+        ff_acc(v[z][0], i > 0 ? rs : 0.f, i > 0 ? rq : 0.f);
+        row(dst, 0, z, v[z][0]);
+        row(dst, 1, z, v[z][1]);
+      }
+    };
+    corners(s_out, out);
+    if (ACC == 2 && a.diag) {
+      // the cell's diagonal (a preconditioner: FP32 per cell is enough): monomial of a
+      // corner with itself, entry (p, p)
+      FF dg[2][2];
+#pragma unroll
+      for (int z = 0; z < 2; z++)
+#pragma unroll
+        for (int xx = 0; xx < 2; xx++)
+          dg[z][xx] = FF{fmaf(K.m[0], tm[lc * AMPS_CELLM + 9 * (2 * xx + 6 * set + 18 * z) + 4 * p], K.dg), 0.f};
+      corners(s_dg, dg);
     }
     if (tid == 0) s_next = t3;
     __syncthreads();  // s_out, s_next complete; this buffer is not read again
     // scatter with P^T: one FP64 reduction per tile corner and component
     if (tid < kFFCorners) {
+      if (ACC == 2 && a.diag && idc >= 0) {
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+          atomicAdd(a.diag + d * a.nvc + idc, (double)s_dg[d][tid].x + (double)s_dg[d][tid].y);
+      }
 #pragma unroll
       for (int d = 0; d < 3; d++) {
         const FF o{s_out[d][tid].x, s_out[d][tid].y};
@@ -691,15 +715,17 @@ __global__ void __launch_bounds__(256) k_amr_finish_ff(long long nvc, Hang h, un
   }
 }
 
-// hanging rows: y_h = x_h - (P x)_h (operator) or 0 (rhs)
-__global__ void __launch_bounds__(256) k_amr_constraint(long long nvc, Hang h,
-                                                        const double* __restrict__ x,
+// constraint rows (hanging, boundary; rows lists them among others):
+// y_h = x_h - (P x)_h (operator) or 0 (rhs)
+__global__ void __launch_bounds__(256) k_amr_constraint(int nrows, const int* __restrict__ rows, long long nvc,
+                                                        Hang h, const double* __restrict__ x,
                                                         const double* __restrict__ dinv,
                                                         double* __restrict__ y, int rhs_mode,
                                                         int* __restrict__ next) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0;  // for the next tile kernel
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nvc) return;
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t0 >= nrows) return;
+  const int c = rows[t0];
   int s = h.hs[c], e = h.hs[c + 1];
   const int* col = h.hp;
   const double* w = h.hw;
@@ -726,64 +752,67 @@ __global__ void __launch_bounds__(256) k_amr_constraint(long long nvc, Hang h,
   }
 }
 
-// Jacobi diagonal (free corners: sum over their cells of the cell diagonal)
-// Jacobi diagonal (a preconditioner: FP32 arithmetic is enough; per cell size
-// s: base[s] = V (1/8 + th2dt2 / (8 dx^2)), fv[s] = f V)
-struct DiagK {
-  float base[kMaxScale], fv[kMaxScale];
-};
-__global__ void __launch_bounds__(256) k_amr_diag(long long ncell, long long nvc, const int* ctab,
-                                                  Hang h, const int* bscale, const float* cellM, DiagK K,
-                                                  double* diag) {
-  const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (cell >= ncell) return;
-  const int b = (int)(cell >> 9), l = (int)(cell & 511);
-  const int i = l & 7, j = (l >> 3) & 7, k = l >> 6;
-  const int sc = min(__ffs(bscale[b]) - 1, kMaxScale - 1);
-  const float base = K.base[sc], fv = K.fv[sc];
-  const float* mm = cellM + cell * AMPS_CELLM;
-#pragma unroll
-  for (int c = 0; c < 8; c++) {
-    const int cc = ctab[b * 729 + (i + c_off[c][0]) + 9 * ((j + c_off[c][1]) + 9 * (k + c_off[c][2]))];
-    const float* blk = mm + pair_monomial(c, c) * 9;
-    const float m0 = blk[0], m1 = blk[4], m2 = blk[8];
-    if (h.hs[cc + 1] > h.hs[cc]) continue;
-    atomicAdd(diag + cc, (double)fmaf(fv, m0, base));
-    atomicAdd(diag + nvc + cc, (double)fmaf(fv, m1, base));
-    atomicAdd(diag + 2 * nvc + cc, (double)fmaf(fv, m2, base));
-  }
-}
-
-__global__ void __launch_bounds__(256) k_amr_invert_diag(long long nvc, Hang h, double* diag) {
+// 1 / the Jacobi diagonal that the RHS kernel summed
+__global__ void __launch_bounds__(256) k_amr_invert_diag(long long nvc, Hang h, const double* __restrict__ diag,
+                                                         double* __restrict__ dinv) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nvc) return;
   const bool hang = h.hs[c + 1] > h.hs[c] || is_bnd(h, c);  // constraint rows: scaling 1
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     const float v = (float)diag[d * nvc + c];  // a preconditioner: FP32 reciprocal
-    diag[d * nvc + c] = (hang || v == 0.f) ? 1.0 : (double)(1.0f / v);
+    dinv[d * nvc + c] = (hang || v == 0.f) ? 1.0 : (double)(1.0f / v);
   }
 }
 
+// B^{n+1} = B^n - dt curl E^{n+theta}, one CTA per block: each corner value is
+// gathered once into shared memory (hanging ones interpolated there), and the face
+// sums of the curl share their partial sums along the third axis: 24 FP64 additions
+// per cell instead of 42.  FP64 (a 64th of the FP32 rate) and the gathers' latency
+// bound it.  491,520 cells: 49 us (one thread per cell gathering its 8 corners: 85).
 __global__ void __launch_bounds__(256) k_amr_update_b(long long ncell, long long nvc,
-                                                      const int* ctab, Hang h, const double* bdx,
-                                                      const double* Eh, const double* Bn,
-                                                      double* Bnew, double dt) {
-  const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (cell >= ncell) return;
-  const int b = (int)(cell >> 9), l = (int)(cell & 511);
-  const int i = l & 7, j = (l >> 3) & 7, k = l >> 6;
-  double e[8][3];
+                                                      const int* __restrict__ ctabh, Hang h,
+                                                      const double* __restrict__ bdx,
+                                                      const double* __restrict__ Eh,
+                                                      const double* __restrict__ Bn,
+                                                      double* __restrict__ Bnew, double dt) {
+  __shared__ double s_e[3][729];
+  const int b = blockIdx.x;
+  for (int q = threadIdx.x; q < 729; q += 256) {
+    const int id = ctabh[b * 729 + q];
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    const int cc = ctab[b * 729 + (i + c_off[c][0]) + 9 * ((j + c_off[c][1]) + 9 * (k + c_off[c][2]))];
-#pragma unroll
-    for (int d = 0; d < 3; d++) e[c][d] = cval(Eh, nullptr, nvc, cc, d, h);
+    for (int d = 0; d < 3; d++) s_e[d][q] = id >= 0 ? Eh[d * nvc + id] : cval(Eh, nullptr, nvc, ~id, d, h);
   }
-  double cu[3];
-  cell_curl<double>(e, 0.25 / bdx[b], cu);
+  const long long cell0 = (long long)b * AMPS_CPB + threadIdx.x;
+  double B[2][3];
 #pragma unroll
-  for (int d = 0; d < 3; d++) Bnew[d * ncell + cell] = Bn[d * ncell + cell] - dt * cu[d];
+  for (int k = 0; k < 2; k++)
+#pragma unroll
+    for (int d = 0; d < 3; d++) B[k][d] = Bn[d * ncell + cell0 + 256 * k];
+  const double f = dt * 0.25 / bdx[b];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int l = threadIdx.x + 256 * k;
+    const int c0 = (l & 7) + 9 * (((l >> 3) & 7) + 9 * (l >> 6));
+    // diff[d][e]: 4 dx times the mean difference of component d along axis e
+    auto diffs = [&](int d, int sa, int sb, int sc, double& da, double& db) {
+      // sums along the stride sc, then differences along sa and sb
+      const double* e = s_e[d] + c0;
+      const double s00 = e[0] + e[sc], s10 = e[sa] + e[sa + sc];
+      const double s01 = e[sb] + e[sb + sc], s11 = e[sa + sb] + e[sa + sb + sc];
+      const double t1 = s11 - s00, t2 = s10 - s01;
+      da = t1 + t2;
+      db = t1 - t2;
+    };
+    double xy, xz, yx, yz, zx, zy;  // xy: of E_x along y
+    diffs(0, 9, 81, 1, xy, xz);
+    diffs(1, 1, 81, 9, yx, yz);
+    diffs(2, 1, 9, 81, zx, zy);
+    Bnew[cell0 + 256 * k] = B[k][0] - f * (zy - yz);
+    Bnew[ncell + cell0 + 256 * k] = B[k][1] - f * (xz - zx);
+    Bnew[2 * ncell + cell0 + 256 * k] = B[k][2] - f * (yx - xy);
+  }
 }
 
 // UpdateB's boundary branch on meshes with open axes
@@ -837,88 +866,57 @@ __global__ void __launch_bounds__(256) k_amr_bnd_b(long long ncell, const int* _
   for (int q = 0; q < 3; q++) Bnew[q * ncell + cell] = acc[q] / nface;
 }
 
-// C2N: accumulate V*B and V on the corners (P^T for hanging is not used: their
-// value is re-interpolated afterwards)
-__global__ void __launch_bounds__(256) k_amr_c2n_acc(long long ncell, long long nvc,
-                                                     const int* ctab, const double* bdx,
-                                                     const double* Bcen, double* acc,
-                                                     double* wsum) {
-  const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (cell >= ncell) return;
-  const int b = (int)(cell >> 9), l = (int)(cell & 511);
-  const int i = l & 7, j = (l >> 3) & 7, k = l >> 6;
+// C2N, corner B = sum of V B over the corner's cells / sum of V (cinv, the mesh's
+// own), one CTA per block: the block's cells are summed onto its 729 corners axis by
+// axis in shared memory (11 FP64 additions per cell), corners inside the block are
+// written, those on its faces added to the other blocks' shares.  Hanging corners
+// are interpolated afterwards.  491,520 cells: 33 us with the hanging corners (8
+// reductions per cell and component, and the volumes summed again each time: 70).
+__global__ void __launch_bounds__(256) k_amr_c2n(long long ncell, long long nvc,
+                                                 const int* __restrict__ ctab,
+                                                 const double* __restrict__ bdx,
+                                                 const double* __restrict__ cinv,
+                                                 const double* __restrict__ Bcen, double* __restrict__ acc) {
+  __shared__ double s_c[512], s_x[576], s_y[648];
+  const int b = blockIdx.x, tid = threadIdx.x;
   const double dx = bdx[b], V = dx * dx * dx;
-  const double B[3] = {Bcen[cell], Bcen[ncell + cell], Bcen[2 * ncell + cell]};
+  int cc[3];
+  double w[3];
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    const int cc = ctab[b * 729 + (i + c_off[c][0]) + 9 * ((j + c_off[c][1]) + 9 * (k + c_off[c][2]))];
-    atomicAdd(wsum + cc, V);
-#pragma unroll
-    for (int d = 0; d < 3; d++) atomicAdd(acc + d * nvc + cc, V * B[d]);
+  for (int r = 0; r < 3; r++) {
+    const int q = tid + 256 * r;
+    cc[r] = q < 729 ? ctab[b * 729 + q] : 0;
+    w[r] = V * cinv[cc[r]];
   }
-}
-
-__global__ void __launch_bounds__(256) k_amr_c2n_div(long long nvc, const double* wsum,
-                                                     double* acc) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nvc) return;
-  const double w = wsum[c];
-#pragma unroll
-  for (int d = 0; d < 3; d++) acc[d * nvc + c] = w > 0.0 ? acc[d * nvc + c] / w : 0.0;
-}
-
-// hanging corners of a field take the interpolation of their (free) parents
-__global__ void __launch_bounds__(256) k_amr_fix_hanging(long long nvc, Hang h, double* F) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nvc) return;
-  const int s = h.hs[c], e = h.hs[c + 1];
-  if (s == e) return;
-#pragma unroll
   for (int d = 0; d < 3; d++) {
-    double v = 0.0;
-    for (int t = s; t < e; t++) v += h.hw[t] * F[d * nvc + h.hp[t]];
-    F[d * nvc + c] = v;
+#pragma unroll
+    for (int k = 0; k < 2; k++) s_c[tid + 256 * k] = Bcen[d * ncell + (long long)b * AMPS_CPB + tid + 256 * k];
+    __syncthreads();
+    for (int q = tid; q < 576; q += 256) {
+      const int i = q % 9, r = q / 9;  // corner i of row r
+      s_x[q] = (i > 0 ? s_c[8 * r + i - 1] : 0.0) + (i < 8 ? s_c[8 * r + i] : 0.0);
+    }
+    __syncthreads();
+    for (int q = tid; q < 648; q += 256) {
+      const int i = q % 9, j = q / 9 % 9, k = q / 81;
+      s_y[q] = (j > 0 ? s_x[i + 9 * (j - 1 + 8 * k)] : 0.0) + (j < 8 ? s_x[i + 9 * (j + 8 * k)] : 0.0);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const int q = tid + 256 * r;
+      if (q >= 729) break;
+      const int i = q % 9, j = q / 9 % 9, k = q / 81;
+      const double v = w[r] * ((k > 0 ? s_y[q - 81] : 0.0) + (k < 8 ? s_y[q] : 0.0));
+      double* o = acc + d * nvc + cc[r];
+      if (i > 0 && i < 8 && j > 0 && j < 8 && k > 0 && k < 8) *o = v;
+      else atomicAdd(o, v);
+    }
   }
 }
 
-__global__ void __launch_bounds__(256) k_amr_update_e(long long nvc, const double* Eh, double* En,
-                                                      double theta) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nvc) return;
-#pragma unroll
-  for (int d = 0; d < 3; d++)
-    En[d * nvc + c] = (Eh[d * nvc + c] - (1.0 - theta) * En[d * nvc + c]) / theta;
-}
-
-// wave energy sum_cells V (sum_corners |E|^2/8 + |B|^2) / (8 pi)
-__global__ void __launch_bounds__(256) k_amr_wave_energy(long long ncell, long long nvc,
-                                                         const int* ctab, const double* bdx,
-                                                         const double* En, const double* Bcen,
-                                                         double* energy) {
-  const long long cell = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double en = 0.0;
-  if (cell < ncell) {
-    const int b = (int)(cell >> 9), l = (int)(cell & 511);
-    const int i = l & 7, j = (l >> 3) & 7, k = l >> 6;
-    const double dx = bdx[b], V = dx * dx * dx;
-    double e2 = 0.0;
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const int cc = ctab[b * 729 + (i + c_off[c][0]) + 9 * ((j + c_off[c][1]) + 9 * (k + c_off[c][2]))];
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        const double v = En[d * nvc + cc];
-        e2 += v * v;
-      }
-    }
-    double b2 = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      const double v = Bcen[d * ncell + cell];
-      b2 += v * v;
-    }
-    en = (0.125 * e2 + b2) * V * 0.125 / kPi;
-  }
+// sum of en over the grid into *energy (256 threads per CTA)
+__device__ __forceinline__ void add_energy(double en, double* energy) {
   __shared__ double s[8];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) en += __shfl_xor_sync(0xffffffffu, en, o);
@@ -929,6 +927,67 @@ __global__ void __launch_bounds__(256) k_amr_wave_energy(long long ncell, long l
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += s[w];
     atomicAdd(energy, t);
   }
+}
+
+// hanging corners of a field take the interpolation of their (free) parents; rows
+// lists them among others.  cvol (optional): their share of the wave energy.
+__global__ void __launch_bounds__(256) k_amr_fix_hanging(int nrows, const int* __restrict__ rows, long long nvc,
+                                                         Hang h, double* F, const double* __restrict__ cvol,
+                                                         double* energy) {
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  double en = 0.0;
+  if (t0 < nrows) {
+    const int c = rows[t0], s = h.hs[c], e = h.hs[c + 1];
+    if (s < e) {
+      double v[3] = {0.0, 0.0, 0.0};
+      for (int t = s; t < e; t++) {
+        const double w = h.hw[t];
+        const int p = h.hp[t];
+#pragma unroll
+        for (int d = 0; d < 3; d++) v[d] += w * F[d * nvc + p];
+      }
+#pragma unroll
+      for (int d = 0; d < 3; d++) F[d * nvc + c] = v[d];
+      if (cvol) en = -cvol[c] * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) * 0.015625 / kPi;
+    }
+  }
+  if (cvol) add_energy(en, energy);
+}
+
+// E^{n+1} = ri E^{n+theta} - r1 E^n, and the wave energy sum_cells V (sum_corners
+// |E|^2/8 + |B|^2) / (8 pi) per corner with the volume of its cells (cvol; hanging
+// corners carry it negative: their E and its energy follow in k_amr_fix_hanging).
+// The FP64 pipe bounds it.  491,520 cells: 42 us with k_amr_fix_hanging (a pass over
+// the cells' 8 corners each, and all corners looked at for hanging ones: 85).
+__global__ void __launch_bounds__(256) k_amr_update_e(long long ncell, long long nvc,
+                                                      const double* __restrict__ Eh, double* __restrict__ En,
+                                                      double ri, double r1, const double* __restrict__ cvol,
+                                                      const double* __restrict__ bdx,
+                                                      const double* __restrict__ Bcen, double* energy) {
+  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  double ee = 0.0, eb = 0.0;
+  for (long long c = t0; c < nvc; c += step) {
+    double e2 = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const double v = ri * Eh[d * nvc + c] - r1 * En[d * nvc + c];
+      En[d * nvc + c] = v;
+      e2 += v * v;
+    }
+    const double w = cvol[c];
+    ee += w > 0.0 ? w * e2 : 0.0;
+  }
+  for (long long cell = t0; cell < ncell; cell += step) {
+    const double dx = bdx[cell >> 9];
+    double b2 = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const double v = Bcen[d * ncell + cell];
+      b2 += v * v;
+    }
+    eb += dx * dx * dx * b2;
+  }
+  add_energy((0.125 * ee + eb) * 0.125 / kPi, energy);
 }
 
 __global__ void k_amr_pack(long long nvc, const int* ctab, Hang h, const double* Eh,
@@ -993,6 +1052,7 @@ static ApplyArgs apply_args(amps_gpu_ctx* c) {
     split(0.125 * V, K.id);
     split(a.f * V, K.m);
     split(a.thdt * V * 0.25 / dx, K.bb);
+    K.dg = (float)(V * (0.125 + a.th2dt2 / (8.0 * dx * dx)));
   }
   split(a.f, a.fj);
   return a;
@@ -1065,7 +1125,8 @@ cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* di
   TimedLaunch t(c, "matvec", 3);
   if ((e = split_input(c, x, dinv, a)) != cudaSuccess) return e;
   if ((e = launch_tile<1>(c, a, y)) != cudaSuccess) return e;
-  k_amr_constraint<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, x, dinv, y, 0, c->d_next);
+  k_amr_constraint<<<g1(std::max(c->nsrows, 1)), 256, 0, c->stream>>>(c->nsrows, c->d_srows, c->nvc, a.h,
+                                                                      x, dinv, y, 0, c->d_next);
   return cudaGetLastError();
 }
 
@@ -1088,42 +1149,34 @@ cudaError_t launch_amr_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, f
   return cudaGetLastError();
 }
 
-cudaError_t launch_amr_rhs(amps_gpu_ctx* c) {
+// diag: also sum the Jacobi diagonal, for launch_amr_jacobi
+cudaError_t launch_amr_rhs(amps_gpu_ctx* c, bool diag) {
   cudaError_t e = cudaMemsetAsync(c->d_rhs, 0, sizeof(double) * 3 * c->nvc, c->stream);
+  if (e == cudaSuccess && diag) e = cudaMemsetAsync(c->d_diag, 0, sizeof(double) * 3 * c->nvc, c->stream);
   if (e != cudaSuccess) return e;
   ApplyArgs a = apply_args(c);
+  a.diag = diag ? c->d_diag : nullptr;
   a.x = c->d_En;
   a.dinv = nullptr;
   a.Bcen = c->d_Bc;
   TimedLaunch t(c, "rhs", 3);
   if ((e = split_input(c, c->d_En, nullptr, a)) != cudaSuccess) return e;
   if ((e = launch_tile<2>(c, a, c->d_rhs)) != cudaSuccess) return e;
-  k_amr_constraint<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, nullptr, nullptr, c->d_rhs, 1, c->d_next);
+  k_amr_constraint<<<g1(std::max(c->nsrows, 1)), 256, 0, c->stream>>>(c->nsrows, c->d_srows, c->nvc, a.h,
+                                                                      nullptr, nullptr, c->d_rhs, 1, c->d_next);
   return cudaGetLastError();
 }
 
 cudaError_t launch_amr_jacobi(amps_gpu_ctx* c) {
-  cudaError_t e = cudaMemsetAsync(c->d_dinv, 0, sizeof(double) * 3 * c->nvc, c->stream);
-  if (e != cudaSuccess) return e;
-  ApplyArgs a = apply_args(c);
-  TimedLaunch t(c, "jacobi", 2);
-  DiagK K{};
-  for (int sc = 0; sc < kMaxScale; sc++) {
-    const double dx = c->dxf * (double)(1 << sc), V = dx * dx * dx;
-    K.base[sc] = (float)(V * (0.125 + a.th2dt2 / (8.0 * dx * dx)));
-    K.fv[sc] = (float)(a.f * V);
-  }
-  k_amr_diag<<<g1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_ctab, a.h, c->d_bscale,
-                                                  c->d_cellM, K, c->d_dinv);
-  k_amr_invert_diag<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, a.h, c->d_dinv);
+  TimedLaunch t(c, "jacobi");
+  k_amr_invert_diag<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, hang_of(c), c->d_diag, c->d_dinv);
   return cudaGetLastError();
 }
 
 cudaError_t launch_amr_update_b(amps_gpu_ctx* c) {
   TimedLaunch t(c, "update_b");
-  k_amr_update_b<<<g1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_ctab, hang_of(c),
-                                                      c->d_bdx, c->d_Eh, c->d_Bc, c->d_Bc2,
-                                                      c->cfg.dt);
+  k_amr_update_b<<<c->nb, 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_ctabh, hang_of(c), c->d_bdx, c->d_Eh,
+                                               c->d_Bc, c->d_Bc2, c->cfg.dt);
   if (c->mesh_open) {
     const int* nf = c->amrdev.nfine;
     for (int pass = 0; pass <= (c->neumann ? 3 : 0); pass++)
@@ -1133,34 +1186,36 @@ cudaError_t launch_amr_update_b(amps_gpu_ctx* c) {
   return cudaGetLastError();
 }
 
+// hanging corners of F, optionally with their wave energy
+static cudaError_t fix_hanging(amps_gpu_ctx* c, double* F, const double* cvol, double* energy) {
+  if (c->nsrows == 0) return cudaSuccess;
+  k_amr_fix_hanging<<<g1(c->nsrows), 256, 0, c->stream>>>(c->nsrows, c->d_srows, c->nvc, hang_of(c), F, cvol,
+                                                          energy);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_amr_c2n(amps_gpu_ctx* c, const double* Bcen, double* Bcor) {
-  // the GMRES work vector holds the weights (3*nvc >= nvc doubles)
-  double* wsum = c->d_w;
   cudaError_t e = cudaMemsetAsync(Bcor, 0, sizeof(double) * 3 * c->nvc, c->stream);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(wsum, 0, sizeof(double) * c->nvc, c->stream);
-  if (e != cudaSuccess) return e;
-  TimedLaunch t(c, "c2n", 3);
-  k_amr_c2n_acc<<<g1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_ctab, c->d_bdx, Bcen,
-                                                     Bcor, wsum);
-  k_amr_c2n_div<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, wsum, Bcor);
-  k_amr_fix_hanging<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, hang_of(c), Bcor);
-  return cudaGetLastError();
+  TimedLaunch t(c, "c2n", 2);
+  k_amr_c2n<<<c->nb, 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_ctab, c->d_bdx, c->d_cinv, Bcen, Bcor);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  return fix_hanging(c, Bcor, nullptr, nullptr);
 }
 
 cudaError_t launch_amr_update_e(amps_gpu_ctx* c) {
   cudaError_t e = cudaMemsetAsync(c->d_energy + 1, 0, sizeof(double), c->stream);
   if (e != cudaSuccess) return e;
-  TimedLaunch t(c, "update_e", 3);
-  k_amr_update_e<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, c->d_Eh, c->d_En, c->cfg.theta);
-  k_amr_fix_hanging<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, hang_of(c), c->d_En);
-  k_amr_wave_energy<<<g1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_ctab, c->d_bdx,
-                                                         c->d_En, c->d_Bc, c->d_energy + 1);
-  return cudaGetLastError();
+  TimedLaunch t(c, "update_e", 2);
+  const double th = c->cfg.theta;
+  const unsigned grid = (unsigned)std::min<long long>((std::max(c->nvc, c->ncor) + 255) / 256, 152LL * 8);
+  k_amr_update_e<<<grid, 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_Eh, c->d_En, 1.0 / th, (1.0 - th) / th, c->d_cvol,
+                                              c->d_bdx, c->d_Bc, c->d_energy + 1);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  return fix_hanging(c, c->d_En, c->d_cvol, c->d_energy + 1);
 }
 
 // E^{n+theta} = E^n + dE with hanging corners re-interpolated
 cudaError_t launch_amr_fix_hanging(amps_gpu_ctx* c, double* F) {
-  k_amr_fix_hanging<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, hang_of(c), F);
-  return cudaGetLastError();
+  return fix_hanging(c, F, nullptr, nullptr);
 }

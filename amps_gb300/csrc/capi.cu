@@ -314,7 +314,7 @@ bool alloc_context(amps_gpu_ctx* c) {
        !dalloc(&c->d_Bcor_cur, 3 * nv);
   if (!c->amr) ok = ok && !dalloc(&c->d_J, 3 * nc) && !dalloc(&c->d_M, 243 * nc);
   if (c->amr)
-    ok = ok && !dalloc(&c->d_y32, 3 * nv) && !dalloc(&c->d_next, 1) &&
+    ok = ok && !dalloc(&c->d_y32, 3 * nv) && !dalloc(&c->d_next, 1) && !dalloc(&c->d_diag, 3 * nv) &&
          cudaMemsetAsync(c->d_next, 0, sizeof(int), c->stream) == cudaSuccess &&
          cudaMemsetAsync(c->d_y32, 0, sizeof(float) * 3 * nv, c->stream) == cudaSuccess;
   ok = ok && !dalloc(&c->d_rhs, 3 * nv) && !dalloc(&c->d_x, 3 * nv) &&
@@ -658,12 +658,18 @@ amps_gpu_status amps_gpu_create_amr(const amps_gpu_config* cfg, const amps_amr_m
     for (long long r = 0; r < nv; r++)
       if (sdiag[(size_t)r].x == 0.f) srows.push_back((int)r);
     c->nsrows = (int)srows.size();
+    // volume of the cells at each corner (hanging corners negative) and its inverse
+    std::vector<double> cvol((size_t)nv), cinv((size_t)nv);
+    for (size_t r = 0; r < cvol.size(); r++) {
+      cinv[r] = D[r] > 0.0 ? 0.125 / D[r] : 0.0;
+      cvol[r] = (hs[r + 1] > hs[r] ? -8.0 : 8.0) * D[r];
+    }
     std::vector<int> ctabh(m->corner_tab.begin(), m->corner_tab.end());
     for (int& q : ctabh)
       if (hs[(size_t)q + 1] > hs[(size_t)q]) q = ~q;
     ok = ok && upload(&c->d_ss, ss) && upload(&c->d_sc, sc) && upload(&c->d_sv, sv) &&
          upload(&c->d_svh, svh) && upload(&c->d_svl, svl) && upload(&c->d_sdiag, sdiag) && upload(&c->d_srows, srows) &&
-         upload(&c->d_ctabh, ctabh);
+         upload(&c->d_ctabh, ctabh) && upload(&c->d_cvol, cvol) && upload(&c->d_cinv, cinv);
   }
   if (!ok) {
     cudaGetLastError();
@@ -728,7 +734,7 @@ amps_gpu_status amps_gpu_destroy(amps_gpu_ctx* c) {
   c->d_hstage = nullptr;
   void* ptrs[] = {c->d_nbr, c->d_En, c->d_Eh, c->d_Bc, c->d_Bc2, c->d_Bcor_prev, c->d_Bcor_cur,
                   c->d_J, c->d_M, c->d_rhs, c->d_x, c->d_V, c->d_w, c->d_dinv, c->d_red, c->d_arn, c->d_xs, c->d_step,
-                  c->d_Z, c->d_y32, c->d_next,
+                  c->d_Z, c->d_y32, c->d_next, c->d_diag, c->d_cvol, c->d_cinv,
                   c->d_stencil_push, c->d_stencil_dep, c->d_stencil_cprev, c->d_stencil_ccur, c->d_key, c->d_rank, c->d_base, c->d_cnt,
                   c->d_arr, c->d_stay, c->d_tmp, c->d_count, c->d_scan_part, c->d_flags,
                   c->d_cellM, c->d_cellJ, c->d_energy, c->d_ctab, c->d_hs, c->d_hp, c->d_hw, c->d_hwh, c->d_hwl,
@@ -1025,7 +1031,7 @@ amps_gpu_status amps_gpu_field_solve(amps_gpu_ctx* c, double tol, int maxit, int
   // report bounded-wait timeouts in the flags
   const bool watch = precond == 2 || c->amr;
   if (watch && (s = reset_flags(c))) return s;
-  if ((s = cuda_check(c, launch_rhs(c), "rhs"))) return s;
+  if ((s = cuda_check(c, launch_rhs(c, precond != 0), "rhs"))) return s;
   amps_gpu_status gs = gmres_solve(c, tol, maxit, precond, &st);
   if (gs != AMPS_GPU_OK && gs != AMPS_GPU_GMRES_NOT_CONVERGED) return gs;
   if (watch && (s = check_flags(c, nullptr, nullptr, nullptr))) return s;

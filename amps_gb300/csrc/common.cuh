@@ -120,6 +120,9 @@ struct amps_gpu_ctx {
   float* d_dff = nullptr;       // 2n: the Jacobi scaling as FP32 pairs (hi n, lo n)
   double* d_tmpv = nullptr;     // 2n doubles: FP64 copies of Krylov vectors for the
                                 // learned network, its sample harvest and the FP64 inner operator
+  double* d_diag = nullptr;     // 3*nvc: the AMR operator's diagonal, summed by the RHS kernel
+  double* d_cvol = nullptr;     // nvc: volume of the cells at each AMR corner (hanging: negative)
+  double* d_cinv = nullptr;     // nvc: 1 / |d_cvol|
   int* d_next = nullptr;        // next tile of the persistent AMR operator in pairs (zero between launches)
   float* d_y32 = nullptr;       // 3*nvc FP32 accumulation of the inner AMR operator (zero between
                                 // applications)
@@ -320,7 +323,7 @@ cudaError_t launch_export(amps_gpu_ctx* c, double* d_x, double* d_v, uint8_t* d_
                           int32_t* d_blk, int32_t* d_cel, uint32_t* d_id);
 
 // ---- field launchers (field.cu) ----
-cudaError_t launch_rhs(amps_gpu_ctx* c);
+cudaError_t launch_rhs(amps_gpu_ctx* c, bool diag);  // diag: for a solve with launch_jacobi_diag
 cudaError_t launch_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y);
 // Input of the inner operator on a Krylov vector: v as FP32 pairs (vh, vl) or,
 // for the flexible directions, as doubles (vd); the scaling D as FP32 pairs
@@ -354,7 +357,7 @@ amps_gpu_status field_autotune(amps_gpu_ctx* c, double* ms);
 cudaError_t launch_amr_pack(amps_gpu_ctx* c, const double* Eh, const double* Bprev,
                             const double* Bcur);
 cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y);
-cudaError_t launch_amr_rhs(amps_gpu_ctx* c);
+cudaError_t launch_amr_rhs(amps_gpu_ctx* c, bool diag);
 cudaError_t launch_amr_jacobi(amps_gpu_ctx* c);
 cudaError_t launch_amr_update_b(amps_gpu_ctx* c);
 cudaError_t launch_amr_c2n(amps_gpu_ctx* c, const double* Bcen, double* Bcor);

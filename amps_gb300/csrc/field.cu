@@ -1250,8 +1250,8 @@ cudaError_t launch_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, float
   return cudaGetLastError();
 }
 
-cudaError_t launch_rhs(amps_gpu_ctx* c) {
-  if (c->amr) return launch_amr_rhs(c);
+cudaError_t launch_rhs(amps_gpu_ctx* c, bool diag) {
+  if (c->amr) return launch_amr_rhs(c, diag);
   const TapsFF T = taps_ff(make_taps(c->cfg, false));
   double c4[3];
   for (int d = 0; d < 3; d++) c4[d] = 0.25 * (c->cfg.dt / c->cfg.dx[d] * c->cfg.theta);

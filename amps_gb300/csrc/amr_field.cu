@@ -302,11 +302,6 @@ __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigne
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
                                                    unsigned long long c) {
   unsigned long long r;

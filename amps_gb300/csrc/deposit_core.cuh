@@ -49,18 +49,46 @@ SpeciesTab make_species(const amps_gpu_config& c) {
   return t;
 }
 
+// a, b in both halves of a register pair; a * b per half
+__device__ __forceinline__ unsigned long long dup2(float a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// the larger and the smaller magnitude, NaN if either is
+__device__ __forceinline__ float abs_max(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(fabsf(a)), "f"(fabsf(b)));
+  return r;
+}
+__device__ __forceinline__ float abs_min(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(fabsf(a)), "f"(fabsf(b)));
+  return r;
+}
+
 // en += the kinetic energy 0.5 m W v^2 of one particle (ProcessCell :2238,
-// summed in FP64 by the reference) as a float pair: the squares and the
-// weight-correction product exact by FMA, sums by TwoSum, the FP64 species
-// factor 0.5 m w as two floats (FF, common.cuh).  Error ~1e-14 of the sum.
+// summed in FP64 by the reference) as a float pair: the squares are added to the
+// largest one, so that what a sum loses is its difference to the larger operand
+// (Dekker's fast two-sum, exact) and the square's error comes with it from one FMA;
+// the weight-correction product exact by FMA, the last sum by TwoSum, the FP64 species
+// factor 0.5 m w as two floats (FF, common.cuh).  Error ~1e-14 of the sum.  29
+// operations (TwoSum for each square: 40).
 __device__ __forceinline__ void kinetic_energy(FF& en, float v0, float v1, float v2, float wcorr,
                                                int s, const SpeciesTab& st) {
-  const float p0 = __fmul_rn(v0, v0);
-  FF t{p0, fmaf(v0, v0, -p0)};
-  ff_add(t, v1, v1, 0.f);
-  ff_add(t, v2, v2, 0.f);
-  const FF tw = ff_mul(t.s, t.q, wcorr, 0.f);
-  ff_add2(en, st.keh[s], st.kel[s], tw.s, tw.q);
+  const float m0 = abs_max(v0, v1), n0 = abs_min(v0, v1);
+  const float m = abs_max(m0, v2), n1 = abs_min(m0, v2);
+  const float p = __fmul_rn(m, m), ep = fmaf(m, m, -p);
+  const float s0 = fmaf(n0, n0, p), e0 = fmaf(n0, n0, __fsub_rn(p, s0));
+  const float s1 = fmaf(n1, n1, s0), e1 = fmaf(n1, n1, __fsub_rn(s0, s1));
+  const float q = __fadd_rn(ep, __fadd_rn(e0, e1));
+  const float th = __fmul_rn(s1, wcorr), tl = fmaf(q, wcorr, fmaf(s1, wcorr, -th));
+  ff_add2(en, st.keh[s], st.kel[s], th, tl);
 }
 
 // Stage one bulk copy per stencil into shared memory; returns false on timeout.
@@ -183,22 +211,16 @@ __device__ __forceinline__ void stage_fields(float* __restrict__ rec, int pos,
     B1 = Bs[0][1] + Bs[1][1];
     B2 = Bs[0][2] + Bs[1][2];
   }
+  // b = h B: alpha = c0 (1 + b b^T + [. x b]), c0 = 1 / (1 + b^2)
   const float h = st.qdt2m[s];
-  const float h2 = h * h;
-  const float c0 = 1.0f / (1.0f + h2 * (B0 * B0 + B1 * B1 + B2 * B2));
-  const float P0 = -h * B0, P1 = -h * B1, P2 = -h * B2;
-  float al[9];
-  al[0] = c0 * (1.f + h2 * B0 * B0);
-  al[1] = c0 * (-P2 + h2 * B0 * B1);
-  al[2] = c0 * (P1 + h2 * B0 * B2);
-  al[3] = c0 * (P2 + h2 * B1 * B0);
-  al[4] = c0 * (1.f + h2 * B1 * B1);
-  al[5] = c0 * (-P0 + h2 * B1 * B2);
-  al[6] = c0 * (-P1 + h2 * B2 * B0);
-  al[7] = c0 * (P0 + h2 * B2 * B1);
-  al[8] = c0 * (1.f + h2 * B2 * B2);
+  const float b0 = h * B0, b1 = h * B1, b2 = h * B2;
+  const float c0 = 1.0f / (1.0f + (b0 * b0 + b1 * b1 + b2 * b2));
   const float qW = st.qw[s] * wq;
-  const float kc = qW * h * inv_vol;
+  const float K = qW * h * inv_vol * c0;  // k alpha = K (..)
+  const float k0 = K * b0, k1 = K * b1, k2 = K * b2;
+  const float ka[9] = {fmaf(k0, b0, K),  fmaf(k0, b1, k2),  fmaf(k0, b2, -k1),
+                       fmaf(k0, b1, -k2), fmaf(k1, b1, K),  fmaf(k1, b2, k0),
+                       fmaf(k0, b2, k1), fmaf(k1, b2, -k0), fmaf(k2, b2, K)};
   float* r = rec + pos;
   {
     const float X[3] = {gx * gx, gx * fx, fx * fx};
@@ -214,16 +236,14 @@ __device__ __forceinline__ void stage_fields(float* __restrict__ rec, int pos,
       }
   }
 #pragma unroll
-  for (int e = 0; e < 9; e++) r[(27 + e) * FS] = kc * al[e];
+  for (int e = 0; e < 9; e++) r[(27 + e) * FS] = ka[e];
 #pragma unroll
   for (int c = 0; c < 8; c++) r[(36 + c) * FS] = w[c];
   r[44 * FS] = 0.f;
-  const float vr0 = al[0] * v0 + al[1] * v1 + al[2] * v2;
-  const float vr1 = al[3] * v0 + al[4] * v1 + al[5] * v2;
-  const float vr2 = al[6] * v0 + al[7] * v1 + al[8] * v2;
-  r[45 * FS] = qW * vr0;
-  r[46 * FS] = qW * vr1;
-  r[47 * FS] = qW * vr2;
+  const float qc = qW * c0, bv = fmaf(b0, v0, fmaf(b1, v1, b2 * v2));
+  r[45 * FS] = qc * fmaf(v1, b2, fmaf(-v2, b1, fmaf(b0, bv, v0)));
+  r[46 * FS] = qc * fmaf(v2, b0, fmaf(-v0, b2, fmaf(b1, bv, v1)));
+  r[47 * FS] = qc * fmaf(v0, b1, fmaf(-v1, b0, fmaf(b2, bv, v2)));
   kinetic_energy(en, v0, v1, v2, wq, s, st);
 }
 

@@ -230,24 +230,41 @@ __device__ __forceinline__ void lapenta(float h, const float E[3], const float B
   v[2] = 2.f * a2 - v[2];
 }
 
+constexpr int kPushWarps = 4;       // warps per CTA (one row of 8 cells each)
+constexpr int kSlabSC = 2 * 81;     // a layer of cells sees two planes of corners
+constexpr int kSlabCSC = 3 * 100;   // and three planes of centres
+// What bounds it: the shared-memory return path (80 % of its cycles while the kernel
+// runs: the tile accumulation's 48 16-byte loads per 32 particles, 37 % of the time)
+// with issue at 53 % and the FMA pipe at 40 %.  A CTA takes half a layer of a block and
+// stages the layer's two planes of corners (7.8 KB, where the block's nine took 35), so
+// four CTAs of four warps share an SM at 128 registers: the same 16 warps as two of
+// eight, with shorter waits at a CTA's start and end.  More warps only lose: five CTAs
+// (96 registers) 2.59 ms, six (80) 2.61 ms.  67.1M particles on the refined mesh: 2.54 ms
+// (2.61 before), 4.2M on 64 uniform blocks 190 us (206), 60 blocks with centre B 98 us
+// (108).
 // CB: the particles see B interpolated from the cell centres (B^n from the
 // centre stencil for the push, B^{n+1} for the deposit); E from the corners.
 template <bool DEP, bool AMR, bool CB = false>
-__global__ void __launch_bounds__(256, 2) k_push_deposit(StepArgs a) {
+__global__ void __launch_bounds__(kPushWarps * 32, 4) k_push_deposit(StepArgs a) {
   extern __shared__ __align__(16) float4 s_dyn[];
-  constexpr int kDepSC = CB ? AMPS_CSC : AMPS_SC;
-  float4* s_push = s_dyn;                         // 729 x 2 float4
-  float4* s_dep = s_dyn + 2 * AMPS_SC;            // 729 float4 corners, or 1000 centres (CB)
-  float4* s_cprev = s_dep + kDepSC;               // 1000 float4 centres of B^n (CB)
-  float* s_rec = reinterpret_cast<float*>(s_cprev + (CB ? AMPS_CSC : 0));  // kWarps x kFields x kFS
+  constexpr int kDepSC = CB ? kSlabCSC : kSlabSC;
+  const int b = blockIdx.x, k = blockIdx.y / (AMPS_NC / kPushWarps);
+  // the layer's slab of the stencils; the pointers count from the block's first corner
+  // or centre
+  float4* const t_push = s_dyn;              // kSlabSC x 2 float4
+  float4* const t_dep = s_dyn + 2 * kSlabSC; // corners, or centres (CB)
+  float4* const t_cprev = t_dep + kDepSC;    // centres of B^n (CB)
+  const float4* s_push = t_push - 2 * 81 * k;
+  const float4* s_dep = t_dep - (CB ? 100 : 81) * k;
+  const float4* s_cprev = t_cprev - 100 * k;
+  float* s_rec = reinterpret_cast<float*>(t_cprev + (CB ? kSlabCSC : 0));  // kPushWarps x kFields x kFS
   __shared__ __align__(8) uint64_t bar;
-  __shared__ double s_en[kWarps];
-  const int b = blockIdx.x, k = blockIdx.y;
+  __shared__ double s_en[kPushWarps];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint32_t bp = AMPS_SC * AMPS_PUSH_STRIDE * sizeof(float);
+  const uint32_t bp = kSlabSC * AMPS_PUSH_STRIDE * sizeof(float);
   const uint32_t bd = DEP ? kDepSC * 4 * sizeof(float) : 0;
-  const uint32_t bc = CB ? AMPS_CSC * sizeof(float4) : 0;
-  const int j = wid;
+  const uint32_t bc = CB ? kSlabCSC * sizeof(float4) : 0;
+  const int j = wid + kPushWarps * (blockIdx.y % (AMPS_NC / kPushWarps));
   // slot range and occupancy of the row's 8 cells, one lane per cell
   int mb0 = 0, mn0 = 0;
   if (lane < AMPS_NC) {
@@ -276,17 +293,16 @@ __global__ void __launch_bounds__(256, 2) k_push_deposit(StepArgs a) {
     }
   };
   prefetch(0, lane);  // in flight while the stencils are staged
-  const void* dep_src = CB ? (const void*)(a.st_ccur + (size_t)b * AMPS_CSC)
-                           : (const void*)(a.st_dep + (size_t)b * AMPS_SC * AMPS_DEP_STRIDE);
-  if (!stage_stencils(&bar, s_push, a.st_push + (size_t)b * AMPS_SC * AMPS_PUSH_STRIDE, bp, s_dep,
-                      dep_src, bd, a.flags, s_cprev, CB ? a.st_cprev + (size_t)b * AMPS_CSC : nullptr,
-                      bc))
+  const size_t cor = (size_t)b * AMPS_SC + 81 * k, cen = (size_t)b * AMPS_CSC + 100 * k;
+  const void* dep_src = CB ? (const void*)(a.st_ccur + cen) : (const void*)(a.st_dep + cor * AMPS_DEP_STRIDE);
+  if (!stage_stencils(&bar, t_push, a.st_push + cor * AMPS_PUSH_STRIDE, bp, t_dep, dep_src, bd, a.flags,
+                      t_cprev, CB ? a.st_cprev + cen : nullptr, bc))
     return;
   float* rec = s_rec + wid * kFields * kFS;
   int fA, fB;
   lane_fields(lane, fA, fB);
   FF en_row{0.f, 0.f};  // float pair across the row's cells, FP64 in the CTA reduction
-  unsigned long long n_far = 0, n_near = 0, n_del = 0;
+  unsigned n_far = 0, n_near = 0, n_del = 0;
   const float inv_vol = block_inv_vol(a, b);
   const float bdtdx = AMR ? __ldg(a.amr.bdtdx + b) : 0.0f;
   for (int i = 0; i < AMPS_NC; i++) {
@@ -308,36 +324,34 @@ __global__ void __launch_bounds__(256, 2) k_push_deposit(StepArgs a) {
       else if (i + 1 < AMPS_NC)
         prefetch(i + 1, lane);
       if (act) {
-        // gather E^{n+theta}, B^n at the old position
+        // gather E^{n+theta}, B^n at the old position, which lies in this cell (every
+        // writer of a particle files it under (int)u): the corners' addresses are the
+        // warp's
         int ic[3];
-        float f[3];
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-          ic[d] = min(max((int)u[d], 0), AMPS_NC - 1);
-          f[d] = u[d] - (float)ic[d];
-        }
+        const float f[3] = {u[0] - (float)i, u[1] - (float)j, u[2] - (float)k};
+        const float xy[4] = {(1.f - f[0]) * (1.f - f[1]), f[0] * (1.f - f[1]), (1.f - f[0]) * f[1],
+                             f[0] * f[1]};
+        const unsigned long long zz[2] = {dup2(1.f - f[2]), dup2(f[2])};
         // E and B as three packed pairs (E0 E1) (E2 B0) (B1 B2), the layout of a
-        // stencil corner's two float4s, accumulated by packed FMAs
+        // stencil corner's two float4s, accumulated by packed FMAs; the weights come
+        // out doubled for them
         unsigned long long eb[2][3] = {{0ull, 0ull, 0ull}, {0ull, 0ull, 0ull}};  // z = 0, 1 layers
 #pragma unroll
-        for (int cc = 0; cc < 2; cc++)
+        for (int ab = 0; ab < 4; ab++) {
+          const unsigned long long w2 = dup2(xy[ab]);
 #pragma unroll
-          for (int bb = 0; bb < 2; bb++)
-#pragma unroll
-            for (int aa = 0; aa < 2; aa++) {
-              const float w = (aa ? f[0] : 1.f - f[0]) * (bb ? f[1] : 1.f - f[1]) *
-                              (cc ? f[2] : 1.f - f[2]);
-              const int sidx = (ic[0] + aa) + 9 * (ic[1] + bb) + 81 * (ic[2] + cc);
-              const ulonglong2 q0v = reinterpret_cast<const ulonglong2*>(s_push)[2 * sidx];
-              unsigned long long ww;
-              asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
-              ffma2(eb[cc][0], ww, q0v.x);
-              ffma2(eb[cc][1], ww, q0v.y);
-              if (!CB) {
-                const ulonglong2 q1v = reinterpret_cast<const ulonglong2*>(s_push)[2 * sidx + 1];
-                ffma2(eb[cc][2], ww, q1v.x);
-              }
+          for (int cc = 0; cc < 2; cc++) {
+            const unsigned long long ww = mul2(w2, zz[cc]);
+            const int sidx = (i + (ab & 1)) + 9 * (j + (ab >> 1)) + 81 * (k + cc);
+            const ulonglong2 q0v = reinterpret_cast<const ulonglong2*>(s_push)[2 * sidx];
+            ffma2(eb[cc][0], ww, q0v.x);
+            ffma2(eb[cc][1], ww, q0v.y);
+            if (!CB) {
+              const ulonglong2 q1v = reinterpret_cast<const ulonglong2*>(s_push)[2 * sidx + 1];
+              ffma2(eb[cc][2], ww, q1v.x);
             }
+          }
+        }
         float eb_f[6];
 #pragma unroll
         for (int t = 0; t < 3; t++) {
@@ -357,33 +371,48 @@ __global__ void __launch_bounds__(256, 2) k_push_deposit(StepArgs a) {
 #pragma unroll
           for (int d = 0; d < 3; d++) {
             u[d] = fmaf(v[d], bdtdx, u[d]);
-            const int od = (int)floorf(u[d] * 0.125f);
-            if (od > 1 || od < -1) far = true;
             if (!(u[d] >= 0.0f && u[d] < 8.0f)) out = true;
             ic[d] = min((int)u[d], AMPS_NC - 1);
           }
-          if (out) nbk = amr_dest(a.amr, b, u, ic, a.open);
+          if (out) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+              const int od = (int)floorf(u[d] * 0.125f);
+              if (od > 1 || od < -1) far = true;
+            }
+            nbk = amr_dest(a.amr, b, u, ic, a.open);
+          }
 #pragma unroll
           for (int d = 0; d < 3; d++)
             if (fabsf(u[d] - rintf(u[d])) < 4.76837158203125e-7f) nearf = true;
         } else {
-          int o[3];
+          bool out = false;
 #pragma unroll
           for (int d = 0; d < 3; d++) {
-            float un = fmaf(v[d], a.dtdx[d], u[d]);
-            int od = (int)floorf(un * 0.125f);
-            if (od > 1 || od < -1) far = true;
-            od = max(-1, min(1, od));
-            un -= 8.0f * (float)od;
-            un = clamp_below8(fmaxf(un, 0.0f));
-            o[d] = od;
-            u[d] = un;
-            ic[d] = min((int)un, AMPS_NC - 1);
-            if (fabsf(un - rintf(un)) < 4.76837158203125e-7f) nearf = true;
+            u[d] = fmaf(v[d], a.dtdx[d], u[d]);
+            if (!(u[d] >= 0.0f && u[d] < 8.0f)) out = true;
           }
-          if (o[0] | o[1] | o[2])
-            nbk = (a.open && leaves_open_face(a, b, o)) ? -1
-                                                        : __ldg(a.nbr + b * 27 + nbr_slot(o[0], o[1], o[2]));
+          if (out) {
+            int o[3];
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+              float un = u[d];
+              int od = (int)floorf(un * 0.125f);
+              if (od > 1 || od < -1) far = true;
+              od = max(-1, min(1, od));
+              un -= 8.0f * (float)od;
+              u[d] = clamp_below8(fmaxf(un, 0.0f));
+              o[d] = od;
+            }
+            if (o[0] | o[1] | o[2])
+              nbk = (a.open && leaves_open_face(a, b, o)) ? -1
+                                                          : __ldg(a.nbr + b * 27 + nbr_slot(o[0], o[1], o[2]));
+          }
+#pragma unroll
+          for (int d = 0; d < 3; d++) {
+            ic[d] = min((int)u[d], AMPS_NC - 1);
+            if (fabsf(u[d] - rintf(u[d])) < 4.76837158203125e-7f) nearf = true;
+          }
         }
         if (far) n_far++;
         if (nearf) n_near++;
@@ -408,9 +437,12 @@ __global__ void __launch_bounds__(256, 2) k_push_deposit(StepArgs a) {
       }
       // every lane stages its position; only stayers carry weight (movers are
       // deposited by k_arrivals in their destination cell)
-      if (DEP)
-        stage_fields<kFS, CB>(rec, lane, s_dep, u[0], u[1], u[2], v[0], v[1], v[2], act ? s : 0,
-                          stays ? wcv : 0.f, i, j, k, a.st, inv_vol, en_row);
+      // (centre B: the slab reaches the cell's own positions only)
+      if (DEP) {
+        const bool at = !CB || stays;
+        stage_fields<kFS, CB>(rec, lane, s_dep, at ? u[0] : i + 0.5f, at ? u[1] : j + 0.5f, at ? u[2] : k + 0.5f,
+                              v[0], v[1], v[2], act ? s : 0, stays ? wcv : 0.f, i, j, k, a.st, inv_vol, en_row);
+      }
       // movers: slack of the destination cell, else the overflow list
       const bool mover = act && !stays && key >= 0;
       // one reservation per mover (a chunk has a few): no warp-wide key match
@@ -451,9 +483,9 @@ __global__ void __launch_bounds__(256, 2) k_push_deposit(StepArgs a) {
     if (lane == 0) a.stay[cid] = nst;
     if (DEP) tile.flush(lane, a.cellM, a.cellJ, cid);
   }
-  if (n_far) atomicAdd(a.flags + 0, n_far);
-  if (n_near) atomicAdd(a.flags + 1, n_near);
-  if (n_del) atomicAdd(a.flags + 5, n_del);
+  if (n_far) atomicAdd(a.flags + 0, (unsigned long long)n_far);
+  if (n_near) atomicAdd(a.flags + 1, (unsigned long long)n_near);
+  if (n_del) atomicAdd(a.flags + 5, (unsigned long long)n_del);
   if (DEP) reduce_energy(ff_value(en_row), s_en, a.energy);
 }
 
@@ -1692,8 +1724,8 @@ StepArgs step_args(amps_gpu_ctx* c) {
 }
 
 size_t smem_push(bool dep, bool cb = false) {
-  return (size_t)(2 * AMPS_SC + (cb ? 2 * AMPS_CSC : AMPS_SC)) * sizeof(float4) +
-         (dep ? kWarps * kFields * kFS * sizeof(float) : 0);
+  return (size_t)(2 * kSlabSC + (cb ? 2 * kSlabCSC : kSlabSC)) * sizeof(float4) +
+         (dep ? kPushWarps * kFields * kFS * sizeof(float) : 0);
 }
 size_t smem_dep(bool cb = false) {
   return (size_t)(cb ? AMPS_CSC : AMPS_SC) * sizeof(float4) + kWarps * kFields * kFS * sizeof(float);
@@ -1911,24 +1943,24 @@ cudaError_t launch_push_step(amps_gpu_ctx* c, bool deposit) {
     if (e != cudaSuccess) return e;
   }
   StepArgs a = step_args(c);
-  const dim3 grid(c->nb, AMPS_NC);
+  const dim3 grid(c->nb, AMPS_NC), pgrid(c->nb, AMPS_NC * AMPS_NC / kPushWarps);
   {
     TimedLaunch t(c, deposit ? "push_deposit" : "push");
     if (c->amr) {
       if (deposit)
-        k_push_deposit<true, true><<<grid, kWarps * 32, smem_push(true), c->stream>>>(a);
+        k_push_deposit<true, true><<<pgrid, kPushWarps * 32, smem_push(true), c->stream>>>(a);
       else
-        k_push_deposit<false, true><<<grid, kWarps * 32, smem_push(false), c->stream>>>(a);
+        k_push_deposit<false, true><<<pgrid, kPushWarps * 32, smem_push(false), c->stream>>>(a);
     } else if (c->b_center) {
       if (deposit)
-        k_push_deposit<true, false, true><<<grid, kWarps * 32, smem_push(true, true), c->stream>>>(a);
+        k_push_deposit<true, false, true><<<pgrid, kPushWarps * 32, smem_push(true, true), c->stream>>>(a);
       else
-        k_push_deposit<false, false, true><<<grid, kWarps * 32, smem_push(false, true), c->stream>>>(a);
+        k_push_deposit<false, false, true><<<pgrid, kPushWarps * 32, smem_push(false, true), c->stream>>>(a);
     } else {
       if (deposit)
-        k_push_deposit<true, false><<<grid, kWarps * 32, smem_push(true), c->stream>>>(a);
+        k_push_deposit<true, false><<<pgrid, kPushWarps * 32, smem_push(true), c->stream>>>(a);
       else
-        k_push_deposit<false, false><<<grid, kWarps * 32, smem_push(false), c->stream>>>(a);
+        k_push_deposit<false, false><<<pgrid, kPushWarps * 32, smem_push(false), c->stream>>>(a);
     }
   }
   e = cudaGetLastError();

@@ -749,14 +749,17 @@ __global__ void __launch_bounds__(256) k_amr_constraint(int nrows, const int* __
 
 // 1 / the Jacobi diagonal that the RHS kernel summed
 __global__ void __launch_bounds__(256) k_amr_invert_diag(long long nvc, Hang h, const double* __restrict__ diag,
-                                                         double* __restrict__ dinv) {
+                                                         double* __restrict__ dinv, float* __restrict__ dff) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nvc) return;
   const bool hang = h.hs[c + 1] > h.hs[c] || is_bnd(h, c);  // constraint rows: scaling 1
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     const float v = (float)diag[d * nvc + c];  // a preconditioner: FP32 reciprocal
-    dinv[d * nvc + c] = (hang || v == 0.f) ? 1.0 : (double)(1.0f / v);
+    const float r = (hang || v == 0.f) ? 1.f : 1.0f / v;
+    dinv[d * nvc + c] = (double)r;
+    dff[d * nvc + c] = r;  // as pairs: FP32 values
+    dff[3 * nvc + d * nvc + c] = 0.f;
   }
 }
 
@@ -770,9 +773,11 @@ __global__ void __launch_bounds__(256) k_amr_update_b(long long ncell, long long
                                                       const double* __restrict__ bdx,
                                                       const double* __restrict__ Eh,
                                                       const double* __restrict__ Bn,
-                                                      double* __restrict__ Bnew, double dt) {
+                                                      double* __restrict__ Bnew, double dt,
+                                                      double* __restrict__ energy) {
   __shared__ double s_e[3][729];
   const int b = blockIdx.x;
+  if (b == 0 && threadIdx.x == 0) *energy = 0.0;  // for k_amr_update_e
   for (int q = threadIdx.x; q < 729; q += 256) {
     const int id = ctabh[b * 729 + q];
 #pragma unroll
@@ -1111,14 +1116,19 @@ static cudaError_t launch_tile32(amps_gpu_ctx* c, const ApplyArgs& a, float* y32
   return cudaGetLastError();
 }
 
-cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y) {
+cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y, bool pairs) {
   cudaError_t e = cudaMemsetAsync(y, 0, sizeof(double) * 3 * c->nvc, c->stream);
   if (e != cudaSuccess) return e;
   ApplyArgs a = apply_args(c);
   a.x = x;
   a.dinv = dinv;
-  TimedLaunch t(c, "matvec", 3);
-  if ((e = split_input(c, x, dinv, a)) != cudaSuccess) return e;
+  TimedLaunch t(c, "matvec", pairs ? 2 : 3);
+  if (pairs) {
+    a.xh = c->d_xs;
+    a.xl = c->d_xs + 3 * c->nvc;
+  } else if ((e = split_input(c, x, dinv, a)) != cudaSuccess) {
+    return e;
+  }
   if ((e = launch_tile<1>(c, a, y)) != cudaSuccess) return e;
   k_amr_constraint<<<g1(std::max(c->nsrows, 1)), 256, 0, c->stream>>>(c->nsrows, c->d_srows, c->nvc, a.h,
                                                                       x, dinv, y, 0, c->d_next);
@@ -1164,14 +1174,14 @@ cudaError_t launch_amr_rhs(amps_gpu_ctx* c, bool diag) {
 
 cudaError_t launch_amr_jacobi(amps_gpu_ctx* c) {
   TimedLaunch t(c, "jacobi");
-  k_amr_invert_diag<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, hang_of(c), c->d_diag, c->d_dinv);
+  k_amr_invert_diag<<<g1(c->nvc), 256, 0, c->stream>>>(c->nvc, hang_of(c), c->d_diag, c->d_dinv, c->d_dff);
   return cudaGetLastError();
 }
 
 cudaError_t launch_amr_update_b(amps_gpu_ctx* c) {
   TimedLaunch t(c, "update_b");
   k_amr_update_b<<<c->nb, 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_ctabh, hang_of(c), c->d_bdx, c->d_Eh,
-                                               c->d_Bc, c->d_Bc2, c->cfg.dt);
+                                               c->d_Bc, c->d_Bc2, c->cfg.dt, c->d_energy + 1);
   if (c->mesh_open) {
     const int* nf = c->amrdev.nfine;
     for (int pass = 0; pass <= (c->neumann ? 3 : 0); pass++)
@@ -1199,8 +1209,7 @@ cudaError_t launch_amr_c2n(amps_gpu_ctx* c, const double* Bcen, double* Bcor) {
 }
 
 cudaError_t launch_amr_update_e(amps_gpu_ctx* c) {
-  cudaError_t e = cudaMemsetAsync(c->d_energy + 1, 0, sizeof(double), c->stream);
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
   TimedLaunch t(c, "update_e", 2);
   const double th = c->cfg.theta;
   const unsigned grid = (unsigned)std::min<long long>((std::max(c->nvc, c->ncor) + 255) / 256, 152LL * 8);

@@ -181,7 +181,7 @@ amps_gpu_status reset_flags(amps_gpu_ctx* c) {
 }
 
 // The launch sequence of one particle step: flag reset, stencil pack, push
-// (+ deposit), arrivals (+ assembly), flag read-back.
+// (+ deposit), arrivals (+ assembly), read-back of the flags and the energy.
 cudaError_t enqueue_particle_step(amps_gpu_ctx* c, bool deposit) {
   cudaError_t e = cudaMemsetAsync(c->d_flags, 0, 7 * sizeof(unsigned long long), c->stream);
   if (e == cudaSuccess) e = launch_pack_stencils(c, c->d_Eh, c->d_Bcor_prev, c->d_Bcor_cur);
@@ -189,6 +189,8 @@ cudaError_t enqueue_particle_step(amps_gpu_ctx* c, bool deposit) {
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(c->h_flags, c->d_flags, 7 * sizeof(unsigned long long),
                         cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess && deposit)
+    e = cudaMemcpyAsync(c->h_energy, c->d_energy, sizeof(double), cudaMemcpyDeviceToHost, c->stream);
   return e;
 }
 
@@ -277,6 +279,10 @@ amps_gpu_status particle_step(amps_gpu_ctx* c, bool deposit, long long* out_of_b
     if ((s = cuda_check(c, particles_place_overflow(c, ovf, deposit, &left), "overflow placement")))
       return s;
     if (left > 0 && (s = cuda_check(c, particles_relayout(c, ovf), "overflow relayout"))) return s;
+    // with the arrivals deposited here
+    if (deposit && (s = cuda_check(c, cudaMemcpyAsync(c->h_energy, c->d_energy, sizeof(double),
+                                                      cudaMemcpyDeviceToHost, c->stream), "energy")))
+      return s;
     if ((s = check_flags(c, nullptr, nullptr, nullptr))) return s;
   }
   if (deposit && (s = cuda_check(c, launch_species_moments(c), "species moments"))) return s;
@@ -320,7 +326,8 @@ bool alloc_context(amps_gpu_ctx* c) {
   ok = ok && !dalloc(&c->d_rhs, 3 * nv) && !dalloc(&c->d_x, 3 * nv) &&
        !dalloc(&c->d_V, (size_t)(c->restart + 1) * ((3 * nv + 3) & ~3LL)) &&
        !dalloc(&c->d_w, (3 * nv + 3) & ~3LL) &&
-       !dalloc(&c->d_dinv, 3 * nv) && !dalloc(&c->d_red, 12288);
+       !dalloc(&c->d_dinv, 3 * nv) && !dalloc(&c->d_red, 12288) &&
+       cudaMemsetAsync(c->d_red, 0, sizeof(double) * 12288, c->stream) == cudaSuccess;
   ok = ok && cudaMallocHost(&c->h_red, 128 * sizeof(double)) == cudaSuccess;
   ok = ok && !dalloc(&c->d_stencil_push, (size_t)c->nb * AMPS_SC * AMPS_PUSH_STRIDE) &&
        !dalloc(&c->d_stencil_dep, (size_t)c->nb * AMPS_SC * AMPS_DEP_STRIDE);
@@ -1010,18 +1017,15 @@ amps_gpu_status amps_gpu_push_deposit(amps_gpu_ctx* c, double* particle_energy) 
   cudaSetDevice(c->cfg.device);
   amps_gpu_status s = particle_step(c, true, nullptr, nullptr);
   if (s) return s;
-  if (particle_energy) {
-    if ((s = cuda_check(c, cudaMemcpy(c->h_energy, c->d_energy, sizeof(double),
-                                      cudaMemcpyDeviceToHost), "energy")))
-      return s;
-    *particle_energy = c->h_energy[0];
-  }
+  if (particle_energy) *particle_energy = c->h_energy[0];
   c->have_moments = true;
   return AMPS_GPU_OK;
 }
 
-amps_gpu_status amps_gpu_field_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
-                                     amps_gpu_solve_stats* stats) {
+// wait: the wave energy in stats is final on return; otherwise it follows in
+// h_energy[1] once the stream has been waited for
+static amps_gpu_status field_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
+                                   amps_gpu_solve_stats* stats, bool wait) {
   if (!c || tol <= 0.0 || maxit <= 0 || precond < 0 || precond > 2)
     return set_err(c, AMPS_GPU_INVALID_ARG, "field_solve: bad arguments");
   cudaSetDevice(c->cfg.device);
@@ -1032,26 +1036,33 @@ amps_gpu_status amps_gpu_field_solve(amps_gpu_ctx* c, double tol, int maxit, int
   const bool watch = precond == 2 || c->amr;
   if (watch && (s = reset_flags(c))) return s;
   if ((s = cuda_check(c, launch_rhs(c, precond != 0), "rhs"))) return s;
-  amps_gpu_status gs = gmres_solve(c, tol, maxit, precond, &st);
+  bool eh_done = false;
+  amps_gpu_status gs = gmres_solve(c, tol, maxit, precond, &st, &eh_done);
   if (gs != AMPS_GPU_OK && gs != AMPS_GPU_GMRES_NOT_CONVERGED) return gs;
   if (watch && (s = check_flags(c, nullptr, nullptr, nullptr))) return s;
   // ProcessFinalSolution: E^{n+theta} = E^n + dE
-  if ((s = cuda_check(c, launch_add(c, c->d_En, c->d_x, c->d_Eh, 3 * c->nvc), "E_half"))) return s;
+  if (!eh_done && (s = cuda_check(c, launch_add(c, c->d_En, c->d_x, c->d_Eh, 3 * c->nvc), "E_half"))) return s;
   if ((s = cuda_check(c, launch_update_b(c), "update_b"))) return s;
   std::swap(c->d_Bc, c->d_Bc2);
   std::swap(c->d_Bcor_prev, c->d_Bcor_cur);
-  if ((s = cuda_check(c, launch_c2n(c, c->d_Bc, c->d_Bcor_cur), "c2n"))) return s;
-  if ((s = cuda_check(c, launch_update_e(c), "update_e"))) return s;
+  if ((s = cuda_check(c, launch_c2n_update_e(c, c->d_Bc, c->d_Bcor_cur), "c2n, update_e"))) return s;
   if ((s = cuda_check(c, cudaMemcpyAsync(c->h_energy + 1, c->d_energy + 1, sizeof(double),
                                          cudaMemcpyDeviceToHost, c->stream), "wave energy")))
     return s;
-  if ((s = cuda_check(c, cudaStreamSynchronize(c->stream), "sync"))) return s;
-  st.wave_energy = c->h_energy[1];
+  if (wait) {
+    if ((s = cuda_check(c, cudaStreamSynchronize(c->stream), "sync"))) return s;
+    st.wave_energy = c->h_energy[1];
+  }
   if (stats) *stats = st;
   if (gs == AMPS_GPU_GMRES_NOT_CONVERGED)
     return set_err(c, gs, "GMRES did not converge: iterations " + std::to_string(st.iterations) +
                               ", relative residual " + std::to_string(st.rel_residual));
   return AMPS_GPU_OK;
+}
+
+amps_gpu_status amps_gpu_field_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
+                                     amps_gpu_solve_stats* stats) {
+  return field_solve(c, tol, maxit, precond, stats, true);
 }
 
 amps_gpu_status amps_gpu_step(amps_gpu_ctx* c, double tol, int maxit, int precond,
@@ -1062,12 +1073,11 @@ amps_gpu_status amps_gpu_step(amps_gpu_ctx* c, double tol, int maxit, int precon
   if (!c->have_moments) {
     if ((s = amps_gpu_update_j_mass_matrix(c, nullptr))) return s;
   }
-  amps_gpu_status fs = amps_gpu_field_solve(c, tol, maxit, precond, &st.solve);
+  amps_gpu_status fs = field_solve(c, tol, maxit, precond, &st.solve, false);
   if (fs != AMPS_GPU_OK && fs != AMPS_GPU_GMRES_NOT_CONVERGED) return fs;
+  // waits for the solve's field update too
   if ((s = particle_step(c, true, &st.out_of_block, &st.ulp_face))) return s;
-  if ((s = cuda_check(c, cudaMemcpy(c->h_energy, c->d_energy, sizeof(double),
-                                    cudaMemcpyDeviceToHost), "energy")))
-    return s;
+  st.solve.wave_energy = c->h_energy[1];
   st.particle_energy = c->h_energy[0];
   c->have_moments = true;
   if (stats) *stats = st;

@@ -324,7 +324,8 @@ cudaError_t launch_export(amps_gpu_ctx* c, double* d_x, double* d_v, uint8_t* d_
 
 // ---- field launchers (field.cu) ----
 cudaError_t launch_rhs(amps_gpu_ctx* c, bool diag);  // diag: for a solve with launch_jacobi_diag
-cudaError_t launch_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y);
+// pairs: d_xs holds x as FP32 pairs already
+cudaError_t launch_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y, bool pairs = false);
 // Input of the inner operator on a Krylov vector: v as FP32 pairs (vh, vl) or,
 // for the flexible directions, as doubles (vd); the scaling D as FP32 pairs
 // (dh, dl) or none.  The operator computes w = A (D v) and writes it as FP32
@@ -344,10 +345,10 @@ cudaError_t launch_in_f32(amps_gpu_ctx* c, const OpIn& in, float* xf);
 cudaError_t launch_amr_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, float* wl);
 cudaError_t launch_jacobi_diag(amps_gpu_ctx* c);
 cudaError_t launch_update_b(amps_gpu_ctx* c);
-cudaError_t launch_c2n(amps_gpu_ctx* c, const double* Bcen, double* Bcor);
-cudaError_t launch_update_e(amps_gpu_ctx* c);
+cudaError_t launch_c2n_update_e(amps_gpu_ctx* c, const double* Bcen, double* Bcor);
+// eh_done: d_Eh holds E^n + x already
 amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
-                            amps_gpu_solve_stats* st);
+                            amps_gpu_solve_stats* st, bool* eh_done);
 // times candidate launch shapes of the operator and reduction kernels on the
 // context's own data and keeps the fastest; ms[6] receives the timings
 amps_gpu_status field_autotune(amps_gpu_ctx* c, double* ms);
@@ -356,7 +357,7 @@ amps_gpu_status field_autotune(amps_gpu_ctx* c, double* ms);
 //      them when the context holds an AMR mesh ----
 cudaError_t launch_amr_pack(amps_gpu_ctx* c, const double* Eh, const double* Bprev,
                             const double* Bcur);
-cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y);
+cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y, bool pairs);
 cudaError_t launch_amr_rhs(amps_gpu_ctx* c, bool diag);
 cudaError_t launch_amr_jacobi(amps_gpu_ctx* c);
 cudaError_t launch_amr_update_b(amps_gpu_ctx* c);

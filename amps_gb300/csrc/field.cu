@@ -15,8 +15,9 @@
 //               re-orthogonalisation; each Arnoldi step is matvec + one
 //               cooperative kernel on FP32-pair vectors (k_arnoldi_tile)
 //               (the external linear_solver_wrapper of LinearSystemCornerNode.h:3282)
-//   k_update_b  UpdateB (:5160-5711), k_c2n InterpolateB_C2N (:5715),
-//   k_update_e  UpdateE with the wave-energy sum (:5909-6001)
+//   k_update_b  UpdateB (:5160-5711)
+//   k_c2n_update_e  InterpolateB_C2N (:5715), UpdateE with the wave-energy sum
+//   (:5909-6001)
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -281,14 +282,20 @@ __global__ void __launch_bounds__(32 * kOpMaxWarps) k_rhs(long long ncor, const 
 }
 
 __global__ void __launch_bounds__(256) k_jacobi(long long ncor, const float* __restrict__ M,
-                                                double* __restrict__ dinv, double k00, double k11,
-                                                double k22, double f) {
+                                                double* __restrict__ dinv, float* __restrict__ dff, double k00,
+                                                double k11, double k22, double f) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncor) return;
   // a preconditioner: FP32 arithmetic (FP64 division is slow on this part)
-  dinv[c] = (double)(1.0f / fmaf((float)f, M[(size_t)0 * ncor + c], (float)k00));
-  dinv[ncor + c] = (double)(1.0f / fmaf((float)f, M[(size_t)4 * ncor + c], (float)k11));
-  dinv[2 * ncor + c] = (double)(1.0f / fmaf((float)f, M[(size_t)8 * ncor + c], (float)k22));
+  const float v[3] = {1.0f / fmaf((float)f, M[(size_t)0 * ncor + c], (float)k00),
+                      1.0f / fmaf((float)f, M[(size_t)4 * ncor + c], (float)k11),
+                      1.0f / fmaf((float)f, M[(size_t)8 * ncor + c], (float)k22)};
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    dinv[d * ncor + c] = (double)v[d];
+    dff[d * ncor + c] = v[d];  // as pairs: FP32 values
+    dff[3 * ncor + d * ncor + c] = 0.f;
+  }
 }
 
 // ---- reductions ------------------------------------------------------------
@@ -318,24 +325,6 @@ __device__ __forceinline__ void block_store_partials(double* acc, int nv, double
   }
 }
 
-__global__ void k_reduce_partials(const double* __restrict__ partial, int nblk, int nv,
-                                  double* __restrict__ out, const double* __restrict__ add) {
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (w >= nv) return;
-  double t = 0.0;
-  for (int bk = lane; bk < nblk; bk += 32) t += partial[bk * kMaxV + w];
-  t = warp_sum(t);
-  if (lane == 0) out[w] = t + (add ? add[w] : 0.0);
-}
-
-// r = b - r (in place on r)
-__global__ void __launch_bounds__(256) k_residual(long long n, const double* __restrict__ b,
-                                                  double* __restrict__ r) {
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x)
-    r[t] = b[t] - r[t];
-}
-
 // x += dinv .* sum_i y_i V_i  (nv from *d_nv when given)
 __global__ void __launch_bounds__(256) k_combine(long long n, const double* __restrict__ V,
                                                  const double* __restrict__ y, int nv,
@@ -354,16 +343,6 @@ __global__ void __launch_bounds__(256) k_combine(long long n, const double* __re
   }
 }
 
-// partial norms of one vector
-__global__ void __launch_bounds__(256) k_norm2(long long n, const double* __restrict__ v,
-                                               double* __restrict__ partial) {
-  double acc[1] = {0.0};
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x)
-    acc[0] += v[t] * v[t];
-  block_store_partials<1>(acc, 1, partial);
-}
-
 // GMRES least-squares state on the device: the Hessenberg columns after the
 // Givens rotations (row stride kMaxV), the rotations, the rotated right-hand
 // side g (|g[j]| = residual norm after j steps), the solution y, and the
@@ -376,7 +355,8 @@ struct GmState {
   double target;
   int jj;    // columns processed in this cycle
   int done;  // |g[jj]| <= target, or breakdown
-  double bn2, rn2;  // graph cycle (k_gm_first, k_gm_status): ||b||^2, end-of-cycle ||r||^2
+  double bn2, rn2;  // ||b||^2 (k_first), end-of-cycle ||r||^2 (k_residual)
+  unsigned ticket;  // CTAs of a reducing kernel that have stored their share (0 between kernels)
 };
 static_assert(kGmOffset * sizeof(double) + sizeof(GmState) <= 12288 * sizeof(double),
               "GmState must fit in d_red");
@@ -392,23 +372,75 @@ __global__ void k_gm_start(GmState* __restrict__ S, const double* __restrict__ n
   S->done = 0;
 }
 
-// start of the first cycle from x0 = 0 (r = b): g = (||b||, 0, ...), target
-// tol ||b|| on the device; keeps ||b||^2 for the host's single read
-__global__ void k_gm_first(GmState* __restrict__ S, const double* __restrict__ n2, double tol) {
-  if (threadIdx.x != 0) return;
-  for (int i = 0; i <= kMaxV; i++) S->g[i] = 0.0;
-  const double b2 = *n2;
-  S->g[0] = sqrt(b2);
-  S->target = tol * sqrt(b2);
-  S->jj = 0;
-  S->done = 0;
-  S->bn2 = b2;
-  S->rn2 = -1.0;
+// Sum of acc over the grid, returned in every thread of the CTA that stores its share
+// last (true there); partial sums are added in the order of the CTAs.  256 threads.
+__device__ __forceinline__ bool grid_sum(double acc, double* __restrict__ partial, unsigned* ticket, double& sum) {
+  __shared__ double s_sum;
+  __shared__ int s_last;
+  double a[1] = {acc};
+  block_store_partials<1>(a, 1, partial);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return false;
+  __threadfence();
+  if (threadIdx.x < 32) {
+    double t = 0.0;
+    for (int bk = threadIdx.x; bk < (int)gridDim.x; bk += 32) t += __ldcg(partial + bk * kMaxV);
+    t = warp_sum(t);
+    if (threadIdx.x == 0) {
+      s_sum = t;
+      *ticket = 0u;
+    }
+  }
+  __syncthreads();
+  sum = s_sum;
+  return true;
 }
 
-// end of the graph cycle: the true residual's ||r||^2 next to jj, done, ||b||^2
-__global__ void k_gm_status(GmState* __restrict__ S, const double* __restrict__ n2) {
-  if (threadIdx.x == 0) S->rn2 = *n2;
+// Start of a solve from x0 = 0: r = b (in w), x = 0, ||b||^2, and the state of a first
+// cycle with the target tol ||b||.  (One launch: the copy, the clearing, the norm, its
+// reduction and the state took five, ~4 us each on a small mesh.)
+__global__ void __launch_bounds__(256) k_first(long long n, const double* __restrict__ b, double* __restrict__ w,
+                                               double* __restrict__ x, double* __restrict__ partial,
+                                               double* __restrict__ n2, GmState* __restrict__ S, double tol) {
+  double acc = 0.0;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
+       t += (long long)gridDim.x * blockDim.x) {
+    const double v = b[t];
+    w[t] = v;
+    x[t] = 0.0;
+    acc += v * v;
+  }
+  double b2;
+  if (!grid_sum(acc, partial, &S->ticket, b2)) return;
+  if (threadIdx.x <= kMaxV) S->g[threadIdx.x] = threadIdx.x == 0 ? sqrt(b2) : 0.0;
+  if (threadIdx.x == 0) {
+    *n2 = b2;
+    S->target = tol * sqrt(b2);
+    S->jj = 0;
+    S->done = 0;
+    S->bn2 = b2;
+    S->rn2 = -1.0;
+  }
+}
+
+// r = b - r (in place on r) and ||r||^2
+__global__ void __launch_bounds__(256) k_residual(long long n, const double* __restrict__ b,
+                                                  double* __restrict__ r, double* __restrict__ partial,
+                                                  double* __restrict__ n2, GmState* __restrict__ S) {
+  double acc = 0.0;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
+       t += (long long)gridDim.x * blockDim.x) {
+    const double v = b[t] - r[t];
+    r[t] = v;
+    acc += v * v;
+  }
+  double r2;
+  if (!grid_sum(acc, partial, &S->ticket, r2) || threadIdx.x != 0) return;
+  *n2 = r2;
+  S->rn2 = r2;
 }
 
 // Arnoldi column jj: h = h1 + h2 (the two CGS passes), h[jj+1] = ||w||; apply
@@ -440,16 +472,32 @@ __device__ void gm_update(GmState* __restrict__ S, int jj, const double* h1, con
   if (fabs(S->g[jj + 1]) <= S->target || hn == 0.0) S->done = 1;
 }
 
-// y = R^-1 g on the processed columns (back substitution)
-__global__ void k_gm_solve(GmState* __restrict__ S) {
-  if (threadIdx.x != 0) return;
-  const int j = S->jj;
-  for (int i = j - 1; i >= 0; i--) {
-    double t = S->g[i];
-    for (int q = i + 1; q < j; q++) t -= S->H[i * kMaxV + q] * S->y[q];
-    const double d = S->H[i * kMaxV + i];
-    S->y[i] = d != 0.0 ? t / d : 0.0;
+// y = R^-1 g on the processed columns, by the whole CTA: R staged, then one lane per
+// row and a back substitution by columns (reciprocals of the diagonal first, so the
+// chain holds a product and an FMA per column).  s_y: kMaxV values.
+__device__ __forceinline__ void gm_solve(const GmState* __restrict__ S, double* s_y) {
+  __shared__ double s_h[kMaxV][kMaxV + 1];
+  const int j = min(S->jj, kMaxV);
+  for (int q = threadIdx.x; q < j * j; q += blockDim.x) s_h[q / j][q % j] = S->H[(q / j) * kMaxV + q % j];
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const double d = lane < j ? s_h[lane][lane] : 0.0;
+    const double inv = d != 0.0 ? 1.0 / d : 0.0;
+    double g = lane < j ? S->g[lane] : 0.0;
+    for (int i = j - 1; i >= 0; i--) {
+      const double y = __shfl_sync(0xffffffffu, g * inv, i);
+      if (lane == i) g = y;
+      if (lane < i) g -= s_h[lane][i] * y;
+    }
+    s_y[lane] = g;
   }
+  __syncthreads();
+}
+__global__ void __launch_bounds__(256) k_gm_solve(GmState* __restrict__ S) {
+  __shared__ double s_y[kMaxV];
+  gm_solve(S, s_y);
+  if (threadIdx.x < kMaxV) S->y[threadIdx.x] = s_y[threadIdx.x];
 }
 
 // ---- Krylov vectors in FP32 pairs ----------------------------------------------
@@ -984,19 +1032,23 @@ __global__ void __launch_bounds__(256) k_from_ff(long long n, const float* __res
     x[t] = (double)v[t] + (double)v[ff_ld(n) + t];
 }
 
-// x += D sum_i y_i V_i, V pair vectors, D as pairs (or none); nv from *d_nv
-// (at most NVM: the loads of all vectors are issued before the pair sums)
+// x += D sum_i y_i V_i with y of the least-squares state, V pair vectors, D as pairs (or
+// none); at most NVM vectors (the loads of all of them are issued before the pair
+// sums).  Every CTA solves for y itself (a launch less); xs (optional): the new x as
+// pairs, the input of the residual's operator; eo (optional): en + x, E^{n+theta}.
 template <int NVM>
 __global__ void __launch_bounds__(256) k_combine_ff(long long n, const float* __restrict__ V,
-                                                    const double* __restrict__ y,
-                                                    const int* __restrict__ d_nv,
-                                                    const float* __restrict__ dff,
-                                                    double* __restrict__ x) {
+                                                    const GmState* __restrict__ S,
+                                                    const float* __restrict__ dff, double* __restrict__ x,
+                                                    float* __restrict__ xs, const double* __restrict__ en,
+                                                    double* __restrict__ eo) {
   __shared__ float s_y[kMaxV][2];
+  __shared__ double s_yd[kMaxV];
   const long long ld = ff_ld(n);
-  const int nv = min(*d_nv, NVM);
+  const int nv = min(S->jj, NVM);
+  gm_solve(S, s_yd);
   if (threadIdx.x < kMaxV) {
-    const double v = threadIdx.x < nv ? y[threadIdx.x] : 0.0;
+    const double v = threadIdx.x < nv ? s_yd[threadIdx.x] : 0.0;
     s_y[threadIdx.x][0] = (float)v;
     s_y[threadIdx.x][1] = (float)(v - (double)s_y[threadIdx.x][0]);
   }
@@ -1019,30 +1071,27 @@ __global__ void __launch_bounds__(256) k_combine_ff(long long n, const float* __
       }
     a = ff_norm(a);
     if (dff) a = ff_mul(a.s, a.q, dff[t], dff[n + t]);
-    x[t] += ff_value(a);
+    const double v = x[t] + ff_value(a);
+    x[t] = v;
+    if (eo) eo[t] = en[t] + v;
+    if (xs) {
+      const float h = (float)v;
+      xs[t] = h;
+      xs[n + t] = (float)(v - (double)h);
+    }
   }
 }
 
-void launch_combine_ff(cudaStream_t s, unsigned gr, long long n, const float* V, const double* y,
-                       const int* d_nv, int nv_host, const float* dff, double* x) {
+void launch_combine_ff(cudaStream_t s, unsigned gr, long long n, const float* V, const GmState* S, int nv_host,
+                       const float* dff, double* x, float* xs, const double* en, double* eo) {
   if (nv_host <= 4)
-    k_combine_ff<4><<<gr, 256, 0, s>>>(n, V, y, d_nv, dff, x);
+    k_combine_ff<4><<<gr, 256, 0, s>>>(n, V, S, dff, x, xs, en, eo);
   else if (nv_host <= 8)
-    k_combine_ff<8><<<gr, 256, 0, s>>>(n, V, y, d_nv, dff, x);
+    k_combine_ff<8><<<gr, 256, 0, s>>>(n, V, S, dff, x, xs, en, eo);
   else if (nv_host <= 16)
-    k_combine_ff<16><<<gr, 256, 0, s>>>(n, V, y, d_nv, dff, x);
+    k_combine_ff<16><<<gr, 256, 0, s>>>(n, V, S, dff, x, xs, en, eo);
   else
-    k_combine_ff<32><<<gr, 256, 0, s>>>(n, V, y, d_nv, dff, x);
-}
-
-// the Jacobi scaling D as pairs
-__global__ void __launch_bounds__(256) k_dff(long long n, const double* __restrict__ d, float* __restrict__ v) {
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const float h = (float)d[t];
-    v[t] = h;
-    v[n + t] = (float)(d[t] - (double)h);
-  }
+    k_combine_ff<32><<<gr, 256, 0, s>>>(n, V, S, dff, x, xs, en, eo);
 }
 
 // xf = fp32(D v)
@@ -1102,8 +1151,9 @@ __global__ void __launch_bounds__(256) k_update_b(long long ncor, const int* __r
                                                   const double* __restrict__ Eh,
                                                   const double* __restrict__ Bn,
                                                   double* __restrict__ Bnew, double c4x,
-                                                  double c4y, double c4z) {
+                                                  double c4y, double c4z, double* __restrict__ energy) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c == 0) *energy = 0.0;  // for k_c2n_update_e
   if (c >= ncor) return;
   int b, i, j, k;
   corner_ijk(c, b, i, j, k);
@@ -1133,43 +1183,41 @@ __global__ void __launch_bounds__(256) k_update_b(long long ncor, const int* __r
   Bnew[2 * ncor + c] = Bn[2 * ncor + c] + t2;
 }
 
-__global__ void __launch_bounds__(256) k_c2n(long long ncor, const int* __restrict__ nbr,
-                                             const double* __restrict__ Bc,
-                                             double* __restrict__ Bcor) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncor) return;
-  int b, i, j, k;
-  corner_ijk(c, b, i, j, k);
-  double t[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-  for (int kk = -1; kk <= 0; kk++)
-#pragma unroll
-    for (int jj = -1; jj <= 0; jj++)
-#pragma unroll
-      for (int ii = -1; ii <= 0; ii++) {
-        const int id = local_id(nbr, b, i + ii, j + jj, k + kk);
-#pragma unroll
-        for (int d = 0; d < 3; d++) t[d] += Bc[d * ncor + id];
-      }
-#pragma unroll
-  for (int d = 0; d < 3; d++) Bcor[d * ncor + c] = t[d] / 8.0;
-}
-
-__global__ void __launch_bounds__(256) k_update_e(long long ncor, const double* __restrict__ Eh,
-                                                  double* __restrict__ En,
-                                                  const double* __restrict__ Bc, double theta,
-                                                  double vol_over_8pi, double* __restrict__ energy) {
+// Corner B^{n+1} from the 8 cells of a corner, E^{n+1} and the wave energy: one thread
+// per corner and cell (one launch: each of the two took 5 us on a small mesh, most of
+// it its own start)
+__global__ void __launch_bounds__(256) k_c2n_update_e(long long ncor, const int* __restrict__ nbr,
+                                                      const double* __restrict__ Bc,
+                                                      double* __restrict__ Bcor,
+                                                      const double* __restrict__ Eh, double* __restrict__ En,
+                                                      double theta, double vol_over_8pi,
+                                                      double* __restrict__ energy) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double en = 0.0;
   if (c < ncor) {
-    double e2 = 0.0, b2 = 0.0;
+    int b, i, j, k;
+    corner_ijk(c, b, i, j, k);
+    double t[3] = {0.0, 0.0, 0.0}, b2 = 0.0, e2 = 0.0;
+#pragma unroll
+    for (int kk = -1; kk <= 0; kk++)
+#pragma unroll
+      for (int jj = -1; jj <= 0; jj++)
+#pragma unroll
+        for (int ii = -1; ii <= 0; ii++) {
+          const int id = local_id(nbr, b, i + ii, j + jj, k + kk);
+#pragma unroll
+          for (int d = 0; d < 3; d++) {
+            const double v = Bc[d * ncor + id];
+            t[d] += v;
+            if (ii == 0 && jj == 0 && kk == 0) b2 += v * v;  // cell c itself
+          }
+        }
 #pragma unroll
     for (int d = 0; d < 3; d++) {
+      Bcor[d * ncor + c] = t[d] * 0.125;
       const double e = (Eh[d * ncor + c] - (1.0 - theta) * En[d * ncor + c]) / theta;
       En[d * ncor + c] = e;
       e2 += e * e;
-      const double bb = Bc[d * ncor + c];
-      b2 += bb * bb;
     }
     en = (e2 + b2) * vol_over_8pi;
   }
@@ -1216,11 +1264,11 @@ static cudaError_t split_input(amps_gpu_ctx* c, const double* x, const double* d
   return cudaGetLastError();
 }
 
-cudaError_t launch_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y) {
-  if (c->amr) return launch_amr_matvec(c, x, dinv, y);
+cudaError_t launch_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, double* y, bool pairs) {
+  if (c->amr) return launch_amr_matvec(c, x, dinv, y, pairs);
   const TapsFF T = taps_ff(make_taps(c->cfg, true));
-  TimedLaunch t(c, "matvec", 2);
-  cudaError_t e = split_input(c, x, dinv);
+  TimedLaunch t(c, "matvec", pairs ? 1 : 2);
+  cudaError_t e = pairs ? cudaSuccess : split_input(c, x, dinv);
   if (e != cudaSuccess) return e;
   const long long n = 3 * c->ncor;
   k_matvec<<<(unsigned)(c->ncor / 32), c->tune_tb, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_M, c->d_xs,
@@ -1269,7 +1317,7 @@ cudaError_t launch_jacobi_diag(amps_gpu_ctx* c) {
   if (c->amr) return launch_amr_jacobi(c);
   Taps T = make_taps(c->cfg, true);
   TimedLaunch t(c, "jacobi");
-  k_jacobi<<<grid1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->d_M, c->d_dinv, T.K[0][0][0],
+  k_jacobi<<<grid1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->d_M, c->d_dinv, c->d_dff, T.K[0][0][0],
                                                    T.K[1][1][0], T.K[2][2][0], T.f);
   return cudaGetLastError();
 }
@@ -1280,26 +1328,20 @@ cudaError_t launch_update_b(amps_gpu_ctx* c) {
   for (int d = 0; d < 3; d++) c4[d] = 0.25 * (c->cfg.dt / c->cfg.dx[d]);
   TimedLaunch t(c, "update_b");
   k_update_b<<<grid1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_Eh, c->d_Bc,
-                                                     c->d_Bc2, c4[0], c4[1], c4[2]);
+                                                     c->d_Bc2, c4[0], c4[1], c4[2], c->d_energy + 1);
   return cudaGetLastError();
 }
 
-cudaError_t launch_c2n(amps_gpu_ctx* c, const double* Bcen, double* Bcor) {
-  if (c->amr) return launch_amr_c2n(c, Bcen, Bcor);
-  TimedLaunch t(c, "c2n");
-  k_c2n<<<grid1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->d_nbr, Bcen, Bcor);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_update_e(amps_gpu_ctx* c) {
-  if (c->amr) return launch_amr_update_e(c);
+// after launch_update_b, which clears the wave energy
+cudaError_t launch_c2n_update_e(amps_gpu_ctx* c, const double* Bcen, double* Bcor) {
+  if (c->amr) {
+    const cudaError_t e = launch_amr_c2n(c, Bcen, Bcor);
+    return e == cudaSuccess ? launch_amr_update_e(c) : e;
+  }
   const double vol = c->cfg.dx[0] * c->cfg.dx[1] * c->cfg.dx[2];
-  cudaError_t e = cudaMemsetAsync(c->d_energy + 1, 0, sizeof(double), c->stream);
-  if (e != cudaSuccess) return e;
-  TimedLaunch t(c, "update_e");
-  k_update_e<<<grid1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->d_Eh, c->d_En, c->d_Bc,
-                                                     c->cfg.theta, vol * 0.125 / kPi,
-                                                     c->d_energy + 1);
+  TimedLaunch t(c, "c2n_update_e");
+  k_c2n_update_e<<<grid1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->d_nbr, Bcen, Bcor, c->d_Eh, c->d_En,
+                                                        c->cfg.theta, vol / (8.0 * kPi), c->d_energy + 1);
   return cudaGetLastError();
 }
 
@@ -1319,7 +1361,7 @@ cudaError_t launch_update_e(amps_gpu_ctx* c) {
 // Device scratch layout of d_red: [0, kRedBlocks*kMaxV) partials, then h1
 // (kMaxV), h2 (kMaxV), nrm2 (8), y (kMaxV); GmState at kGmOffset.
 amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
-                            amps_gpu_solve_stats* st) {
+                            amps_gpu_solve_stats* st, bool* eh_done) {
   const long long n = 3 * c->nvc;
   const int m = std::min(c->restart, kMaxV);
   double* partial = c->d_red;
@@ -1363,7 +1405,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
   // (nothing that writes d_xs -- split_input, k_rhs, the AMR operators -- runs
   // between a step that writes it and the inner_matvec that reads it)
   const bool pre_xf = !flexible && c->inner_fp32;
-  if (pre_xf && !c->d_xs) CK(cudaMalloc(reinterpret_cast<void**>(&c->d_xs), sizeof(float) * 2 * n));
+  if (!c->d_xs) CK(cudaMalloc(reinterpret_cast<void**>(&c->d_xs), sizeof(float) * 2 * n));
   float* xf_next = pre_xf ? c->d_xs : nullptr;
   auto inner_matvec = [&](int jj, const double* zj) -> cudaError_t {
     if (c->inner_fp32) {
@@ -1390,29 +1432,15 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     k_to_ff<<<gr, 256, 0, s>>>(n, c->d_tmpv + n, wf);
     return cudaGetLastError();
   };
-  auto norm_to = [&](const double* v) {
-    k_norm2<<<gr, 256, 0, s>>>(n, v, partial);
-    k_reduce_partials<<<1, 32, 0, s>>>(partial, gr, 1, d_n2, nullptr);
-  };
-  auto read_norm = [&](const double* v, double* out) -> cudaError_t {
-    norm_to(v);
-    cudaError_t ee = cudaMemcpyAsync(c->h_red, d_n2, sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (ee != cudaSuccess) return ee;
-    ee = cudaStreamSynchronize(s);
-    *out = std::sqrt(c->h_red[0]);
-    return ee;
-  };
-  // the Jacobi scaling, x0 = 0, r0 = b
+  double* w = c->d_w;  // between cycles: the FP64 residual
+  // the Jacobi scaling, x0 = 0, r0 = b, ||b|| and the first cycle's state
   auto prologue = [&]() -> cudaError_t {
     if (dinv) {
       cudaError_t ee = launch_jacobi_diag(c);
       if (ee != cudaSuccess) return ee;
-      k_dff<<<gr, 256, 0, s>>>(n, dinv, c->d_dff);
     }
-    cudaError_t ee = cudaMemsetAsync(c->d_x, 0, sizeof(double) * n, s);
-    if (ee == cudaSuccess)
-      ee = cudaMemcpyAsync(c->d_w, c->d_rhs, sizeof(double) * n, cudaMemcpyDeviceToDevice, s);
-    return ee;
+    k_first<<<gr, 256, 0, s>>>(n, c->d_rhs, w, c->d_x, partial, d_n2, gs, tol);
+    return cudaGetLastError();
   };
   // Arnoldi step jj: the operator (after the network for flexible directions),
   // then the cooperative CGS2 + normalisation + Givens step
@@ -1436,20 +1464,20 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     TimedLaunch t(c, "gmres_orth");
     return launch_arnoldi(s, n, Vf, wf, nv, vf(nv), c->d_arn, gs, jj, xf_next, dh, c->d_flags);
   };
-  // end of a cycle of at most nv_max steps: least squares, x += (D) V y, the
-  // true FP64 residual into w and its squared norm into d_n2
-  double* w = c->d_w;  // between cycles: the FP64 residual
+  // end of a cycle of at most nv_max steps: least squares, x += (D) V y (with its pairs
+  // in d_xs and E^{n+theta} = E^n + x), the true FP64 residual into w and its squared
+  // norm into d_n2
   auto cycle_end = [&](int nv_max) -> cudaError_t {
-    k_gm_solve<<<1, 32, 0, s>>>(gs);
-    if (flexible)
+    if (flexible) {
+      k_gm_solve<<<1, 256, 0, s>>>(gs);
       k_combine<<<gr, 256, 0, s>>>(n, c->d_Z, gs->y, kMaxV, &gs->jj, nullptr, c->d_x);
-    else
-      launch_combine_ff(s, gr, n, Vf, gs->y, &gs->jj, nv_max, dinv ? c->d_dff : nullptr, c->d_x);
+    } else {
+      launch_combine_ff(s, gr, n, Vf, gs, nv_max, dinv ? c->d_dff : nullptr, c->d_x, c->d_xs, c->d_En, c->d_Eh);
+    }
     cudaError_t ee = cudaGetLastError();
-    if (ee == cudaSuccess) ee = launch_matvec(c, c->d_x, nullptr, w);
+    if (ee == cudaSuccess) ee = launch_matvec(c, c->d_x, nullptr, w, !flexible);
     if (ee != cudaSuccess) return ee;
-    k_residual<<<gr, 256, 0, s>>>(n, c->d_rhs, w);
-    norm_to(w);
+    k_residual<<<gr, 256, 0, s>>>(n, c->d_rhs, w, partial, d_n2, gs);
     return cudaGetLastError();
   };
 
@@ -1478,17 +1506,13 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
       if (ee == cudaSuccess) {
         cudaError_t e1 = prologue();
         if (e1 == cudaSuccess) {
-          norm_to(c->d_rhs);
-          k_gm_first<<<1, 32, 0, s>>>(gs, d_n2, tol);
           k_start_ff<<<gr, 256, 0, s>>>(n, w, d_n2, vf(0), xf_next, dh);
           for (int jj = 0; jj < K && e1 == cudaSuccess; jj++) e1 = arnoldi_step(jj);
         }
         if (e1 == cudaSuccess) e1 = cycle_end(K);
-        if (e1 == cudaSuccess) {
-          k_gm_status<<<1, 32, 0, s>>>(gs, d_n2);
+        if (e1 == cudaSuccess)
           e1 = cudaMemcpyAsync(c->h_red, &gs->jj, 2 * sizeof(int) + 2 * sizeof(double),
                                cudaMemcpyDeviceToHost, s);
-        }
         ee = cudaStreamEndCapture(s, &gr_cap);
         if (ee == cudaSuccess && e1 == cudaSuccess)
           ee = cudaGraphInstantiate(&exec, gr_cap, 0);
@@ -1522,8 +1546,9 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
   }
   if (!graph_done) {
     CK(prologue());
-    CK(read_norm(c->d_rhs, &bnorm));
-    beta = bnorm;
+    CK(cudaMemcpyAsync(c->h_red, d_n2, sizeof(double), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    beta = bnorm = std::sqrt(c->h_red[0]);
   }
   while (true) {
     rel = bnorm > 0.0 ? beta / bnorm : 0.0;
@@ -1560,6 +1585,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     CK(cudaStreamSynchronize(s));
     beta = std::sqrt(c->h_red[0]);
   }
+  *eh_done = cycles > 0 && !flexible;  // cycle_end left E^n + x in d_Eh
   // the next solve's first cycle queues as many steps as this solve took
   if (conv) c->gm_guess[precond] = std::max(1, std::min(it, m));
   // the solve's own pair (b, x)
@@ -1620,17 +1646,17 @@ amps_gpu_status field_autotune(amps_gpu_ctx* c, double* ms) {
   // the shape of the solve's grid-stride vector passes
   GmState* gs = reinterpret_cast<GmState*>(c->d_red + kGmOffset);
   const int eight = 8;
+  if ((e = cudaMemsetAsync(gs, 0, sizeof(GmState), s)) != cudaSuccess) fail(e, "autotune");
   if ((e = cudaMemcpyAsync(&gs->jj, &eight, sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess)
     fail(e, "autotune");
-  if ((e = cudaMemsetAsync(gs->y, 0, sizeof(gs->y), s)) != cudaSuccess) fail(e, "autotune");
   const float* Vf = reinterpret_cast<const float*>(c->d_V);
   best = 1e30;
   int best_cap = c->tune_red;
   for (int q = 0; q < 3 && !st; q++) {
     const unsigned gr = gridr(n, caps[q], 4);
-    launch_combine_ff(s, gr, n, Vf, gs->y, &gs->jj, 8, nullptr, x);
+    launch_combine_ff(s, gr, n, Vf, gs, 8, nullptr, x, nullptr, nullptr, nullptr);
     cudaEventRecord(a, s);
-    for (int r = 0; r < 5; r++) launch_combine_ff(s, gr, n, Vf, gs->y, &gs->jj, 8, nullptr, x);
+    for (int r = 0; r < 5; r++) launch_combine_ff(s, gr, n, Vf, gs, 8, nullptr, x, nullptr, nullptr, nullptr);
     cudaEventRecord(b, s);
     if ((e = cudaEventSynchronize(b)) != cudaSuccess) fail(e, "autotune sweep");
     float t = 0.f;

@@ -22,10 +22,8 @@
 namespace {
 
 constexpr double kPi = 3.14159265358979323846264338327950288;
-__constant__ int c_off[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
-                                {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
-
-// offset bit d of corner c in the table order above
+// offset bit d of corner c of a cell, in the order (x, y) = (0,0) (1,0) (1,1) (0,1)
+// on the lower face, then on the upper
 __host__ __device__ constexpr int off_bit(int c, int d) {
   return d == 0 ? (((c + 1) >> 1) & 1) : (d == 1 ? ((c >> 1) & 1) : (c >> 2));
 }
@@ -139,88 +137,108 @@ constexpr int kTileCells = 32;
 constexpr int kTileThreads = 3 * kTileCells;
 constexpr uint32_t kTileBytes = kTileCells * AMPS_CELLM * 4;  // 31,104
 constexpr int kTC = 90;  // tile corners, (i, j, k) at i + 9 (j + 5 k)
+constexpr int kT32Threads = 2 * kTileThreads;
 
 // The FP32 inner operator (curl-curl + mass; identity added in pairs by
 // k_amr_finish_ff).  Bound: reading the partials (478 MB at 491,520 cells).
-// Persistent CTAs, three per SM with two tile buffers each: the next tile's
-// bulk copy, its corner values and the corner ids of the one after are in
-// flight while a tile is computed (one tile per CTA, six CTAs per SM, held its
-// buffer through the whole chain of dependent loads: 3.8 TB/s).  Each corner
-// value is gathered once per tile; the corner table carries hanging corners as
-// ~id, so the common corner needs no look at the constraint rows.  The cells'
-// contributions to a corner are added by shuffles along x and y, and go out as
+// Persistent CTAs, three per SM with two tile buffers each.  Three producer warps
+// gather a tile's 90 corner values (once each; the corner table carries hanging
+// corners as ~id, so the common corner needs no look at the constraint rows) and
+// start the bulk copy of its partials as soon as a buffer is free; three consumer
+// warps, one output component each, wait for nothing but the buffer.  (With the
+// gather in the computing warps and two CTA barriers per tile: 94 us; one tile per
+// CTA, which held its buffer through the whole chain of dependent loads: 132; tiles
+// of 16 cells, six CTAs per SM: 106, as a tile's chain does not shrink with it.)  The
+// cells' contributions to a corner are added by shuffles along x and y, and go out as
 // one global reduction per tile corner and component (P^T for hanging ones).
-// 491,520 cells: 94 us (5.1 TB/s), before 132.
-__global__ void __launch_bounds__(kTileThreads) k_amr_tile32(ApplyArgs a, int tiles, float* __restrict__ y32) {
+// 491,520 cells: 84 us (5.9 TB/s).
+__global__ void __launch_bounds__(kT32Threads) k_amr_tile32(ApplyArgs a, int tiles, float* __restrict__ y32) {
   extern __shared__ __align__(16) float s_m[];  // two tiles of partials
-  __shared__ __align__(8) uint64_t bar[2];
-  __shared__ float s_x[3][kTC];
-  __shared__ int s_id[kTC];
-  const int tid = threadIdx.x, p = tid / 32, lane = tid & 31;
+  // tx: a tile's partials have landed; val: its corners are stored (3 warps); empty:
+  // the 3 consumer warps have read both
+  __shared__ __align__(8) uint64_t tx[2], val[2], empty[2];
+  __shared__ float s_x[2][3][kTC];
+  __shared__ int s_id[2][kTC];
+  const int tid = threadIdx.x, p = tid / 32 % 3, lane = tid & 31;
   const int step = gridDim.x;
   if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
+    for (int q = 0; q < 2; q++) {
+      mbar_init(&tx[q], 1);
+      mbar_init(&val[q], 3);
+      mbar_init(&empty[q], 3);
+    }
     fence_mbar_init();
   }
   __syncthreads();
-  auto copy = [&](int tile, int buf) {
-    mbar_arrive_expect_tx(&bar[buf], kTileBytes);
-    bulk_copy_g2s(s_m + (size_t)buf * (kTileBytes / 4), a.cellM + (size_t)tile * kTileCells * AMPS_CELLM,
-                  kTileBytes, &bar[buf]);
+  auto arrive = [&](uint64_t* bar) {
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
   };
-  // thread t < 90 owns tile corner t
-  const int ti = tid % 9, tj = (tid / 9) % 5, tk = tid / 45;
-  auto corner_id = [&](int tile) {
-    if (tile >= tiles || tid >= kTC) return 0;
-    const int b = tile >> 4, l = (tile & 15) * kTileCells;  // 16 tiles per block
-    return __ldg(a.ctabh + b * 729 + ti + 9 * (((l >> 3) & 7) + tj + 9 * ((l >> 6) + tk)));
+  // a wait that runs out is counted, and the warp leaves its loop
+  auto wait = [&](uint64_t* bar, int phase) {
+    const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase, kWaitLimit)) != 0;
+    if (!ok && lane == 0) atomicAdd(a.flags + 2, 1ull);
+    return ok;
   };
-  auto corner_values = [&](int id, float (&x)[3]) {
-    if (id >= 0) {
+  if (tid >= kTileThreads) {
+    // ---- producers: warp p brings 30 of a tile's 90 corners, the first the partials
+    const int t = 30 * p + lane, ti = t % 9, tj = (t / 9) % 5, tk = t / 45;
+    const bool act = lane < 30;
+    auto corner_id = [&](int tile) {
+      if (tile >= tiles || !act) return 0;
+      const int b = tile >> 4, l = (tile & 15) * kTileCells;  // 16 tiles per block
+      return __ldg(a.ctabh + b * 729 + ti + 9 * (((l >> 3) & 7) + tj + 9 * ((l >> 6) + tk)));
+    };
+    float x[3] = {0.f, 0.f, 0.f};
+    auto corner_values = [&](int id) {
+      if (!act) return;
+      if (id >= 0) {
 #pragma unroll
-      for (int d = 0; d < 3; d++) x[d] = a.xf[d * a.nvc + id];
-    } else {
-      const int h = ~id, s = a.h.hs[h], e = a.h.hs[h + 1];
+        for (int d = 0; d < 3; d++) x[d] = a.xf[d * a.nvc + id];
+      } else {
+        const int h = ~id, s = a.h.hs[h], e = a.h.hs[h + 1];
 #pragma unroll
-      for (int d = 0; d < 3; d++) x[d] = 0.f;
-      for (int t = s; t < e; t++) {
-        const float w = a.h.hwh[t];
-        const int q = a.h.hp[t];
+        for (int d = 0; d < 3; d++) x[d] = 0.f;
+        for (int r = s; r < e; r++) {
+          const float w = a.h.hwh[r];
+          const int q = a.h.hp[r];
 #pragma unroll
-        for (int d = 0; d < 3; d++) x[d] = fmaf(w, a.xf[d * a.nvc + q], x[d]);
+          for (int d = 0; d < 3; d++) x[d] = fmaf(w, a.xf[d * a.nvc + q], x[d]);
+        }
       }
-    }
-  };
-  int tile = blockIdx.x;  // grid <= tiles
-  if (tid == 0) copy(tile, 0);
-  int id = corner_id(tile), id1 = corner_id(tile + step);
-  float x[3] = {0.f, 0.f, 0.f};
-  if (tid < kTC) corner_values(id, x);
-  int n = 0;  // tiles done
-  for (; tile < tiles; tile += step, n++) {
-    const int buf = n & 1;
-    const bool more = tile + step < tiles;
-    if (tid == 0 && more) copy(tile + step, buf ^ 1);
-    if (tid < kTC) {
-      s_id[tid] = id;
+    };
+    int id = corner_id(blockIdx.x), n = 0;
+    corner_values(id);
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < tiles; tile += step, n++) {
+      const int buf = n & 1;
+      const int idn = corner_id(tile + step);
+      if (n >= 2) ok = wait(&empty[buf], ((n >> 1) - 1) & 1);
+      if (!ok) break;
+      if (p == 0 && lane == 0) {
+        mbar_arrive_expect_tx(&tx[buf], kTileBytes);
+        bulk_copy_g2s(s_m + (size_t)buf * (kTileBytes / 4), a.cellM + (size_t)tile * kTileCells * AMPS_CELLM,
+                      kTileBytes, &tx[buf]);
+      }
+      if (act) {
+        s_id[buf][t] = id;
 #pragma unroll
-      for (int d = 0; d < 3; d++) s_x[d][tid] = x[d];
+        for (int d = 0; d < 3; d++) s_x[buf][d][t] = x[d];
+      }
+      arrive(&val[buf]);
+      id = idn;
+      if (tile + step < tiles) corner_values(id);
     }
-    // in flight over this tile's arithmetic
-    const int id2 = corner_id(tile + 2 * step);
-    if (tid < kTC && more) corner_values(id1, x);
-    id = id1;
-    id1 = id2;
-    // CTA-uniform: every thread leaves together on a timeout
-    const bool ok = __syncthreads_and(mbar_wait_bounded(&bar[buf], (n >> 1) & 1, kWaitLimit)) != 0;
-    if (!ok) {
-      if (tid == 0) atomicAdd(a.flags + 2, 1ull);
-      // let the copies land before exiting
-      mbar_wait_bounded(&bar[buf], (n >> 1) & 1, kWaitLimit);
-      if (more) mbar_wait_bounded(&bar[buf ^ 1], ((n + 1) >> 1) & 1, kWaitLimit);
-      return;
-    }
+    // the last copies land before the CTA's shared memory goes, whoever gave up
+    if (p == 0)
+      for (int q = max(0, n - 2); q < n; q++) mbar_wait_bounded(&tx[q & 1], (q >> 1) & 1, kWaitLimit);
+    return;
+  }
+  // ---- consumers: warp p takes component p
+  int n = 0;
+  for (int tile = blockIdx.x; tile < tiles; tile += step, n++) {
+    const int buf = n & 1;
+    if (!wait(&val[buf], (n >> 1) & 1) || !wait(&tx[buf], (n >> 1) & 1)) return;
     const LevelK& K = a.lk[min(__ffs(__ldg(a.bscale + (tile >> 4))) - 1, kMaxScale - 1)];
     const int i = lane & 7, j = lane >> 3;
     float e[8][3], out[8];
@@ -229,7 +247,7 @@ __global__ void __launch_bounds__(kTileThreads) k_amr_tile32(ApplyArgs a, int ti
       out[c] = 0.f;
       const int tc = (i + off_bit(c, 0)) + 9 * ((j + off_bit(c, 1)) + 5 * off_bit(c, 2));
 #pragma unroll
-      for (int d = 0; d < 3; d++) e[c][d] = s_x[d][tc];
+      for (int d = 0; d < 3; d++) e[c][d] = s_x[buf][d][tc];
     }
     // mass term, monomial by monomial: the ordered corner pairs that share it
     const float* mm = s_m + (size_t)buf * (kTileBytes / 4) + lane * AMPS_CELLM + 3 * p;
@@ -252,7 +270,7 @@ __global__ void __launch_bounds__(kTileThreads) k_amr_tile32(ApplyArgs a, int ti
     else cell_curl_t_row<float>(cu, K.cc[0], 2, out);
     // out[c] in the table order (0,0) (1,0) (1,1) (0,1), z: add along x and y
     auto put = [&](int tc, float v) {
-      const int q = s_id[tc];
+      const int q = s_id[buf][tc];
       if (q >= 0) {
         atomicAdd(y32 + p * a.nvc + q, v);
       } else {
@@ -273,7 +291,7 @@ __global__ void __launch_bounds__(kTileThreads) k_amr_tile32(ApplyArgs a, int ti
       if (j == 3) put(i + 9 * (4 + 5 * z), c1);
       if (i == 7 && j == 3) put(8 + 9 * (4 + 5 * z), e1);
     }
-    __syncthreads();  // s_x, s_id and this buffer are rewritten
+    arrive(&empty[buf]);
   }
 }
 
@@ -1075,7 +1093,7 @@ static cudaError_t split_input(amps_gpu_ctx* c, const double* x, const double* d
 // CTAs of a persistent tile kernel that the device holds at a time (asked once per
 // device and kernel)
 template <typename Kernel>
-static cudaError_t tile_grid(Kernel kernel, uint32_t smem, int (&grid)[64], int& n) {
+static cudaError_t tile_grid(Kernel kernel, int threads, uint32_t smem, int (&grid)[64], int& n) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
@@ -1084,7 +1102,7 @@ static cudaError_t tile_grid(Kernel kernel, uint32_t smem, int (&grid)[64], int&
     cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kTileThreads, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
     if (e != cudaSuccess) return e;
     grid[dev] = sms * std::max(per, 1);
   }
@@ -1097,7 +1115,7 @@ template <int ACC>
 static cudaError_t launch_tile(amps_gpu_ctx* c, const ApplyArgs& a, double* y64) {
   static int grid[64] = {0};
   int n = 0;
-  cudaError_t e = tile_grid(k_amr_tile_ff<ACC>, 2 * tile_ff_bytes<ACC>(), grid, n);
+  cudaError_t e = tile_grid(k_amr_tile_ff<ACC>, kTileThreads, 2 * tile_ff_bytes<ACC>(), grid, n);
   if (e != cudaSuccess) return e;
   // AMR meshes hold whole 512-cell blocks: ncell is a multiple of the tile
   const int tiles = (int)(c->ncor / kFFCells);
@@ -1109,10 +1127,10 @@ static cudaError_t launch_tile(amps_gpu_ctx* c, const ApplyArgs& a, double* y64)
 static cudaError_t launch_tile32(amps_gpu_ctx* c, const ApplyArgs& a, float* y32) {
   static int grid[64] = {0};
   int n = 0;
-  cudaError_t e = tile_grid(k_amr_tile32, 2 * kTileBytes, grid, n);
+  cudaError_t e = tile_grid(k_amr_tile32, kT32Threads, 2 * kTileBytes, grid, n);
   if (e != cudaSuccess) return e;
   const int tiles = (int)(c->ncor / kTileCells);
-  k_amr_tile32<<<std::min(n, tiles), kTileThreads, 2 * kTileBytes, c->stream>>>(a, tiles, y32);
+  k_amr_tile32<<<std::min(n, tiles), kT32Threads, 2 * kTileBytes, c->stream>>>(a, tiles, y32);
   return cudaGetLastError();
 }
 

@@ -207,18 +207,27 @@ __global__ void __launch_bounds__(kT32Threads) k_amr_tile32(ApplyArgs a, int til
         }
       }
     };
+    auto copy = [&](int tile, int buf) {
+      if (p != 0 || lane != 0) return;
+      mbar_arrive_expect_tx(&tx[buf], kTileBytes);
+      bulk_copy_g2s(s_m + (size_t)buf * (kTileBytes / 4), a.cellM + (size_t)tile * kTileCells * AMPS_CELLM,
+                    kTileBytes, &tx[buf]);
+    };
+    // the partials don't change within a solve: the first two tiles' before the wait
+    for (int q = 0; q < 2; q++)
+      if ((int)blockIdx.x + q * step < tiles) copy(blockIdx.x + q * step, q);
     int id = corner_id(blockIdx.x), n = 0;
+    pdl_wait();
+    pdl_next();
     corner_values(id);
     bool ok = true;
     for (int tile = blockIdx.x; tile < tiles; tile += step, n++) {
       const int buf = n & 1;
       const int idn = corner_id(tile + step);
-      if (n >= 2) ok = wait(&empty[buf], ((n >> 1) - 1) & 1);
-      if (!ok) break;
-      if (p == 0 && lane == 0) {
-        mbar_arrive_expect_tx(&tx[buf], kTileBytes);
-        bulk_copy_g2s(s_m + (size_t)buf * (kTileBytes / 4), a.cellM + (size_t)tile * kTileCells * AMPS_CELLM,
-                      kTileBytes, &tx[buf]);
+      if (n >= 2) {
+        ok = wait(&empty[buf], ((n >> 1) - 1) & 1);
+        if (!ok) break;
+        copy(tile, buf);
       }
       if (act) {
         s_id[buf][t] = id;
@@ -229,12 +238,14 @@ __global__ void __launch_bounds__(kT32Threads) k_amr_tile32(ApplyArgs a, int til
       id = idn;
       if (tile + step < tiles) corner_values(id);
     }
-    // the last copies land before the CTA's shared memory goes, whoever gave up
+    // the last copies land before the CTA's shared memory goes, whoever gave up (n is
+    // 0, or the two last copies are of tiles n - 2 and n - 1)
     if (p == 0)
       for (int q = max(0, n - 2); q < n; q++) mbar_wait_bounded(&tx[q & 1], (q >> 1) & 1, kWaitLimit);
     return;
   }
   // ---- consumers: warp p takes component p
+  pdl_wait();
   int n = 0;
   for (int tile = blockIdx.x; tile < tiles; tile += step, n++) {
     const int buf = n & 1;
@@ -366,6 +377,8 @@ template <int ACC>
 constexpr uint32_t tile_ff_bytes() { return kFFBytes + (ACC == 2 ? kFFJBytes : 0); }
 template <int ACC>
 __global__ void __launch_bounds__(kTileThreads, ACC == 2 ? 5 : 6) k_amr_tile_ff(ApplyArgs a, int tiles, double* __restrict__ y64) {
+  pdl_wait();
+  pdl_next();
   extern __shared__ __align__(16) float s_m[];  // two tiles of partials (and currents)
   constexpr uint32_t kBytes = tile_ff_bytes<ACC>();
   __shared__ __align__(8) uint64_t bar[2];
@@ -607,6 +620,8 @@ __global__ void __launch_bounds__(kTileThreads, ACC == 2 ? 5 : 6) k_amr_tile_ff(
 __global__ void __launch_bounds__(256) k_amr_split(long long n, const double* __restrict__ x,
                                                    const double* __restrict__ dinv,
                                                    float* __restrict__ xh, float* __restrict__ xl) {
+  pdl_wait();
+  pdl_next();
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     const double v = dinv ? dinv[t] * x[t] : x[t];
@@ -647,11 +662,13 @@ __global__ void __launch_bounds__(256) k_amr_finish_ff(long long nvc, Hang h, un
       const long long c = min(c0 + 256 * k, nvc - 1);
       dg[k] = diag[c];
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        y[k][d] = y32[d * nvc + c];
-        v[k][d] = opin_value(in, d * nvc + c);
-      }
+      for (int d = 0; d < 3; d++) v[k][d] = opin_value(in, d * nvc + c);
     }
+    pdl_wait();  // the tiles' sums
+#pragma unroll
+    for (int k = 0; k < kFinPer; k++)
+#pragma unroll
+      for (int d = 0; d < 3; d++) y[k][d] = y32[d * nvc + min(c0 + 256 * k, nvc - 1)];
 #pragma unroll
     for (int k = 0; k < kFinPer; k++) {
       const long long c = c0 + 256 * k;
@@ -714,6 +731,7 @@ __global__ void __launch_bounds__(256) k_amr_finish_ff(long long nvc, Hang h, un
       const float bs = __shfl_xor_sync(0xffffffffu, acc[d].s, k), bq = __shfl_xor_sync(0xffffffffu, acc[d].q, k);
       ff_acc(acc[d], bs, bq);
     }
+  pdl_wait();
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     if (!act || lane != d) continue;
@@ -735,6 +753,8 @@ __global__ void __launch_bounds__(256) k_amr_constraint(int nrows, const int* __
                                                         const double* __restrict__ dinv,
                                                         double* __restrict__ y, int rhs_mode,
                                                         int* __restrict__ next) {
+  pdl_wait();
+  pdl_next();
   if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0;  // for the next tile kernel
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
   if (t0 >= nrows) return;
@@ -793,6 +813,8 @@ __global__ void __launch_bounds__(256) k_amr_update_b(long long ncell, long long
                                                       const double* __restrict__ Bn,
                                                       double* __restrict__ Bnew, double dt,
                                                       double* __restrict__ energy) {
+  pdl_wait();
+  pdl_next();
   __shared__ double s_e[3][729];
   const int b = blockIdx.x;
   if (b == 0 && threadIdx.x == 0) *energy = 0.0;  // for k_amr_update_e
@@ -895,6 +917,8 @@ __global__ void __launch_bounds__(256) k_amr_c2n(long long ncell, long long nvc,
                                                  const double* __restrict__ bdx,
                                                  const double* __restrict__ cinv,
                                                  const double* __restrict__ Bcen, double* __restrict__ acc) {
+  pdl_wait();
+  pdl_next();
   __shared__ double s_c[512], s_x[576], s_y[648];
   const int b = blockIdx.x, tid = threadIdx.x;
   const double dx = bdx[b], V = dx * dx * dx;
@@ -952,6 +976,8 @@ __device__ __forceinline__ void add_energy(double en, double* energy) {
 __global__ void __launch_bounds__(256) k_amr_fix_hanging(int nrows, const int* __restrict__ rows, long long nvc,
                                                          Hang h, double* F, const double* __restrict__ cvol,
                                                          double* energy) {
+  pdl_wait();
+  pdl_next();
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
   double en = 0.0;
   if (t0 < nrows) {
@@ -982,6 +1008,8 @@ __global__ void __launch_bounds__(256) k_amr_update_e(long long ncell, long long
                                                       double ri, double r1, const double* __restrict__ cvol,
                                                       const double* __restrict__ bdx,
                                                       const double* __restrict__ Bcen, double* energy) {
+  pdl_wait();
+  pdl_next();
   const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
   double ee = 0.0, eb = 0.0;
   for (long long c = t0; c < nvc; c += step) {
@@ -1010,6 +1038,8 @@ __global__ void __launch_bounds__(256) k_amr_update_e(long long ncell, long long
 
 __global__ void k_amr_pack(long long nvc, const int* ctab, Hang h, const double* Eh,
                            const double* Bprev, const double* Bcur, float* sp, float* sd) {
+  pdl_wait();
+  pdl_next();
   const int b = blockIdx.x;
   for (int s = threadIdx.x; s < AMPS_SC; s += blockDim.x) {
     const int cc = ctab[b * 729 + s];
@@ -1036,7 +1066,7 @@ unsigned g1(long long n) { return (unsigned)((n + 255) / 256); }
 cudaError_t launch_amr_pack(amps_gpu_ctx* c, const double* Eh, const double* Bprev,
                             const double* Bcur) {
   TimedLaunch t(c, "pack_stencils");
-  k_amr_pack<<<c->nb, 256, 0, c->stream>>>(c->nvc, c->d_ctab, hang_of(c), Eh, Bprev, Bcur,
+  launch_pdl(k_amr_pack, dim3(c->nb), dim3(256), 0, c->stream, c->nvc, c->d_ctab, hang_of(c), Eh, Bprev, Bcur,
                                             c->d_stencil_push, c->d_stencil_dep);
   return cudaGetLastError();
 }
@@ -1084,7 +1114,7 @@ static cudaError_t split_input(amps_gpu_ctx* c, const double* x, const double* d
     return e;
   a.xh = c->d_xs;
   a.xl = c->d_xs + n;
-  k_amr_split<<<(unsigned)std::min<long long>((n + 255) / 256, 152LL * 16), 256, 0, c->stream>>>(n, x, dinv,
+  launch_pdl(k_amr_split, dim3((unsigned)(std::min<long long>((n + 255) / 256, 152LL * 16))), dim3(256), 0, c->stream, n, x, dinv,
                                                                                                 c->d_xs,
                                                                                                 c->d_xs + n);
   return cudaGetLastError();
@@ -1119,7 +1149,7 @@ static cudaError_t launch_tile(amps_gpu_ctx* c, const ApplyArgs& a, double* y64)
   if (e != cudaSuccess) return e;
   // AMR meshes hold whole 512-cell blocks: ncell is a multiple of the tile
   const int tiles = (int)(c->ncor / kFFCells);
-  k_amr_tile_ff<ACC><<<std::min(n, tiles), kTileThreads, 2 * tile_ff_bytes<ACC>(), c->stream>>>(a, tiles, y64);
+  launch_pdl(k_amr_tile_ff<ACC>, dim3(std::min(n, tiles)), dim3(kTileThreads), 2 * tile_ff_bytes<ACC>(), c->stream, a, tiles, y64);
   return cudaGetLastError();
 }
 
@@ -1130,7 +1160,7 @@ static cudaError_t launch_tile32(amps_gpu_ctx* c, const ApplyArgs& a, float* y32
   cudaError_t e = tile_grid(k_amr_tile32, kT32Threads, 2 * kTileBytes, grid, n);
   if (e != cudaSuccess) return e;
   const int tiles = (int)(c->ncor / kTileCells);
-  k_amr_tile32<<<std::min(n, tiles), kT32Threads, 2 * kTileBytes, c->stream>>>(a, tiles, y32);
+  launch_pdl(k_amr_tile32, dim3(std::min(n, tiles)), dim3(kT32Threads), 2 * kTileBytes, c->stream, a, tiles, y32);
   return cudaGetLastError();
 }
 
@@ -1148,7 +1178,7 @@ cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* di
     return e;
   }
   if ((e = launch_tile<1>(c, a, y)) != cudaSuccess) return e;
-  k_amr_constraint<<<g1(std::max(c->nsrows, 1)), 256, 0, c->stream>>>(c->nsrows, c->d_srows, c->nvc, a.h,
+  launch_pdl(k_amr_constraint, dim3(g1(std::max(c->nsrows, 1))), dim3(256), 0, c->stream, c->nsrows, c->d_srows, c->nvc, a.h,
                                                                       x, dinv, y, 0, c->d_next);
   return cudaGetLastError();
 }
@@ -1166,7 +1196,7 @@ cudaError_t launch_amr_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, f
   if ((e = launch_tile32(c, a, c->d_y32)) != cudaSuccess) return e;
   const unsigned plain = (unsigned)((c->nvc + 256 * kFinPer - 1) / (256 * kFinPer));
   const int per = 256 / kRowLanes;
-  k_amr_finish_ff<<<plain + (unsigned)((c->nsrows + per - 1) / per), 256, 0, c->stream>>>(
+  launch_pdl(k_amr_finish_ff, dim3(plain + (unsigned)((c->nsrows + per - 1) / per)), dim3(256), 0, c->stream, 
       c->nvc, a.h, plain, c->nsrows, c->d_srows, c->d_ss, c->d_sc, c->d_svh, c->d_svl, c->d_sdiag,
       c->d_y32, in, wh, wl);
   return cudaGetLastError();
@@ -1185,7 +1215,7 @@ cudaError_t launch_amr_rhs(amps_gpu_ctx* c, bool diag) {
   TimedLaunch t(c, "rhs", 3);
   if ((e = split_input(c, c->d_En, nullptr, a)) != cudaSuccess) return e;
   if ((e = launch_tile<2>(c, a, c->d_rhs)) != cudaSuccess) return e;
-  k_amr_constraint<<<g1(std::max(c->nsrows, 1)), 256, 0, c->stream>>>(c->nsrows, c->d_srows, c->nvc, a.h,
+  launch_pdl(k_amr_constraint, dim3(g1(std::max(c->nsrows, 1))), dim3(256), 0, c->stream, c->nsrows, c->d_srows, c->nvc, a.h,
                                                                       nullptr, nullptr, c->d_rhs, 1, c->d_next);
   return cudaGetLastError();
 }
@@ -1198,7 +1228,7 @@ cudaError_t launch_amr_jacobi(amps_gpu_ctx* c) {
 
 cudaError_t launch_amr_update_b(amps_gpu_ctx* c) {
   TimedLaunch t(c, "update_b");
-  k_amr_update_b<<<c->nb, 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_ctabh, hang_of(c), c->d_bdx, c->d_Eh,
+  launch_pdl(k_amr_update_b, dim3(c->nb), dim3(256), 0, c->stream, c->ncor, c->nvc, c->d_ctabh, hang_of(c), c->d_bdx, c->d_Eh,
                                                c->d_Bc, c->d_Bc2, c->cfg.dt, c->d_energy + 1);
   if (c->mesh_open) {
     const int* nf = c->amrdev.nfine;
@@ -1212,7 +1242,7 @@ cudaError_t launch_amr_update_b(amps_gpu_ctx* c) {
 // hanging corners of F, optionally with their wave energy
 static cudaError_t fix_hanging(amps_gpu_ctx* c, double* F, const double* cvol, double* energy) {
   if (c->nsrows == 0) return cudaSuccess;
-  k_amr_fix_hanging<<<g1(c->nsrows), 256, 0, c->stream>>>(c->nsrows, c->d_srows, c->nvc, hang_of(c), F, cvol,
+  launch_pdl(k_amr_fix_hanging, dim3(g1(c->nsrows)), dim3(256), 0, c->stream, c->nsrows, c->d_srows, c->nvc, hang_of(c), F, cvol,
                                                           energy);
   return cudaGetLastError();
 }
@@ -1221,7 +1251,7 @@ cudaError_t launch_amr_c2n(amps_gpu_ctx* c, const double* Bcen, double* Bcor) {
   cudaError_t e = cudaMemsetAsync(Bcor, 0, sizeof(double) * 3 * c->nvc, c->stream);
   if (e != cudaSuccess) return e;
   TimedLaunch t(c, "c2n", 2);
-  k_amr_c2n<<<c->nb, 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_ctab, c->d_bdx, c->d_cinv, Bcen, Bcor);
+  launch_pdl(k_amr_c2n, dim3(c->nb), dim3(256), 0, c->stream, c->ncor, c->nvc, c->d_ctab, c->d_bdx, c->d_cinv, Bcen, Bcor);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   return fix_hanging(c, Bcor, nullptr, nullptr);
 }
@@ -1231,7 +1261,7 @@ cudaError_t launch_amr_update_e(amps_gpu_ctx* c) {
   TimedLaunch t(c, "update_e", 2);
   const double th = c->cfg.theta;
   const unsigned grid = (unsigned)std::min<long long>((std::max(c->nvc, c->ncor) + 255) / 256, 152LL * 8);
-  k_amr_update_e<<<grid, 256, 0, c->stream>>>(c->ncor, c->nvc, c->d_Eh, c->d_En, 1.0 / th, (1.0 - th) / th, c->d_cvol,
+  launch_pdl(k_amr_update_e, grid, dim3(256), 0, c->stream, c->ncor, c->nvc, c->d_Eh, c->d_En, 1.0 / th, (1.0 - th) / th, c->d_cvol,
                                               c->d_bdx, c->d_Bc, c->d_energy + 1);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   return fix_hanging(c, c->d_En, c->d_cvol, c->d_energy + 1);

@@ -184,6 +184,7 @@ amps_gpu_status reset_flags(amps_gpu_ctx* c) {
 // (+ deposit), arrivals (+ assembly), read-back of the flags and the energy.
 cudaError_t enqueue_particle_step(amps_gpu_ctx* c, bool deposit) {
   cudaError_t e = cudaMemsetAsync(c->d_flags, 0, 7 * sizeof(unsigned long long), c->stream);
+  if (e == cudaSuccess && deposit) e = cudaMemsetAsync(c->d_energy, 0, sizeof(double), c->stream);
   if (e == cudaSuccess) e = launch_pack_stencils(c, c->d_Eh, c->d_Bcor_prev, c->d_Bcor_cur);
   if (e == cudaSuccess) e = launch_push_step(c, deposit);
   if (e == cudaSuccess)

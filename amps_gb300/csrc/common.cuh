@@ -12,6 +12,7 @@
 //   and deposit kernels, contiguous per block so one bulk TMA copy stages them.
 #pragma once
 
+#include <utility>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -379,6 +380,29 @@ __host__ __device__ inline int nbr_slot(int ox, int oy, int oz) {
 // combined in FP64.  Error ~1e-14 of the sum of |terms| for 81 terms.  The
 // arithmetic uses the _rn intrinsics, which the compiler never contracts into
 // FMAs (a contraction would break the error-free transformations).
+// Programmatic dependent launch: a kernel launched by launch_pdl may start while the
+// kernel before it on the stream is still running, and waits for that one's completion
+// (and so for all before it) in pdl_wait(), before it touches anything the other reads or
+// writes; a kernel lets the next one start early by pdl_next(), after its own pdl_wait().
+// It hides a launch's latency (1 to 2 us), of which a step of a small mesh has two
+// dozen, and whatever a kernel can load or copy before its wait.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 struct FF {
   float s, q;
 };

@@ -125,6 +125,8 @@ TapsFF taps_ff(const Taps& T) {
 __global__ void __launch_bounds__(256) k_split(long long n, const double* __restrict__ x,
                                                const double* __restrict__ dinv,
                                                float* __restrict__ xh, float* __restrict__ xl) {
+  pdl_wait();
+  pdl_next();
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     const double v = dinv ? dinv[t] * x[t] : x[t];
@@ -225,6 +227,8 @@ __global__ void __launch_bounds__(32 * kOpMaxWarps) k_matvec(long long ncor, con
                                                              const float* __restrict__ xl,
                                                              double* __restrict__ y,
                                                              const __grid_constant__ TapsFF T) {
+  pdl_wait();
+  pdl_next();
   __shared__ float2 s_row[6][kOpMaxWarps][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const long long c = (long long)blockIdx.x * 32 + lane;
@@ -246,6 +250,8 @@ __global__ void __launch_bounds__(32 * kOpMaxWarps) k_rhs(long long ncor, const 
                                                           double* __restrict__ rhs,
                                                           const __grid_constant__ TapsFF T, double c4x,
                                                           double c4y, double c4z) {
+  pdl_wait();
+  pdl_next();
   __shared__ float2 s_row[6][kOpMaxWarps][32];
   __shared__ double s_cb[3][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -405,6 +411,8 @@ __device__ __forceinline__ bool grid_sum(double acc, double* __restrict__ partia
 __global__ void __launch_bounds__(256) k_first(long long n, const double* __restrict__ b, double* __restrict__ w,
                                                double* __restrict__ x, double* __restrict__ partial,
                                                double* __restrict__ n2, GmState* __restrict__ S, double tol) {
+  pdl_wait();
+  pdl_next();
   double acc = 0.0;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
@@ -430,6 +438,8 @@ __global__ void __launch_bounds__(256) k_first(long long n, const double* __rest
 __global__ void __launch_bounds__(256) k_residual(long long n, const double* __restrict__ b,
                                                   double* __restrict__ r, double* __restrict__ partial,
                                                   double* __restrict__ n2, GmState* __restrict__ S) {
+  pdl_wait();
+  pdl_next();
   double acc = 0.0;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
@@ -616,6 +626,7 @@ __global__ void __launch_bounds__(kArnBlock, 2) k_arnoldi_tile(
   float2* s_part = reinterpret_cast<float2*>(s_w + 4 * T);
   auto tile_of = [&](int k) { return (long long)blockIdx.x + (long long)k * nblk; };
   auto count_of = [&](int k) { return (int)min((long long)T, n - tile_of(k) * T); };
+  pdl_next();
   if (tid == 0) {
     for (int s = 0; s < stages; s++) {
       mbar_init(&full[s], 1);
@@ -1005,6 +1016,8 @@ cudaError_t launch_arnoldi(cudaStream_t s, long long n, const float* V, float* w
 __global__ void __launch_bounds__(256) k_start_ff(long long n, const double* __restrict__ r,
                                                   const double* __restrict__ nrm2, float* __restrict__ v,
                                                   float* __restrict__ xf, const float* __restrict__ dh) {
+  pdl_wait();
+  pdl_next();
   const double sc = *nrm2 > 0.0 ? 1.0 / sqrt(*nrm2) : 0.0;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
@@ -1027,6 +1040,8 @@ __global__ void __launch_bounds__(256) k_to_ff(long long n, const double* __rest
   }
 }
 __global__ void __launch_bounds__(256) k_from_ff(long long n, const float* __restrict__ v, double* __restrict__ x) {
+  pdl_wait();
+  pdl_next();
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x)
     x[t] = (double)v[t] + (double)v[ff_ld(n) + t];
@@ -1042,6 +1057,8 @@ __global__ void __launch_bounds__(256) k_combine_ff(long long n, const float* __
                                                     const float* __restrict__ dff, double* __restrict__ x,
                                                     float* __restrict__ xs, const double* __restrict__ en,
                                                     double* __restrict__ eo) {
+  pdl_wait();
+  pdl_next();
   __shared__ float s_y[kMaxV][2];
   __shared__ double s_yd[kMaxV];
   const long long ld = ff_ld(n);
@@ -1085,17 +1102,19 @@ __global__ void __launch_bounds__(256) k_combine_ff(long long n, const float* __
 void launch_combine_ff(cudaStream_t s, unsigned gr, long long n, const float* V, const GmState* S, int nv_host,
                        const float* dff, double* x, float* xs, const double* en, double* eo) {
   if (nv_host <= 4)
-    k_combine_ff<4><<<gr, 256, 0, s>>>(n, V, S, dff, x, xs, en, eo);
+    launch_pdl(k_combine_ff<4>, dim3(gr), dim3(256), 0, s, n, V, S, dff, x, xs, en, eo);
   else if (nv_host <= 8)
-    k_combine_ff<8><<<gr, 256, 0, s>>>(n, V, S, dff, x, xs, en, eo);
+    launch_pdl(k_combine_ff<8>, dim3(gr), dim3(256), 0, s, n, V, S, dff, x, xs, en, eo);
   else if (nv_host <= 16)
-    k_combine_ff<16><<<gr, 256, 0, s>>>(n, V, S, dff, x, xs, en, eo);
+    launch_pdl(k_combine_ff<16>, dim3(gr), dim3(256), 0, s, n, V, S, dff, x, xs, en, eo);
   else
-    k_combine_ff<32><<<gr, 256, 0, s>>>(n, V, S, dff, x, xs, en, eo);
+    launch_pdl(k_combine_ff<32>, dim3(gr), dim3(256), 0, s, n, V, S, dff, x, xs, en, eo);
 }
 
 // xf = fp32(D v)
 __global__ void __launch_bounds__(256) k_in_f32(long long n, OpIn in, float* __restrict__ xf) {
+  pdl_wait();
+  pdl_next();
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x)
     xf[t] = in.vd ? (float)in.vd[t] : (in.dh ? in.vh[t] * in.dh[t] : in.vh[t]);
@@ -1110,6 +1129,8 @@ __global__ void __launch_bounds__(32 * kOpMaxWarps) k_matvec32_ff(long long ncor
                                                                   const float* __restrict__ xf, OpIn in,
                                                                   float* __restrict__ wh, float* __restrict__ wl,
                                                                   const __grid_constant__ TapsF T) {
+  pdl_wait();
+  pdl_next();
   __shared__ float s_row[3][kOpMaxWarps][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const long long c = (long long)blockIdx.x * 32 + lane;
@@ -1152,6 +1173,8 @@ __global__ void __launch_bounds__(256) k_update_b(long long ncor, const int* __r
                                                   const double* __restrict__ Bn,
                                                   double* __restrict__ Bnew, double c4x,
                                                   double c4y, double c4z, double* __restrict__ energy) {
+  pdl_wait();
+  pdl_next();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c == 0) *energy = 0.0;  // for k_c2n_update_e
   if (c >= ncor) return;
@@ -1192,6 +1215,8 @@ __global__ void __launch_bounds__(256) k_c2n_update_e(long long ncor, const int*
                                                       const double* __restrict__ Eh, double* __restrict__ En,
                                                       double theta, double vol_over_8pi,
                                                       double* __restrict__ energy) {
+  pdl_wait();
+  pdl_next();
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double en = 0.0;
   if (c < ncor) {
@@ -1260,7 +1285,7 @@ static cudaError_t split_input(amps_gpu_ctx* c, const double* x, const double* d
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&c->d_xs), sizeof(float) * 2 * n);
     if (e != cudaSuccess) return e;
   }
-  k_split<<<gridr(n), 256, 0, c->stream>>>(n, x, dinv, c->d_xs, c->d_xs + n);
+  launch_pdl(k_split, dim3(gridr(n)), dim3(256), 0, c->stream, n, x, dinv, c->d_xs, c->d_xs + n);
   return cudaGetLastError();
 }
 
@@ -1271,14 +1296,14 @@ cudaError_t launch_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, 
   cudaError_t e = pairs ? cudaSuccess : split_input(c, x, dinv);
   if (e != cudaSuccess) return e;
   const long long n = 3 * c->ncor;
-  k_matvec<<<(unsigned)(c->ncor / 32), c->tune_tb, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_M, c->d_xs,
+  launch_pdl(k_matvec, dim3((unsigned)((c->ncor / 32))), dim3(c->tune_tb), 0, c->stream, c->ncor, c->d_nbr, c->d_M, c->d_xs,
                                                                    c->d_xs + n, y, T);
   return cudaGetLastError();
 }
 
 cudaError_t launch_in_f32(amps_gpu_ctx* c, const OpIn& in, float* xf) {
   const long long n = 3 * c->nvc;
-  k_in_f32<<<gridr(n), 256, 0, c->stream>>>(n, in, xf);
+  launch_pdl(k_in_f32, dim3(gridr(n)), dim3(256), 0, c->stream, n, in, xf);
   return cudaGetLastError();
 }
 
@@ -1293,7 +1318,7 @@ cudaError_t launch_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, float
   TimedLaunch t(c, "matvec32", in.xf_ready ? 1 : 2);
   cudaError_t e = in.xf_ready ? cudaSuccess : launch_in_f32(c, in, c->d_xs);
   if (e != cudaSuccess) return e;
-  k_matvec32_ff<<<(unsigned)(c->ncor / 32), c->tune_tb, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_M, c->d_xs,
+  launch_pdl(k_matvec32_ff, dim3((unsigned)((c->ncor / 32))), dim3(c->tune_tb), 0, c->stream, c->ncor, c->d_nbr, c->d_M, c->d_xs,
                                                                         in, wh, wl, T);
   return cudaGetLastError();
 }
@@ -1307,7 +1332,7 @@ cudaError_t launch_rhs(amps_gpu_ctx* c, bool diag) {
   cudaError_t e = split_input(c, c->d_En, nullptr);
   if (e != cudaSuccess) return e;
   const long long n = 3 * c->ncor;
-  k_rhs<<<(unsigned)(c->ncor / 32), c->tune_tb, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_M, c->d_xs,
+  launch_pdl(k_rhs, dim3((unsigned)((c->ncor / 32))), dim3(c->tune_tb), 0, c->stream, c->ncor, c->d_nbr, c->d_M, c->d_xs,
                                                                 c->d_xs + n, c->d_Bc, c->d_J, c->d_rhs, T,
                                                                 c4[0], c4[1], c4[2]);
   return cudaGetLastError();
@@ -1327,7 +1352,7 @@ cudaError_t launch_update_b(amps_gpu_ctx* c) {
   double c4[3];
   for (int d = 0; d < 3; d++) c4[d] = 0.25 * (c->cfg.dt / c->cfg.dx[d]);
   TimedLaunch t(c, "update_b");
-  k_update_b<<<grid1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->d_nbr, c->d_Eh, c->d_Bc,
+  launch_pdl(k_update_b, dim3(grid1(c->ncor)), dim3(256), 0, c->stream, c->ncor, c->d_nbr, c->d_Eh, c->d_Bc,
                                                      c->d_Bc2, c4[0], c4[1], c4[2], c->d_energy + 1);
   return cudaGetLastError();
 }
@@ -1340,7 +1365,7 @@ cudaError_t launch_c2n_update_e(amps_gpu_ctx* c, const double* Bcen, double* Bco
   }
   const double vol = c->cfg.dx[0] * c->cfg.dx[1] * c->cfg.dx[2];
   TimedLaunch t(c, "c2n_update_e");
-  k_c2n_update_e<<<grid1(c->ncor), 256, 0, c->stream>>>(c->ncor, c->d_nbr, Bcen, Bcor, c->d_Eh, c->d_En,
+  launch_pdl(k_c2n_update_e, dim3(grid1(c->ncor)), dim3(256), 0, c->stream, c->ncor, c->d_nbr, Bcen, Bcor, c->d_Eh, c->d_En,
                                                         c->cfg.theta, vol / (8.0 * kPi), c->d_energy + 1);
   return cudaGetLastError();
 }
@@ -1424,7 +1449,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     // FP64 inner operator, through FP64 copies
     const double* x = zj;
     if (!zj) {
-      k_from_ff<<<gr, 256, 0, s>>>(n, vf(jj), c->d_tmpv);
+      launch_pdl(k_from_ff, dim3(gr), dim3(256), 0, s, n, vf(jj), c->d_tmpv);
       x = c->d_tmpv;
     }
     cudaError_t ee = launch_matvec(c, x, zj ? nullptr : dinv, c->d_tmpv + n);
@@ -1439,7 +1464,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
       cudaError_t ee = launch_jacobi_diag(c);
       if (ee != cudaSuccess) return ee;
     }
-    k_first<<<gr, 256, 0, s>>>(n, c->d_rhs, w, c->d_x, partial, d_n2, gs, tol);
+    launch_pdl(k_first, dim3(gr), dim3(256), 0, s, n, c->d_rhs, w, c->d_x, partial, d_n2, gs, tol);
     return cudaGetLastError();
   };
   // Arnoldi step jj: the operator (after the network for flexible directions),
@@ -1449,15 +1474,15 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     cudaError_t ee;
     if (flexible) {
       double* zj = c->d_Z + (size_t)jj * n;
-      k_from_ff<<<gr, 256, 0, s>>>(n, vf(jj), c->d_tmpv);  // v_j in FP64 for the network
+      launch_pdl(k_from_ff, dim3(gr), dim3(256), 0, s, n, vf(jj), c->d_tmpv);  // v_j in FP64 for the network
       if ((ee = launch_precond_net(c, c->d_tmpv, zj)) != cudaSuccess) return ee;
       if ((ee = inner_matvec(jj, zj)) != cudaSuccess) return ee;
     } else {
       if ((ee = inner_matvec(jj, nullptr)) != cudaSuccess) return ee;
       // training pairs for the learned preconditioner: (A D v_j, D v_j)
       if (harvest) {
-        k_from_ff<<<gr, 256, 0, s>>>(n, wf, c->d_tmpv);
-        k_from_ff<<<gr, 256, 0, s>>>(n, vf(jj), c->d_tmpv + n);
+        launch_pdl(k_from_ff, dim3(gr), dim3(256), 0, s, n, wf, c->d_tmpv);
+        launch_pdl(k_from_ff, dim3(gr), dim3(256), 0, s, n, vf(jj), c->d_tmpv + n);
         if ((ee = precond_harvest_pairs(c, c->d_tmpv, c->d_tmpv + n, 1)) != cudaSuccess) return ee;
       }
     }
@@ -1477,7 +1502,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     cudaError_t ee = cudaGetLastError();
     if (ee == cudaSuccess) ee = launch_matvec(c, c->d_x, nullptr, w, !flexible);
     if (ee != cudaSuccess) return ee;
-    k_residual<<<gr, 256, 0, s>>>(n, c->d_rhs, w, partial, d_n2, gs);
+    launch_pdl(k_residual, dim3(gr), dim3(256), 0, s, n, c->d_rhs, w, partial, d_n2, gs);
     return cudaGetLastError();
   };
 
@@ -1506,7 +1531,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
       if (ee == cudaSuccess) {
         cudaError_t e1 = prologue();
         if (e1 == cudaSuccess) {
-          k_start_ff<<<gr, 256, 0, s>>>(n, w, d_n2, vf(0), xf_next, dh);
+          launch_pdl(k_start_ff, dim3(gr), dim3(256), 0, s, n, w, d_n2, vf(0), xf_next, dh);
           for (int jj = 0; jj < K && e1 == cudaSuccess; jj++) e1 = arnoldi_step(jj);
         }
         if (e1 == cudaSuccess) e1 = cycle_end(K);
@@ -1564,7 +1589,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     const double target = tol * bnorm;
     // V0 = r / ||r|| (d_n2 holds ||r||^2)
     k_gm_start<<<1, 32, 0, s>>>(gs, d_n2, target);
-    k_start_ff<<<gr, 256, 0, s>>>(n, w, d_n2, vf(0), xf_next, dh);
+    launch_pdl(k_start_ff, dim3(gr), dim3(256), 0, s, n, w, d_n2, vf(0), xf_next, dh);
     int launched = 0, used = 0;
     bool done = false;
     const int first_read = cycles == 1 ? std::max(1, std::min(c->gm_guess[precond], m)) : 1;

@@ -151,6 +151,8 @@ __global__ void k_pack_stencils(int nb, long long ncor, const int* __restrict__ 
                                 float* __restrict__ sd, const double* __restrict__ Bcp,
                                 const double* __restrict__ Bcc, float4* __restrict__ cp,
                                 float4* __restrict__ cc) {
+  pdl_wait();
+  pdl_next();
   const int b = blockIdx.x;
   if (cp) {
     for (int s = threadIdx.x; s < AMPS_CSC; s += blockDim.x) {
@@ -293,6 +295,8 @@ __global__ void __launch_bounds__(kPushWarps * 32, 4) k_push_deposit(StepArgs a)
     }
   };
   prefetch(0, lane);  // in flight while the stencils are staged
+  pdl_wait();  // the stencils
+  pdl_next();
   const size_t cor = (size_t)b * AMPS_SC + 81 * k, cen = (size_t)b * AMPS_CSC + 100 * k;
   const void* dep_src = CB ? (const void*)(a.st_ccur + cen) : (const void*)(a.st_dep + cor * AMPS_DEP_STRIDE);
   if (!stage_stencils(&bar, t_push, a.st_push + cor * AMPS_PUSH_STRIDE, bp, t_dep, dep_src, bd, a.flags,
@@ -732,6 +736,8 @@ constexpr int kLayer = AMPS_NC * AMPS_NC;
 
 template <bool DEP, int CHUNK, bool CB = false>
 __global__ void __launch_bounds__(256, CHUNK == 16 ? 4 : 2) k_arrivals(StepArgs a) {
+  pdl_wait();
+  pdl_next();
   constexpr int FS = CHUNK + 4;  // field stride of the staged fields
   extern __shared__ __align__(16) float4 s_dyn[];
   float* s_rec = reinterpret_cast<float*>(s_dyn);
@@ -1010,6 +1016,8 @@ __global__ void __launch_bounds__(kAsmThreads, 2) k_assemble(long long ncor, con
                                                           const float* __restrict__ cellM,
                                                           const float* __restrict__ cellJ, double inv_vol,
                                                           float* __restrict__ M, double* __restrict__ J) {
+  pdl_wait();
+  pdl_next();
   extern __shared__ __align__(16) float4 s_dyn[];
   float* s_c = reinterpret_cast<float*>(s_dyn);
   const int b = blockIdx.x / kAsmPerBlock, tile = blockIdx.x % kAsmPerBlock;
@@ -1829,7 +1837,7 @@ cudaError_t launch_pack_stencils(amps_gpu_ctx* c, const double* Eh, const double
   // centre B: B^n in the scratch slot d_Bc2 (the field solve swaps it there;
   // the field import copies the imported centres into it), B^{n+1} in d_Bc
   const bool cb = c->b_center;
-  k_pack_stencils<<<c->nb, 256, 0, c->stream>>>(
+  launch_pdl(k_pack_stencils, dim3(c->nb), dim3(256), 0, c->stream, 
       c->nb, c->ncor, c->d_nbr, Eh, Bprev, Bcur, c->d_stencil_push, c->d_stencil_dep,
       cb ? c->d_Bc2 : nullptr, cb ? c->d_Bc : nullptr,
       cb ? reinterpret_cast<float4*>(c->d_stencil_cprev) : nullptr,
@@ -1842,7 +1850,7 @@ static cudaError_t launch_assemble(amps_gpu_ctx* c) {
   if (c->amr) return cudaSuccess;
   TimedLaunch t(c, "assemble");
   const double inv_vol = 1.0 / (c->cfg.dx[0] * c->cfg.dx[1] * c->cfg.dx[2]);
-  k_assemble<<<(unsigned)(c->nb * kAsmPerBlock), kAsmThreads, kAsmSmem, c->stream>>>(
+  launch_pdl(k_assemble, dim3((unsigned)((c->nb * kAsmPerBlock))), dim3(kAsmThreads), kAsmSmem, c->stream, 
       c->ncor, c->d_nbr, c->d_cellM, c->d_cellJ, inv_vol, c->d_M, c->d_J);
   return cudaGetLastError();
 }
@@ -1938,29 +1946,25 @@ cudaError_t launch_inject(amps_gpu_ctx* c, const StepArgs& a) {
 cudaError_t launch_push_step(amps_gpu_ctx* c, bool deposit) {
   set_smem_attrs();
   cudaError_t e;
-  if (deposit) {
-    e = cudaMemsetAsync(c->d_energy, 0, sizeof(double), c->stream);
-    if (e != cudaSuccess) return e;
-  }
   StepArgs a = step_args(c);
   const dim3 grid(c->nb, AMPS_NC), pgrid(c->nb, AMPS_NC * AMPS_NC / kPushWarps);
   {
     TimedLaunch t(c, deposit ? "push_deposit" : "push");
     if (c->amr) {
       if (deposit)
-        k_push_deposit<true, true><<<pgrid, kPushWarps * 32, smem_push(true), c->stream>>>(a);
+        launch_pdl(k_push_deposit<true, true>, pgrid, dim3(kPushWarps * 32), smem_push(true), c->stream, a);
       else
-        k_push_deposit<false, true><<<pgrid, kPushWarps * 32, smem_push(false), c->stream>>>(a);
+        launch_pdl(k_push_deposit<false, true>, pgrid, dim3(kPushWarps * 32), smem_push(false), c->stream, a);
     } else if (c->b_center) {
       if (deposit)
-        k_push_deposit<true, false, true><<<pgrid, kPushWarps * 32, smem_push(true, true), c->stream>>>(a);
+        launch_pdl(k_push_deposit<true, false, true>, pgrid, dim3(kPushWarps * 32), smem_push(true, true), c->stream, a);
       else
-        k_push_deposit<false, false, true><<<pgrid, kPushWarps * 32, smem_push(false, true), c->stream>>>(a);
+        launch_pdl(k_push_deposit<false, false, true>, pgrid, dim3(kPushWarps * 32), smem_push(false, true), c->stream, a);
     } else {
       if (deposit)
-        k_push_deposit<true, false><<<pgrid, kPushWarps * 32, smem_push(true), c->stream>>>(a);
+        launch_pdl(k_push_deposit<true, false>, pgrid, dim3(kPushWarps * 32), smem_push(true), c->stream, a);
       else
-        k_push_deposit<false, false><<<pgrid, kPushWarps * 32, smem_push(false), c->stream>>>(a);
+        launch_pdl(k_push_deposit<false, false>, pgrid, dim3(kPushWarps * 32), smem_push(false), c->stream, a);
     }
   }
   e = cudaGetLastError();
@@ -1981,10 +1985,10 @@ cudaError_t launch_push_step(amps_gpu_ctx* c, bool deposit) {
     const size_t sm = smem_arr(chunk);
     const int v = (chunk == 32 ? 1 : 0) | (deposit ? 2 : 0) | (c->b_center ? 4 : 0);
     switch (v) {
-      case 0: k_arrivals<false, 16><<<grid, kWarps * 32, sm, c->stream>>>(a); break;
-      case 1: k_arrivals<false, 32><<<grid, kWarps * 32, sm, c->stream>>>(a); break;
-      case 2: k_arrivals<true, 16><<<grid, kWarps * 32, sm, c->stream>>>(a); break;
-      case 3: k_arrivals<true, 32><<<grid, kWarps * 32, sm, c->stream>>>(a); break;
+      case 0: launch_pdl(k_arrivals<false, 16>, grid, dim3(kWarps * 32), sm, c->stream, a); break;
+      case 1: launch_pdl(k_arrivals<false, 32>, grid, dim3(kWarps * 32), sm, c->stream, a); break;
+      case 2: launch_pdl(k_arrivals<true, 16>, grid, dim3(kWarps * 32), sm, c->stream, a); break;
+      case 3: launch_pdl(k_arrivals<true, 32>, grid, dim3(kWarps * 32), sm, c->stream, a); break;
       case 4: k_arrivals<false, 16, true><<<grid, kWarps * 32, sm, c->stream>>>(a); break;
       case 5: k_arrivals<false, 32, true><<<grid, kWarps * 32, sm, c->stream>>>(a); break;
       case 6: k_arrivals<true, 16, true><<<grid, kWarps * 32, sm, c->stream>>>(a); break;

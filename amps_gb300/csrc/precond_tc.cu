@@ -254,8 +254,25 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kThreads, 1)
     mbar_arrive_expect_tx(&bar[2], kWBytes);
     bulk_copy_g2s(wsm, wimg + (size_t)wset * (kWBytes / 2), kWBytes, &bar[2]);
   }
-  // layer-1 input, channels 0..2 of channel plane 0: on its way while the planes are
-  // zeroed
+  // zero the channel planes of the first layer, and of the others the rows before
+  // planes 0 and 4, the lowest of the two CTAs (the lower ring); the rest is written
+  // before it is read for a voxel of R
+  for (int q = tid; q < 2 * kRows; q += kThreads)
+    reinterpret_cast<uint4*>(act)[q] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid < 4 * kLead)
+    reinterpret_cast<uint4*>(act)[(2 + tid / kLead % 2) * kRows + tid / (2 * kLead) * 4 * 128 + tid % kLead] =
+        make_uint4(0u, 0u, 0u, 0u);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tslot)),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  // everything up to here overlaps the end of the kernel before
+  pdl_wait();
+  pdl_next();
+  // layer-1 input, channels 0..2 of channel plane 0
   constexpr int kPer = (1000 + kThreads - 1) / kThreads;
   const float* xs = x + (size_t)s * 1000 * 3;
   float xv[kPer][3];
@@ -275,21 +292,6 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kThreads, 1)
         for (int ch = 0; ch < 3; ch++) xv[q][ch] = __ldg(xs + 3 * v + ch);
       }
     }
-  }
-  // zero the channel planes of the first layer, and of the others the rows before
-  // planes 0 and 4, the lowest of the two CTAs (the lower ring); the rest is written
-  // before it is read for a voxel of R
-  for (int q = tid; q < 2 * kRows; q += kThreads)
-    reinterpret_cast<uint4*>(act)[q] = make_uint4(0u, 0u, 0u, 0u);
-  if (tid < 4 * kLead)
-    reinterpret_cast<uint4*>(act)[(2 + tid / kLead % 2) * kRows + tid / (2 * kLead) * 4 * 128 + tid % kLead] =
-        make_uint4(0u, 0u, 0u, 0u);
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tslot)),
-                 "r"(kTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   __syncthreads();
 #pragma unroll
@@ -498,6 +500,6 @@ cudaError_t precond_apply_tc_mesh(PrecondState* P, cudaStream_t st, int nb, cons
   cudaError_t e = set_tc_attr();
   if (e != cudaSuccess) return e;
   MeshIO io{v, dinv, in_map, hs, hp, hw, out_map, set, nvc, z};
-  k_precond_tc<<<nb * kSplit, kThreads, kSmem, st>>>(nullptr, nullptr, P->wtc, P->flags, io);
-  return cudaGetLastError();
+  // (the weights were packed long before: only the input is of the kernel before)
+  return launch_pdl(k_precond_tc, dim3(nb * kSplit), dim3(kThreads), kSmem, st, nullptr, nullptr, P->wtc, P->flags, io);
 }

@@ -1432,11 +1432,12 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
   const bool pre_xf = !flexible && c->inner_fp32;
   if (!c->d_xs) CK(cudaMalloc(reinterpret_cast<void**>(&c->d_xs), sizeof(float) * 2 * n));
   float* xf_next = pre_xf ? c->d_xs : nullptr;
-  auto inner_matvec = [&](int jj, const double* zj) -> cudaError_t {
+  auto inner_matvec = [&](int jj, const double* zj, bool zf) -> cudaError_t {
     if (c->inner_fp32) {
       OpIn in{};
       if (zj) {
         in.vd = zj;
+        in.xf_ready = zf;  // the network left fp32(z) in d_xs
       } else {
         in.vh = vf(jj);
         in.vl = vf(jj) + ld;
@@ -1475,10 +1476,11 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     if (flexible) {
       double* zj = c->d_Z + (size_t)jj * n;
       launch_pdl(k_from_ff, dim3(gr), dim3(256), 0, s, n, vf(jj), c->d_tmpv);  // v_j in FP64 for the network
-      if ((ee = launch_precond_net(c, c->d_tmpv, zj)) != cudaSuccess) return ee;
-      if ((ee = inner_matvec(jj, zj)) != cudaSuccess) return ee;
+      bool zf = false;
+      if ((ee = launch_precond_net(c, c->d_tmpv, zj, c->d_xs, &zf)) != cudaSuccess) return ee;
+      if ((ee = inner_matvec(jj, zj, zf)) != cudaSuccess) return ee;
     } else {
-      if ((ee = inner_matvec(jj, nullptr)) != cudaSuccess) return ee;
+      if ((ee = inner_matvec(jj, nullptr, false)) != cudaSuccess) return ee;
       // training pairs for the learned preconditioner: (A D v_j, D v_j)
       if (harvest) {
         launch_pdl(k_from_ff, dim3(gr), dim3(256), 0, s, n, wf, c->d_tmpv);

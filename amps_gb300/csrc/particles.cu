@@ -235,9 +235,11 @@ __device__ __forceinline__ void lapenta(float h, const float E[3], const float B
 constexpr int kPushWarps = 4;       // warps per CTA (one row of 8 cells each)
 constexpr int kSlabSC = 2 * 81;     // a layer of cells sees two planes of corners
 constexpr int kSlabCSC = 3 * 100;   // and three planes of centres
-// What bounds it: the shared-memory return path (80 % of its cycles while the kernel
-// runs: the tile accumulation's 48 16-byte loads per 32 particles, 37 % of the time)
-// with issue at 53 % and the FMA pipe at 40 %.  A CTA takes half a layer of a block and
+// What bounds it: no single unit; the shared-memory return path is at 80 % while the
+// kernel runs, issue at 53 %, the FMA pipe at 40 %, and the tile accumulation (48 16-byte
+// shared loads and 144 packed FMAs per 32 particles) takes 37 % of the time.  (Tiles of
+// 27 x 12 sums that halve the loads' cost need a third more packed FMAs: 2.60 to 2.82
+// ms.)  A CTA takes half a layer of a block and
 // stages the layer's two planes of corners (7.8 KB, where the block's nine took 35), so
 // four CTAs of four warps share an SM at 128 registers: the same 16 warps as two of
 // eight, with shorter waits at a CTA's start and end.  More warps only lose: five CTAs

@@ -200,12 +200,16 @@ __global__ void __launch_bounds__(256) k_scatter_z(int nb, long long nvc,
 __global__ void __launch_bounds__(256) k_pc_jacobi(long long n, const int* __restrict__ ids,
                                                    long long nvc, const double* __restrict__ vin,
                                                    const double* __restrict__ dinv,
-                                                   double* __restrict__ z) {
+                                                   double* __restrict__ z, float* __restrict__ xf) {
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n;
        q += (long long)gridDim.x * blockDim.x) {
     const long long id = ids[q];
 #pragma unroll
-    for (int ch = 0; ch < 3; ch++) z[ch * nvc + id] = dinv[ch * nvc + id] * vin[ch * nvc + id];
+    for (int ch = 0; ch < 3; ch++) {
+      const double v = dinv[ch * nvc + id] * vin[ch * nvc + id];
+      z[ch * nvc + id] = v;
+      xf[ch * nvc + id] = (float)v;
+    }
   }
 }
 
@@ -355,20 +359,21 @@ cudaError_t precond_harvest_pairs(amps_gpu_ctx* c, const double* r, const double
 }
 
 // z = D v + N(D v) on the mesh
-cudaError_t launch_precond_net(amps_gpu_ctx* c, const double* v, double* z) {
+cudaError_t launch_precond_net(amps_gpu_ctx* c, const double* v, double* z, float* xf, bool* xf_ready) {
   PrecondState* P = c->pn;
   if (!P) return cudaErrorInvalidValue;
+  *xf_ready = P->use_tc;
   cudaError_t e;
   if (c->pc_njac > 0) {
     TimedLaunch t(c, "precond_jacobi_hanging");
     k_pc_jacobi<<<(unsigned)std::min<long long>((c->pc_njac + 255) / 256, 1216), 256, 0, c->stream>>>(
-        c->pc_njac, c->d_pc_jac, c->nvc, v, c->d_dinv, z);
+        c->pc_njac, c->d_pc_jac, c->nvc, v, c->d_dinv, z, xf);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (P->use_tc) {
     TimedLaunch t(c, "precond_net_tc");
     return precond_apply_tc_mesh(P, c->stream, c->nb, c->d_pc_in, c->d_hs, c->d_hp, c->d_hw,
-                                 c->d_pc_out, c->d_pc_set, c->nvc, v, c->d_dinv, z);
+                                 c->d_pc_out, c->d_pc_set, c->nvc, v, c->d_dinv, z, xf);
   }
   if ((e = precond_work(P, c->nb)) != cudaSuccess) return e;
   {

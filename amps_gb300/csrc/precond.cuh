@@ -67,7 +67,8 @@ cudaError_t precond_forward_tc(PrecondState* P, cudaStream_t st, int S, const fl
 cudaError_t precond_apply_tc_mesh(PrecondState* P, cudaStream_t st, int nb, const int* in_map,
                                   const int* hs, const int* hp, const double* hw,
                                   const int* out_map, const int* set, long long nvc,
-                                  const double* v, const double* dinv, double* z);
+                                  const double* v, const double* dinv, double* z, float* xf);
 // GMRES hooks (field.cu)
-cudaError_t launch_precond_net(amps_gpu_ctx* c, const double* v, double* z);
+// xf_ready: the FP32 operator's input fp32(z) was left in xf too (tensor-core path)
+cudaError_t launch_precond_net(amps_gpu_ctx* c, const double* v, double* z, float* xf, bool* xf_ready);
 cudaError_t precond_harvest_pairs(amps_gpu_ctx* c, const double* r, const double* e, int e_scaled);

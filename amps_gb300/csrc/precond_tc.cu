@@ -231,6 +231,7 @@ struct MeshIO {
   const int* set;
   long long nvc;
   double* z;
+  float* xf;  // z in FP32, the operator's input
 };
 
 __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kThreads, 1)
@@ -389,9 +390,12 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kThreads, 1)
             const long long id = mesh.out_map[(size_t)s * 512 + (i - 1) + 8 * ((j - 1) + 8 * (k - 1))];
             if (id >= 0) {
 #pragma unroll
-              for (int ch = 0; ch < 3; ch++)
-                mesh.z[ch * mesh.nvc + id] = mesh.dinv[ch * mesh.nvc + id] * mesh.v[ch * mesh.nvc + id] +
-                                             (double)__uint_as_float(r[g][0][ch]);
+              for (int ch = 0; ch < 3; ch++) {
+                const double z = mesh.dinv[ch * mesh.nvc + id] * mesh.v[ch * mesh.nvc + id] +
+                                 (double)__uint_as_float(r[g][0][ch]);
+                mesh.z[ch * mesh.nvc + id] = z;
+                mesh.xf[ch * mesh.nvc + id] = (float)z;
+              }
             }
           } else {
             float* dst = y + ((size_t)s * 1000 + (k * 10 + j) * 10 + i) * 3;
@@ -486,7 +490,7 @@ cudaError_t precond_forward_tc(PrecondState* P, cudaStream_t st, int S, const fl
   if (!P->tc_ready || !P->flags) return cudaErrorInvalidValue;
   cudaError_t e = set_tc_attr();
   if (e != cudaSuccess) return e;
-  MeshIO none{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr};
+  MeshIO none{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr};
   k_precond_tc<<<S * kSplit, kThreads, kSmem, st>>>(x, y, P->wtc + (size_t)P->active * (kWBytes / 2),
                                                     P->flags, none);
   return cudaGetLastError();
@@ -495,11 +499,11 @@ cudaError_t precond_forward_tc(PrecondState* P, cudaStream_t st, int S, const fl
 cudaError_t precond_apply_tc_mesh(PrecondState* P, cudaStream_t st, int nb, const int* in_map,
                                   const int* hs, const int* hp, const double* hw,
                                   const int* out_map, const int* set, long long nvc,
-                                  const double* v, const double* dinv, double* z) {
+                                  const double* v, const double* dinv, double* z, float* xf) {
   if (!P->tc_ready || !P->flags) return cudaErrorInvalidValue;
   cudaError_t e = set_tc_attr();
   if (e != cudaSuccess) return e;
-  MeshIO io{v, dinv, in_map, hs, hp, hw, out_map, set, nvc, z};
+  MeshIO io{v, dinv, in_map, hs, hp, hw, out_map, set, nvc, z, xf};
   // (the weights were packed long before: only the input is of the kernel before)
   return launch_pdl(k_precond_tc, dim3(nb * kSplit), dim3(kThreads), kSmem, st, nullptr, nullptr, P->wtc, P->flags, io);
 }

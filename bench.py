@@ -41,11 +41,11 @@ METRIC = "particle-steps/s (push+deposit)"
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the
 # particle-step kernels on the default workload, from a one-pass ncu capture
 # of this bench command; "version" names the kernel revision it was taken on
-MEASURED_TRAFFIC = {"amr_64c_128ppc": {"version": "push_deposit packed-FMA 3x3 tiles on SoA "
-                                                  "records, FP32 chunk sums, unrolled full chunks; "
-                                                  "arrivals from a "
+MEASURED_TRAFFIC = {"amr_64c_128ppc": {"version": "push_deposit on half-layer CTAs with "
+                                                  "slab stencils, packed-FMA 3x3 tiles on SoA "
+                                                  "records, FP32 chunk sums; arrivals from a "
                                                   "per-layer cell list",
-                                       "push_deposit": 4.663e9, "arrivals": 1.015e9}}
+                                       "push_deposit": 4.526e9, "arrivals": 1.015e9}}
 UNIT = "particle-steps/s"
 
 
@@ -196,8 +196,9 @@ def kernel_bytes(n, ncell, nb, name, b_center=False):
     if name == "push_deposit":
         # particles: read u,v (24) + species (1), write u,v (24); per cell: base, cnt
         # (8), stay (4), partials 267 floats (27 monomials x 9 + 8 corners x 3);
-        # stencils 23.3 + 11.7 KB per CTA (centre B: 23.3 + 2 x 16 KB)
-        return n * 49 + ncell * (12 + 267 * 4) + ctas * (23328 + (32000 if b_center else 11664))
+        # stencils of half a layer of a block: two planes of 81 corners, 32 + 16 B each
+        # (centre B: 32 B, and three planes of 100 centres twice, 16 B each)
+        return n * 49 + ncell * (12 + 267 * 4) + 2 * ctas * (162 * 32 + (9600 if b_center else 162 * 16))
     if name == "arrivals":
         # per cell: base, base+1, cnt, stay, arr (20) and cnt/arr writes (8); the
         # ~1% arrivals and their partial read-modify-write; stencil per CTA

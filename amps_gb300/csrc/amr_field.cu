@@ -1036,22 +1036,25 @@ __global__ void __launch_bounds__(256) k_amr_update_e(long long ncell, long long
   add_energy((0.125 * ee + eb) * 0.125 / kPi, energy);
 }
 
-__global__ void k_amr_pack(long long nvc, const int* ctab, Hang h, const double* Eh,
-                           const double* Bprev, const double* Bcur, float* sp, float* sd) {
+// three CTAs per block, a corner per thread (ctabh: hanging corners as ~id); 960 blocks:
+// 33 us (one CTA per block and two looks at the constraint rows per value: 41)
+__global__ void __launch_bounds__(256) k_amr_pack(long long nvc, const int* __restrict__ ctabh, Hang h,
+                                                  const double* __restrict__ Eh, const double* __restrict__ Bprev,
+                                                  const double* __restrict__ Bcur, float* __restrict__ sp,
+                                                  float* __restrict__ sd) {
   pdl_wait();
   pdl_next();
-  const int b = blockIdx.x;
-  for (int s = threadIdx.x; s < AMPS_SC; s += blockDim.x) {
-    const int cc = ctab[b * 729 + s];
-    float4* op = reinterpret_cast<float4*>(sp + ((size_t)b * AMPS_SC + s) * AMPS_PUSH_STRIDE);
-    op[0] = make_float4((float)cval(Eh, nullptr, nvc, cc, 0, h), (float)cval(Eh, nullptr, nvc, cc, 1, h),
-                        (float)cval(Eh, nullptr, nvc, cc, 2, h), (float)cval(Bprev, nullptr, nvc, cc, 0, h));
-    op[1] = make_float4((float)cval(Bprev, nullptr, nvc, cc, 1, h),
-                        (float)cval(Bprev, nullptr, nvc, cc, 2, h), 0.f, 0.f);
-    reinterpret_cast<float4*>(sd)[(size_t)b * AMPS_SC + s] =
-        make_float4((float)cval(Bcur, nullptr, nvc, cc, 0, h), (float)cval(Bcur, nullptr, nvc, cc, 1, h),
-                    (float)cval(Bcur, nullptr, nvc, cc, 2, h), 0.f);
-  }
+  const int b = blockIdx.x, s = blockIdx.y * 256 + threadIdx.x;
+  if (s >= AMPS_SC) return;
+  const int id = ctabh[b * 729 + s];
+  auto val = [&](const double* F, int d) {
+    return (float)(id >= 0 ? F[d * nvc + id] : cval(F, nullptr, nvc, ~id, d, h));
+  };
+  float4* op = reinterpret_cast<float4*>(sp + ((size_t)b * AMPS_SC + s) * AMPS_PUSH_STRIDE);
+  op[0] = make_float4(val(Eh, 0), val(Eh, 1), val(Eh, 2), val(Bprev, 0));
+  op[1] = make_float4(val(Bprev, 1), val(Bprev, 2), 0.f, 0.f);
+  reinterpret_cast<float4*>(sd)[(size_t)b * AMPS_SC + s] =
+      make_float4(val(Bcur, 0), val(Bcur, 1), val(Bcur, 2), 0.f);
 }
 
 Hang hang_of(const amps_gpu_ctx* c) {
@@ -1066,7 +1069,7 @@ unsigned g1(long long n) { return (unsigned)((n + 255) / 256); }
 cudaError_t launch_amr_pack(amps_gpu_ctx* c, const double* Eh, const double* Bprev,
                             const double* Bcur) {
   TimedLaunch t(c, "pack_stencils");
-  launch_pdl(k_amr_pack, dim3(c->nb), dim3(256), 0, c->stream, c->nvc, c->d_ctab, hang_of(c), Eh, Bprev, Bcur,
+  launch_pdl(k_amr_pack, dim3(c->nb, 3), dim3(256), 0, c->stream, c->nvc, c->d_ctabh, hang_of(c), Eh, Bprev, Bcur,
                                             c->d_stencil_push, c->d_stencil_dep);
   return cudaGetLastError();
 }

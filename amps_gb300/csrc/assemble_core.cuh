@@ -65,37 +65,43 @@ __device__ __forceinline__ void asm_stage(float* s_c, const float* __restrict__ 
   __syncthreads();
 }
 
+// slot of corner `lane` of the tile: acc[9]
+__device__ __forceinline__ void asm_slot(const float* __restrict__ s_c, int slot, int lane, float (&acc)[9]) {
+  const int i = lane & 7, j = lane >> 3;
+  int d[3] = {slot % 3, (slot / 3) % 3, slot / 9};
+  int lo[3], hi[3];  // the corner's offset bits in the slot's cells
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    d[a] = d[a] == 0 ? 0 : (d[a] == 1 ? -1 : 1);
+    lo[a] = d[a] < 0 ? 1 : 0;
+    hi[a] = d[a] > 0 ? 0 : 1;
+  }
+#pragma unroll
+  for (int e = 0; e < 9; e++) acc[e] = 0.f;
+  for (int lz = lo[2]; lz <= hi[2]; lz++)
+    for (int ly = lo[1]; ly <= hi[1]; ly++)
+      for (int lx = lo[0]; lx <= hi[0]; lx++) {
+        const int mono = (2 * lx + d[0]) + 3 * (2 * ly + d[1]) + 9 * (2 * lz + d[2]);
+        const int row = (j - ly + 1) + 5 * (1 - lz), ii = i - lx;
+        const float* src = (ii >= 0 ? s_c + row * kAsmRowF + ii * AMPS_CELLM
+                                    : s_c + kAsmRows * kAsmRowF + row * AMPS_CELLM) +
+                           mono * 9;
+#pragma unroll
+        for (int e = 0; e < 9; e++) acc[e] += src[e];
+      }
+}
+
 // The warp's slots of corner `lane` of the tile: out(slot, acc[9])
 template <class Out>
 __device__ __forceinline__ void asm_slots(const float* __restrict__ s_c, int wid, int lane, const Out& out) {
-  const int i = lane & 7, j = lane >> 3;
   for (int q = c_asm_first[wid]; q < c_asm_first[wid + 1]; q++) {
     const int slot = c_asm_slot[q];
-    int d[3] = {slot % 3, (slot / 3) % 3, slot / 9};
-    int lo[3], hi[3];  // the corner's offset bits in the slot's cells
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      d[a] = d[a] == 0 ? 0 : (d[a] == 1 ? -1 : 1);
-      lo[a] = d[a] < 0 ? 1 : 0;
-      hi[a] = d[a] > 0 ? 0 : 1;
-    }
     float acc[9];
-#pragma unroll
-    for (int e = 0; e < 9; e++) acc[e] = 0.f;
-    for (int lz = lo[2]; lz <= hi[2]; lz++)
-      for (int ly = lo[1]; ly <= hi[1]; ly++)
-        for (int lx = lo[0]; lx <= hi[0]; lx++) {
-          const int mono = (2 * lx + d[0]) + 3 * (2 * ly + d[1]) + 9 * (2 * lz + d[2]);
-          const int row = (j - ly + 1) + 5 * (1 - lz), ii = i - lx;
-          const float* src = (ii >= 0 ? s_c + row * kAsmRowF + ii * AMPS_CELLM
-                                      : s_c + kAsmRows * kAsmRowF + row * AMPS_CELLM) +
-                             mono * 9;
-#pragma unroll
-          for (int e = 0; e < 9; e++) acc[e] += src[e];
-        }
+    asm_slot(s_c, slot, lane, acc);
     out(slot, acc);
   }
 }
+constexpr int kAsmMaxSlots = 8;  // of a warp
 
 // component d of corner (i, j, k)'s current: the sum over its 8 cells
 template <class CellId>

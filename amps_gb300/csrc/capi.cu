@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -268,8 +269,10 @@ amps_gpu_status particle_step(amps_gpu_ctx* c, bool deposit, long long* out_of_b
       c->arr_tune_ms[c->arr_tune_cur] += ms;
       c->arr_tune_n[c->arr_tune_cur]++;
     }
+    // means equal to 0.1 us, below what the events resolve, keep 16
+    auto mean = [&](int q) { return std::nearbyint(c->arr_tune_ms[q] / c->arr_tune_n[q] * 1e4); };
     if (--c->arr_tune_left == 0 && c->arr_tune_n[0] > 0 && c->arr_tune_n[1] > 0)
-      c->arr_chunk = c->arr_tune_ms[1] / c->arr_tune_n[1] < c->arr_tune_ms[0] / c->arr_tune_n[0] ? 32 : 16;
+      c->arr_chunk = mean(1) < mean(0) ? 32 : 16;
     c->arr_tune_cur = -1;
   }
   if (ovf > 0) {

@@ -248,7 +248,8 @@ constexpr int kSlabCSC = 3 * 100;   // and three planes of centres
 // (108).
 // CB: the particles see B interpolated from the cell centres (B^n from the
 // centre stencil for the push, B^{n+1} for the deposit); E from the corners.
-template <bool DEP, bool AMR, bool CB = false>
+// PARTS: a warp takes a row's 8 cells, or one of PARTS parts of them (push_parts).
+template <bool DEP, bool AMR, bool CB = false, int PARTS = 1>
 __global__ void __launch_bounds__(kPushWarps * 32, 4) k_push_deposit(StepArgs a) {
   extern __shared__ __align__(16) float4 s_dyn[];
   constexpr int kDepSC = CB ? kSlabCSC : kSlabSC;
@@ -269,6 +270,8 @@ __global__ void __launch_bounds__(kPushWarps * 32, 4) k_push_deposit(StepArgs a)
   const uint32_t bd = DEP ? kDepSC * 4 * sizeof(float) : 0;
   const uint32_t bc = CB ? kSlabCSC * sizeof(float4) : 0;
   const int j = wid + kPushWarps * (blockIdx.y % (AMPS_NC / kPushWarps));
+  constexpr int kCells = AMPS_NC / PARTS;
+  const int i0 = PARTS == 1 ? 0 : blockIdx.z * kCells, i1 = i0 + kCells;  // of the row
   // slot range and occupancy of the row's 8 cells, one lane per cell
   int mb0 = 0, mn0 = 0;
   if (lane < AMPS_NC) {
@@ -283,7 +286,7 @@ __global__ void __launch_bounds__(kPushWarps * 32, 4) k_push_deposit(StepArgs a)
   int ps = 0;
   float pwc = 1.0f;
   uint32_t pid = 0;
-  int pf_cell = 0;  // cell whose chunk the prefetch registers hold
+  int pf_cell = i0;  // cell whose chunk the prefetch registers hold
   auto prefetch = [&](int c, int q) {
     const int cb = __shfl_sync(0xffffffffu, mb0, c), cn = __shfl_sync(0xffffffffu, mn0, c);
     pf_cell = c;
@@ -296,7 +299,7 @@ __global__ void __launch_bounds__(kPushWarps * 32, 4) k_push_deposit(StepArgs a)
       pid = a.p.id ? a.p.id[pn] : 0u;
     }
   };
-  prefetch(0, lane);  // in flight while the stencils are staged
+  prefetch(i0, lane);  // in flight while the stencils are staged
   pdl_wait();  // the stencils
   pdl_next();
   const size_t cor = (size_t)b * AMPS_SC + 81 * k, cen = (size_t)b * AMPS_CSC + 100 * k;
@@ -311,7 +314,7 @@ __global__ void __launch_bounds__(kPushWarps * 32, 4) k_push_deposit(StepArgs a)
   unsigned n_far = 0, n_near = 0, n_del = 0;
   const float inv_vol = block_inv_vol(a, b);
   const float bdtdx = AMR ? __ldg(a.amr.bdtdx + b) : 0.0f;
-  for (int i = 0; i < AMPS_NC; i++) {
+  for (int i = i0; i < i1; i++) {
     const long long cid = (long long)b * AMPS_CPB + i + AMPS_NC * (j + AMPS_NC * k);
     const int b0 = __shfl_sync(0xffffffffu, mb0, i), n0 = __shfl_sync(0xffffffffu, mn0, i);
     Tile tile;
@@ -327,7 +330,7 @@ __global__ void __launch_bounds__(kPushWarps * 32, 4) k_push_deposit(StepArgs a)
       uint32_t idv = pid;
       if (q0 + 32 < n0)
         prefetch(i, q0 + 32 + lane);
-      else if (i + 1 < AMPS_NC)
+      else if (i + 1 < i1)
         prefetch(i + 1, lane);
       if (act) {
         // gather E^{n+theta}, B^n at the old position, which lies in this cell (every
@@ -1733,10 +1736,12 @@ StepArgs step_args(amps_gpu_ctx* c) {
   return a;
 }
 
-size_t smem_push(bool dep, bool cb = false) {
+// (below the 48 KB that need no attribute)
+constexpr size_t smem_push(bool dep, bool cb = false) {
   return (size_t)(2 * kSlabSC + (cb ? 2 * kSlabCSC : kSlabSC)) * sizeof(float4) +
          (dep ? kPushWarps * kFields * kFS * sizeof(float) : 0);
 }
+static_assert(smem_push(true, true) <= 48 * 1024, "");
 size_t smem_dep(bool cb = false) {
   return (size_t)(cb ? AMPS_CSC : AMPS_SC) * sizeof(float4) + kWarps * kFields * kFS * sizeof(float);
 }
@@ -1745,20 +1750,12 @@ size_t smem_arr(int chunk) { return (size_t)kWarps * kFields * (chunk + 4) * siz
 void set_smem_attrs() {
   static bool done = false;
   if (done) return;
-  cudaFuncSetAttribute(k_push_deposit<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_push(true));
-  cudaFuncSetAttribute(k_push_deposit<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_push(false));
-  cudaFuncSetAttribute(k_push_deposit<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_push(true));
-  cudaFuncSetAttribute(k_push_deposit<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_push(false));
   cudaFuncSetAttribute(k_arrivals<true, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_arr(16));
   cudaFuncSetAttribute(k_arrivals<false, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_arr(16));
   cudaFuncSetAttribute(k_arrivals<true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_arr(32));
   cudaFuncSetAttribute(k_arrivals<false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_arr(32));
   cudaFuncSetAttribute(k_deposit<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dep(false));
   cudaFuncSetAttribute(k_deposit<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dep(true));
-  cudaFuncSetAttribute(k_push_deposit<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem_push(true, true));
-  cudaFuncSetAttribute(k_push_deposit<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem_push(false, true));
   cudaFuncSetAttribute(k_arrivals<true, 16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_arr(16));
   cudaFuncSetAttribute(k_arrivals<false, 16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_arr(16));
   cudaFuncSetAttribute(k_arrivals<true, 32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_arr(32));
@@ -1946,28 +1943,45 @@ cudaError_t launch_inject(amps_gpu_ctx* c, const StepArgs& a) {
   return cudaGetLastError();
 }
 
+// A warp's time is its cells' chain, so a mesh whose CTAs all run at once (four per SM on
+// 152 SMs: up to 9 blocks) splits its rows in four: one block 10 us, 20 with whole rows.
+// Beyond, whole rows are as fast or faster (64 blocks 186 us against 184 to 188, 960
+// refined 2.54 ms against 2.65).
+constexpr int kParts = 4;
+static int push_parts(const amps_gpu_ctx* c) {
+  return (long long)kParts * c->nb * AMPS_NC * AMPS_NC / kPushWarps <= 4 * 152 ? kParts : 1;
+}
+template <bool DEP, bool AMR, bool CB>
+static cudaError_t launch_push(amps_gpu_ctx* c, const StepArgs& a) {
+  const int parts = push_parts(c);
+  const dim3 grid(c->nb, AMPS_NC * AMPS_NC / kPushWarps, parts), block(kPushWarps * 32);
+  return parts == kParts
+             ? launch_pdl(k_push_deposit<DEP, AMR, CB, kParts>, grid, block, smem_push(DEP, CB), c->stream, a)
+             : launch_pdl(k_push_deposit<DEP, AMR, CB, 1>, grid, block, smem_push(DEP, CB), c->stream, a);
+}
+
 cudaError_t launch_push_step(amps_gpu_ctx* c, bool deposit) {
   set_smem_attrs();
   cudaError_t e;
   StepArgs a = step_args(c);
-  const dim3 grid(c->nb, AMPS_NC), pgrid(c->nb, AMPS_NC * AMPS_NC / kPushWarps);
+  const dim3 grid(c->nb, AMPS_NC);
   {
     TimedLaunch t(c, deposit ? "push_deposit" : "push");
     if (c->amr) {
       if (deposit)
-        launch_pdl(k_push_deposit<true, true>, pgrid, dim3(kPushWarps * 32), smem_push(true), c->stream, a);
+        launch_push<true, true, false>(c, a);
       else
-        launch_pdl(k_push_deposit<false, true>, pgrid, dim3(kPushWarps * 32), smem_push(false), c->stream, a);
+        launch_push<false, true, false>(c, a);
     } else if (c->b_center) {
       if (deposit)
-        launch_pdl(k_push_deposit<true, false, true>, pgrid, dim3(kPushWarps * 32), smem_push(true, true), c->stream, a);
+        launch_push<true, false, true>(c, a);
       else
-        launch_pdl(k_push_deposit<false, false, true>, pgrid, dim3(kPushWarps * 32), smem_push(false, true), c->stream, a);
+        launch_push<false, false, true>(c, a);
     } else {
       if (deposit)
-        launch_pdl(k_push_deposit<true, false>, pgrid, dim3(kPushWarps * 32), smem_push(true), c->stream, a);
+        launch_push<true, false, false>(c, a);
       else
-        launch_pdl(k_push_deposit<false, false>, pgrid, dim3(kPushWarps * 32), smem_push(false), c->stream, a);
+        launch_push<false, false, false>(c, a);
     }
   }
   e = cudaGetLastError();

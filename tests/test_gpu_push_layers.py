@@ -18,7 +18,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("centre", [False, True])
-@pytest.mark.parametrize("nb", [(1, 1, 1), (2, 1, 3)])
+@pytest.mark.parametrize("nb", [(1, 1, 1), (2, 1, 3), (3, 3, 1), (5, 2, 1)])  # rows in parts up to 9 blocks
 def test_slab_edges_and_velocity_orders(nb, centre):
     wl, _, _, f = G.make_case(nb=nb, ppc=1, seed=51)
     n3 = np.array(wl.mesh.shape)

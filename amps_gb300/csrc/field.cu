@@ -1364,7 +1364,7 @@ cudaError_t launch_c2n_update_e(amps_gpu_ctx* c, const double* Bcen, double* Bco
     return e == cudaSuccess ? launch_amr_update_e(c) : e;
   }
   const double vol = c->cfg.dx[0] * c->cfg.dx[1] * c->cfg.dx[2];
-  TimedLaunch t(c, "c2n_update_e");
+  TimedLaunch t(c, "update_e");  // C2N with it
   launch_pdl(k_c2n_update_e, dim3(grid1(c->ncor)), dim3(256), 0, c->stream, c->ncor, c->d_nbr, Bcen, Bcor, c->d_Eh, c->d_En,
                                                         c->cfg.theta, vol / (8.0 * kPi), c->d_energy + 1);
   return cudaGetLastError();

@@ -1440,10 +1440,10 @@ __device__ __forceinline__ double boris_rel(double qm, double gyro, double ic2, 
   const double gam = rsqrt(1.0 - (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]) * ic2);
   const double b2 = B[0] * B[0] + B[1] * B[1] + B[2] * B[2];
   // the gyro period gyro gam / |B|, compared squared: its root is formed only
-  // where it limits the step
+  // where it limits the step (and may round to above rem, which bounds it)
   double dt = rem;
   const double gg = gyro * gam;
-  if (b2 > 1.0e-50 && gg * gg < rem * rem * b2) dt = gg * rsqrt(b2);
+  if (b2 > 1.0e-50 && gg * gg < rem * rem * b2) dt = fmin(rem, gg * rsqrt(b2));
   const double h = 0.5 * qm * dt;
   double um[3], t[3], up[3], uf[3], l = 0.0;
   for (int d = 0; d < 3; d++) um[d] = gam * v[d] + h * E[d];
@@ -1478,8 +1478,9 @@ __global__ void __launch_bounds__(256) k_relboris(RelBorisArgs a) {
       v[d] = widen(a.d.v[d][p]);
     }
     double rem = a.dt_total;
+    bool left = false;  // through an open face
     long long ns = 0;
-    while (rem > 0.0) {
+    while (rem > 0.0 && !left) {
       if (ns >= a.max_sub) {
         atomicAdd(a.flags + 2, 1ull);
         break;
@@ -1517,7 +1518,7 @@ __global__ void __launch_bounds__(256) k_relboris(RelBorisArgs a) {
           // (long long)o saturates; one bound keeps the sum in range for any o
           const long long bb = bx[d] + max(min((long long)o, 1LL << 40), -(1LL << 40));
           if (bb < 0 || bb >= a.nbk[d]) {
-            if ((a.open >> d) & 1) rem = -1.0;
+            if ((a.open >> d) & 1) left = true;
             const long long r = bb % a.nbk[d];
             bx[d] = (int)(r < 0 ? r + a.nbk[d] : r);
           } else {
@@ -1534,7 +1535,7 @@ __global__ void __launch_bounds__(256) k_relboris(RelBorisArgs a) {
       ns++;
     }
     my_sub += (unsigned long long)ns;
-    if (rem < 0.0) {  // left the domain through an open face
+    if (left) {
       a.key[p] = -1;
       atomicAdd(a.flags + 6, 1ull);
       continue;
@@ -1613,8 +1614,9 @@ __global__ void __launch_bounds__(256) k_amr_relboris(AmrRelBorisArgs a) {
       v[d] = a.d.v[d][p];
     }
     double rem = a.dt_total;
+    bool left = false;  // through an open face
     long long ns = 0;
-    while (rem > 0.0) {
+    while (rem > 0.0 && !left) {
       if (ns >= a.max_sub) {
         atomicAdd(a.flags + 2, 1ull);
         break;
@@ -1660,7 +1662,7 @@ __global__ void __launch_bounds__(256) k_amr_relboris(AmrRelBorisArgs a) {
         for (int d = 0; d < 3; d++) {
           x[d] += dt * v[d];
           if (((a.open >> d) & 1) && (x[d] < a.x0[d] || x[d] >= a.x0[d] + a.m.nfine[d] * a.dxf))
-            rem = -1.0;
+            left = true;
         }
         ns++;
         continue;
@@ -1670,12 +1672,12 @@ __global__ void __launch_bounds__(256) k_amr_relboris(AmrRelBorisArgs a) {
       for (int d = 0; d < 3; d++) {
         x[d] += v[d] * dt;
         if (((a.open >> d) & 1) && (x[d] < a.x0[d] || x[d] >= a.x0[d] + a.m.nfine[d] * a.dxf))
-          rem = -1.0;
+          left = true;
       }
       ns++;
     }
     my_sub += (unsigned long long)ns;
-    if (rem < 0.0) {  // left the domain through an open face
+    if (left) {
       a.key[p] = -1;
       atomicAdd(a.flags + 6, 1ull);
       continue;

@@ -555,13 +555,15 @@ __device__ __forceinline__ FF ff_warp_sum(FF a) {
 //     are fewer vectors than warps), so the register cost does not grow with
 //     nv and no sums cross warps inside the sweep.
 // The staged tile serves both halves of the second sweep (w' and then h2), the
-// third sweep needs V's hi halves only and sums V h2 in FP32 (h2 is of the order
-// of the pair arithmetic's own rounding, 2^-48 |w|; relative errors of 2^-24 in
-// V h2 are far below the last bit of w''), and tiles are walked in alternating directions so
-// a sweep starts on what the last one left in L2: 2.5 basis reads per step.
-// ||w''||^2 = ||w'||^2 - ||h2||^2 (V orthonormal) spares a sweep and a grid
-// barrier; where the second projection took more than half of ||w'||^2 (w in
-// the span of V) it is summed instead, from a sweep with the full pairs.
+// third sweep needs V's hi halves only and sums V h2 in FP32, and tiles are walked
+// in alternating directions so a sweep starts on what the last one left in L2: 2.5
+// basis reads per step.  ||w''||^2 = ||w'||^2 - ||h2||^2 (V orthonormal) spares a
+// sweep and a grid barrier.  Both hold where h2 is no more than the first
+// projection's rounding, a few 2^-48 |w|: FP32 is wrong by 2^-24 of V h2, which
+// ||h2|| <= 2^-28 ||w'|| (kArnSmallH2, its square) keeps under the pairs' own
+// last bit.  Any larger h2 (|w'| far below |w|, or a basis that lost its
+// orthogonality) takes the third sweep in full pairs and the norm from its sum, one
+// more grid barrier.
 // A CTA whose tiles all fit its stages reads them once.  1.34M unknowns, mean
 // step of a 55-iteration solve (1 to 30 vectors): 103 us, 4 us per vector (the
 // rate of HBM) on ~45 us of barriers and start-up.  Before: 304 us with
@@ -578,6 +580,7 @@ constexpr size_t kArnSmem = 108 * 1024;
 constexpr size_t arn_extra(int T) { return sizeof(float) * (T < kArnCons ? 8 : 4) * T; }
 constexpr size_t arn_ring(int T) { return kArnSmem - arn_extra(T); }
 constexpr int kArnDots = kMaxV;             // dots per sweep: nv, and ||w'||^2
+constexpr double kArnSmallH2 = 0x1p-56;     // of ||h2||^2 / ||w'||^2
 constexpr int kArnRounds = kArnDots / kArnWarps;  // vectors per warp at most
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -844,7 +847,7 @@ __global__ void __launch_bounds__(kArnBlock, 2) k_arnoldi_tile(
     t = warp_sum(t);
     if (lane == 0) {
       const double w2 = s_n2, n2 = w2 - t;
-      s_slow = !(n2 >= 0.5 * w2) || !(n2 > 0.0);
+      s_slow = !(t <= kArnSmallH2 * w2) || !(n2 > 0.0);
       s_n2 = n2;
       s_inv = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
     }
@@ -896,7 +899,7 @@ __global__ void __launch_bounds__(kArnBlock, 2) k_arnoldi_tile(
     if (!resident) release(c);
   }
   if (!slow) return;
-  // w was (nearly) in the span of V: its remainder's norm from the sum itself
+  // the second projection counts: the norm from the remainder's sum itself
   float2* part3 = part2 + (size_t)kArnDots * nblk;
   dots_n = 1;
   dots_p = 1;
@@ -951,7 +954,7 @@ bool arn_map(CUtensorMap* m, const float* base, long long cols, long long pitch,
 }
 
 template <int T>
-cudaError_t launch_arnoldi_t(cudaStream_t s, int sms, long long n, const float* V, float* w, int nv,
+cudaError_t launch_arnoldi_t(cudaStream_t s, int ctas, long long n, const float* V, float* w, int nv,
                              float* vnext, double* d_arn, GmState* gs, int jj, float* xf, const float* dh,
                              unsigned long long* flags) {
   static unsigned long long ready = 0;             // per device
@@ -968,7 +971,7 @@ cudaError_t launch_arnoldi_t(cudaStream_t s, int sms, long long n, const float* 
     ready |= 1ull << dev;
   }
   const long long tiles = (n + T - 1) / T;
-  const unsigned g = (unsigned)std::max<long long>(1, std::min<long long>(2 * sms, tiles));
+  const unsigned g = (unsigned)std::max<long long>(1, std::min<long long>(ctas, tiles));
   const size_t stage = sizeof(float) * 2 * T * (size_t)(nv + 1);
   const long long most = (tiles + g - 1) / g;  // tiles of a CTA
   int stages = (int)std::min<long long>({(long long)kArnMaxStages, (long long)(arn_ring(T) / stage), most});
@@ -987,11 +990,15 @@ cudaError_t launch_arnoldi_t(cudaStream_t s, int sms, long long n, const float* 
 // Tile length: the longest of 1024, 512, 256, 128 elements at which a CTA's ring
 // holds kArnMinStages tiles and, above 128, every CTA gets 4 (a tile costs a
 // barrier or two and the warps' latency: short bases need long tiles, short
-// vectors need tiles for every SM).
+// vectors need tiles for every SM).  tile, ctas: force a length, bound the grid
+// (0: by the rules).
 constexpr int kArnMinStages = 2;
+bool arn_fits(int T, int nv) {
+  return nv + 1 <= kArnDots && kArnMinStages * sizeof(float) * 2 * T * (size_t)(nv + 1) <= arn_ring(T);
+}
 cudaError_t launch_arnoldi(cudaStream_t s, long long n, const float* V, float* w, int nv, float* vnext,
                            double* d_arn, GmState* gs, int jj, float* xf, const float* dh,
-                           unsigned long long* flags) {
+                           unsigned long long* flags, int tile = 0, int ctas = 0) {
   static int sms[64] = {0};  // per device
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1003,13 +1010,14 @@ cudaError_t launch_arnoldi(cudaStream_t s, long long n, const float* V, float* w
     sms[dev] = std::min(v, kArnMaxGrid / 2);
   }
   if (nv + 1 > kArnDots) return cudaErrorInvalidValue;
-  auto fits = [&](int T) {
-    return kArnMinStages * sizeof(float) * 2 * T * (size_t)(nv + 1) <= arn_ring(T) && n >= 8LL * sms[dev] * T;
+  auto takes = [&](int T) {
+    return tile ? tile == T : T == 128 || (arn_fits(T, nv) && n >= 8LL * sms[dev] * T);
   };
-  if (fits(1024)) return launch_arnoldi_t<1024>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
-  if (fits(512)) return launch_arnoldi_t<512>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
-  if (fits(256)) return launch_arnoldi_t<256>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
-  return launch_arnoldi_t<128>(s, sms[dev], n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  const int g = ctas > 0 ? std::min(ctas, 2 * sms[dev]) : 2 * sms[dev];
+  if (takes(1024)) return launch_arnoldi_t<1024>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  if (takes(512)) return launch_arnoldi_t<512>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  if (takes(256)) return launch_arnoldi_t<256>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  return launch_arnoldi_t<128>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
 }
 
 // V0 = r / ||r|| as a pair vector (nrm2: ||r||^2)
@@ -1703,4 +1711,74 @@ amps_gpu_status field_autotune(amps_gpu_ctx* c, double* ms) {
 cudaError_t launch_add(amps_gpu_ctx* c, const double* a, const double* b, double* o, long long n) {
   k_add<<<gridr(n), 256, 0, c->stream>>>(n, a, b, o);
   return cudaGetLastError();
+}
+
+// One Arnoldi step on host vectors, for checks of k_arnoldi_tile by itself: pairs
+// of V and w, a least-squares state whose rotations are the identity (so that its
+// column is h and the norm), the step, and everything back.
+extern "C" amps_gpu_status amps_gpu_arnoldi_step(int device, long long n, int nv, const double* V, const double* w,
+                                                 const double* d, int tile, int ctas, double* h, double* norm,
+                                                 double* vnext, float* xf) {
+  if (n < kArnCons || nv < 1 || nv + 1 > kArnDots || !V || !w || !h || !norm || !vnext || !xf || ctas < 0)
+    return AMPS_GPU_INVALID_ARG;
+  if (tile != 0 && ((tile != 128 && tile != 256 && tile != 512 && tile != 1024) || !arn_fits(tile, nv)))
+    return AMPS_GPU_INVALID_ARG;
+  int ndev = 0;
+  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) return AMPS_GPU_NO_DEVICE;
+  if (device < 0 || device >= ndev) return AMPS_GPU_INVALID_ARG;
+  cudaSetDevice(device);
+  const long long ld = ff_ld(n);
+  const size_t vec = 2 * (size_t)ld * sizeof(float);  // bytes of a pair vector
+  cudaStream_t s = nullptr;
+  char* mem = nullptr;
+  // the basis and V_nv, w, D as a pair vector, one FP64 vector, xf, then the step's scratch
+  const size_t arn = sizeof(double) * 3 * kArnMaxGrid * kMaxV, state = (sizeof(GmState) + 63) & ~(size_t)63;
+  const size_t bytes = vec * (nv + 5) + arn + state + 64;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&mem), bytes);
+  float* dV = reinterpret_cast<float*>(mem);
+  float* dvn = dV + 2 * (size_t)nv * ld;
+  float* dw = dvn + 2 * ld;
+  float* dd = dw + 2 * ld;
+  double* d64 = reinterpret_cast<double*>(dd + 2 * ld);
+  float* dxf = reinterpret_cast<float*>(d64 + ld);
+  double* darn = reinterpret_cast<double*>(mem + vec * (nv + 5));
+  GmState* gs = reinterpret_cast<GmState*>(reinterpret_cast<char*>(darn) + arn);
+  unsigned long long* flags = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(gs) + state);
+  if (e == cudaSuccess) e = cudaMemsetAsync(mem, 0, bytes, s);
+  auto up = [&](const double* src, float* dst) {
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d64, src, sizeof(double) * n, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return;
+    k_to_ff<<<gridr(n), 256, 0, s>>>(n, d64, dst);
+    e = cudaGetLastError();
+  };
+  for (int i = 0; i < nv; i++) up(V + (size_t)i * n, dV + 2 * (size_t)i * ld);
+  up(w, dw);
+  if (d) up(d, dd);
+  std::vector<GmState> S(1);
+  std::fill_n(S[0].cs, kMaxV, 1.0);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(gs, S.data(), sizeof(GmState), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess)
+    e = launch_arnoldi(s, n, dV, dw, nv, dvn, darn, gs, nv - 1, dxf, d ? dd : nullptr, flags, tile, ctas);
+  if (e == cudaSuccess) {
+    launch_pdl(k_from_ff, dim3(gridr(n)), dim3(256), 0, s, n, dvn, d64);
+    e = cudaGetLastError();
+  }
+  unsigned long long timeouts = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(vnext, d64, sizeof(double) * n, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(xf, dxf, sizeof(float) * n, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(S.data(), gs, sizeof(GmState), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&timeouts, flags + 2, sizeof(timeouts), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaFree(mem);
+  if (s) cudaStreamDestroy(s);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return AMPS_GPU_CUDA_ERROR;
+  }
+  const int jj = nv - 1;
+  for (int i = 0; i < jj; i++) h[i] = S[0].H[i * kMaxV + jj];
+  h[jj] = S[0].H[jj * kMaxV + jj] * S[0].cs[jj];
+  *norm = S[0].H[jj * kMaxV + jj] * S[0].sn[jj];
+  return timeouts ? AMPS_GPU_DEVICE_TIMEOUT : AMPS_GPU_OK;
 }

@@ -527,6 +527,19 @@ amps_gpu_status amps_gpu_set_arrivals_chunk(amps_gpu_ctx* ctx, int chunk);
 amps_gpu_status amps_gpu_get_particle_tuning(amps_gpu_ctx* ctx, int* arrivals_chunk, int* pending,
                                              double* ms);
 
+/* ---- the solver's Arnoldi step by itself, on host vectors ----
+ * One step of the field solve's GMRES (two classical Gram-Schmidt projections,
+ * normalisation) of w[n] against the basis V[nv][n], n >= 256, 1 <= nv <= 31, in the pair
+ * arithmetic of the solve (48 significant bits; V and w are rounded to it):
+ * h[nv], the sum of both projections' coefficients, *norm = ||w''||, vnext[n] =
+ * w'' / *norm (zeros when *norm is 0) and xf[n] = fp32(D vnext), D = d or 1 when
+ * d is null.  tile: elements per tile of the kernel (128, 256, 512 or 1024; 0: as
+ * a solve of this size takes it; a length whose tiles of nv vectors do not fit on
+ * chip is AMPS_GPU_INVALID_ARG), ctas: CTAs at most (0: as a solve takes it). */
+amps_gpu_status amps_gpu_arnoldi_step(int device, long long n, int nv, const double* V,
+                                      const double* w, const double* d, int tile, int ctas,
+                                      double* h, double* norm, double* vnext, float* xf);
+
 /* ---- per-kernel device timing on the context stream (CUDA events) ---- */
 amps_gpu_status amps_gpu_set_kernel_timing(amps_gpu_ctx* ctx, int enable);
 /* Fills up to cap entries; names are static strings.  Returns the count in *n. */

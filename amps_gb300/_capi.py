@@ -172,6 +172,7 @@ SIGNATURES = {
     "amps_ic_count": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]),
     "amps_ic_maxwellian": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, D,
                                      C.c_ulonglong, C.c_int, F, F, U8, I32]),
+    "amps_gpu_set_wait_limit": (C.c_int, [P, C.c_uint]),
     "amps_gpu_arnoldi_step": (C.c_int, [C.c_int, C.c_longlong, C.c_int, D, D, D, C.c_int, C.c_int,
                                         D, D, D, F]),
     "amps_gpu_trace_dipole": (C.c_int, [C.c_int, C.c_longlong, D, D, I32, I64, C.c_double,

@@ -1036,7 +1036,7 @@ static amps_gpu_status field_solve(amps_gpu_ctx* c, double tol, int maxit, int p
   amps_gpu_status s;
   amps_gpu_solve_stats st{};
   // the tensor-core preconditioner and the AMR operator's staged copies
-  // report bounded-wait timeouts in the flags
+  // report bounded-wait timeouts in the flags (the Arnoldi step in its state)
   const bool watch = precond == 2 || c->amr;
   if (watch && (s = reset_flags(c))) return s;
   if ((s = cuda_check(c, launch_rhs(c, precond != 0), "rhs"))) return s;
@@ -1061,6 +1061,15 @@ static amps_gpu_status field_solve(amps_gpu_ctx* c, double tol, int maxit, int p
   if (gs == AMPS_GPU_GMRES_NOT_CONVERGED)
     return set_err(c, gs, "GMRES did not converge: iterations " + std::to_string(st.iterations) +
                               ", relative residual " + std::to_string(st.rel_residual));
+  return AMPS_GPU_OK;
+}
+
+amps_gpu_status amps_gpu_set_wait_limit(amps_gpu_ctx* c, unsigned polls) {
+  if (!c) return AMPS_GPU_INVALID_ARG;
+  c->wait_limit = polls;
+  // the captured cycles hold the old limit
+  for (auto& g : c->solve_graphs) cudaGraphExecDestroy(g.exec);
+  c->solve_graphs.clear();
   return AMPS_GPU_OK;
 }
 

@@ -51,6 +51,8 @@ struct AmrDev {
 
 struct PrecondState;
 
+constexpr uint32_t kWaitLimit = 1u << 24;  // polls of a bounded wait (ptx.cuh)
+
 struct amps_gpu_ctx {
   amps_gpu_config cfg;
   int nb = 0;               // blocks
@@ -196,6 +198,7 @@ struct amps_gpu_ctx {
   float* d_xs = nullptr;        // FP32 pair split (hi, lo) of an operator input, 2 x 3*nvc
   double* h_red = nullptr;      // pinned
   int restart = 30;
+  uint32_t wait_limit = kWaitLimit;  // polls of a wait of the Arnoldi step
   int gm_guess[3] = {0, 0, 0};  // per preconditioner: Arnoldi steps of the last first cycle
                                 // (steps queued before the host first waits)
 

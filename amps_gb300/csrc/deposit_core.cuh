@@ -12,7 +12,6 @@
 #include "ptx.cuh"
 
 namespace {
-constexpr uint32_t kWaitLimit = 1u << 24;
 // Staged deposition fields, a structure of arrays per warp: field f of the
 // record at position p is rec[f * FS + p].  A chunk stages one record per
 // lane (position = lane); particles that do not deposit stage zero weight.

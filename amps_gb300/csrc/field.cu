@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <vector>
 
 #include "common.cuh"
@@ -40,7 +41,6 @@ constexpr int kMaxV = 32;
 constexpr int kRedBlocks = 304;  // 2 x 152 SMs
 constexpr int kGmOffset = 10240;  // doubles into d_red (12288 doubles)
 constexpr int kArnMaxGrid = 1024;  // CTAs of the cooperative Arnoldi step (at most)
-constexpr uint32_t kWaitLimit = 1u << 24;
 
 struct Taps {
   double K[3][3][27];  // operator taps without the mass matrix
@@ -362,8 +362,16 @@ struct GmState {
   int jj;    // columns processed in this cycle
   int done;  // |g[jj]| <= target, or breakdown
   double bn2, rn2;  // ||b||^2 (k_first), end-of-cycle ||r||^2 (k_residual)
+  unsigned long long timeouts;  // bounded waits that ran out in the solve's Arnoldi steps
   unsigned ticket;  // CTAs of a reducing kernel that have stored their share (0 between kernels)
 };
+// what the host reads at a time: jj, done, bn2, rn2, timeouts
+struct GmStatus {
+  int jj, done;
+  double bn2, rn2;
+  unsigned long long timeouts;
+};
+static_assert(offsetof(GmState, timeouts) - offsetof(GmState, jj) == offsetof(GmStatus, timeouts), "GmStatus layout");
 static_assert(kGmOffset * sizeof(double) + sizeof(GmState) <= 12288 * sizeof(double),
               "GmState must fit in d_red");
 static_assert(kRedBlocks * kMaxV + 2 * kMaxV + 8 + kMaxV <= kGmOffset, "d_red layout");
@@ -431,6 +439,7 @@ __global__ void __launch_bounds__(256) k_first(long long n, const double* __rest
     S->done = 0;
     S->bn2 = b2;
     S->rn2 = -1.0;
+    S->timeouts = 0ull;
   }
 }
 
@@ -564,7 +573,12 @@ __device__ __forceinline__ FF ff_warp_sum(FF a) {
 // last bit.  Any larger h2 (|w'| far below |w|, or a basis that lost its
 // orthogonality) takes the third sweep in full pairs and the norm from its sum, one
 // more grid barrier.
-// A CTA whose tiles all fit its stages reads them once.  1.34M unknowns, mean
+// A CTA whose tiles all fit its stages reads them once.
+// Waits give up after `limit` polls (counted in the state): a producer whose stage
+// is not freed issues nothing more, a consumer warp whose tile does not come goes on
+// without waiting or freeing, so that a stage is never filled over a copy still in
+// flight; all take part in every barrier, and the producer leaves when its last
+// copies have landed.  1.34M unknowns, mean
 // step of a 55-iteration solve (1 to 30 vectors): 103 us, 4 us per vector (the
 // rate of HBM) on ~45 us of barriers and start-up.  Before: 304 us with
 // per-thread streams, four basis reads and three barriers; 150 us with one CTA
@@ -603,7 +617,7 @@ template <int T>
 __global__ void __launch_bounds__(kArnBlock, 2) k_arnoldi_tile(
     const __grid_constant__ ArnMaps maps, long long n, long long ld, float* __restrict__ w, int nv,
     float* __restrict__ vnext, float2* __restrict__ part, GmState* gs, int jj, float* __restrict__ xf,
-    const float* __restrict__ dh, int stages, unsigned long long* flags) {
+    const float* __restrict__ dh, int stages, uint32_t limit) {
   cg::grid_group grid = cg::this_grid();
   extern __shared__ __align__(128) float s_ring[];
   __shared__ __align__(8) uint64_t full[kArnMaxStages], empty[kArnMaxStages];
@@ -642,10 +656,17 @@ __global__ void __launch_bounds__(kArnBlock, 2) k_arnoldi_tile(
   if (wid == kArnWarps) {
     // ---- producer warp: tile k of the sweep as the ring's use number c; pairs of
     // V, or its hi halves (and D)
+    int issued = 0;
+    bool stop = false;
     auto issue = [&](int c, int k, bool pairs, const float* D) {
+      if (stop) return;
       const int s = c % stages;
-      if (c >= stages && !mbar_wait_bounded(&empty[s], ((c / stages) - 1) & 1, kWaitLimit) && lane == 0)
-        atomicAdd(flags + 2, 1ull);
+      if (c >= stages && !__all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], ((c / stages) - 1) & 1, limit))) {
+        if (lane == 0) atomicAdd(&gs->timeouts, 1ull);
+        stop = true;
+        return;
+      }
+      issued = c + 1;
       if (lane == 0) {
         const long long e0 = tile_of(k) * T;
         const int count = count_of(k);
@@ -678,18 +699,24 @@ __global__ void __launch_bounds__(kArnBlock, 2) k_arnoldi_tile(
       bar_all();  // s_n2
     }
     if (blockIdx.x == 0 && lane == 0) gm_update(gs, jj, s_h1, s_h2, s_n2);
+    for (int c = max(0, issued - stages); c < issued; c++)
+      mbar_wait_bounded(&full[c % stages], (c / stages) & 1, kWaitLimit);
     return;
   }
 
   // ---- consumers
+  bool bad = false;  // this warp gave up on a tile
   auto acquire = [&](int c) -> float* {
     const int s = c % stages;
-    if (!mbar_wait_bounded(&full[s], (c / stages) & 1, kWaitLimit) && lane == 0) atomicAdd(flags + 2, 1ull);
+    if (!bad && !__all_sync(0xffffffffu, mbar_wait_bounded(&full[s], (c / stages) & 1, limit))) {
+      if (lane == 0) atomicAdd(&gs->timeouts, 1ull);
+      bad = true;
+    }
     return s_ring + (size_t)s * stage_f;
   };
   auto release = [&](int c) {
     __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[c % stages]);
+    if (lane == 0 && !bad) mbar_arrive(&empty[c % stages]);
   };
   // dots of the staged w with nd vectors (number nv: w itself): warp -> vector
   // and, with fewer vectors than warps, element range
@@ -956,7 +983,7 @@ bool arn_map(CUtensorMap* m, const float* base, long long cols, long long pitch,
 template <int T>
 cudaError_t launch_arnoldi_t(cudaStream_t s, int ctas, long long n, const float* V, float* w, int nv,
                              float* vnext, double* d_arn, GmState* gs, int jj, float* xf, const float* dh,
-                             unsigned long long* flags) {
+                             uint32_t limit) {
   static unsigned long long ready = 0;             // per device
   int dev = 0;
   cudaGetDevice(&dev);
@@ -982,7 +1009,7 @@ cudaError_t launch_arnoldi_t(cudaStream_t s, int ctas, long long n, const float*
   if (!arn_map(&maps.v, V, ld, ld, 2 * nv, width) || !arn_map(&maps.h, V, ld, 2 * ld, nv, width) ||
       !arn_map(&maps.w, w, ld, ld, 2, width))
     return cudaErrorInvalidValue;
-  void* args[] = {&maps, &n, &ld, &w, &nv, &vnext, &part, &gs, &jj, &xf, &dh, &stages, &flags};
+  void* args[] = {&maps, &n, &ld, &w, &nv, &vnext, &part, &gs, &jj, &xf, &dh, &stages, &limit};
   return cudaLaunchCooperativeKernel((const void*)k_arnoldi_tile<T>, dim3(g), dim3(kArnBlock), args,
                                      stage * stages + arn_extra(T), s);
 }
@@ -998,7 +1025,7 @@ bool arn_fits(int T, int nv) {
 }
 cudaError_t launch_arnoldi(cudaStream_t s, long long n, const float* V, float* w, int nv, float* vnext,
                            double* d_arn, GmState* gs, int jj, float* xf, const float* dh,
-                           unsigned long long* flags, int tile = 0, int ctas = 0) {
+                           uint32_t limit, int tile = 0, int ctas = 0) {
   static int sms[64] = {0};  // per device
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1014,10 +1041,10 @@ cudaError_t launch_arnoldi(cudaStream_t s, long long n, const float* V, float* w
     return tile ? tile == T : T == 128 || (arn_fits(T, nv) && n >= 8LL * sms[dev] * T);
   };
   const int g = ctas > 0 ? std::min(ctas, 2 * sms[dev]) : 2 * sms[dev];
-  if (takes(1024)) return launch_arnoldi_t<1024>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
-  if (takes(512)) return launch_arnoldi_t<512>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
-  if (takes(256)) return launch_arnoldi_t<256>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
-  return launch_arnoldi_t<128>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, flags);
+  if (takes(1024)) return launch_arnoldi_t<1024>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, limit);
+  if (takes(512)) return launch_arnoldi_t<512>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, limit);
+  if (takes(256)) return launch_arnoldi_t<256>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, limit);
+  return launch_arnoldi_t<128>(s, g, n, V, w, nv, vnext, d_arn, gs, jj, xf, dh, limit);
 }
 
 // V0 = r / ||r|| as a pair vector (nrm2: ||r||^2)
@@ -1497,7 +1524,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
       }
     }
     TimedLaunch t(c, "gmres_orth");
-    return launch_arnoldi(s, n, Vf, wf, nv, vf(nv), c->d_arn, gs, jj, xf_next, dh, c->d_flags);
+    return launch_arnoldi(s, n, Vf, wf, nv, vf(nv), c->d_arn, gs, jj, xf_next, dh, c->wait_limit);
   };
   // end of a cycle of at most nv_max steps: least squares, x += (D) V y (with its pairs
   // in d_xs and E^{n+theta} = E^n + x), the true FP64 residual into w and its squared
@@ -1516,6 +1543,12 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     return cudaGetLastError();
   };
 
+  const GmStatus& stat = *reinterpret_cast<const GmStatus*>(c->h_red);  // after its copy
+  // every read of the step count carries the steps' timeouts
+  auto gave_up = [&]() {
+    return set_err(c, AMPS_GPU_DEVICE_TIMEOUT,
+                   "field solve: " + std::to_string(stat.timeouts) + " bounded waits of the Arnoldi step ran out");
+  };
   int it = 0, cycles = 0;
   bool conv = false;
   double rel = 0.0, bnorm = 0.0, beta = 0.0;
@@ -1546,8 +1579,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
         }
         if (e1 == cudaSuccess) e1 = cycle_end(K);
         if (e1 == cudaSuccess)
-          e1 = cudaMemcpyAsync(c->h_red, &gs->jj, 2 * sizeof(int) + 2 * sizeof(double),
-                               cudaMemcpyDeviceToHost, s);
+          e1 = cudaMemcpyAsync(c->h_red, &gs->jj, sizeof(GmStatus), cudaMemcpyDeviceToHost, s);
         ee = cudaStreamEndCapture(s, &gr_cap);
         if (ee == cudaSuccess && e1 == cudaSuccess)
           ee = cudaGraphInstantiate(&exec, gr_cap, 0);
@@ -1571,11 +1603,11 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     if (exec) {
       CK(cudaGraphLaunch(exec, s));
       CK(cudaStreamSynchronize(s));
-      const int* stat = reinterpret_cast<const int*>(c->h_red);
-      it = stat[0];
+      it = stat.jj;
       cycles = 1;
-      bnorm = std::sqrt(c->h_red[1]);
-      beta = std::sqrt(std::max(0.0, c->h_red[2]));
+      bnorm = std::sqrt(stat.bn2);
+      beta = std::sqrt(std::max(0.0, stat.rn2));
+      if (stat.timeouts) return gave_up();
       graph_done = true;
     }
   }
@@ -1607,11 +1639,11 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
       CK(arnoldi_step(launched++));
       CK(cudaGetLastError());
       if (launched >= first_read || launched == m || it + launched >= maxit) {
-        CK(cudaMemcpyAsync(c->h_red, &gs->jj, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(c->h_red, &gs->jj, sizeof(GmStatus), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        const int* stat = reinterpret_cast<const int*>(c->h_red);
-        used = stat[0];
-        done = stat[1] != 0;
+        if (stat.timeouts) return gave_up();
+        used = stat.jj;
+        done = stat.done != 0;
       }
     }
     it += used;
@@ -1733,7 +1765,7 @@ extern "C" amps_gpu_status amps_gpu_arnoldi_step(int device, long long n, int nv
   char* mem = nullptr;
   // the basis and V_nv, w, D as a pair vector, one FP64 vector, xf, then the step's scratch
   const size_t arn = sizeof(double) * 3 * kArnMaxGrid * kMaxV, state = (sizeof(GmState) + 63) & ~(size_t)63;
-  const size_t bytes = vec * (nv + 5) + arn + state + 64;
+  const size_t bytes = vec * (nv + 5) + arn + state;
   cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&mem), bytes);
   float* dV = reinterpret_cast<float*>(mem);
@@ -1744,7 +1776,6 @@ extern "C" amps_gpu_status amps_gpu_arnoldi_step(int device, long long n, int nv
   float* dxf = reinterpret_cast<float*>(d64 + ld);
   double* darn = reinterpret_cast<double*>(mem + vec * (nv + 5));
   GmState* gs = reinterpret_cast<GmState*>(reinterpret_cast<char*>(darn) + arn);
-  unsigned long long* flags = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(gs) + state);
   if (e == cudaSuccess) e = cudaMemsetAsync(mem, 0, bytes, s);
   auto up = [&](const double* src, float* dst) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(d64, src, sizeof(double) * n, cudaMemcpyHostToDevice, s);
@@ -1759,16 +1790,14 @@ extern "C" amps_gpu_status amps_gpu_arnoldi_step(int device, long long n, int nv
   std::fill_n(S[0].cs, kMaxV, 1.0);
   if (e == cudaSuccess) e = cudaMemcpyAsync(gs, S.data(), sizeof(GmState), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess)
-    e = launch_arnoldi(s, n, dV, dw, nv, dvn, darn, gs, nv - 1, dxf, d ? dd : nullptr, flags, tile, ctas);
+    e = launch_arnoldi(s, n, dV, dw, nv, dvn, darn, gs, nv - 1, dxf, d ? dd : nullptr, kWaitLimit, tile, ctas);
   if (e == cudaSuccess) {
     launch_pdl(k_from_ff, dim3(gridr(n)), dim3(256), 0, s, n, dvn, d64);
     e = cudaGetLastError();
   }
-  unsigned long long timeouts = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(vnext, d64, sizeof(double) * n, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(xf, dxf, sizeof(float) * n, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(S.data(), gs, sizeof(GmState), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&timeouts, flags + 2, sizeof(timeouts), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   cudaFree(mem);
   if (s) cudaStreamDestroy(s);
@@ -1780,5 +1809,5 @@ extern "C" amps_gpu_status amps_gpu_arnoldi_step(int device, long long n, int nv
   for (int i = 0; i < jj; i++) h[i] = S[0].H[i * kMaxV + jj];
   h[jj] = S[0].H[jj * kMaxV + jj] * S[0].cs[jj];
   *norm = S[0].H[jj * kMaxV + jj] * S[0].sn[jj];
-  return timeouts ? AMPS_GPU_DEVICE_TIMEOUT : AMPS_GPU_OK;
+  return S[0].timeouts ? AMPS_GPU_DEVICE_TIMEOUT : AMPS_GPU_OK;
 }

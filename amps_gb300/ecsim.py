@@ -501,6 +501,10 @@ class EcsimContext:
         """GMRES inner operator in FP64 (True) or FP32 with FP64 refinement (False)."""
         self._check(self.lib.amps_gpu_set_inner_fp64(self.h, 1 if on else 0), "set_inner_fp64")
 
+    def set_wait_limit(self, polls):
+        """Polls of a wait of the solve's Arnoldi step before it gives up (default 2^24)."""
+        self._check(self.lib.amps_gpu_set_wait_limit(self.h, polls), "set_wait_limit")
+
     def precond_num_sets(self):
         """Weight sets of the network: 1 on a uniform mesh, one per level on AMR."""
         n = C.c_int()

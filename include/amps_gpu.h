@@ -416,6 +416,10 @@ amps_gpu_status amps_gpu_push_deposit(amps_gpu_ctx* ctx, double* particle_energy
  * each restart (default), 1 FP64 throughout.  No reference counterpart (the
  * reference's solve is FP64). */
 amps_gpu_status amps_gpu_set_inner_fp64(amps_gpu_ctx* ctx, int fp64);
+/* Polls that a wait of the field solve's Arnoldi step makes for a tile before it
+ * gives up (default 2^24; 0: at once); a solve in which one gave up returns
+ * AMPS_GPU_DEVICE_TIMEOUT and keeps E^n and B. */
+amps_gpu_status amps_gpu_set_wait_limit(amps_gpu_ctx* ctx, unsigned polls);
 
 /* ---- learned right preconditioner for the field solve (no reference
  *      counterpart: the reference's GMRES takes PrecondParam 0/1 only) ----

@@ -194,6 +194,7 @@ struct amps_gpu_ctx {
   int arr_tune_n[2] = {0, 0};
   cudaEvent_t arr_ev[2] = {nullptr, nullptr};
   double* d_red = nullptr;      // partial reductions
+  double red_tol = 0.0;         // tolerance of the solve in d_red (field.cu)
   double* d_arn = nullptr;      // per-CTA partial sums of the cooperative Arnoldi step
   float* d_xs = nullptr;        // FP32 pair split (hi, lo) of an operator input, 2 x 3*nvc
   double* h_red = nullptr;      // pinned

@@ -40,6 +40,7 @@ constexpr double kPi = 3.14159265358979323846264338327950288;
 constexpr int kMaxV = 32;
 constexpr int kRedBlocks = 304;  // 2 x 152 SMs
 constexpr int kGmOffset = 10240;  // doubles into d_red (12288 doubles)
+constexpr int kTolOffset = 12287;  // the solve's tolerance, read by k_first
 constexpr int kArnMaxGrid = 1024;  // CTAs of the cooperative Arnoldi step (at most)
 
 struct Taps {
@@ -372,7 +373,7 @@ struct GmStatus {
   unsigned long long timeouts;
 };
 static_assert(offsetof(GmState, timeouts) - offsetof(GmState, jj) == offsetof(GmStatus, timeouts), "GmStatus layout");
-static_assert(kGmOffset * sizeof(double) + sizeof(GmState) <= 12288 * sizeof(double),
+static_assert(kGmOffset * sizeof(double) + sizeof(GmState) <= kTolOffset * sizeof(double),
               "GmState must fit in d_red");
 static_assert(kRedBlocks * kMaxV + 2 * kMaxV + 8 + kMaxV <= kGmOffset, "d_red layout");
 
@@ -414,11 +415,13 @@ __device__ __forceinline__ bool grid_sum(double acc, double* __restrict__ partia
 }
 
 // Start of a solve from x0 = 0: r = b (in w), x = 0, ||b||^2, and the state of a first
-// cycle with the target tol ||b||.  (One launch: the copy, the clearing, the norm, its
+// cycle with the target *tol ||b|| (in memory: a captured launch serves any tolerance).
+// (One launch: the copy, the clearing, the norm, its
 // reduction and the state took five, ~4 us each on a small mesh.)
 __global__ void __launch_bounds__(256) k_first(long long n, const double* __restrict__ b, double* __restrict__ w,
                                                double* __restrict__ x, double* __restrict__ partial,
-                                               double* __restrict__ n2, GmState* __restrict__ S, double tol) {
+                                               double* __restrict__ n2, GmState* __restrict__ S,
+                                               const double* __restrict__ tol) {
   pdl_wait();
   pdl_next();
   double acc = 0.0;
@@ -434,7 +437,7 @@ __global__ void __launch_bounds__(256) k_first(long long n, const double* __rest
   if (threadIdx.x <= kMaxV) S->g[threadIdx.x] = threadIdx.x == 0 ? sqrt(b2) : 0.0;
   if (threadIdx.x == 0) {
     *n2 = b2;
-    S->target = tol * sqrt(b2);
+    S->target = *tol * sqrt(b2);
     S->jj = 0;
     S->done = 0;
     S->bn2 = b2;
@@ -1500,7 +1503,7 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
       cudaError_t ee = launch_jacobi_diag(c);
       if (ee != cudaSuccess) return ee;
     }
-    launch_pdl(k_first, dim3(gr), dim3(256), 0, s, n, c->d_rhs, w, c->d_x, partial, d_n2, gs, tol);
+    launch_pdl(k_first, dim3(gr), dim3(256), 0, s, n, c->d_rhs, w, c->d_x, partial, d_n2, gs, c->d_red + kTolOffset);
     return cudaGetLastError();
   };
   // Arnoldi step jj: the operator (after the network for flexible directions),
@@ -1549,6 +1552,10 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
     return set_err(c, AMPS_GPU_DEVICE_TIMEOUT,
                    "field solve: " + std::to_string(stat.timeouts) + " bounded waits of the Arnoldi step ran out");
   };
+  if (c->red_tol != tol) {  // zero at creation, when no solve's tolerance is
+    CK(cudaMemcpyAsync(c->d_red + kTolOffset, &tol, sizeof(double), cudaMemcpyHostToDevice, s));
+    c->red_tol = tol;
+  }
   int it = 0, cycles = 0;
   bool conv = false;
   double rel = 0.0, bnorm = 0.0, beta = 0.0;

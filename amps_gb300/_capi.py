@@ -172,6 +172,7 @@ SIGNATURES = {
     "amps_ic_count": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]),
     "amps_ic_maxwellian": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, D,
                                      C.c_ulonglong, C.c_int, F, F, U8, I32]),
+    "amps_gpu_set_tuning": (C.c_int, [P, C.c_int, C.c_int]),
     "amps_gpu_set_wait_limit": (C.c_int, [P, C.c_uint]),
     "amps_gpu_arnoldi_step": (C.c_int, [C.c_int, C.c_longlong, C.c_int, D, D, D, C.c_int, C.c_int,
                                         D, D, D, F]),

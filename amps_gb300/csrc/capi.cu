@@ -1230,6 +1230,15 @@ amps_gpu_status amps_gpu_get_tuning(amps_gpu_ctx* c, int* threads_per_cta, int* 
   return AMPS_GPU_OK;
 }
 
+amps_gpu_status amps_gpu_set_tuning(amps_gpu_ctx* c, int threads_per_cta, int reduction_ctas) {
+  if (!c || (threads_per_cta != 64 && threads_per_cta != 128 && threads_per_cta != 256) || reduction_ctas < 1 ||
+      reduction_ctas > 304)
+    return set_err(c, AMPS_GPU_INVALID_ARG, "set_tuning: 64, 128 or 256 threads, 1 to 304 CTAs");
+  c->tune_tb = threads_per_cta;
+  c->tune_red = reduction_ctas;
+  return AMPS_GPU_OK;
+}
+
 amps_gpu_status amps_gpu_set_kernel_timing(amps_gpu_ctx* c, int enable) {
   if (!c) return AMPS_GPU_INVALID_ARG;
   flush_timers(c);

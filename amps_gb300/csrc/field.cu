@@ -153,16 +153,17 @@ TapsF taps_f32(const Taps& T) {
 
 // ---- the 27-point operator ---------------------------------------------------
 // A CTA takes 32 consecutive corners (ncor is a multiple of 512) and splits the
-// 27 slots over its W = blockDim / 32 warps (slot s: warp s mod W); lane = corner,
-// so the 243 coefficient planes of M are read in whole lines, and a slot's
-// neighbour values serve the three components.  The warps' partial sums meet in
-// shared memory and are added in warp order.  Bound: latency on small meshes --
+// 27 slots into 8 groups (slot s: group s mod 8) over its 2, 4 or 8 warps; lane =
+// corner, so the 243 coefficient planes of M are read in whole lines, and a slot's
+// neighbour values serve the three components.  The groups' sums meet in shared
+// memory and are added in their order, so that a row has the same bits at any CTA
+// size (the autotuner chooses it by time).  Bound: latency on small meshes --
 // one thread per (component, corner) walked all 27 slots, nine rounds of
 // dependent loads -- and reading M (HBM) on large ones.  us per application,
 // before and now, at 512 and at 32,768 corners: FP32 operator 15.6 -> 8.5, 18.5 ->
 // 15.9; residual operator with its input split 23.2 -> 16.1, 30.5 -> 27.2; RHS
 // likewise 27 -> 16.8, 42 -> 37.
-constexpr int kOpMaxWarps = 8;
+constexpr int kOpGroups = 8;  // of slots; a CTA has at most a warp per group
 
 __device__ __forceinline__ void slot_offset(int s, int& di, int& dj, int& dk) {
   const int d0 = s % 3, d1 = (s / 3) % 3, d2 = s / 9;
@@ -171,20 +172,19 @@ __device__ __forceinline__ void slot_offset(int s, int& di, int& dj, int& dk) {
   dk = d2 == 0 ? 0 : (d2 == 1 ? -1 : 1);
 }
 
-// This warp's slots of (K + f M) x at corner c, all three rows, to FP64 accuracy:
+// The slots of a group of (K + f M) x at corner c, all three rows, to FP64 accuracy:
 // sk the taps, sm the mass matrix's FP32 coefficients, against the split input.
 struct RowFF {
   FF sk[3], sm[3];
 };
 __device__ __forceinline__ RowFF rows_ff(long long ncor, const int* __restrict__ nbr, const float* __restrict__ M,
                                          const float* __restrict__ xh, const float* __restrict__ xl,
-                                         const TapsFF& T, long long c, int b, int i, int j, int k, int wid,
-                                         int warps) {
+                                         const TapsFF& T, long long c, int b, int i, int j, int k, int group) {
   RowFF r;
 #pragma unroll
   for (int p = 0; p < 3; p++) r.sk[p] = r.sm[p] = FF{0.f, 0.f};
 #pragma unroll 2
-  for (int s = wid; s < 27; s += warps) {
+  for (int s = group; s < 27; s += kOpGroups) {
     int di, dj, dk;
     slot_offset(s, di, dj, dk);
     const int nb = local_id(nbr, b, i + di, j + dj, k + dk);
@@ -203,26 +203,33 @@ __device__ __forceinline__ RowFF rows_ff(long long ncor, const int* __restrict__
   }
   return r;
 }
-// The warps' rows into s_row[6][warps][32], and component p of the sum at lane
-// (after the barrier)
-__device__ __forceinline__ void rows_store(const RowFF& r, float2 (*s_row)[kOpMaxWarps][32], int wid, int lane) {
+// The groups' rows into s_row[6][kOpGroups][32], a warp's after one another, and
+// component p of the sum at lane (after the barrier)
+__device__ __forceinline__ void rows_store(long long ncor, const int* __restrict__ nbr, const float* __restrict__ M,
+                                           const float* __restrict__ xh, const float* __restrict__ xl,
+                                           const TapsFF& T, long long c, int b, int i, int j, int k,
+                                           float2 (*s_row)[kOpGroups][32], int wid, int warps, int lane) {
+  for (int g = wid; g < kOpGroups; g += warps) {
+    const RowFF r = rows_ff(ncor, nbr, M, xh, xl, T, c, b, i, j, k, g);
 #pragma unroll
-  for (int p = 0; p < 3; p++) {
-    s_row[p][wid][lane] = make_float2(r.sk[p].s, r.sk[p].q);
-    s_row[3 + p][wid][lane] = make_float2(r.sm[p].s, r.sm[p].q);
+    for (int p = 0; p < 3; p++) {
+      s_row[p][g][lane] = make_float2(r.sk[p].s, r.sk[p].q);
+      s_row[3 + p][g][lane] = make_float2(r.sm[p].s, r.sm[p].q);
+    }
   }
 }
-__device__ __forceinline__ double rows_sum(float2 (*s_row)[kOpMaxWarps][32], int warps, int p, int lane, double f) {
+__device__ __forceinline__ double rows_sum(float2 (*s_row)[kOpGroups][32], int p, int lane, double f) {
   FF a{0.f, 0.f}, m{0.f, 0.f};
-  for (int w = 0; w < warps; w++) {
-    ff_acc(a, s_row[p][w][lane].x, s_row[p][w][lane].y);
-    ff_acc(m, s_row[3 + p][w][lane].x, s_row[3 + p][w][lane].y);
+#pragma unroll
+  for (int g = 0; g < kOpGroups; g++) {
+    ff_acc(a, s_row[p][g][lane].x, s_row[p][g][lane].y);
+    ff_acc(m, s_row[3 + p][g][lane].x, s_row[3 + p][g][lane].y);
   }
   return ff_value(a) + f * ff_value(m);
 }
 
 // y = A (dinv .* x) to FP64 accuracy from the split input (outer residuals)
-__global__ void __launch_bounds__(32 * kOpMaxWarps) k_matvec(long long ncor, const int* __restrict__ nbr,
+__global__ void __launch_bounds__(32 * kOpGroups) k_matvec(long long ncor, const int* __restrict__ nbr,
                                                              const float* __restrict__ M,
                                                              const float* __restrict__ xh,
                                                              const float* __restrict__ xl,
@@ -230,19 +237,19 @@ __global__ void __launch_bounds__(32 * kOpMaxWarps) k_matvec(long long ncor, con
                                                              const __grid_constant__ TapsFF T) {
   pdl_wait();
   pdl_next();
-  __shared__ float2 s_row[6][kOpMaxWarps][32];
+  __shared__ float2 s_row[6][kOpGroups][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const long long c = (long long)blockIdx.x * 32 + lane;
   int b, i, j, k;
   corner_ijk(c, b, i, j, k);
-  rows_store(rows_ff(ncor, nbr, M, xh, xl, T, c, b, i, j, k, wid, warps), s_row, wid, lane);
+  rows_store(ncor, nbr, M, xh, xl, T, c, b, i, j, k, s_row, wid, warps, lane);
   __syncthreads();
-  for (int p = wid; p < 3; p += warps) y[p * ncor + c] = rows_sum(s_row, warps, p, lane, T.f);
+  for (int p = wid; p < 3; p += warps) y[p * ncor + c] = rows_sum(s_row, p, lane, T.f);
 }
 
 // RHS: theta c dt curl B^n - f J - (curl-curl + f M) E^n, the last term to
 // FP64 accuracy from the split E^n (taps without the identity)
-__global__ void __launch_bounds__(32 * kOpMaxWarps) k_rhs(long long ncor, const int* __restrict__ nbr,
+__global__ void __launch_bounds__(32 * kOpGroups) k_rhs(long long ncor, const int* __restrict__ nbr,
                                                           const float* __restrict__ M,
                                                           const float* __restrict__ Eh,
                                                           const float* __restrict__ El,
@@ -253,7 +260,7 @@ __global__ void __launch_bounds__(32 * kOpMaxWarps) k_rhs(long long ncor, const 
                                                           double c4y, double c4z) {
   pdl_wait();
   pdl_next();
-  __shared__ float2 s_row[6][kOpMaxWarps][32];
+  __shared__ float2 s_row[6][kOpGroups][32];
   __shared__ double s_cb[3][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const long long c = (long long)blockIdx.x * 32 + lane;
@@ -283,9 +290,9 @@ __global__ void __launch_bounds__(32 * kOpMaxWarps) k_rhs(long long ncor, const 
       }
     s_cb[p][lane] = cb - T.f * J[p * ncor + c];
   }
-  rows_store(rows_ff(ncor, nbr, M, Eh, El, T, c, b, i, j, k, wid, warps), s_row, wid, lane);
+  rows_store(ncor, nbr, M, Eh, El, T, c, b, i, j, k, s_row, wid, warps, lane);
   __syncthreads();
-  for (int p = wid; p < 3; p += warps) rhs[p * ncor + c] = s_cb[p][lane] - rows_sum(s_row, warps, p, lane, T.f);
+  for (int p = wid; p < 3; p += warps) rhs[p * ncor + c] = s_cb[p][lane] - rows_sum(s_row, p, lane, T.f);
 }
 
 __global__ void __launch_bounds__(256) k_jacobi(long long ncor, const float* __restrict__ M,
@@ -1162,40 +1169,43 @@ __global__ void __launch_bounds__(256) k_in_f32(long long n, OpIn in, float* __r
 // mass-matrix terms, a small fraction of A on ECSIM time steps) in FP32
 // arithmetic: the inner operator of the refined GMRES, which never decides
 // convergence.  xf = fp32(D v).
-__global__ void __launch_bounds__(32 * kOpMaxWarps) k_matvec32_ff(long long ncor, const int* __restrict__ nbr,
+__global__ void __launch_bounds__(32 * kOpGroups) k_matvec32_ff(long long ncor, const int* __restrict__ nbr,
                                                                   const float* __restrict__ M,
                                                                   const float* __restrict__ xf, OpIn in,
                                                                   float* __restrict__ wh, float* __restrict__ wl,
                                                                   const __grid_constant__ TapsF T) {
   pdl_wait();
   pdl_next();
-  __shared__ float s_row[3][kOpMaxWarps][32];
+  __shared__ float s_row[3][kOpGroups][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const long long c = (long long)blockIdx.x * 32 + lane;
   int b, i, j, k;
   corner_ijk(c, b, i, j, k);
-  float acc[3] = {0.f, 0.f, 0.f};
+  for (int g = wid; g < kOpGroups; g += warps) {
+    float acc[3] = {0.f, 0.f, 0.f};
 #pragma unroll 4
-  for (int s = wid; s < 27; s += warps) {
-    int di, dj, dk;
-    slot_offset(s, di, dj, dk);
-    const int nb = local_id(nbr, b, i + di, j + dj, k + dk);
-    float x[3], m[9];
+    for (int s = g; s < 27; s += kOpGroups) {
+      int di, dj, dk;
+      slot_offset(s, di, dj, dk);
+      const int nb = local_id(nbr, b, i + di, j + dj, k + dk);
+      float x[3], m[9];
 #pragma unroll
-    for (int q = 0; q < 3; q++) x[q] = xf[q * ncor + nb];
+      for (int q = 0; q < 3; q++) x[q] = xf[q * ncor + nb];
 #pragma unroll
-    for (int e = 0; e < 9; e++) m[e] = M[(size_t)(9 * s + e) * ncor + c];
+      for (int e = 0; e < 9; e++) m[e] = M[(size_t)(9 * s + e) * ncor + c];
 #pragma unroll
-    for (int p = 0; p < 3; p++)
+      for (int p = 0; p < 3; p++)
 #pragma unroll
-      for (int q = 0; q < 3; q++) acc[p] = fmaf(fmaf(T.f, m[3 * p + q], T.K[p][q][s]), x[q], acc[p]);
+        for (int q = 0; q < 3; q++) acc[p] = fmaf(fmaf(T.f, m[3 * p + q], T.K[p][q][s]), x[q], acc[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < 3; p++) s_row[p][g][lane] = acc[p];
   }
-#pragma unroll
-  for (int p = 0; p < 3; p++) s_row[p][wid][lane] = acc[p];
   __syncthreads();
   for (int p = wid; p < 3; p += warps) {
     float a = 0.f;
-    for (int w = 0; w < warps; w++) a += s_row[p][w][lane];
+#pragma unroll
+    for (int g = 0; g < kOpGroups; g++) a += s_row[p][g][lane];
     const long long t = p * ncor + c;
     FF y = opin_value(in, t);
     ff_acc(y, a, 0.f);

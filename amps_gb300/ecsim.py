@@ -621,6 +621,10 @@ class EcsimContext:
                 "sweep_ms_cta76_152_304": ms[3:].round(4).tolist(),
                 "threads_per_cta": tb.value, "reduction_ctas": red.value}
 
+    def set_tuning(self, threads_per_cta, reduction_ctas):
+        """The launch shapes autotune chooses, set by hand (a run that repeats another's bits)."""
+        self._check(self.lib.amps_gpu_set_tuning(self.h, threads_per_cta, reduction_ctas), "set_tuning")
+
     # ---- timing ----
     def set_kernel_timing(self, on=True):
         self._check(self.lib.amps_gpu_set_kernel_timing(self.h, 1 if on else 0), "timing")

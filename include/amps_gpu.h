@@ -517,10 +517,15 @@ amps_gpu_status amps_gpu_update_j_mass_matrix_noalloc(const amps_gpu_config* cfg
  * field buffers it reads; graphs are not used while kernel timing is on.
  * autotune: times 3 CTA sizes of the field operator kernels and 3 grid sizes of
  * the GMRES sweeps on this context's data and keeps the fastest; ms[6]
- * (optional) receives the candidates' times. get_tuning reads the choice. */
+ * (optional) receives the candidates' times. get_tuning reads the choice,
+ * set_tuning sets it (threads 64, 128 or 256; reduction CTAs 1 to 304).  On a
+ * uniform mesh the operator's rows have the same bits at any CTA size; the sums of
+ * the norms are of the reduction CTAs, so a solve repeats bit for bit at equal
+ * reduction CTAs. */
 amps_gpu_status amps_gpu_set_graphs(amps_gpu_ctx* ctx, int on);
 amps_gpu_status amps_gpu_autotune(amps_gpu_ctx* ctx, double* ms);
 amps_gpu_status amps_gpu_get_tuning(amps_gpu_ctx* ctx, int* threads_per_cta, int* reduction_ctas);
+amps_gpu_status amps_gpu_set_tuning(amps_gpu_ctx* ctx, int threads_per_cta, int reduction_ctas);
 /* The particle side of the autotuner: amps_gpu_autotune also arms a
  * comparison of the arrivals kernel staging 16 or 32 arrivals at a time over
  * the next 6 particle steps (3 each, stream launches timed by events; the

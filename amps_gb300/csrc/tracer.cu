@@ -17,6 +17,7 @@
 // ~1e-2 of |x|, so plain FP32 sums would lose ~1e-5 of every displacement.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -253,23 +254,28 @@ __global__ void k_set_queue(unsigned long long* queue, unsigned long long first)
 // The caller's interleaved SI arrays <-> normalised component arrays (FP64
 // divisions and products rounded as written, then to T): a host loop over them,
 // six pageable copies each way and nine allocations took longer than the tracing
-// (call of 262,144 FP32 particles x 2000 steps: 6.2 ms, now 4.4).
+// (call of 262,144 FP32 particles x 2000 steps: 6.2 ms, now 4.4).  The SI values
+// cross in chunks of kTraceChunk particles (s: the chunk's first in the states of n
+// particles), so they take 12.6 MB at any n beside the 36 (FP32) or 60 bytes of a
+// particle's state, status and step count; a chunk's 6 MB per array take ten times
+// its launch.
+constexpr long long kTraceChunk = 1 << 18;
 template <class T>
-__global__ void __launch_bounds__(256) k_trace_in(long long n, const double* __restrict__ x,
+__global__ void __launch_bounds__(256) k_trace_in(long long count, long long n, const double* __restrict__ x,
                                                   const double* __restrict__ p, double r_e, double pscale,
                                                   T* __restrict__ s) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * n) return;
+  if (t >= 3 * count) return;
   const long long i = t / 3, d = t - 3 * i;
   s[d * n + i] = (T)(x[t] / r_e);
   s[(3 + d) * n + i] = (T)__dmul_rn(p[t], pscale);
 }
 template <class T>
-__global__ void __launch_bounds__(256) k_trace_out(long long n, const T* __restrict__ s, double r_e,
-                                                   double pscale, double* __restrict__ x,
+__global__ void __launch_bounds__(256) k_trace_out(long long count, long long n, const T* __restrict__ s,
+                                                   double r_e, double pscale, double* __restrict__ x,
                                                    double* __restrict__ p) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * n) return;
+  if (t >= 3 * count) return;
   const long long i = t / 3, d = t - 3 * i;
   x[t] = __dmul_rn((double)s[d * n + i], r_e);
   p[t] = (double)s[(3 + d) * n + i] / pscale;
@@ -281,9 +287,9 @@ amps_gpu_status run_trace(long long n, double* x, double* p, int32_t* status, in
                           double r_in, double r_out, long long max_steps, double dphi_max,
                           double dt_max, long long* total_steps, double* kernel_ms) {
   const double pscale = 1.0 / (m0 * kC);
-  // one allocation: control words, SI arrays, step counts, state, status
-  const size_t sn = (size_t)n;
-  const size_t bytes = 64 + sn * (6 * sizeof(double) + sizeof(int64_t) + 6 * sizeof(T) + sizeof(int32_t));
+  // one allocation: control words, a chunk's SI arrays, step counts, state, status
+  const size_t sn = (size_t)n, ch = (size_t)std::min(n, kTraceChunk);
+  const size_t bytes = 64 + ch * 6 * sizeof(double) + sn * (sizeof(int64_t) + 6 * sizeof(T) + sizeof(int32_t));
   char* mem = nullptr;
   cudaStream_t s = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -298,20 +304,24 @@ amps_gpu_status run_trace(long long n, double* x, double* p, int32_t* status, in
   ok = ok && cudaEventCreate(&e0) == cudaSuccess && cudaEventCreate(&e1) == cudaSuccess;
   unsigned long long* d_ctl = reinterpret_cast<unsigned long long*>(mem);
   double* d_x = reinterpret_cast<double*>(mem + 64);
-  double* d_p = d_x + 3 * sn;
-  int64_t* d_steps = reinterpret_cast<int64_t*>(d_p + 3 * sn);
+  double* d_p = d_x + 3 * ch;
+  int64_t* d_steps = reinterpret_cast<int64_t*>(d_p + 3 * ch);
   T* d = reinterpret_cast<T*>(d_steps + sn);
   int32_t* d_st = reinterpret_cast<int32_t*>(d + 6 * sn);
-  ok = ok && cudaMemcpyAsync(d_x, x, sizeof(double) * 3 * sn, cudaMemcpyHostToDevice, s) == cudaSuccess;
-  ok = ok && cudaMemcpyAsync(d_p, p, sizeof(double) * 3 * sn, cudaMemcpyHostToDevice, s) == cudaSuccess;
   ok = ok && cudaMemsetAsync(d_ctl, 0, 64, s) == cudaSuccess;
+  auto cgrid = [](long long count) { return (unsigned)((3 * count + 255) / 256); };
+  for (long long i = 0; ok && i < n; i += kTraceChunk) {
+    const long long count = std::min(n - i, kTraceChunk);
+    const size_t b = sizeof(double) * 3 * (size_t)count;
+    ok = cudaMemcpyAsync(d_x, x + 3 * i, b, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+         cudaMemcpyAsync(d_p, p + 3 * i, b, cudaMemcpyHostToDevice, s) == cudaSuccess;
+    if (ok) k_trace_in<T><<<cgrid(count), 256, 0, s>>>(count, n, d_x, d_p, r_e, pscale, d + i);
+  }
   if (!ok) {
     cudaGetLastError();
     cleanup();
     return AMPS_GPU_CUDA_ERROR;
   }
-  const unsigned cgrid = (unsigned)((3 * n + 255) / 256);
-  k_trace_in<T><<<cgrid, 256, 0, s>>>(n, d_x, d_p, r_e, pscale, d);
   TraceArgs<T> a;
   a.x = d; a.y = d + sn; a.z = d + 2 * sn; a.px = d + 3 * sn; a.py = d + 4 * sn; a.pz = d + 5 * sn;
   a.status = d_st; a.steps = d_steps; a.n = n;
@@ -336,13 +346,16 @@ amps_gpu_status run_trace(long long n, double* x, double* p, int32_t* status, in
   k_set_queue<<<1, 1, 0, s>>>(a.queue, (unsigned long long)(32 * warps));
   k_trace<T><<<grid, NT, 0, s>>>(a);
   cudaEventRecord(e1, s);
-  k_trace_out<T><<<cgrid, 256, 0, s>>>(n, d, r_e, pscale, d_x, d_p);
   unsigned long long ctl[4];
   cudaError_t err = cudaGetLastError();
+  for (long long i = 0; err == cudaSuccess && i < n; i += kTraceChunk) {
+    const long long count = std::min(n - i, kTraceChunk);
+    const size_t b = sizeof(double) * 3 * (size_t)count;
+    k_trace_out<T><<<cgrid(count), 256, 0, s>>>(count, n, d + i, r_e, pscale, d_x, d_p);
+    if ((err = cudaGetLastError()) == cudaSuccess) err = cudaMemcpyAsync(x + 3 * i, d_x, b, cudaMemcpyDeviceToHost, s);
+    if (err == cudaSuccess) err = cudaMemcpyAsync(p + 3 * i, d_p, b, cudaMemcpyDeviceToHost, s);
+  }
   if (err == cudaSuccess) err = cudaMemcpyAsync(ctl, d_ctl, sizeof(ctl), cudaMemcpyDeviceToHost, s);
-  if (err == cudaSuccess) err = cudaStreamSynchronize(s);
-  if (err == cudaSuccess) err = cudaMemcpyAsync(x, d_x, sizeof(double) * 3 * sn, cudaMemcpyDeviceToHost, s);
-  if (err == cudaSuccess) err = cudaMemcpyAsync(p, d_p, sizeof(double) * 3 * sn, cudaMemcpyDeviceToHost, s);
   if (err == cudaSuccess) err = cudaMemcpyAsync(status, d_st, sizeof(int32_t) * sn, cudaMemcpyDeviceToHost, s);
   if (err == cudaSuccess) err = cudaMemcpyAsync(steps, d_steps, sizeof(int64_t) * sn, cudaMemcpyDeviceToHost, s);
   if (err == cudaSuccess) err = cudaStreamSynchronize(s);

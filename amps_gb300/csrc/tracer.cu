@@ -340,8 +340,11 @@ amps_gpu_status run_trace(long long n, double* x, double* p, int32_t* status, in
   const int grid = nsm * TraceShape<T>::kPerSM;
   const long long warps = (long long)grid * (NT / 32);
   // a CTA ends when its particles have; the cap is a safety net far above that:
-  // the even share of particles of a lane, each at full length, 8 times over
-  a.iter_cap = 8 * ((n + 32 * warps - 1) / (32 * warps) + 2) * ((max_steps + kRefill - 1) / kRefill + 2) + n + 16;
+  // the even share of particles of a lane, each at full length, 8 times over (as far
+  // as 63 bits go: max_steps may be any)
+  const double cap = 8.0 * (double)((n + 32 * warps - 1) / (32 * warps) + 2) * ((double)(max_steps / kRefill) + 3.0) +
+                     (double)n + 16.0;
+  a.iter_cap = cap < 9.0e18 ? (long long)cap : 9000000000000000000LL;
   cudaEventRecord(e0, s);
   k_set_queue<<<1, 1, 0, s>>>(a.queue, (unsigned long long)(32 * warps));
   k_trace<T><<<grid, NT, 0, s>>>(a);

@@ -184,40 +184,50 @@ amps_gpu_status layout_upload(amps_gpu_ctx* c, const double* host, void* dev, lo
   return cuda_check(c, e, "upload");
 }
 
-// Fields between the device and host arrays (null: skipped), one wait at the end
+// Fields between the device and host arrays (null: skipped), one wait at the end.
+// The staging of pageable arrays stays with the context, so those that together take
+// more than kBatchStage (whose copies take far longer than the launches and waits
+// saved), or more than the device has left, go one by one through staging for one.
+constexpr size_t kBatchStage = 64u << 20;
 amps_gpu_status layout_vec3_many(amps_gpu_ctx* c, bool to_host, int count, double* const* host,
                                  double* const* dev, const long long* n) {
   Vec3Jobs j{};
   double* stage[kMaxVec3] = {nullptr};  // pageable arrays cross through staging
   double* user[kMaxVec3] = {nullptr};
+  double* map[kMaxVec3] = {nullptr};
+  bool single[kMaxVec3] = {false};
   size_t need = 0;
   int jobs = 0;
   long long most = 0;
   if (count > kMaxVec3) return set_err(c, AMPS_GPU_INVALID_ARG, "layout: too many fields");
   for (int q = 0; q < count; q++) {
     if (!host[q] || n[q] <= 0) continue;
+    map[q] = mapped(host[q]);
+    const size_t bytes = sizeof(double) * 3 * (size_t)n[q];
+    single[q] = !map[q] && need + bytes > kBatchStage;
+    if (!map[q] && !single[q]) need += bytes;
+  }
+  double* buf = need ? host_stage(c, need) : nullptr;
+  for (int q = 0; q < count; q++) {
+    if (!host[q] || n[q] <= 0) continue;
+    if (!map[q] && !buf) single[q] = true;
+    if (single[q]) continue;
     user[jobs] = host[q];
-    j.host[jobs] = mapped(host[q]);
+    j.host[jobs] = map[q];
     j.dev[jobs] = dev[q];
     j.n[jobs] = n[q];
-    if (!j.host[jobs]) need += sizeof(double) * 3 * (size_t)n[q];
     most = most < n[q] ? n[q] : most;
     jobs++;
   }
-  if (!jobs) return AMPS_GPU_OK;
   cudaError_t e = cudaSuccess;
-  if (need) {
-    double* buf = host_stage(c, need);
-    if (!buf) return set_err(c, AMPS_GPU_CUDA_ERROR, "layout staging allocation failed");
-    for (int q = 0; q < jobs; q++) {
-      if (j.host[q]) continue;
-      stage[q] = j.host[q] = buf;
-      buf += 3 * j.n[q];
-      if (!to_host && e == cudaSuccess)
-        e = cudaMemcpyAsync(stage[q], user[q], sizeof(double) * 3 * (size_t)j.n[q], cudaMemcpyHostToDevice, c->stream);
-    }
+  for (int q = 0; q < jobs; q++) {
+    if (j.host[q]) continue;
+    stage[q] = j.host[q] = buf;
+    buf += 3 * j.n[q];
+    if (!to_host && e == cudaSuccess)
+      e = cudaMemcpyAsync(stage[q], user[q], sizeof(double) * 3 * (size_t)j.n[q], cudaMemcpyHostToDevice, c->stream);
   }
-  if (e == cudaSuccess) {
+  if (e == cudaSuccess && jobs) {
     const dim3 grid(grid_of(3 * most), jobs);
     if (to_host)
       k_vec3_many<true><<<grid, 256, 0, c->stream>>>(j, perm_of(c));
@@ -228,8 +238,13 @@ amps_gpu_status layout_vec3_many(amps_gpu_ctx* c, bool to_host, int count, doubl
   for (int q = 0; q < jobs && to_host && e == cudaSuccess; q++)
     if (stage[q])
       e = cudaMemcpyAsync(user[q], stage[q], sizeof(double) * 3 * (size_t)j.n[q], cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  return cuda_check(c, e, to_host ? "download fields" : "upload fields");
+  if (e == cudaSuccess && jobs) e = cudaStreamSynchronize(c->stream);
+  amps_gpu_status st = cuda_check(c, e, to_host ? "download fields" : "upload fields");
+  for (int q = 0; q < count && !st; q++)
+    if (single[q])
+      st = to_host ? layout_download(c, dev[q], host[q], n[q], 3, false)
+                   : layout_upload(c, host[q], dev[q], n[q], 3, false);
+  return st;
 }
 
 amps_gpu_status layout_download(amps_gpu_ctx* c, const void* dev, double* host, long long n,

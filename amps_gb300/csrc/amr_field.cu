@@ -105,22 +105,17 @@ constexpr int kMaxScale = 8;
 
 struct ApplyArgs {
   long long ncell, nvc;
-  const int* ctab;
-  const int* ctabh;     // ctab with hanging corners as ~id
+  const int* ctabh;     // block corner -> corner, hanging ones as ~id
   Hang h;
   const int* bscale;
   LevelK lk[kMaxScale];
   float fj[2];          // f as a pair (the current term of the RHS)
-  const float* xh;      // ACC 1/2 input as FP32 pairs (dinv applied)
+  const float* xh;      // ACC 1/2 input as FP32 pairs (the scaling applied)
   const float* xl;
-  const double* bdx;
   const float* cellM;
   const float* cellJ;
-  const double* x;     // input field (component-major)
-  const float* xf;     // the same times dinv, in FP32 (the FP32 inner operator)
-  const double* dinv;  // optional right preconditioner
-  const double* Bcen;  // RHS: centre B (component-major over cells)
-  double th2dt2, f, thdt;
+  const float* xf;      // the same in FP32 (the FP32 inner operator)
+  const double* Bcen;   // RHS: centre B (component-major over cells)
   unsigned long long* flags;  // [2]: bounded-wait timeouts
   double* diag;               // RHS: += the Jacobi diagonal of free corners (null: not wanted)
   int* next;                  // tiles handed out beyond the first two per CTA
@@ -1069,8 +1064,8 @@ unsigned g1(long long n) { return (unsigned)((n + 255) / 256); }
 cudaError_t launch_amr_pack(amps_gpu_ctx* c, const double* Eh, const double* Bprev,
                             const double* Bcur) {
   TimedLaunch t(c, "pack_stencils");
-  launch_pdl(k_amr_pack, dim3(c->nb, 3), dim3(256), 0, c->stream, c->nvc, c->d_ctabh, hang_of(c), Eh, Bprev, Bcur,
-                                            c->d_stencil_push, c->d_stencil_dep);
+  launch_pdl(k_amr_pack, dim3(c->nb, 3), dim3(256), 0, c->stream, c->nvc, c->d_ctabh, hang_of(c), Eh, Bprev,
+             Bcur, c->d_stencil_push, c->d_stencil_dep);
   return cudaGetLastError();
 }
 
@@ -1078,16 +1073,12 @@ static ApplyArgs apply_args(amps_gpu_ctx* c) {
   ApplyArgs a{};
   a.ncell = c->ncor;
   a.nvc = c->nvc;
-  a.ctab = c->d_ctab;
   a.ctabh = c->d_ctabh;
   a.h = hang_of(c);
-  a.bdx = c->d_bdx;
   a.cellM = c->d_cellM;
   a.cellJ = c->d_cellJ;
   const double th = c->cfg.theta, dt = c->cfg.dt;
-  a.th2dt2 = th * th * dt * dt;
-  a.f = 4.0 * kPi * dt * th;
-  a.thdt = th * dt;
+  const double th2dt2 = th * th * dt * dt, f = 4.0 * kPi * dt * th, thdt = th * dt;
   a.flags = c->d_flags;
   a.next = c->d_next;
   a.bscale = c->d_bscale;
@@ -1099,13 +1090,13 @@ static ApplyArgs apply_args(amps_gpu_ctx* c) {
     const double dx = c->dxf * (double)(1 << sc), V = dx * dx * dx;
     LevelK& K = a.lk[sc];
     split(0.25 / dx, K.curl);
-    split(a.th2dt2 * V * 0.25 / dx, K.cc);
+    split(th2dt2 * V * 0.25 / dx, K.cc);
     split(0.125 * V, K.id);
-    split(a.f * V, K.m);
-    split(a.thdt * V * 0.25 / dx, K.bb);
-    K.dg = (float)(V * (0.125 + a.th2dt2 / (8.0 * dx * dx)));
+    split(f * V, K.m);
+    split(thdt * V * 0.25 / dx, K.bb);
+    K.dg = (float)(V * (0.125 + th2dt2 / (8.0 * dx * dx)));
   }
-  split(a.f, a.fj);
+  split(f, a.fj);
   return a;
 }
 
@@ -1117,9 +1108,8 @@ static cudaError_t split_input(amps_gpu_ctx* c, const double* x, const double* d
     return e;
   a.xh = c->d_xs;
   a.xl = c->d_xs + n;
-  launch_pdl(k_amr_split, dim3((unsigned)(std::min<long long>((n + 255) / 256, 152LL * 16))), dim3(256), 0, c->stream, n, x, dinv,
-                                                                                                c->d_xs,
-                                                                                                c->d_xs + n);
+  launch_pdl(k_amr_split, dim3((unsigned)(std::min<long long>((n + 255) / 256, 152LL * 16))), dim3(256), 0,
+             c->stream, n, x, dinv, c->d_xs, c->d_xs + n);
   return cudaGetLastError();
 }
 
@@ -1152,7 +1142,8 @@ static cudaError_t launch_tile(amps_gpu_ctx* c, const ApplyArgs& a, double* y64)
   if (e != cudaSuccess) return e;
   // AMR meshes hold whole 512-cell blocks: ncell is a multiple of the tile
   const int tiles = (int)(c->ncor / kFFCells);
-  launch_pdl(k_amr_tile_ff<ACC>, dim3(std::min(n, tiles)), dim3(kTileThreads), 2 * tile_ff_bytes<ACC>(), c->stream, a, tiles, y64);
+  launch_pdl(k_amr_tile_ff<ACC>, dim3(std::min(n, tiles)), dim3(kTileThreads), 2 * tile_ff_bytes<ACC>(),
+             c->stream, a, tiles, y64);
   return cudaGetLastError();
 }
 
@@ -1163,7 +1154,8 @@ static cudaError_t launch_tile32(amps_gpu_ctx* c, const ApplyArgs& a, float* y32
   cudaError_t e = tile_grid(k_amr_tile32, kT32Threads, 2 * kTileBytes, grid, n);
   if (e != cudaSuccess) return e;
   const int tiles = (int)(c->ncor / kTileCells);
-  launch_pdl(k_amr_tile32, dim3(std::min(n, tiles)), dim3(kT32Threads), 2 * kTileBytes, c->stream, a, tiles, y32);
+  launch_pdl(k_amr_tile32, dim3(std::min(n, tiles)), dim3(kT32Threads), 2 * kTileBytes, c->stream, a, tiles,
+             y32);
   return cudaGetLastError();
 }
 
@@ -1171,8 +1163,6 @@ cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* di
   cudaError_t e = cudaMemsetAsync(y, 0, sizeof(double) * 3 * c->nvc, c->stream);
   if (e != cudaSuccess) return e;
   ApplyArgs a = apply_args(c);
-  a.x = x;
-  a.dinv = dinv;
   TimedLaunch t(c, "matvec", pairs ? 2 : 3);
   if (pairs) {
     a.xh = c->d_xs;
@@ -1181,8 +1171,8 @@ cudaError_t launch_amr_matvec(amps_gpu_ctx* c, const double* x, const double* di
     return e;
   }
   if ((e = launch_tile<1>(c, a, y)) != cudaSuccess) return e;
-  launch_pdl(k_amr_constraint, dim3(g1(std::max(c->nsrows, 1))), dim3(256), 0, c->stream, c->nsrows, c->d_srows, c->nvc, a.h,
-                                                                      x, dinv, y, 0, c->d_next);
+  launch_pdl(k_amr_constraint, dim3(g1(std::max(c->nsrows, 1))), dim3(256), 0, c->stream, c->nsrows,
+             c->d_srows, c->nvc, a.h, x, dinv, y, 0, c->d_next);
   return cudaGetLastError();
 }
 
@@ -1199,9 +1189,9 @@ cudaError_t launch_amr_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, f
   if ((e = launch_tile32(c, a, c->d_y32)) != cudaSuccess) return e;
   const unsigned plain = (unsigned)((c->nvc + 256 * kFinPer - 1) / (256 * kFinPer));
   const int per = 256 / kRowLanes;
-  launch_pdl(k_amr_finish_ff, dim3(plain + (unsigned)((c->nsrows + per - 1) / per)), dim3(256), 0, c->stream, 
-      c->nvc, a.h, plain, c->nsrows, c->d_srows, c->d_ss, c->d_sc, c->d_svh, c->d_svl, c->d_sdiag,
-      c->d_y32, in, wh, wl);
+  launch_pdl(k_amr_finish_ff, dim3(plain + (unsigned)((c->nsrows + per - 1) / per)), dim3(256), 0,
+             c->stream, c->nvc, a.h, plain, c->nsrows, c->d_srows, c->d_ss, c->d_sc, c->d_svh, c->d_svl,
+             c->d_sdiag, c->d_y32, in, wh, wl);
   return cudaGetLastError();
 }
 
@@ -1212,14 +1202,12 @@ cudaError_t launch_amr_rhs(amps_gpu_ctx* c, bool diag) {
   if (e != cudaSuccess) return e;
   ApplyArgs a = apply_args(c);
   a.diag = diag ? c->d_diag : nullptr;
-  a.x = c->d_En;
-  a.dinv = nullptr;
   a.Bcen = c->d_Bc;
   TimedLaunch t(c, "rhs", 3);
   if ((e = split_input(c, c->d_En, nullptr, a)) != cudaSuccess) return e;
   if ((e = launch_tile<2>(c, a, c->d_rhs)) != cudaSuccess) return e;
-  launch_pdl(k_amr_constraint, dim3(g1(std::max(c->nsrows, 1))), dim3(256), 0, c->stream, c->nsrows, c->d_srows, c->nvc, a.h,
-                                                                      nullptr, nullptr, c->d_rhs, 1, c->d_next);
+  launch_pdl(k_amr_constraint, dim3(g1(std::max(c->nsrows, 1))), dim3(256), 0, c->stream, c->nsrows,
+             c->d_srows, c->nvc, a.h, nullptr, nullptr, c->d_rhs, 1, c->d_next);
   return cudaGetLastError();
 }
 
@@ -1231,8 +1219,8 @@ cudaError_t launch_amr_jacobi(amps_gpu_ctx* c) {
 
 cudaError_t launch_amr_update_b(amps_gpu_ctx* c) {
   TimedLaunch t(c, "update_b");
-  launch_pdl(k_amr_update_b, dim3(c->nb), dim3(256), 0, c->stream, c->ncor, c->nvc, c->d_ctabh, hang_of(c), c->d_bdx, c->d_Eh,
-                                               c->d_Bc, c->d_Bc2, c->cfg.dt, c->d_energy + 1);
+  launch_pdl(k_amr_update_b, dim3(c->nb), dim3(256), 0, c->stream, c->ncor, c->nvc, c->d_ctabh, hang_of(c),
+             c->d_bdx, c->d_Eh, c->d_Bc, c->d_Bc2, c->cfg.dt, c->d_energy + 1);
   if (c->mesh_open) {
     const int* nf = c->amrdev.nfine;
     for (int pass = 0; pass <= (c->neumann ? 3 : 0); pass++)
@@ -1245,8 +1233,8 @@ cudaError_t launch_amr_update_b(amps_gpu_ctx* c) {
 // hanging corners of F, optionally with their wave energy
 static cudaError_t fix_hanging(amps_gpu_ctx* c, double* F, const double* cvol, double* energy) {
   if (c->nsrows == 0) return cudaSuccess;
-  launch_pdl(k_amr_fix_hanging, dim3(g1(c->nsrows)), dim3(256), 0, c->stream, c->nsrows, c->d_srows, c->nvc, hang_of(c), F, cvol,
-                                                          energy);
+  launch_pdl(k_amr_fix_hanging, dim3(g1(c->nsrows)), dim3(256), 0, c->stream, c->nsrows, c->d_srows, c->nvc,
+             hang_of(c), F, cvol, energy);
   return cudaGetLastError();
 }
 
@@ -1254,7 +1242,8 @@ cudaError_t launch_amr_c2n(amps_gpu_ctx* c, const double* Bcen, double* Bcor) {
   cudaError_t e = cudaMemsetAsync(Bcor, 0, sizeof(double) * 3 * c->nvc, c->stream);
   if (e != cudaSuccess) return e;
   TimedLaunch t(c, "c2n", 2);
-  launch_pdl(k_amr_c2n, dim3(c->nb), dim3(256), 0, c->stream, c->ncor, c->nvc, c->d_ctab, c->d_bdx, c->d_cinv, Bcen, Bcor);
+  launch_pdl(k_amr_c2n, dim3(c->nb), dim3(256), 0, c->stream, c->ncor, c->nvc, c->d_ctab, c->d_bdx,
+             c->d_cinv, Bcen, Bcor);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   return fix_hanging(c, Bcor, nullptr, nullptr);
 }
@@ -1264,13 +1253,8 @@ cudaError_t launch_amr_update_e(amps_gpu_ctx* c) {
   TimedLaunch t(c, "update_e", 2);
   const double th = c->cfg.theta;
   const unsigned grid = (unsigned)std::min<long long>((std::max(c->nvc, c->ncor) + 255) / 256, 152LL * 8);
-  launch_pdl(k_amr_update_e, grid, dim3(256), 0, c->stream, c->ncor, c->nvc, c->d_Eh, c->d_En, 1.0 / th, (1.0 - th) / th, c->d_cvol,
-                                              c->d_bdx, c->d_Bc, c->d_energy + 1);
+  launch_pdl(k_amr_update_e, grid, dim3(256), 0, c->stream, c->ncor, c->nvc, c->d_Eh, c->d_En, 1.0 / th,
+             (1.0 - th) / th, c->d_cvol, c->d_bdx, c->d_Bc, c->d_energy + 1);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   return fix_hanging(c, c->d_En, c->d_cvol, c->d_energy + 1);
-}
-
-// E^{n+theta} = E^n + dE with hanging corners re-interpolated
-cudaError_t launch_amr_fix_hanging(amps_gpu_ctx* c, double* F) {
-  return fix_hanging(c, F, nullptr, nullptr);
 }

@@ -678,9 +678,9 @@ amps_gpu_status amps_gpu_create_amr(const amps_gpu_config* cfg, const amps_amr_m
     std::vector<int> ctabh(m->corner_tab.begin(), m->corner_tab.end());
     for (int& q : ctabh)
       if (hs[(size_t)q + 1] > hs[(size_t)q]) q = ~q;
-    ok = ok && upload(&c->d_ss, ss) && upload(&c->d_sc, sc) && upload(&c->d_sv, sv) &&
-         upload(&c->d_svh, svh) && upload(&c->d_svl, svl) && upload(&c->d_sdiag, sdiag) && upload(&c->d_srows, srows) &&
-         upload(&c->d_ctabh, ctabh) && upload(&c->d_cvol, cvol) && upload(&c->d_cinv, cinv);
+    ok = ok && upload(&c->d_ss, ss) && upload(&c->d_sc, sc) && upload(&c->d_svh, svh) && upload(&c->d_svl, svl) &&
+         upload(&c->d_sdiag, sdiag) && upload(&c->d_srows, srows) && upload(&c->d_ctabh, ctabh) &&
+         upload(&c->d_cvol, cvol) && upload(&c->d_cinv, cinv);
   }
   if (!ok) {
     cudaGetLastError();
@@ -751,7 +751,7 @@ amps_gpu_status amps_gpu_destroy(amps_gpu_ctx* c) {
                   c->d_cellM, c->d_cellJ, c->d_energy, c->d_ctab, c->d_hs, c->d_hp, c->d_hw, c->d_hwh, c->d_hwl,
                   c->d_bflag, c->d_bs, c->d_bc, c->d_bw, c->d_bwh, c->d_bwl,
                   c->d_fine_map, c->d_borg, c->d_bscale, c->d_bdx, c->d_bdtdx, c->d_binvvol,
-                  c->d_ss, c->d_sc, c->d_sv, c->d_svh, c->d_svl, c->d_sdiag, c->d_srows, c->d_ctabh, c->d_dff, c->d_tmpv, c->d_pc_in, c->d_pc_out_v[0], c->d_pc_out_v[1],
+                  c->d_ss, c->d_sc, c->d_svh, c->d_svl, c->d_sdiag, c->d_srows, c->d_ctabh, c->d_dff, c->d_tmpv, c->d_pc_in, c->d_pc_out_v[0], c->d_pc_out_v[1],
                   c->d_pc_set, c->d_pc_jac_v[0], c->d_pc_jac_v[1]};
   for (void* p : ptrs) cudaFree(p);
   for (int b = 0; b < 2; b++) {

@@ -95,7 +95,6 @@ struct amps_gpu_ctx {
   float* d_binvvol = nullptr; // 1/dx^3 per block
   int* d_ss = nullptr;        // identity part of the AMR operator, CSR rows (nvc+1)
   int* d_sc = nullptr;        //   columns
-  double* d_sv = nullptr;     //   values
   float* d_svh = nullptr;     //   values as FP32 pairs
   float* d_svl = nullptr;
   float2* d_sdiag = nullptr;  //   the diagonal of rows that are nothing else, as pairs (0: others)
@@ -368,22 +367,12 @@ cudaError_t launch_amr_jacobi(amps_gpu_ctx* c);
 cudaError_t launch_amr_update_b(amps_gpu_ctx* c);
 cudaError_t launch_amr_c2n(amps_gpu_ctx* c, const double* Bcen, double* Bcor);
 cudaError_t launch_amr_update_e(amps_gpu_ctx* c);
-cudaError_t launch_amr_fix_hanging(amps_gpu_ctx* c, double* F);
 
 // ---- device helpers ----
 __host__ __device__ inline int nbr_slot(int ox, int oy, int oz) {
   return (ox + 1) + 3 * (oy + 1) + 9 * (oz + 1);
 }
 
-// FP64-accurate sums of products at FP32 throughput (GB300 issues FP32 FMAs at
-// 64x its FP64 rate): x = xh + xl split into FP32 (xh = fp32(x)); a product
-// with an FP32 coefficient m is m xh exactly (its rounding error recovered by
-// an FMA) plus m xl.  The leading parts are summed with an error-free TwoSum
-// per step (Knuth), whose exact errors go with the small parts into a second
-// FP32 sum (the cascaded summation of Ogita, Rump and Oishi); the two are
-// combined in FP64.  Error ~1e-14 of the sum of |terms| for 81 terms.  The
-// arithmetic uses the _rn intrinsics, which the compiler never contracts into
-// FMAs (a contraction would break the error-free transformations).
 // Programmatic dependent launch: a kernel launched by launch_pdl may start while the
 // kernel before it on the stream is still running, and waits for that one's completion
 // (and so for all before it) in pdl_wait(), before it touches anything the other reads or
@@ -393,7 +382,8 @@ __host__ __device__ inline int nbr_slot(int ox, int oy, int oz) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              A&&... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -407,6 +397,15 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// FP64-accurate sums of products at FP32 throughput (GB300 issues FP32 FMAs at
+// 64x its FP64 rate): x = xh + xl split into FP32 (xh = fp32(x)); a product
+// with an FP32 coefficient m is m xh exactly (its rounding error recovered by
+// an FMA) plus m xl.  The leading parts are summed with an error-free TwoSum
+// per step (Knuth), whose exact errors go with the small parts into a second
+// FP32 sum (the cascaded summation of Ogita, Rump and Oishi); the two are
+// combined in FP64.  Error ~1e-14 of the sum of |terms| for 81 terms.  The
+// arithmetic uses the _rn intrinsics, which the compiler never contracts into
+// FMAs (a contraction would break the error-free transformations).
 struct FF {
   float s, q;
 };

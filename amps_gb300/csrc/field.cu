@@ -382,7 +382,7 @@ struct GmStatus {
 static_assert(offsetof(GmState, timeouts) - offsetof(GmState, jj) == offsetof(GmStatus, timeouts), "GmStatus layout");
 static_assert(kGmOffset * sizeof(double) + sizeof(GmState) <= kTolOffset * sizeof(double),
               "GmState must fit in d_red");
-static_assert(kRedBlocks * kMaxV + 2 * kMaxV + 8 + kMaxV <= kGmOffset, "d_red layout");
+static_assert(kRedBlocks * kMaxV < kGmOffset, "d_red layout");
 
 // start of a cycle: g = (||r||, 0, ...); *n2 = ||r||^2
 __global__ void k_gm_start(GmState* __restrict__ S, const double* __restrict__ n2, double target) {
@@ -1344,8 +1344,8 @@ cudaError_t launch_matvec(amps_gpu_ctx* c, const double* x, const double* dinv, 
   cudaError_t e = pairs ? cudaSuccess : split_input(c, x, dinv);
   if (e != cudaSuccess) return e;
   const long long n = 3 * c->ncor;
-  launch_pdl(k_matvec, dim3((unsigned)((c->ncor / 32))), dim3(c->tune_tb), 0, c->stream, c->ncor, c->d_nbr, c->d_M, c->d_xs,
-                                                                   c->d_xs + n, y, T);
+  launch_pdl(k_matvec, dim3((unsigned)(c->ncor / 32)), dim3(c->tune_tb), 0, c->stream, c->ncor, c->d_nbr,
+             c->d_M, c->d_xs, c->d_xs + n, y, T);
   return cudaGetLastError();
 }
 
@@ -1366,8 +1366,8 @@ cudaError_t launch_matvec32_ff(amps_gpu_ctx* c, const OpIn& in, float* wh, float
   TimedLaunch t(c, "matvec32", in.xf_ready ? 1 : 2);
   cudaError_t e = in.xf_ready ? cudaSuccess : launch_in_f32(c, in, c->d_xs);
   if (e != cudaSuccess) return e;
-  launch_pdl(k_matvec32_ff, dim3((unsigned)((c->ncor / 32))), dim3(c->tune_tb), 0, c->stream, c->ncor, c->d_nbr, c->d_M, c->d_xs,
-                                                                        in, wh, wl, T);
+  launch_pdl(k_matvec32_ff, dim3((unsigned)(c->ncor / 32)), dim3(c->tune_tb), 0, c->stream, c->ncor,
+             c->d_nbr, c->d_M, c->d_xs, in, wh, wl, T);
   return cudaGetLastError();
 }
 
@@ -1380,9 +1380,8 @@ cudaError_t launch_rhs(amps_gpu_ctx* c, bool diag) {
   cudaError_t e = split_input(c, c->d_En, nullptr);
   if (e != cudaSuccess) return e;
   const long long n = 3 * c->ncor;
-  launch_pdl(k_rhs, dim3((unsigned)((c->ncor / 32))), dim3(c->tune_tb), 0, c->stream, c->ncor, c->d_nbr, c->d_M, c->d_xs,
-                                                                c->d_xs + n, c->d_Bc, c->d_J, c->d_rhs, T,
-                                                                c4[0], c4[1], c4[2]);
+  launch_pdl(k_rhs, dim3((unsigned)(c->ncor / 32)), dim3(c->tune_tb), 0, c->stream, c->ncor, c->d_nbr,
+             c->d_M, c->d_xs, c->d_xs + n, c->d_Bc, c->d_J, c->d_rhs, T, c4[0], c4[1], c4[2]);
   return cudaGetLastError();
 }
 
@@ -1401,7 +1400,7 @@ cudaError_t launch_update_b(amps_gpu_ctx* c) {
   for (int d = 0; d < 3; d++) c4[d] = 0.25 * (c->cfg.dt / c->cfg.dx[d]);
   TimedLaunch t(c, "update_b");
   launch_pdl(k_update_b, dim3(grid1(c->ncor)), dim3(256), 0, c->stream, c->ncor, c->d_nbr, c->d_Eh, c->d_Bc,
-                                                     c->d_Bc2, c4[0], c4[1], c4[2], c->d_energy + 1);
+             c->d_Bc2, c4[0], c4[1], c4[2], c->d_energy + 1);
   return cudaGetLastError();
 }
 
@@ -1413,8 +1412,8 @@ cudaError_t launch_c2n_update_e(amps_gpu_ctx* c, const double* Bcen, double* Bco
   }
   const double vol = c->cfg.dx[0] * c->cfg.dx[1] * c->cfg.dx[2];
   TimedLaunch t(c, "update_e");  // C2N with it
-  launch_pdl(k_c2n_update_e, dim3(grid1(c->ncor)), dim3(256), 0, c->stream, c->ncor, c->d_nbr, Bcen, Bcor, c->d_Eh, c->d_En,
-                                                        c->cfg.theta, vol / (8.0 * kPi), c->d_energy + 1);
+  launch_pdl(k_c2n_update_e, dim3(grid1(c->ncor)), dim3(256), 0, c->stream, c->ncor, c->d_nbr, Bcen, Bcor,
+             c->d_Eh, c->d_En, c->cfg.theta, vol / (8.0 * kPi), c->d_energy + 1);
   return cudaGetLastError();
 }
 
@@ -1431,14 +1430,14 @@ cudaError_t launch_c2n_update_e(amps_gpu_ctx* c, const double* Bcen, double* Bco
 // reads the device's convergence flag, then one step per read; steps queued
 // past convergence leave the least-squares state untouched (gm_update is
 // frozen), so they cost time but not accuracy.
-// Device scratch layout of d_red: [0, kRedBlocks*kMaxV) partials, then h1
-// (kMaxV), h2 (kMaxV), nrm2 (8), y (kMaxV); GmState at kGmOffset.
+// Device scratch layout of d_red: [0, kRedBlocks*kMaxV) partials, ||r||^2, GmState at
+// kGmOffset, the tolerance at kTolOffset.
 amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
                             amps_gpu_solve_stats* st, bool* eh_done) {
   const long long n = 3 * c->nvc;
   const int m = std::min(c->restart, kMaxV);
   double* partial = c->d_red;
-  double* d_n2 = c->d_red + kRedBlocks * kMaxV + 2 * kMaxV;
+  double* d_n2 = c->d_red + kRedBlocks * kMaxV;
   GmState* gs = reinterpret_cast<GmState*>(c->d_red + kGmOffset);
   const unsigned gr = gridr(n, c->tune_red, c->tune_ept);
   cudaStream_t s = c->stream;
@@ -1513,7 +1512,8 @@ amps_gpu_status gmres_solve(amps_gpu_ctx* c, double tol, int maxit, int precond,
       cudaError_t ee = launch_jacobi_diag(c);
       if (ee != cudaSuccess) return ee;
     }
-    launch_pdl(k_first, dim3(gr), dim3(256), 0, s, n, c->d_rhs, w, c->d_x, partial, d_n2, gs, c->d_red + kTolOffset);
+    launch_pdl(k_first, dim3(gr), dim3(256), 0, s, n, c->d_rhs, w, c->d_x, partial, d_n2, gs,
+               c->d_red + kTolOffset);
     return cudaGetLastError();
   };
   // Arnoldi step jj: the operator (after the network for flexible directions),

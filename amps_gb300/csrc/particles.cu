@@ -1840,10 +1840,10 @@ cudaError_t launch_pack_stencils(amps_gpu_ctx* c, const double* Eh, const double
   const bool cb = c->b_center;
   // a corner (or two centres) per thread: one CTA per block, which took them in turn,
   // took 11 us on 64 blocks and 20 us on 60 with centre B, now 8 and 14
-  launch_pdl(k_pack_stencils, dim3(c->nb, cb ? 4 : 3), dim3(256), 0, c->stream, c->nb, c->ncor, c->d_nbr, Eh, Bprev, Bcur, c->d_stencil_push, c->d_stencil_dep,
-      cb ? c->d_Bc2 : nullptr, cb ? c->d_Bc : nullptr,
-      cb ? reinterpret_cast<float4*>(c->d_stencil_cprev) : nullptr,
-      cb ? reinterpret_cast<float4*>(c->d_stencil_ccur) : nullptr);
+  launch_pdl(k_pack_stencils, dim3(c->nb, cb ? 4 : 3), dim3(256), 0, c->stream, c->nb, c->ncor, c->d_nbr,
+             Eh, Bprev, Bcur, c->d_stencil_push, c->d_stencil_dep, cb ? c->d_Bc2 : nullptr,
+             cb ? c->d_Bc : nullptr, cb ? reinterpret_cast<float4*>(c->d_stencil_cprev) : nullptr,
+             cb ? reinterpret_cast<float4*>(c->d_stencil_ccur) : nullptr);
   return cudaGetLastError();
 }
 
@@ -1852,8 +1852,8 @@ static cudaError_t launch_assemble(amps_gpu_ctx* c) {
   if (c->amr) return cudaSuccess;
   TimedLaunch t(c, "assemble");
   const double inv_vol = 1.0 / (c->cfg.dx[0] * c->cfg.dx[1] * c->cfg.dx[2]);
-  launch_pdl(k_assemble, dim3((unsigned)((c->nb * kAsmPerBlock))), dim3(kAsmThreads), kAsmSmem, c->stream, 
-      c->ncor, c->d_nbr, c->d_cellM, c->d_cellJ, inv_vol, c->d_M, c->d_J);
+  launch_pdl(k_assemble, dim3((unsigned)(c->nb * kAsmPerBlock)), dim3(kAsmThreads), kAsmSmem, c->stream,
+             c->ncor, c->d_nbr, c->d_cellM, c->d_cellJ, inv_vol, c->d_M, c->d_J);
   return cudaGetLastError();
 }
 

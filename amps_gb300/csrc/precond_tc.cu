@@ -505,5 +505,6 @@ cudaError_t precond_apply_tc_mesh(PrecondState* P, cudaStream_t st, int nb, cons
   if (e != cudaSuccess) return e;
   MeshIO io{v, dinv, in_map, hs, hp, hw, out_map, set, nvc, z, xf};
   // (the weights were packed long before: only the input is of the kernel before)
-  return launch_pdl(k_precond_tc, dim3(nb * kSplit), dim3(kThreads), kSmem, st, nullptr, nullptr, P->wtc, P->flags, io);
+  return launch_pdl(k_precond_tc, dim3(nb * kSplit), dim3(kThreads), kSmem, st, nullptr, nullptr, P->wtc,
+                    P->flags, io);
 }

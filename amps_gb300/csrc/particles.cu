@@ -1325,19 +1325,18 @@ __global__ void __launch_bounds__(256) k_import_local(long long n, const float* 
   }
 }
 
-// Export: compact arrays in cell order (out offsets = exclusive scan of cnt), one
-// warp per cell, its lanes over the cell's particles (consecutive loads and
-// stores; a thread per cell walked its particles alone: 276 us for 995,328
-// particles of 13,824 cells, now 53).
-__global__ void __launch_bounds__(256, 4) k_export(long long ncells, const int* __restrict__ base,
+// Export: compact arrays in cell order (out offsets = exclusive scan of cnt), `lanes`
+// lanes (a power of two, export_lanes) per cell over its particles: consecutive
+// loads and stores.
+__global__ void __launch_bounds__(256, 4) k_export(long long ncells, int lanes, const int* __restrict__ base,
                                                 const int* __restrict__ cnt,
                                                 const int* __restrict__ out0, PBuf s, int nbx,
                                                 int nby, double x00, double x01, double x02,
                                                 double dx0, double dx1, double dx2, double* x,
                                                 double* v, uint8_t* sp, int32_t* blk,
                                                 int32_t* cel, uint32_t* id, AmrDev m, double dxf) {
-  const long long cid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+  const long long cid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / lanes;
+  const int lane = threadIdx.x & (lanes - 1);
   if (cid >= ncells) return;
   const int b = (int)(cid / AMPS_CPB), l = (int)(cid % AMPS_CPB);
   double o0, o1, o2;
@@ -1355,7 +1354,7 @@ __global__ void __launch_bounds__(256, 4) k_export(long long ncells, const int* 
   }
   const int b0 = base[cid], n0 = cnt[cid];
   const long long q0 = out0[cid];
-  for (int t = lane; t < n0; t += 32) {
+  for (int t = lane; t < n0; t += lanes) {
     const long long p = b0 + t, q = q0 + t;
     if (x) {
       x[3 * q] = o0 + (double)s.u[0][p] * dx0;
@@ -2258,6 +2257,18 @@ cudaError_t launch_import_local(amps_gpu_ctx* c, const float* d_u, const float* 
   return rebuild_from_list(c, n);
 }
 
+// Lanes per cell of the export: as many as the mean cell has particles, and beyond 8
+// only as long as that puts more threads on the chip (4 CTAs of 256 on 152 SMs).  A
+// thread per cell walks its particles alone, a warp per cell idles and waits where
+// they are few.  us with 1 / 4 / 8 / 32 lanes, 110,592 cells: 4 particles per cell
+// 67 / 35 / 52 / 161, 16: 403 / 95 / 88 / 172, 128: 5188 / 723 / 422 / 509; 4096
+// cells with 1 / 8 / 16 / 32: 128 per cell 474 / 34 / 22 / 22.
+static int export_lanes(long long np, long long ncells) {
+  int lanes = 1;
+  while (lanes < 32 && lanes * ncells < np && (lanes < 8 || lanes * ncells < 152LL * 4 * 256)) lanes *= 2;
+  return lanes;
+}
+
 cudaError_t launch_export(amps_gpu_ctx* c, double* d_x, double* d_v, uint8_t* d_sp,
                           int32_t* d_blk, int32_t* d_cel, uint32_t* d_id) {
   cudaError_t e = cudaMemcpyAsync(c->d_tmp, c->d_cnt, sizeof(int) * c->ncor,
@@ -2268,8 +2279,9 @@ cudaError_t launch_export(amps_gpu_ctx* c, double* d_x, double* d_v, uint8_t* d_
   e = scan_ints(c, c->d_tmp, c->d_tmp, c->ncor + 1);
   if (e != cudaSuccess) return e;
   TimedLaunch t(c, "export");
-  k_export<<<(unsigned)((32 * c->ncor + 255) / 256), 256, 0, c->stream>>>(
-      c->ncor, c->d_base, c->d_cnt, c->d_tmp, pbuf(c, c->cur), c->cfg.nbx, c->cfg.nby,
+  const int lanes = export_lanes(c->np, c->ncor);
+  k_export<<<(unsigned)((lanes * c->ncor + 255) / 256), 256, 0, c->stream>>>(
+      c->ncor, lanes, c->d_base, c->d_cnt, c->d_tmp, pbuf(c, c->cur), c->cfg.nbx, c->cfg.nby,
       c->cfg.x0[0], c->cfg.x0[1], c->cfg.x0[2], c->cfg.dx[0], c->cfg.dx[1], c->cfg.dx[2], d_x, d_v,
       d_sp, d_blk, d_cel, d_id, c->amrdev, c->dxf);
   return cudaGetLastError();

@@ -580,20 +580,21 @@ __device__ __forceinline__ FF ff_warp_sum(FF a) {
 // sweep and a grid barrier.  Both hold where h2 is no more than the first
 // projection's rounding, a few 2^-48 |w|: FP32 is wrong by 2^-24 of V h2, which
 // ||h2|| <= 2^-28 ||w'|| (kArnSmallH2, its square) keeps under the pairs' own
-// last bit.  Any larger h2 (|w'| far below |w|, or a basis that lost its
-// orthogonality) takes the third sweep in full pairs and the norm from its sum, one
-// more grid barrier.
+// last bit (solves: ||h2||^2 / ||w'||^2 of 1e-29 to 1e-23 in all of 181 steps looked
+// at).  Any larger h2 (|w'| far below |w|, or a basis that lost its orthogonality)
+// takes the third sweep in full pairs and the norm from its sum, one more grid barrier.
 // A CTA whose tiles all fit its stages reads them once.
-// Waits give up after `limit` polls (counted in the state): a producer whose stage
-// is not freed issues nothing more, a consumer warp whose tile does not come goes on
-// without waiting or freeing, so that a stage is never filled over a copy still in
-// flight; all take part in every barrier, and the producer leaves when its last
-// copies have landed.  1.34M unknowns, mean
-// step of a 55-iteration solve (1 to 30 vectors): 103 us, 4 us per vector (the
-// rate of HBM) on ~45 us of barriers and start-up.  Before: 304 us with
-// per-thread streams, four basis reads and three barriers; 150 us with one CTA
-// per SM and a bulk copy per row.  1.50M unknowns, 1 to 8 vectors: 59 us, before
-// 81.
+// Waits give up after `limit` polls (counted in the state): a producer whose stage is
+// not freed issues nothing more, a consumer warp whose tile does not come goes on and
+// frees nothing more, so that a stage is never filled over a copy still in flight; all
+// take part in every barrier, and the producer leaves when its last copies have
+// landed.  (64 registers at the tiles of long bases: with 80, which votes or flags at
+// the waits cost, the next kernels' early CTAs find no room beside this one, 14 us a
+// step of a learned solve on 1.1M unknowns.)
+// 1.34M unknowns, mean step of a 55-iteration solve (1 to 30 vectors): 103 us, 4 us
+// per vector (the rate of HBM) on ~45 us of barriers and start-up.  Before: 304 us
+// with per-thread streams, four basis reads and three barriers; 150 us with one CTA
+// per SM and a bulk copy per row.  1.50M unknowns, 1 to 8 vectors: 59 us, before 81.
 constexpr int kArnCons = 256;               // consumer threads (8 warps)
 constexpr int kArnBlock = kArnCons + 32;    // + the producer warp
 constexpr int kArnWarps = kArnCons / 32;
@@ -666,18 +667,14 @@ __global__ void __launch_bounds__(kArnBlock, 2) k_arnoldi_tile(
   if (wid == kArnWarps) {
     // ---- producer warp: tile k of the sweep as the ring's use number c; pairs of
     // V, or its hi halves (and D)
-    int issued = 0;
-    bool stop = false;
+    int end = resident ? nt : 3 * nt;  // of the uses; lower where it gave up
     auto issue = [&](int c, int k, bool pairs, const float* D) {
-      if (stop) return;
       const int s = c % stages;
-      if (c >= stages && !__all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], ((c / stages) - 1) & 1, limit))) {
+      if (c >= stages && !mbar_wait_bounded(&empty[s], ((c / stages) - 1) & 1, limit)) {
         if (lane == 0) atomicAdd(&gs->timeouts, 1ull);
-        stop = true;
-        return;
+        end = min(end, c);
       }
-      issued = c + 1;
-      if (lane == 0) {
+      if (lane == 0 && c < end) {
         const long long e0 = tile_of(k) * T;
         const int count = count_of(k);
         const uint32_t dbytes = D ? (uint32_t)((count + 3) & ~3) * 4u : 0u;
@@ -709,17 +706,18 @@ __global__ void __launch_bounds__(kArnBlock, 2) k_arnoldi_tile(
       bar_all();  // s_n2
     }
     if (blockIdx.x == 0 && lane == 0) gm_update(gs, jj, s_h1, s_h2, s_n2);
-    for (int c = max(0, issued - stages); c < issued; c++)
-      mbar_wait_bounded(&full[c % stages], (c / stages) & 1, kWaitLimit);
+    if (lane == 0)
+      for (int c = max(0, end - stages); c < end; c++)
+        mbar_wait_bounded(&full[c % stages], (c / stages) & 1, kWaitLimit);
     return;
   }
 
   // ---- consumers
-  bool bad = false;  // this warp gave up on a tile
+  bool bad = false;  // this lane gave up on a tile; lane 0 frees only while it saw all land
   auto acquire = [&](int c) -> float* {
     const int s = c % stages;
-    if (!bad && !__all_sync(0xffffffffu, mbar_wait_bounded(&full[s], (c / stages) & 1, limit))) {
-      if (lane == 0) atomicAdd(&gs->timeouts, 1ull);
+    if (!mbar_wait_bounded(&full[s], (c / stages) & 1, limit)) {
+      atomicAdd(&gs->timeouts, 1ull);
       bad = true;
     }
     return s_ring + (size_t)s * stage_f;

@@ -160,9 +160,10 @@ TapsF taps_f32(const Taps& T) {
 // size (the autotuner chooses it by time).  Bound: latency on small meshes --
 // one thread per (component, corner) walked all 27 slots, nine rounds of
 // dependent loads -- and reading M (HBM) on large ones.  us per application,
-// before and now, at 512 and at 32,768 corners: FP32 operator 15.6 -> 8.5, 18.5 ->
-// 15.9; residual operator with its input split 23.2 -> 16.1, 30.5 -> 27.2; RHS
-// likewise 27 -> 16.8, 42 -> 37.
+// before and now, at 512 and at 32,768 corners: FP32 operator 15.6 -> 8.0, 18.5 ->
+// 13.0 (5.0 and 10.6 back to back); residual operator with its input split 23.2 ->
+// 16.1, 30.5 -> 27.2, 9.7 and 21.2 on pairs that are there; RHS with the split of E^n
+// 27 -> 15.4, 42 -> 36.8.
 constexpr int kOpGroups = 8;  // of slots; a CTA has at most a warp per group
 
 __device__ __forceinline__ void slot_offset(int s, int& di, int& dj, int& dk) {

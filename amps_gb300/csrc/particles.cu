@@ -1946,8 +1946,8 @@ cudaError_t launch_inject(amps_gpu_ctx* c, const StepArgs& a) {
 
 // A warp's time is its cells' chain, so a mesh whose CTAs all run at once (four per SM on
 // 152 SMs: up to 9 blocks) splits its rows in four: one block 10 us, 20 with whole rows.
-// Beyond, whole rows are as fast or faster (64 blocks 186 us against 184 to 188, 960
-// refined 2.54 ms against 2.65).
+// Beyond, whole rows are as fast (64 blocks 186 us, 184 to 188 in parts) or faster (960
+// refined blocks 2.54 ms, 2.65 in parts).
 constexpr int kParts = 4;
 static int push_parts(const amps_gpu_ctx* c) {
   return (long long)kParts * c->nb * AMPS_NC * AMPS_NC / kPushWarps <= 4 * 152 ? kParts : 1;

@@ -31,9 +31,10 @@
 // alike (its A rows come from shared memory) and 64 at N = 96, so three dx per MMA
 // count (294 MMAs per CTA instead of 810), and an issue loop in uniform control flow
 // (one elected thread, descriptors in uniform registers; a loop under tid == 0 issues
-// one MMA in 74 cycles); these are 15,000 of the kernel's 25,000 cycles, the chain
-// gather - read-back - exchange the rest.  64 blocks of a mesh: 28 us per
-// application; with an MMA per tap, 4 warps and one commit a layer 60.
+// one MMA in 74 cycles); these are 15,000 of the kernel's 25,000 cycles (13 us, warm),
+// the chain gather - read-back - exchange the rest.  64 blocks of a mesh: 27 us between
+// events around an application in a solve (launch, events and cold inputs included);
+// with an MMA per tap, 4 warps and one commit a layer 60.
 // Shared memory per CTA: 4 channel planes (82,944 B) + the three layers'
 // BF16 weight images (110,592 B, one bulk copy); tensor memory: 256 columns.
 // Every mbarrier wait is bounded; a timeout is counted in flags[2] and the CTA

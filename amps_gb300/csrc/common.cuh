@@ -165,7 +165,8 @@ struct amps_gpu_ctx {
   };
   std::vector<StepGraph> graphs;
   // the first GMRES cycle of a solve as a graph (gmres_solve), keyed by the
-  // preconditioner, the Arnoldi steps and the launch shapes it was captured with
+  // preconditioner, the Arnoldi steps and the launch shapes it was captured with (the
+  // tolerance is read from d_red; set_wait_limit drops them)
   struct SolveGraph {
     int precond, steps, tb, red, ept;
     cudaGraphExec_t exec;

@@ -1761,13 +1761,14 @@ cudaError_t launch_add(amps_gpu_ctx* c, const double* a, const double* b, double
   return cudaGetLastError();
 }
 
-// One Arnoldi step on host vectors, for checks of k_arnoldi_tile by itself: pairs
+// One Arnoldi step on host vectors (as many elements as a tile copy's 32-bit
+// coordinate reaches), for checks of k_arnoldi_tile by itself: pairs
 // of V and w, a least-squares state whose rotations are the identity (so that its
 // column is h and the norm), the step, and everything back.
 extern "C" amps_gpu_status amps_gpu_arnoldi_step(int device, long long n, int nv, const double* V, const double* w,
                                                  const double* d, int tile, int ctas, double* h, double* norm,
                                                  double* vnext, float* xf) {
-  if (n < kArnCons || nv < 1 || nv + 1 > kArnDots || !V || !w || !h || !norm || !vnext || !xf || ctas < 0)
+  if (n < kArnCons || n > (1LL << 31) - 2048 || nv < 1 || nv + 1 > kArnDots || !V || !w || !h || !norm || !vnext || !xf || ctas < 0)
     return AMPS_GPU_INVALID_ARG;
   if (tile != 0 && ((tile != 128 && tile != 256 && tile != 512 && tile != 1024) || !arn_fits(tile, nv)))
     return AMPS_GPU_INVALID_ARG;

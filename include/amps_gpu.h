@@ -538,7 +538,7 @@ amps_gpu_status amps_gpu_get_particle_tuning(amps_gpu_ctx* ctx, int* arrivals_ch
 
 /* ---- the solver's Arnoldi step by itself, on host vectors ----
  * One step of the field solve's GMRES (two classical Gram-Schmidt projections,
- * normalisation) of w[n] against the basis V[nv][n], n >= 256, 1 <= nv <= 31, in the pair
+ * normalisation) of w[n] against the basis V[nv][n], 256 <= n <= 2^31 - 2048, 1 <= nv <= 31, in the pair
  * arithmetic of the solve (48 significant bits; V and w are rounded to it):
  * h[nv], the sum of both projections' coefficients, *norm = ||w''||, vnext[n] =
  * w'' / *norm (zeros when *norm is 0) and xf[n] = fp32(D vnext), D = d or 1 when

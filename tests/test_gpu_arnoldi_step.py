@@ -110,3 +110,10 @@ def test_refused_arguments():
     big = np.zeros((5, 2048))
     assert step(big, np.ones(2048), None, 1024)[0] == 1  # two tiles of 5 vectors do not fit on chip
     assert step(np.zeros((32, 2048)), np.ones(2048))[0] == 1
+
+
+def test_refused_length():
+    """beyond a tile copy's 32-bit coordinates; refused before any vector is read"""
+    lib, a = _capi.load(), np.zeros(4)
+    d, f = a.ctypes.data_as(C.POINTER(C.c_double)), a.ctypes.data_as(C.POINTER(C.c_float))
+    assert lib.amps_gpu_arnoldi_step(0, 2 ** 31, 1, d, d, None, 0, 0, d, d, d, f) == 1
